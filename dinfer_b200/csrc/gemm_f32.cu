@@ -3,8 +3,8 @@
 // bfloat16 model whose file stores a matrix in 32-bit.  A, W and C may each be f32 or bf16 in
 // memory; every product and sum is f32.  Any M, N, K.
 //
-// Two kernels: a 128x128x8 register-tiled one for prompts, and a warp-per-output-column one for
-// the few rows of a decode step.  The reference has no 32-bit path (its weights are bf16 and its
+// Two kernels: a register-tiled one for prompts (packed multiply-adds, K shared by a cluster where tiles are few), and a
+// warp-per-output-column one for the few rows of a decode step.  The reference has no 32-bit path (its weights are bf16 and its
 // products cuBLASLt: crates/kernels/src/gemm.rs:649-690).
 #include "common.cuh"
 
@@ -12,57 +12,169 @@ using namespace dinfer;
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 8;
+constexpr int BM = 64, BN = 128, BK = 16;      // a CTA's tile; k per stage
+constexpr int TILE_THREADS = 128;
+constexpr int LDK = BK + 4;                    // row stride of a staged operand (floats): eight rows' 16-byte pieces of one k
+                                               // lie in different banks
+constexpr int STAGES = 3;
+constexpr int STAGE_FLOATS = (BM + BN) * LDK;
+constexpr int LDC_S = BN + 8;                  // row stride of the partial tile
+constexpr int TILE_SMEM = STAGES * STAGE_FLOATS * 4;
+static_assert(BM * LDC_S <= STAGES * STAGE_FLOATS, "the partial tile takes the stages' place");
+static_assert(TILE_SMEM <= 48 * 1024, "no opt-in");
+constexpr int MAX_SPLITS = 8;                  // CTAs that may share a tile's K (a portable cluster)
 
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 16 bytes, or zeros where `live` is false (nothing is read then)
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+// two independent 32-bit multiply-adds, each rounded once (the packed form is one instruction on this machine)
+__device__ __forceinline__ void fma2(uint64_t& c, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float4 ld_cluster_f4(const float* local, uint32_t rank) {
+  uint32_t remote;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+
+// Stages rows [r0, r0 + ROWS) of an operand, k in [k0, k0 + BK), as [row][k]; rows from `rows` on and k from `k_end` on are
+// zeros.  fast: 32-bit, rows of whole 16-byte pieces (K and the stride multiples of 4, the pointer aligned): cp.async;
+// else through registers, element by element.
+template <typename T, int ROWS>
+__device__ __forceinline__ void stage_rows(float* dst, const T* __restrict__ src, int64_t ld, int r0, int rows, int k0, int k_end,
+                                           bool fast) {
+  if constexpr (sizeof(T) == 4) {
+    if (fast) {
+#pragma unroll
+      for (int i = 0; i < ROWS * (BK / 4) / TILE_THREADS; ++i) {
+        const int idx = threadIdx.x + i * TILE_THREADS;
+        const int r = idx / (BK / 4), k = (idx % (BK / 4)) * 4;
+        const bool live = r0 + r < rows && k0 + k < k_end;
+        cp_async16(dst + r * LDK + k, reinterpret_cast<const float*>(src) + (live ? (int64_t)(r0 + r) * ld + k0 + k : 0), live);
+      }
+      return;
+    }
+  }
+#pragma unroll 4
+  for (int i = 0; i < ROWS * BK / TILE_THREADS; ++i) {
+    const int idx = threadIdx.x + i * TILE_THREADS;
+    const int r = idx / BK, k = idx % BK;
+    dst[r * LDK + k] = (r0 + r < rows && k0 + k < k_end) ? to_f32<T>(src[(int64_t)(r0 + r) * ld + k0 + k]) : 0.f;
+  }
+}
+
+// The tile kernel.  Bound by the rate of the multiply-adds: four warps own 32 x 64 of the tile each, a lane 8 x 8 (rows ly
+// + 4 i, columns lx + 8 j), and a multiply-add works on two k at once (even and odd k have a sum of their own, added at
+// the end), so that the operands are used as they lie in shared memory: 16 16-byte loads feed 128 packed multiply-adds.
+// Three stages of 16 k.  `splits` CTAs, one cluster, share a tile's K where the tiles alone leave SMs idle (a 333-row
+// product of 1024 columns is 48 tiles): each leaves its partial tile in its shared memory and all fold it in split order,
+// a share of the tile each.  333 x 6144 x 1024 and 333 x 1024 x 3072 in 32-bit took 884 us with one 128 x 128 x 8 tile per
+// CTA (plain multiply-adds, one stage, 24 CTAs on the second), 204 us now (31 TFLOP/s); 2048 x 6144 x 1024 644 us (40).
 template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(TILE_THREADS, 2)
 gemm_tile_kernel(const TA* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
-                 TC* __restrict__ C, int64_t ldc, int M, int N, int K, int64_t sa, int64_t sw, int64_t sc) {
-  A += (int64_t)blockIdx.z * sa; W += (int64_t)blockIdx.z * sw; C += (int64_t)blockIdx.z * sc;
-  __shared__ float As[BK][BM];
-  __shared__ float Ws[BK][BN];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
+                 TC* __restrict__ C, int64_t ldc, int M, int N, int K, int64_t sa, int64_t sw, int64_t sc, int splits,
+                 int a_fast, int w_fast, int c_fast) {
+  extern __shared__ __align__(16) float sm[];
+  const int z = blockIdx.z / splits, rank = blockIdx.z % splits;
+  A += (int64_t)z * sa; W += (int64_t)z * sw; C += (int64_t)z * sc;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[8][8];
+  // (lanes 0-7 and 8-15 read the two halves of the columns' pieces: 16 lanes' 16-byte loads then take one pass over the banks)
+  const int ly = ((lane >> 2) & 1) | (lane >> 4 << 1), lx = (lane & 3) | ((lane >> 3 & 1) << 2);
+  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 64;
+  const int tiles = (K + BK - 1) / BK;
+  const int first = (int)((int64_t)tiles * rank / splits), last = (int)((int64_t)tiles * (rank + 1) / splits);
+
+  uint64_t acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
 
-  const int lr = tid >> 1, lk = (tid & 1) * 4;   // this thread loads row lr, k = lk..lk+3 of both tiles
-  for (int k0 = 0; k0 < K; k0 += BK) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + lk + u;
-      const int am = m0 + lr, wn = n0 + lr;
-      As[lk + u][lr] = (am < M && k < K) ? to_f32<TA>(A[(int64_t)am * lda + k]) : 0.f;
-      Ws[lk + u][lr] = (wn < N && k < K) ? to_f32<TW>(W[(int64_t)wn * ldw + k]) : 0.f;
+  auto stage = [&](int t) {
+    if (t < last) {
+      float* s = sm + (t - first) % STAGES * STAGE_FLOATS;
+      stage_rows<TA, BM>(s, A, lda, m0, M, t * BK, K, a_fast);
+      stage_rows<TW, BN>(s + BM * LDK, W, ldw, n0, N, t * BK, K, w_fast);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[8], b[8];
-      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[k][64 + ty * 4]);
-      *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-      *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&Ws[k][64 + tx * 4]);
+  for (int u = 0; u < STAGES - 1; ++u) stage(first + u);
+  for (int t = first; t < last; ++t) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                       // tile t is there, and nobody reads tile t - 1 any more
+    stage(t + STAGES - 1);
+    const float* as = sm + (t - first) % STAGES * STAGE_FLOATS + (wr + ly) * LDK;
+    const float* ws = sm + (t - first) % STAGES * STAGE_FLOATS + (BM + wc + lx) * LDK;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+    for (int k = 0; k < BK; k += 4) {
+      ulonglong2 a[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + 4 * i * LDK + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + 8 * j * LDK + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, b.y);    // (a sum's two steps apart: the first takes a while)
+      }
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();                                         // the stages' memory takes the partial tile
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-    if (m >= M) continue;
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-      if (n < N) C[(int64_t)m * ldc + n] = from_f32<TC>(acc[i][j]);
+      const float lo = __uint_as_float((uint32_t)acc[i][j]), hi = __uint_as_float((uint32_t)(acc[i][j] >> 32));
+      sm[(wr + ly + 4 * i) * LDC_S + wc + lx + 8 * j] = lo + hi;
     }
+  if (splits > 1) {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+  for (int v = rank * TILE_THREADS + tid; v < BM * (BN / 4); v += splits * TILE_THREADS) {
+    const int r = v / (BN / 4), c = (v % (BN / 4)) * 4;
+    const int m = m0 + r, n = n0 + c;
+    if (m >= M || n >= N) continue;
+    const float* own = sm + r * LDC_S + c;
+    float4 t;
+    if (splits > 1) {
+      t = ld_cluster_f4(own, 0);
+      for (int q = 1; q < splits; ++q) {
+        const float4 u = ld_cluster_f4(own, q);
+        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+      }
+    } else {
+      t = *reinterpret_cast<const float4*>(own);
+    }
+    TC* dst = C + (int64_t)m * ldc + n;
+    if (c_fast && n + 3 < N) {
+      if constexpr (sizeof(TC) == 4) {
+        *reinterpret_cast<float4*>(dst) = t;
+      } else {
+        __nv_bfloat162 p[2] = {__floats2bfloat162_rn(t.x, t.y), __floats2bfloat162_rn(t.z, t.w)};
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(p);
+      }
+    } else {
+      const float e[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (n + u < N) dst[u] = from_f32<TC>(e[u]);
+    }
+  }
+  if (splits > 1) {                                        // nobody leaves while others may still read its share
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   }
 }
 
@@ -134,6 +246,15 @@ gemm_rows_bf16x8_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const 
   }
 }
 
+int num_sms() {                                             // of the current device, asked once
+  static const int n = [] {
+    int dev = 0, v = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
 template <typename TA, typename TW> struct both_bf16 { static constexpr bool value = false; };
 template <> struct both_bf16<__nv_bfloat16, __nv_bfloat16> { static constexpr bool value = true; };
 
@@ -162,10 +283,30 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
     gemm_rows_kernel<TA, TW, TC, 32><<<dim3((N + 7) / 8, 1, batch), 256, 0, stream>>>(
         (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
   } else {
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
+    const int64_t tiles = (int64_t)((N + BN - 1) / BN) * ((M + BM - 1) / BM) * batch;
+    // as many CTAs to a tile as find room at once (two to an SM, but a cluster has to fit into what one GPC has left: 48 tiles
+    // of 333 x 1024 x 3072 took 79 us with 5 CTAs each and 98 with 6, where the last clusters wait), each with at least eight
+    // stages of K to itself
+    int splits = 1;
+    const int k_tiles = (K + BK - 1) / BK;
+    while (splits < MAX_SPLITS && tiles * (splits + 1) <= num_sms() * 5 / 3 && k_tiles / (splits + 1) >= 8 &&
+           (int64_t)batch * (splits + 1) <= 65535)
+      ++splits;
+    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch * splits);
     if (grid.y > 65535) return refuse(DINFER_BAD_ARGUMENT, "gemm_f32: M=%d too large", M);
-    gemm_tile_kernel<TA, TW, TC><<<grid, 256, 0, stream>>>(
-        (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
+    const auto fast = [](const void* q, size_t size, int64_t ld, int64_t stride) {
+      return (int)((reinterpret_cast<uintptr_t>(q) % (4 * size)) == 0 && ld % 4 == 0 && stride % 4 == 0);
+    };
+    const int a_fast = fast(A, sizeof(TA), lda, sa) && K % 4 == 0, w_fast = fast(W, sizeof(TW), ldw, sw) && K % 4 == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(TILE_THREADS); cfg.dynamicSmemBytes = TILE_SMEM; cfg.stream = stream;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = splits;
+    cfg.attrs = &cluster; cfg.numAttrs = splits > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, gemm_tile_kernel<TA, TW, TC>, (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw,
+                       sc, splits, a_fast, w_fast, fast(C, sizeof(TC), ldc, sc));
   }
   return cuda_status("gemm_f32");
 }

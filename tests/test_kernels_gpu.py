@@ -95,6 +95,40 @@ def test_gemm_f32(M, N, K, adt, wdt, cdt):
     assert torch.allclose(out.double().cpu(), want, **t)
 
 
+@pytest.mark.parametrize("M,N,K", [(9, 129, 16), (64, 128, 132), (65, 127, 260), (128, 256, 1024), (333, 1024, 3072), (64, 8, 2050),
+                                   (40, 20, 4)])
+@pytest.mark.parametrize("adt,wdt,cdt", [(torch.float32,) * 3, (torch.bfloat16, torch.float32, torch.bfloat16),
+                                         (torch.float32, torch.bfloat16, torch.float32)])
+def test_gemm_f32_tiles_and_splits(M, N, K, adt, wdt, cdt):
+    """Edges of the tile, remainders of a stage, one to eight CTAs to a tile's K, aligned rows and rows that are not.  K
+    products summed in any order in 32-bit are off by at most (K + 1) 2^-24 of the sum of their sizes, plus the rounding of
+    a bfloat16 result (2^-8 of it)."""
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    for pad in (0, 1):                                       # rows of whole 16-byte pieces, and rows that are not
+        a = torch.randn(M, K + pad, generator=g).to(adt)[:, :K]
+        w = torch.randn(N, K + pad, generator=g).to(wdt)[:, :K]
+        out = torch.full((M, N + pad), float("nan"), dtype=cdt, device="cuda")
+        da, dw = dev(torch.cat([a, a[:, :pad]], 1))[:, :K], dev(torch.cat([w, w[:, :pad]], 1))[:, :K]
+        ops.gemm_f32(da, dw, out[:, :N])
+        want = a.double() @ w.double().T
+        bound = (K + 1) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+        if cdt == torch.bfloat16:
+            bound = bound + 2.0 ** -8 * want.abs()
+        assert bool(((out[:, :N].double().cpu() - want).abs() <= bound).all())
+        assert pad == 0 or bool(torch.isnan(out[:, N:]).all())
+    # several problems at once, their rows interleaved
+    a = torch.randn(M, 3, 44, generator=g).to(adt)
+    w = torch.randn(3, N, 44, generator=g).to(wdt)
+    out = torch.full((M, 3, N), float("nan"), dtype=cdt, device="cuda")
+    ops.gemm_f32_batched(dev(a), dev(w), out)
+    want = torch.einsum("mbk,bnk->mbn", a.double(), w.double())
+    bound = 45 * 2.0 ** -24 * torch.einsum("mbk,bnk->mbn", a.double().abs(), w.double().abs())
+    if cdt == torch.bfloat16:
+        bound = bound + 2.0 ** -8 * want.abs()
+    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+
+
 def test_gemm_f32_strided_operands():
     from dinfer_b200.kernels import ops
     g = torch.Generator().manual_seed(3)
