@@ -18,10 +18,11 @@
 // rewritten: the three filters reduce to one keep-threshold on the scaled logits.  The top-k and the
 // top-p threshold are each found by a radix-16 descent over the order-preserving 32-bit image of a
 // float (eight rounds, every round one pass over shared memory): the largest value t such that the
-// kept entries >= t number at least k (have at least the share p of the mass).  A small k (up to 512)
-// takes a short way instead: a histogram names the bin of the k-th largest entry, the entries from
-// there up are collected in every CTA, and both thresholds are counted out among them.  All sums are
-// taken in a fixed order (thread, warp, CTA rank), so the same logits, seed and count give the same token.
+// kept entries >= t number at least k (have at least the share p of the mass).  Where at most CAND_MAX
+// entries decide (nearly always) both take a short way instead: one pass counts (and weighs) the
+// entries above a few cuts below the maximum, the entries above the first cut that is enough are
+// collected in every CTA, sorted, and both thresholds read off.  All sums are taken in a fixed order
+// (segment, warp of segments, CTA rank), so the same logits, seed and count give the same token.
 #include "common.cuh"
 
 using namespace dinfer;
@@ -29,6 +30,15 @@ using namespace dinfer;
 namespace {
 
 constexpr int BLOCK = 1024;
+// A CTA's slice is cut into SEGMENTS runs of neighbouring ids, and 32 neighbouring segments are a warp of segments: what a
+// sum's order is made of, whatever the block's size.  The sampling kernel's blocks have 512 threads with VT = 2 segments each
+// (t and t + 512): at 64 registers a thread two blocks share an SM, so that one works while the other waits at a cluster
+// barrier, and a wave holds twice the rows.  us for 8 / 16 / 64 rows of 151936, temperature alone: 1024 threads 12.2 / 22.8 /
+// 55, 512 threads 11.9 / 13.3 / 28.
+constexpr int SEGMENTS = 1024;
+constexpr int WARPS_OF_SEGMENTS = SEGMENTS / 32;
+constexpr int VT = 2;
+constexpr int NT = SEGMENTS / VT;           // threads of the sampling kernel
 constexpr int ROW_CTAS = 8;                 // cluster size: CTAs that share a row
 constexpr int MAX_SLICE = 48 * 1024;        // floats of a row slice that shared memory holds (192 KB)
 constexpr int XCH = 16;                     // floats a CTA hands to the others per exchange
@@ -77,42 +87,40 @@ __device__ float (*exchange(Shared& sh, float mine, int n, uint32_t rank))[XCH] 
   return sh.xchg[t];
 }
 
-// Deterministic block sum of a per-thread vector v[0..N): warp shuffle tree, then the warps in order.
-// The result is in sh.blk[0..N) for all threads.
-template <int N>
-__device__ void block_sum_vec(Shared& sh, float (&v)[N]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Sum over the whole row of what every segment contributes: fill(segment, v) adds segment's share to v[0..N).  Warps of
+// segments by a shuffle tree, then those in order, then the CTAs in rank order.
+template <int N, typename F>
+__device__ __forceinline__ void row_sum(Shared& sh, uint32_t rank, float (&out)[N], F fill) {
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
+#pragma unroll 1
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x;
+    float v[N];
 #pragma unroll
-  for (int j = 0; j < N; ++j) {
+    for (int j = 0; j < N; ++j) v[j] = 0.f;
+    fill(u, v);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    for (int j = 0; j < N; ++j) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) sh.warp_part[u >> 5][j] = v[j];
+    }
   }
   __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) sh.warp_part[warp][j] = v[j];
-  }
-  __syncthreads();
-  if ((int)threadIdx.x < N) {
-    float s = 0.f;
-    for (int w = 0; w < BLOCK / 32; ++w) s += sh.warp_part[w][threadIdx.x];
-    sh.blk[threadIdx.x] = s;
-  }
-  __syncthreads();
-}
-
-// Sum over the whole row of a per-thread vector: block sum, exchange, CTAs in rank order.
-template <int N>
-__device__ void row_sum_vec(Shared& sh, float (&v)[N], uint32_t rank, float (&out)[N]) {
-  block_sum_vec<N>(sh, v);
-  const float mine = (int)threadIdx.x < N ? sh.blk[threadIdx.x] : 0.f;
+  float mine = 0.f;
+  if ((int)threadIdx.x < N)
+    for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) mine += sh.warp_part[w][threadIdx.x];
   float (*x)[XCH] = exchange(sh, mine, N, rank);
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    float s = 0.f;
+    float t = 0.f;
 #pragma unroll
-    for (int r = 0; r < ROW_CTAS; ++r) s += x[r][j];
-    out[j] = s;
+    for (int r = 0; r < ROW_CTAS; ++r) t += x[r][j];
+    out[j] = t;
   }
 }
 
@@ -131,9 +139,10 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 }
 
 // argmax over the row (ties to the lowest index), the same in every CTA of the cluster
+template <int THREADS>
 __device__ int row_argmax(Shared& sh, const float* xs, int n_mine, int first, uint32_t rank) {
   ArgMax best{-INFINITY, 0x7fffffff};
-  for (int i = threadIdx.x; i < n_mine; i += BLOCK) best = better(best, ArgMax{xs[i], first + i});
+  for (int i = threadIdx.x; i < n_mine; i += THREADS) best = better(best, ArgMax{xs[i], first + i});
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1)
     best = better(best, ArgMax{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
@@ -142,7 +151,7 @@ __device__ int row_argmax(Shared& sh, const float* xs, int n_mine, int first, ui
   if (lane == 0) { sh.warp_part[warp][0] = best.v; sh.warp_part[warp][1] = __int_as_float(best.i); }
   __syncthreads();
   if (warp == 0) {
-    best = ArgMax{sh.warp_part[lane][0], __float_as_int(sh.warp_part[lane][1])};
+    best = lane < THREADS / 32 ? ArgMax{sh.warp_part[lane][0], __float_as_int(sh.warp_part[lane][1])} : ArgMax{-INFINITY, 0x7fffffff};
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
       best = better(best, ArgMax{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
@@ -179,14 +188,16 @@ __device__ float philox_uniform(uint64_t seed, uint64_t offset) {
   return (float)(c0 >> 8) * (1.f / 16777216.f);
 }
 
-// The slice of the row this CTA owns: ids [first, first + n_mine).  Thread t owns the contiguous
-// ids [t*seg, (t+1)*seg) of the slice, so thread order, then CTA rank, is vocabulary order.
+// The slice of the row this CTA owns: ids [first, first + n_mine).  Segment u holds the contiguous
+// ids [u*seg, (u+1)*seg) of the slice, so segment order, then CTA rank, is vocabulary order.
 struct Slice {
   const float* xs;      // scaled values in shared memory, or null: read the row and scale on the fly
   const float* row;
   float inv_t;
   int first, n_mine, seg;
   __device__ __forceinline__ float at(int i) const { return xs ? xs[i] : row[first + i] * inv_t + 0.f; }
+  __device__ __forceinline__ int begin(int u) const { return min(n_mine, u * seg); }
+  __device__ __forceinline__ int end(int u) const { return min(n_mine, (u + 1) * seg); }
 };
 
 // The largest value t such that the entries x >= max(t, floor_) weigh at least `target`, where an
@@ -196,24 +207,22 @@ template <bool MASS>
 __device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, float m, float floor_, float target) {
   uint32_t prefix = 0;
   float above = 0.f;
-  const int i0 = min(sl.n_mine, (int)threadIdx.x * sl.seg), i1 = min(sl.n_mine, i0 + sl.seg);
 #pragma unroll 1
   for (int shift = 28; shift >= 0; shift -= 4) {
-    float h[16];
-#pragma unroll
-    for (int d = 0; d < 16; ++d) h[d] = 0.f;
-    for (int i = i0; i < i1; ++i) {
-      const float x = sl.at(i);
-      if (!(x >= floor_)) continue;
-      const uint32_t k = float_key(x);
-      if (shift < 28 && (k >> (shift + 4)) != (prefix >> (shift + 4))) continue;
-      const float w = MASS ? expf(x - m) : 1.f;
-      const int dgt = (k >> shift) & 15;
-#pragma unroll
-      for (int d = 0; d < 16; ++d) h[d] += dgt == d ? w : 0.f;
-    }
     float tot[16];
-    row_sum_vec<16>(sh, h, rank, tot);
+    row_sum<16>(sh, rank, tot, [&](int u, float (&h)[16]) {
+      const int i1 = sl.end(u);
+      for (int i = sl.begin(u); i < i1; ++i) {
+        const float x = sl.at(i);
+        if (!(x >= floor_)) continue;
+        const uint32_t k = float_key(x);
+        if (shift < 28 && (k >> (shift + 4)) != (prefix >> (shift + 4))) continue;
+        const float w = MASS ? expf(x - m) : 1.f;
+        const int dgt = (k >> shift) & 15;
+#pragma unroll
+        for (int d = 0; d < 16; ++d) h[d] += dgt == d ? w : 0.f;
+      }
+    });
     int chosen = 0;
     float run = above;
     bool found = false;
@@ -231,168 +240,189 @@ __device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, flo
   return key_float(prefix);
 }
 
-// ---- the short way to a top-k threshold (and the top-p threshold behind it) when k is small
-// One pass counts the kept entries by the upper 12 bits of their key (a histogram in shared memory; the CTAs
-// read each other's counts), which names the bin that holds the k-th largest entry; the entries from that bin
-// up, at most CAND_MAX of them, are copied into every CTA in vocabulary order, and the thresholds are found
-// among them by direct counting.  With more entries than that from the bin up, the radix descent does it.
+// ---- the short way to the two thresholds: where at most CAND_MAX entries hold the k largest, or the share p of the mass
 constexpr int CAND_MAX = 1024;
-constexpr int HIST_BITS = 12, HIST_BINS = 1 << HIST_BITS, BINS_PER_CTA = HIST_BINS / ROW_CTAS;
-static_assert(BINS_PER_CTA <= BLOCK, "a thread per bin of a CTA's share");
+constexpr int CUTS = 8;                       // cuts a pass counts at, the last one the floor
+constexpr int CUT_ROUNDS = 3;
+static_assert(CAND_MAX <= SEGMENTS && 2 * CUTS <= XCH, "a candidate per segment; counts and masses in one exchange");
 
 struct Candidates {
-  uint32_t hist[HIST_BINS];
-  float x[CAND_MAX];                  // the candidates, the same list in every CTA of the row
-  float w[CAND_MAX];                  // their weights exp(x - m), 0 below the floor
-  int warp_tot[BLOCK / 32];
-  int n;
-  float thr;
+  float x[CAND_MAX];                  // the candidates, the same list in every CTA of the row, in vocabulary order
+  float s[CAND_MAX];                  // and from the largest down
+  int warp_tot[WARPS_OF_SEGMENTS];
+  float warp_mass[WARPS_OF_SEGMENTS];
+  int found;
 };
 
-__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t local_addr, uint32_t rank) {
-  uint32_t remote, v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
-  return v;
-}
-
-// inclusive prefix sum of v over the threads of the block, in thread order; `total` is the block's sum
-__device__ int block_scan_inclusive(int v, int* warp_tot, int& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = v;
+// inclusive prefix sums of the segments' v, in segment order; `total` is the block's sum
+__device__ __forceinline__ void segment_scan(int (&v)[VT], int* warp_tot, int& total) {
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += u;
+  for (int vt = 0; vt < VT; ++vt) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v[vt], o);
+      if (lane >= o) v[vt] += t;
+    }
+    if (lane == 31) warp_tot[(vt * NT + threadIdx.x) >> 5] = v[vt];
   }
   __syncthreads();
-  if (lane == 31) warp_tot[warp] = incl;
-  __syncthreads();
-  int before = 0, all = 0;
-#pragma unroll
-  for (int w = 0; w < BLOCK / 32; ++w) {
+  int all = 0;
+#pragma unroll 8
+  for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) {
     const int t = warp_tot[w];
-    if (w < warp) before += t;
+#pragma unroll
+    for (int vt = 0; vt < VT; ++vt)
+      if (w < ((vt * NT + (int)threadIdx.x) >> 5)) v[vt] += t;
     all += t;
   }
   total = all;
-  return incl + before;
 }
 
-// Fills c.x with the kept entries (x >= floor_) from the bin of the k-th largest up; returns their number, or -1
-// if they are more than CAND_MAX.  With fewer than k kept entries all of them are candidates.
-__device__ int gather_candidates(Shared& sh, Candidates& c, const Slice& sl, uint32_t rank, float floor_, int k) {
-  const int i0 = min(sl.n_mine, (int)threadIdx.x * sl.seg), i1 = min(sl.n_mine, i0 + sl.seg);
-  for (int i = threadIdx.x; i < HIST_BINS; i += BLOCK) c.hist[i] = 0u;
-  __syncthreads();
-  for (int i = i0; i < i1; ++i) {
-    const float x = sl.at(i);
-    if (x >= floor_) atomicAdd(&c.hist[float_key(x) >> (32 - HIST_BITS)], 1u);
-  }
-  __syncthreads();
-  cluster_sync_all();
-  // this CTA adds up the bins [rank * BINS_PER_CTA, +BINS_PER_CTA) over all CTAs; thread u takes them from the top
-  int v = 0;
-  const int bin = (int)rank * BINS_PER_CTA + (BINS_PER_CTA - 1 - (int)threadIdx.x);
-  if ((int)threadIdx.x < BINS_PER_CTA) {
+// The highest of a few cuts c such that the kept entries (x >= floor_) with x >= c are enough: at least k of them (MASS
+// false), or at least the share p of the mass of all kept ones (true; `denom` is then that mass).  The first pass cuts at
+// fixed distances below the maximum (x is in units of the softmax's exponent), further ones inside the gap where the count
+// goes from too few to more than CAND_MAX.  Returns whether a cut with at most CAND_MAX entries was found.
+template <bool MASS>
+__device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, float lo, float floor_, float need, float& cut,
+                         float& denom) {
+  float c[CUTS] = {m - 1.f, m - 2.f, m - 4.f, m - 6.f, m - 9.f, m - 13.f, m - 18.f, floor_};
 #pragma unroll
-    for (uint32_t r = 0; r < ROW_CTAS; ++r) v += (int)ld_cluster_u32(smem_u32(&c.hist[bin]), r);
+  for (int j = 0; j < CUTS; ++j) c[j] = fmaxf(c[j], floor_);
+  float target = need;
+#pragma unroll 1
+  for (int round = 0; round < CUT_ROUNDS; ++round) {
+    float tot[MASS ? 2 * CUTS : CUTS];
+    row_sum<MASS ? 2 * CUTS : CUTS>(sh, rank, tot, [&](int u, float (&h)[MASS ? 2 * CUTS : CUTS]) {
+      const int i1 = sl.end(u);
+      for (int i = sl.begin(u); i < i1; ++i) {
+        const float x = sl.at(i);
+        const float w = MASS ? (x >= floor_ ? expf(x - m) : 0.f) : 0.f;
+#pragma unroll
+        for (int j = 0; j < CUTS; ++j) {
+          h[j] += x >= c[j] ? 1.f : 0.f;
+          if (MASS) h[CUTS + j] += x >= c[j] ? w : 0.f;
+        }
+      }
+    });
+    if (MASS && round == 0) { denom = tot[(MASS ? CUTS : 0) + CUTS - 1]; target = need * denom; }
+    float hi = m, low = c[CUTS - 1], n_above = 0.f, n = tot[CUTS - 1];
+    bool reached = false;
+#pragma unroll
+    for (int j = 0; j < CUTS; ++j) {
+      const float have = MASS ? tot[(MASS ? CUTS : 0) + j] : tot[j];
+      if (!reached) {
+        if (have >= target || j == CUTS - 1) { reached = true; low = c[j]; n = tot[j]; }
+        else { hi = c[j]; n_above = tot[j]; }
+      }
+    }
+    cut = low;
+    if (n <= (float)CAND_MAX) return true;
+    if (n_above >= (float)CAND_MAX) return false;          // even what is not enough is too many
+    low = fmaxf(low, lo);                                  // (the floor may be -inf)
+#pragma unroll
+    for (int j = 0; j < CUTS - 1; ++j) c[j] = hi - (hi - low) * ((float)(j + 1) * (1.f / CUTS));
+    c[CUTS - 1] = cut;
   }
-  int mine_total;
-  const int incl = block_scan_inclusive(v, c.warp_tot, mine_total);     // entries of my bins from `bin` up
-  float (*x)[XCH] = exchange(sh, threadIdx.x == 0 ? (float)mine_total : 0.f, 1, rank);
-  int above = 0, kept = 0;
+  return false;
+}
+
+// Fills cd.x with the entries from `cut` up (at most CAND_MAX), in vocabulary order, and cd.s with the same from the
+// largest down; returns their number.
+__device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32_t rank, float cut) {
+  int cnt[VT], end[VT], cta_total;
+#pragma unroll
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
+    int n = 0;
+    for (int i = sl.begin(u); i < i1; ++i) n += sl.at(i) >= cut;
+    cnt[vt] = end[vt] = n;
+  }
+  segment_scan(end, cd.warp_tot, cta_total);
+  float (*x)[XCH] = exchange(sh, threadIdx.x == 0 ? (float)cta_total : 0.f, 1, rank);
+  int base = 0, n = 0;
 #pragma unroll
   for (int r = 0; r < ROW_CTAS; ++r) {
-    const int t = (int)x[r][0];
-    kept += t;
-    if (r > (int)rank) above += t;
-  }
-  // the bin where the count from the top reaches k: at most one thread of the row finds it
-  if (threadIdx.x < 2) sh.blk[threadIdx.x] = -1.f;
-  __syncthreads();
-  if ((int)threadIdx.x < BINS_PER_CTA && v > 0 && above + incl - v < k && above + incl >= k) {
-    sh.blk[0] = (float)bin;
-    sh.blk[1] = (float)(above + incl);
-  }
-  __syncthreads();
-  x = exchange(sh, threadIdx.x < 2 ? sh.blk[threadIdx.x] : 0.f, 2, rank);
-  int pivot_bin = 0, n = kept;                           // fewer than k kept: all of them
-#pragma unroll
-  for (int r = 0; r < ROW_CTAS; ++r)
-    if (x[r][0] >= 0.f) { pivot_bin = (int)x[r][0]; n = (int)x[r][1]; }
-  if (n > CAND_MAX) return -1;
-  // copy them into every CTA, in vocabulary order
-  int cnt = 0;
-  for (int i = i0; i < i1; ++i) {
-    const float xv = sl.at(i);
-    cnt += xv >= floor_ && (int)(float_key(xv) >> (32 - HIST_BITS)) >= pivot_bin;
-  }
-  int cta_total;
-  const int my_end = block_scan_inclusive(cnt, c.warp_tot, cta_total);
-  x = exchange(sh, threadIdx.x == 0 ? (float)cta_total : 0.f, 1, rank);
-  int base = 0;
-#pragma unroll
-  for (int r = 0; r < ROW_CTAS; ++r)
     if (r < (int)rank) base += (int)x[r][0];
-  int at = base + my_end - cnt;
-  for (int i = i0; i < i1 && cnt > 0; ++i) {
-    const float xv = sl.at(i);
-    if (xv >= floor_ && (int)(float_key(xv) >> (32 - HIST_BITS)) >= pivot_bin) {
-      const uint32_t dst = smem_u32(&c.x[at]);
+    n += (int)x[r][0];
+  }
 #pragma unroll
-      for (uint32_t r = 0; r < ROW_CTAS; ++r) st_cluster_f32(dst, r, xv);
-      ++at;
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
+    int at = base + end[vt] - cnt[vt];
+    for (int i = sl.begin(u); i < i1 && cnt[vt] > 0; ++i) {
+      const float xv = sl.at(i);
+      if (xv >= cut && at < CAND_MAX) {
+        const uint32_t dst = smem_u32(&cd.x[at]);
+#pragma unroll
+        for (uint32_t r = 0; r < ROW_CTAS; ++r) st_cluster_f32(dst, r, xv);
+        ++at;
+      }
     }
   }
   cluster_sync_all();
+  __syncthreads();
+  // ranks by counting (equal values in vocabulary order): NT / n2 threads to a candidate, n2 the next power of two
+  n = min(n, CAND_MAX);
+  int n2 = 32;
+  while (n2 < n) n2 <<= 1;
+  const int tpc = n2 >= NT ? 1 : min(32, NT / n2);
+  const int per = NT / tpc;                                // candidates a round ranks
+  for (int i0 = 0; i0 < n; i0 += per) {
+    const int i = i0 + (int)threadIdx.x / tpc;
+    const float v = i < n ? cd.x[i] : 0.f;
+    int before = 0;
+    if (i < n)
+      for (int j = threadIdx.x % tpc; j < n; j += tpc) {
+        const float xj = cd.x[j];
+        before += xj > v || (xj == v && j < i);
+      }
+    for (int o = 1; o < tpc; o <<= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (i < n && threadIdx.x % tpc == 0) cd.s[before] = v;
+  }
   __syncthreads();
   return n;
 }
 
-// the k-th largest of the n candidates (all kept if they are fewer than k)
-__device__ float topk_of_candidates(Candidates& c, int n, int k) {
-  if (threadIdx.x == 0) c.thr = -INFINITY;
-  __syncthreads();
-  if (k <= n && (int)threadIdx.x < n) {
-    const float v = c.x[threadIdx.x];
-    int before = 0;                                      // candidates that come before this one, larger first
-    for (int j = 0; j < n; ++j) {
-      const float xj = c.x[j];
-      before += xj > v || (xj == v && j < (int)threadIdx.x);
+// The largest of the sorted candidates v >= floor_ such that those >= v hold at least the share p of `denom` (of the mass
+// of the candidates >= floor_ where denom < 0).
+__device__ float topp_of_sorted(Candidates& cd, int n, float m, float floor_, float p, float denom) {
+  const int lane = threadIdx.x & 31;
+  float cum[VT];
+  if (threadIdx.x == 0) cd.found = n;
+#pragma unroll
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x;
+    cum[vt] = u < n && cd.s[u] >= floor_ ? expf(cd.s[u] - m) : 0.f;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, cum[vt], o);
+      if (lane >= o) cum[vt] += t;
     }
-    if (before == k - 1) c.thr = v;
+    if (lane == 31) cd.warp_mass[u >> 5] = cum[vt];
   }
   __syncthreads();
-  return c.thr;
-}
-
-// the largest candidate value v >= floor_ such that the candidates >= v hold at least the share p of the mass of
-// those >= floor_; every thread adds the masses in the same order
-__device__ float topp_of_candidates(Candidates& c, int n, float m, float floor_, float p) {
-  for (int j = threadIdx.x; j < n; j += BLOCK) c.w[j] = c.x[j] >= floor_ ? expf(c.x[j] - m) : 0.f;
-  __syncthreads();
-  float best = -INFINITY;
-  if ((int)threadIdx.x < n) {
-    const float v = c.x[threadIdx.x];
-    float denom = 0.f, mass = 0.f;
-    for (int j = 0; j < n; ++j) {
-      const float wj = c.w[j];
-      denom += wj;
-      if (c.x[j] >= v) mass += wj;
-    }
-    if (v >= floor_ && mass >= p * denom) best = v;
+  float before[VT], all = 0.f;
+#pragma unroll
+  for (int vt = 0; vt < VT; ++vt) before[vt] = 0.f;
+#pragma unroll 8
+  for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) {
+    const float t = cd.warp_mass[w];
+#pragma unroll
+    for (int vt = 0; vt < VT; ++vt)
+      if (w < ((vt * NT + (int)threadIdx.x) >> 5)) before[vt] += t;
+    all += t;
   }
+  const float target = p * (denom < 0.f ? all : denom);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) best = fmaxf(best, __shfl_xor_sync(0xffffffffu, best, o));
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x;
+    if (u < n && cd.s[u] >= floor_ && before[vt] + cum[vt] >= target) atomicMin(&cd.found, u);
+  }
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) c.w[threadIdx.x >> 5] = best;            // the weights are done with
-  __syncthreads();
-  float all = -INFINITY;
-#pragma unroll
-  for (int w = 0; w < BLOCK / 32; ++w) all = fmaxf(all, c.w[w]);
-  __syncthreads();
-  return all;
+  if (cd.found < n) return cd.s[cd.found];
+  return n > 0 ? fmaxf(floor_, cd.s[n - 1]) : floor_;      // not reached by a rounding: all of them
 }
 
 __global__ void __launch_bounds__(BLOCK)
@@ -408,7 +438,7 @@ argmax_kernel(const float* __restrict__ logits, int64_t ld, int* __restrict__ ou
   if (threadIdx.x == 0) sh.turn = 0;
   __syncthreads();
   cluster_sync_all();                                    // every CTA runs before any writes into its memory
-  const int r = row_argmax(sh, row + first, n_mine, first, rank);
+  const int r = row_argmax<BLOCK>(sh, row + first, n_mine, first, rank);
   if (rank == 0 && threadIdx.x == 0) out[b] = r;
   cluster_sync_all();                                    // nobody leaves while others may still write to it
 }
@@ -452,7 +482,12 @@ argmax_many_kernel(const float* __restrict__ logits, int64_t ld, int* __restrict
   }
 }
 
-__global__ void __launch_bounds__(BLOCK)
+// What bounds it: the instructions of its passes over the row in shared memory and the cluster barriers between them, not
+// the one read of the row (39 MB for 64 rows of 151936: 6 us).  64 rows, greedy / temperature / top-k 20 + top-p 0.95 /
+// top-p 0.9 in turn, took 165 us with eight radix rounds for the top-p threshold, a shared-memory histogram for the top-k
+// one and one block of 1024 threads to an SM; 58 us now.  Alone, at 8 and 64 rows: top-k 20 + top-p 24 and 118 -> 23 and
+// 57 us, top-p 0.9 72 and 359 -> 29 and 77 us.
+__global__ void __launch_bounds__(NT, 2)
 sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
               const uint64_t* __restrict__ seeds, const uint64_t* __restrict__ offsets,
@@ -471,7 +506,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   cluster_sync_all();                                    // every CTA runs before any writes into its memory
   const float temp = temperature[b];
   if (temp <= 1e-5f) {
-    const int r = row_argmax(sh, row + first, n_mine, first, rank);
+    const int r = row_argmax<NT>(sh, row + first, n_mine, first, rank);
     if (rank == 0 && threadIdx.x == 0) out[b] = r;
     cluster_sync_all();
     return;
@@ -479,12 +514,12 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   const float inv_t = 1.f / temp;
   Slice sl;
   sl.row = row; sl.inv_t = inv_t; sl.first = first; sl.n_mine = n_mine;
-  sl.seg = (per + BLOCK - 1) / BLOCK;
+  sl.seg = (per + SEGMENTS - 1) / SEGMENTS;
   sl.xs = cache_slice ? xs_dyn : nullptr;
 
   // one pass over the row: scaled values into shared memory, maximum and smallest finite value
   float m = -INFINITY, lo = INFINITY;
-  for (int i = threadIdx.x; i < n_mine; i += BLOCK) {
+  for (int i = threadIdx.x; i < n_mine; i += NT) {
     const float x = row[first + i] * inv_t + 0.f;        // + 0: -0 becomes +0 (one image per value)
     if (cache_slice) xs_dyn[i] = x;
     m = fmaxf(m, x);
@@ -501,7 +536,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
     __syncthreads();
     if (threadIdx.x < 2) {
       float v = sh.warp_part[0][threadIdx.x];
-      for (int w = 1; w < BLOCK / 32; ++w) v = threadIdx.x == 0 ? fmaxf(v, sh.warp_part[w][0]) : fminf(v, sh.warp_part[w][1]);
+      for (int w = 1; w < NT / 32; ++w) v = threadIdx.x == 0 ? fmaxf(v, sh.warp_part[w][0]) : fminf(v, sh.warp_part[w][1]);
       sh.blk[threadIdx.x] = v;
     }
     __syncthreads();
@@ -517,44 +552,60 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   const float mp = min_p ? min_p[b] : 0.f;
   if (mp > 0.f) thr = m + logf(mp);                      // p_i >= min_p * p_max
   const int k = top_k ? top_k[b] : -1;
+  const bool finite = m < INFINITY && m > -INFINITY;      // else nothing is kept, whatever the thresholds
   int n_cand = -1;                                       // >= 0: cand holds every entry from the top-k threshold up
+  float cut, denom = -1.f;
   if (k > 0 && k < vocab) {
-    if (k <= CAND_MAX / 2) n_cand = gather_candidates(sh, cand, sl, rank, thr, k);
-    if (n_cand >= 0) thr = fmaxf(thr, topk_of_candidates(cand, n_cand, k));
-    else thr = fmaxf(thr, radix_threshold<false>(sh, sl, rank, m, thr, (float)k));
+    if (k <= CAND_MAX / 2 && finite && find_cut<false>(sh, sl, rank, m, lo, thr, (float)k, cut, denom)) {
+      n_cand = gather_sorted(sh, cand, sl, rank, cut);
+      if (k <= n_cand) thr = fmaxf(thr, cand.s[k - 1]);  // else all of them are kept
+    } else {
+      thr = fmaxf(thr, radix_threshold<false>(sh, sl, rank, m, thr, (float)k));
+    }
   }
   const float p = top_p ? top_p[b] : 1.f;
-  const int i0 = min(n_mine, (int)threadIdx.x * sl.seg), i1 = min(n_mine, i0 + sl.seg);
-  if (p < 1.f && p > 0.f && n_cand >= 0) {
-    thr = fmaxf(thr, topp_of_candidates(cand, n_cand, m, thr, p));
-  } else if (p < 1.f && p > 0.f) {
-    float d1[1] = {0.f}, denom[1];
-    for (int i = i0; i < i1; ++i) {
-      const float x = sl.at(i);
-      if (x >= thr) d1[0] += expf(x - m);
+  if (p < 1.f && p > 0.f) {
+    if (n_cand >= 0) {
+      thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, -1.f));
+    } else if (finite && find_cut<true>(sh, sl, rank, m, lo, thr, p, cut, denom)) {
+      n_cand = gather_sorted(sh, cand, sl, rank, cut);
+      thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, denom));
+    } else {
+      float all[1];
+      row_sum<1>(sh, rank, all, [&](int u, float (&v)[1]) {
+        const int i1 = sl.end(u);
+        for (int i = sl.begin(u); i < i1; ++i) {
+          const float x = sl.at(i);
+          if (x >= thr) v[0] += expf(x - m);
+        }
+      });
+      thr = fmaxf(thr, radix_threshold<true>(sh, sl, rank, m, thr, p * all[0]));
     }
-    row_sum_vec<1>(sh, d1, rank, denom);
-    thr = fmaxf(thr, radix_threshold<true>(sh, sl, rank, m, thr, p * denom[0]));
   }
 
-  // inverse CDF in vocabulary order: threads in order within a CTA, CTAs in rank order
-  float mine = 0.f;
-  for (int i = i0; i < i1; ++i) {
-    const float x = sl.at(i);
-    if (x >= thr) mine += expf(x - m);
-  }
+  // inverse CDF in vocabulary order: segments in order within a CTA, CTAs in rank order
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float incl = mine;                                     // inclusive scan over the lanes of the warp
+  float mine[VT], incl[VT];                              // a segment's mass, and its inclusive scan over its warp of segments
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const float v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
+  for (int vt = 0; vt < VT; ++vt) {
+    const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
+    float t = 0.f;
+    for (int i = sl.begin(u); i < i1; ++i) {
+      const float x = sl.at(i);
+      if (x >= thr) t += expf(x - m);
+    }
+    mine[vt] = incl[vt] = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, incl[vt], o);
+      if (lane >= o) incl[vt] += v;
+    }
+    if (lane == 31) sh.warp_tot[u >> 5] = incl[vt];
   }
-  if (lane == 31) sh.warp_tot[warp] = incl;
   __syncthreads();
   if (threadIdx.x == 0) {
     float s = 0.f;
-    for (int w = 0; w < BLOCK / 32; ++w) s += sh.warp_tot[w];
+    for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) s += sh.warp_tot[w];
     sh.blk[0] = s;
   }
   __syncthreads();
@@ -584,7 +635,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
       float w_before = before;
       int w_last = -1;
       float w_before_last = before;
-      for (int w = 0; w < BLOCK / 32; ++w) {
+      for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) {
         const float t = sh.warp_tot[w];
         if (t > 0.f) { w_last = w; w_before_last = cum; }
         if (w_own < 0 && !clamp && t > 0.f && cum + t >= target) { w_own = w; w_before = cum; }
@@ -595,22 +646,25 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
       sh.blk[1] = w_before;
     }
     __syncthreads();
-    if (warp == sh.pick[0]) {
+#pragma unroll
+    for (int vt = 0; vt < VT; ++vt) {
+      if (vt * (NT / 32) + warp != sh.pick[0]) continue;
       const bool clamp_w = sh.pick[2] != 0;
       const float base = sh.blk[1];
-      const float excl = incl - mine;                    // mass of the lanes before this one
-      // the first lane whose inclusive sum reaches the target (or the last lane that keeps anything)
-      const bool hit = !clamp_w && mine > 0.f && base + incl >= target;
+      const float excl = incl[vt] - mine[vt];            // mass of the segments of the warp before this one
+      // the first segment whose inclusive sum reaches the target (or the last one that keeps anything)
+      const bool hit = !clamp_w && mine[vt] > 0.f && base + incl[vt] >= target;
       const unsigned hits = __ballot_sync(0xffffffffu, hit);
-      const unsigned keeps = __ballot_sync(0xffffffffu, mine > 0.f);
+      const unsigned keeps = __ballot_sync(0xffffffffu, mine[vt] > 0.f);
       int l_own;
       bool clamp_l = false;
       if (hits) l_own = __ffs(hits) - 1;
       else { l_own = 31 - __clz(keeps); clamp_l = true; }
       if (lane == l_own) {
+        const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
         float cum = base + excl;
         int last = -1;
-        for (int i = i0; i < i1; ++i) {
+        for (int i = sl.begin(u); i < i1; ++i) {
           const float xv = sl.at(i);
           if (xv >= thr) {
             cum += expf(xv - m);
@@ -747,8 +801,8 @@ __global__ void logprobs_kernel(const float* __restrict__ logits, int64_t ld, co
 }
 
 template <typename... KArgs, typename... Args>
-int launch_rows(void (*kernel)(KArgs...), int rows, size_t smem, cudaStream_t stream, const char* what, Args... args) {
-  cudaError_t e = launch_pdl_cluster(kernel, dim3(rows * ROW_CTAS), dim3(BLOCK), dim3(ROW_CTAS, 1, 1), smem, stream, args...);
+int launch_rows(void (*kernel)(KArgs...), int rows, int threads, size_t smem, cudaStream_t stream, const char* what, Args... args) {
+  cudaError_t e = launch_pdl_cluster(kernel, dim3(rows * ROW_CTAS), dim3(threads), dim3(ROW_CTAS, 1, 1), smem, stream, args...);
   if (e != cudaSuccess) return refuse((int)e, "%s: launch failed: %s", what, cudaGetErrorString(e));
   return cuda_status(what);
 }
@@ -765,7 +819,7 @@ DINFER_API int dinfer_argmax(const float* logits, int64_t ld, int* out, int rows
     if (e != cudaSuccess) return refuse((int)e, "argmax: launch failed: %s", cudaGetErrorString(e));
     return cuda_status("argmax");
   }
-  return launch_rows(argmax_kernel, rows, 0, stream, "argmax", logits, ld, out, vocab);
+  return launch_rows(argmax_kernel, rows, BLOCK, 0, stream, "argmax", logits, ld, out, vocab);
 }
 
 // temperature [rows]; top_k (<=0: off), top_p, min_p may be null; seeds, offsets [rows] uint64.
@@ -784,7 +838,7 @@ DINFER_API int dinfer_sample(const float* logits, int64_t ld, const float* tempe
     if (e != cudaSuccess) return refuse((int)e, "sample: shared memory opt-in failed: %s", cudaGetErrorString(e));
     opted = true;
   }
-  return launch_rows(sample_kernel, rows, smem, stream, "sample", logits, ld, temperature, top_k, top_p, min_p, seeds,
+  return launch_rows(sample_kernel, rows, NT, smem, stream, "sample", logits, ld, temperature, top_k, top_p, min_p, seeds,
                      offsets, out, vocab, cache_slice);
 }
 

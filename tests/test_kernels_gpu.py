@@ -429,6 +429,49 @@ def test_top_k_the_short_way_and_its_fallbacks():
     assert all(100 <= t < 6100 for t in seen) and max(seen) > 100 + 0.9 * 6000
 
 
+@pytest.mark.parametrize("V", [7, 40, 8 * 1024 + 3, 151936])
+def test_sampling_cuts_and_many_rows(V):
+    """Rows whose thresholds lie at the first cuts, in a gap far below the maximum (one certain token), among more entries
+    than the short way takes, between masked entries, across ties; one row at a time and 24 at once: the draw falls into the
+    token's share of the plain sampler's mass, the same tokens both ways."""
+    from dinfer_b200.sampling import sampler as S
+    g = torch.Generator().manual_seed(V)
+    base = torch.randn(V, generator=g) * 2
+    sure = base - 80.0
+    sure[V // 3] = 60.0                                       # everything else 130 and more below
+    spread = torch.linspace(-400.0, 20.0, V)[torch.randperm(V, generator=g)]
+    masked = base.clone()
+    masked[torch.randperm(V, generator=g)[:V - max(2, V // 50)]] = float("-inf")
+    ties = base.round()
+    flat = base * 0.01
+    rows = [(r, k, p, mp) for r in (base, sure, spread, masked, flat)
+            for k, p, mp in ((-1, 0.9, 0.0), (min(20, max(1, V // 2)), 1.0, 0.0), (5, 0.7, 0.0), (-1, 0.999, 1e-4))]
+    rows += [(ties, k, 1.0, mp) for k, mp in ((-1, 0.0), (20, 0.0), (5, 0.1), (600, 0.0))]
+    logits = torch.stack([r[0] for r in rows])
+    R = len(rows)
+    assert R >= 19
+    temps = torch.full((R,), 0.8)
+    topk = torch.tensor([r[1] for r in rows], dtype=torch.int32)
+    topp, minp = torch.tensor([r[2] for r in rows]), torch.tensor([r[3] for r in rows])
+    seeds = torch.arange(R, dtype=torch.int64) + 11
+    d, cols = dev(logits), [dev(t) for t in (temps, seeds, topk, topp, minp)]
+    for off in range(6):
+        offs = dev(torch.full((R,), off, dtype=torch.int64))
+        got = S.sample(d, cols[0], cols[1], offs, top_k=cols[2], top_p=cols[3], min_p=cols[4])
+        alone = torch.cat([S.sample(d[i:i + 1], cols[0][i:i + 1], cols[1][i:i + 1], offs[i:i + 1], top_k=cols[2][i:i + 1],
+                                    top_p=cols[3][i:i + 1], min_p=cols[4][i:i + 1]) for i in range(R)])
+        assert torch.equal(got, alone)
+        for i in range(R):
+            # the token's share of the cumulative mass holds the draw: a sum over a segment, its warp, the block and the
+            # cluster is off by at most (seg + 5 + 32 + 8) 2^-24 of the total, a threshold by an entry at most
+            x = P.filter_logits(logits[i].double() / 0.8, int(topk[i]), float(topp[i]), float(minp[i]))
+            w = torch.exp(x - x.max())
+            t = int(got[i])
+            near = float(w.sum()) * 64 * 2.0 ** -24 + 2 * float(w[w > 0].min())
+            target, upto = P.philox_uniform(int(seeds[i]), off) * float(w.sum()), float(w[:t + 1].sum())
+            assert upto >= target - near and upto - float(w[t]) <= target + near, (i, off)
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_attention_generic_without_pages(dt):
     """A request whose table holds no page (a dummy row of a captured graph) has no keys: its output is zero and
