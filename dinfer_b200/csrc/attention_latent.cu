@@ -204,6 +204,7 @@ struct LatentTcParams {
   const int* block_table; int max_blocks;
   const int* cu_seqlens; const int* seq_lens;
   int num_reqs, H, R, P, block_size, window, splits;
+  int singles;                   // only the requests that bring one token (the portions are somebody else's)
   float scale_log2;
   float* part;                   // [T * H, splits, R] unnormalised sums (splits > 1)
   float* ml;                     // [T * H, splits, 2] maximum (log2 domain) and sum
@@ -244,7 +245,7 @@ attention_latent_tc_kernel(const LatentTcParams p) {
   int b = 0, tile = blockIdx.x, n_q = 0, tiles = 0;
   for (; b < p.num_reqs; ++b) {
     n_q = cu[b + 1] - cu[b];
-    tiles = n_q > 0 ? (n_q * p.H + BM - 1) / BM : 0;
+    tiles = n_q > 0 && (n_q == 1 || !p.singles) ? (n_q * p.H + BM - 1) / BM : 0;
     if (tile < tiles) break;
     tile -= tiles;
   }
@@ -502,13 +503,14 @@ DINFER_API int dinfer_attention_latent_tc_rows(int R, int max_rows_per_req) {
 }
 
 // bfloat16 only.  q [T, H, R + P] (ldq_t, ldq_h), out [T, H, R] (ldo_t, ldo_h), cache [pages, block_size, R + P];
+// singles: requests that bring more than one token are left out (their rows of out hold nothing afterwards).
 // seq_lens [B]: tokens of each request after the step; row_tiles >= sum_b ceil(n_q(b) * H / BM) with BM from
 // dinfer_attention_latent_tc_rows(R, max_q_len * H); splits > 1 needs part [T * H * splits * R] and ml [T * H * splits * 2].
 DINFER_API int dinfer_attention_latent_tc(const void* q, int64_t ldq_t, int64_t ldq_h, void* out, int64_t ldo_t,
                                           int64_t ldo_h, const void* cache, const int* block_table, int max_blocks,
                                           const int* cu_seqlens, const int* seq_lens, int T, int B, int H, int R, int P,
                                           int block_size, float scale, int window, int max_rows_per_req, int row_tiles,
-                                          int splits, float* part, float* ml, const float* sinks, cudaStream_t stream) {
+                                          int splits, float* part, float* ml, const float* sinks, int singles, cudaStream_t stream) {
   if (T < 0 || B <= 0 || H <= 0 || R <= 0 || P < 0 || block_size <= 0 || max_blocks <= 0 || splits <= 0 || row_tiles < 0)
     return refuse(DINFER_BAD_ARGUMENT, "attention_latent_tc: bad sizes T=%d B=%d H=%d R=%d P=%d", T, B, H, R, P);
   if (R % 16 || P % 16 || R > 512 || ldq_t % 8 || ldq_h % 8 || ldo_t % 2 || ldo_h % 2 ||
@@ -523,7 +525,7 @@ DINFER_API int dinfer_attention_latent_tc(const void* q, int64_t ldq_t, int64_t 
   p.cache = (const __nv_bfloat16*)cache; p.block_table = block_table; p.max_blocks = max_blocks;
   p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.num_reqs = B; p.H = H; p.R = R; p.P = P;
   p.block_size = block_size; p.window = window; p.splits = splits; p.scale_log2 = scale * LOG2E;
-  p.part = part; p.ml = ml; p.sinks = sinks;
+  p.part = part; p.ml = ml; p.sinks = sinks; p.singles = singles;
   const int bm = dinfer_attention_latent_tc_rows(R, max_rows_per_req);
   const int nt = (R + 8 * TC_WARPS - 1) / (8 * TC_WARPS);      // n-tiles of the output a warp owns
   int rc;

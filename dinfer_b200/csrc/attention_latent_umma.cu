@@ -6,7 +6,8 @@
 //
 //   latent_rows        the latents of the portions' requests out of their pages: [key][c (R) | rotated part (P)], request
 //                      after request, only those that bring more than one token, with a window from its first visible key
-//                      on; rows behind the last are zeros (up to the bound the caller made the buffer for)
+//                      on; every request filled up with zero rows to whole key tiles, so that no tile holds another request's
+//                      rows (a masked key still meets 0 * V), and zeros behind the last up to the caller's bound
 //   latent_q_turn      the last P elements of every head of q, rotated in place
 //   attention_latent_umma
 //       S = [q_h | q_rot] [k_h | k_rot]^T, softmax, O += P V with k_h, v_h from the expanded rows [key][h][k (D) | v (V)]
@@ -43,12 +44,13 @@ struct Params {
 };
 
 // What request i of the batch contributes: its row-tile pairs, its rows in the gathered latents and the keys in front of them.
-struct Share { int pairs, keys, skip; };
+struct Share { int pairs, keys, rows, skip; };
 __device__ __forceinline__ Share share_of(const int* cu, const int* seq, int i, int window) {
   const int q = cu[i + 1] - cu[i];
-  if (q <= 1) return {0, 0, 0};
+  if (q <= 1) return {0, 0, 0, 0};
   const int skip = window > 0 ? max(0, seq[i] - q - window + 1) : 0;
-  return {(q + 2 * BM - 1) / (2 * BM), seq[i] - skip, skip};
+  const int keys = seq[i] - skip;
+  return {(q + 2 * BM - 1) / (2 * BM), keys, (keys + BN - 1) / BN * BN, skip};
 }
 __device__ __forceinline__ int warp_inclusive(int v, int lane) {
 #pragma unroll
@@ -92,8 +94,8 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
     int before = 0, keys_before = 0;
     for (int i0 = 0; i0 < p.B; i0 += 32) {
       const int i = i0 + lane;
-      const Share sh = i < p.B ? share_of(p.cu_seqlens, p.seq_lens, i, p.window) : Share{0, 0, 0};
-      const int incl = warp_inclusive(sh.pairs, lane), kincl = warp_inclusive(sh.keys, lane);
+      const Share sh = i < p.B ? share_of(p.cu_seqlens, p.seq_lens, i, p.window) : Share{0, 0, 0, 0};
+      const int incl = warp_inclusive(sh.pairs, lane), kincl = warp_inclusive(sh.rows, lane);
       const int chunk = __shfl_sync(0xffffffffu, incl, 31);
       if (y < before + chunk) {
         const unsigned hit = __ballot_sync(0xffffffffu, y >= before + incl - sh.pairs && y < before + incl);
@@ -101,7 +103,7 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
         b = i0 + src;
         pair = y - before - __shfl_sync(0xffffffffu, incl - sh.pairs, src);
         pairs_b = __shfl_sync(0xffffffffu, sh.pairs, src);
-        key0 = keys_before + __shfl_sync(0xffffffffu, kincl - sh.keys, src);
+        key0 = keys_before + __shfl_sync(0xffffffffu, kincl - sh.rows, src);
         break;
       }
       before += chunk;
@@ -224,6 +226,11 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
         if (!ok) break;
         tc_commit(smem_u32(&v_empty[sv]));                     // the stages go back when the products issued so far have read them
         if (j + 1 < n_tiles) tc_commit(smem_u32(&k_empty[s1]));
+      }
+      // the last commits arrive on the stages' barriers: the block's memory has to be there still
+      if (ok && !(mbar_wait(smem_u32(&v_empty[(n_tiles - 1) % VS]), ((n_tiles - 1) / VS) & 1) &&
+                  mbar_wait(smem_u32(&k_empty[(n_tiles - 1) % KS]), ((n_tiles - 1) / KS) & 1))) {
+        *s_abort = 1; atomicExch(p.status, 34);
       }
     }
   } else {
@@ -372,14 +379,15 @@ latent_rows_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restr
   int b = -1, j = 0, before = 0;
   for (int i0 = 0; i0 < B; i0 += 32) {
     const int i = i0 + lane;
-    const Share sh = i < B ? share_of(cu, seq, i, window) : Share{0, 0, 0};
-    const int incl = warp_inclusive(sh.keys, lane);
+    const Share sh = i < B ? share_of(cu, seq, i, window) : Share{0, 0, 0, 0};
+    const int incl = warp_inclusive(sh.rows, lane);
     const int chunk = __shfl_sync(0xffffffffu, incl, 31);
     if (row < before + chunk) {
-      const unsigned hit = __ballot_sync(0xffffffffu, row >= before + incl - sh.keys && row < before + incl);
+      const unsigned hit = __ballot_sync(0xffffffffu, row >= before + incl - sh.rows && row < before + incl);
       const int src = __ffs(hit) - 1;
-      b = i0 + src;
-      j = row - before - __shfl_sync(0xffffffffu, incl - sh.keys, src) + __shfl_sync(0xffffffffu, sh.skip, src);
+      j = row - before - __shfl_sync(0xffffffffu, incl - sh.rows, src);
+      if (j < __shfl_sync(0xffffffffu, sh.keys, src)) b = i0 + src;
+      j += __shfl_sync(0xffffffffu, sh.skip, src);
       break;
     }
     before += chunk;
@@ -445,7 +453,8 @@ bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 
 
 DINFER_DEFINE_LAST_ERROR()
 
-// out [rows, W] bf16, rows >= the keys of all requests that bring more than one token (those beyond the window left out);
+// out [rows, W] bf16, rows >= the sum over the requests that bring more than one token of their keys (those beyond the window
+// left out), each rounded up to a multiple of 128;
 // cache [pages, block_size, W] bf16; block_table [B, max_blocks]; cu_seqlens [B + 1]; seq_lens [B].
 DINFER_API int dinfer_latent_rows(void* out, const void* cache, const int* block_table, int max_blocks, const int* cu_seqlens,
                                   const int* seq_lens, int B, int rows, int W, int block_size, int window, cudaStream_t stream) {

@@ -40,6 +40,7 @@ LIBRARIES: Dict[str, tuple] = {
     "attention_umma64": ("attention_umma64.cu", []),
     "latent_post": ("latent_post.cu", []),
     "attention_latent": ("attention_latent.cu", []),
+    "latent_expanded": ("attention_latent_umma.cu", []),
     "moe": ("moe.cu", []),
     "delta_rule": ("delta_rule.cu", []),
     "retention": ("retention.cu", []),

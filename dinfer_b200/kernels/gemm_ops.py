@@ -50,6 +50,12 @@ STATUS_MEANING = {
     16: "prompt attention: the softmax warps waited for the last P V before writing the output",
     21: "decode attention: the TMA producer waited for a free stage",
     22: "decode attention: the compute warps waited for a key/value tile",
+    31: "attention over expanded latents: a TMA producer waited for a free K or V stage",
+    32: "attention over expanded latents: the MMA thread waited for the Q or the first K tiles",
+    33: "attention over expanded latents: the MMA thread waited for the softmax warps' P tile",
+    34: "attention over expanded latents: the MMA thread waited for a K or V tile",
+    35: "attention over expanded latents: the softmax warps waited for a score tile",
+    36: "attention over expanded latents: the softmax warps waited for the last P V before writing the output",
 }
 
 

@@ -1,4 +1,5 @@
-"""Wrappers of the latent-attention kernels (``csrc/latent_post.cu``, ``csrc/attention_latent.cu``)."""
+"""Wrappers of the latent-attention kernels (``csrc/latent_post.cu``, ``csrc/attention_latent.cu``,
+``csrc/attention_latent_umma.cu``)."""
 from __future__ import annotations
 
 from ctypes import c_float, c_int, c_int64, c_void_p
@@ -137,11 +138,12 @@ def tc_splits(row_tiles: int, max_seq_len: int) -> int:
 def attention_latent_tc(q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                         cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, kv_rank: int, rope_dim: int, scale: float,
                         window: int = 0, max_q_len: int = 1, max_seq_len: int = 1, splits: Optional[int] = None,
-                        sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+                        sinks: Optional[torch.Tensor] = None, singles: bool = False) -> torch.Tensor:
     """The same attention on tensor cores (bfloat16): prompt portions and decoded tokens in one launch.  ``seq_lens`` [B]:
     tokens of each request after the step (a token's position follows from it); ``max_q_len``: the longest portion of
     the batch (chooses the row tile); ``max_seq_len``: the longest request (chooses how many CTAs share a row tile's keys
-    unless ``splits`` says)."""
+    unless ``splits`` says).  ``singles``: only for the requests that bring one token; the rows of the others hold
+    nothing afterwards."""
     T, H = _check_attention(q_lat, out, cache, block_table, cu_seqlens, kv_rank, rope_dim)
     require_cuda(seq_lens)
     _check_sinks(sinks, H)
@@ -150,9 +152,9 @@ def attention_latent_tc(q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Ten
         raise KernelError("attention_latent_tc: seq_lens int32 [B]")
     if not tc_supported(q_lat.dtype, kv_rank, rope_dim, cache.shape[-2]):
         raise KernelError("attention_latent_tc: bfloat16 with kv_rank and rope_dim in multiples of 16 only")
-    rows_per_req = max(1, int(max_q_len)) * H
+    rows_per_req = H if singles else max(1, int(max_q_len)) * H
     bm = tc_row_tile(kv_rank, rows_per_req)
-    row_tiles = (T * H + bm - 1) // bm + B
+    row_tiles = B * ((H + bm - 1) // bm) if singles else (T * H + bm - 1) // bm + B
     if splits is None:
         splits = tc_splits(row_tiles, max_seq_len)
     part = ml = None
@@ -162,12 +164,111 @@ def attention_latent_tc(q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Ten
     lib, f = _fn("attention_latent", "dinfer_attention_latent_tc",
                  [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                   c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                  c_void_p])
+                  c_int, c_void_p])
     check(lib, f(ptr(q_lat), q_lat.stride(0), q_lat.stride(1), ptr(out), out.stride(0), out.stride(1), ptr(cache),
                  ptr(block_table), block_table.shape[1], ptr(cu_seqlens), ptr(seq_lens), T, B, H, kv_rank, rope_dim,
                  cache.shape[-2], float(scale), int(window), rows_per_req, row_tiles, int(splits), ptr(part), ptr(ml),
-                 ptr(sinks), stream_handle()), "attention_latent_tc")
+                 ptr(sinks), int(bool(singles)), stream_handle()), "attention_latent_tc")
     if splits > 1:
         from .lib import add_launches
         add_launches(1)                                   # the fold kernel
+    return out
+
+
+# ---- portions over expanded latents (csrc/attention_latent_umma.cu)
+KEY_TILE = 128                                              # a request's gathered rows are filled up to whole key tiles
+
+
+def expanded_supported(dtype: torch.dtype, kv_rank: int, rope_dim: int, nope_dim: int, v_dim: int) -> bool:
+    """Sizes the kernel over expanded latents takes: bfloat16, keys and values of 64 or 128, a rotated part of at most 64."""
+    return (dtype == torch.bfloat16 and nope_dim == v_dim and nope_dim in (64, 128) and 0 <= rope_dim <= 64
+            and rope_dim % 8 == 0 and kv_rank > 0 and kv_rank % 8 == 0)
+
+
+def expanded_rows(portions, window: int = 0) -> int:
+    """Rows of the gathered latents of ``portions`` = [(new tokens, tokens after the step)], as ``latent_rows`` lays them out."""
+    rows = 0
+    for n, total in portions:
+        keys = total - (max(0, total - n - window + 1) if window > 0 else 0)
+        rows += (keys + KEY_TILE - 1) // KEY_TILE * KEY_TILE
+    return rows
+
+
+def _check_batch(block_table, cu_seqlens, seq_lens):
+    B = cu_seqlens.numel() - 1
+    for t, n in ((block_table, "block_table"), (cu_seqlens, "cu_seqlens"), (seq_lens, "seq_lens")):
+        if t is not None and (t.dtype != torch.int32 or not t.is_contiguous()):
+            raise KernelError(f"latent attention: {n} must be contiguous int32")
+    if seq_lens.numel() < B or (block_table is not None and (block_table.dim() != 2 or block_table.shape[0] < B)):
+        raise KernelError("latent attention: block_table [B, max_blocks], seq_lens [B]")
+    return B
+
+
+def latent_rows(cache: torch.Tensor, block_table: torch.Tensor, cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, rows: int,
+                window: int = 0) -> torch.Tensor:
+    """The cached rows of the requests that bring more than one token, [rows, R + P], request after request, each filled up
+    with zeros to a multiple of ``KEY_TILE``; with a window from the first key on that its portion sees."""
+    require_cuda(cache, block_table, cu_seqlens, seq_lens)
+    B = _check_batch(block_table, cu_seqlens, seq_lens)
+    if cache.dtype != torch.bfloat16 or not cache.is_contiguous() or cache.dim() < 3:
+        raise KernelError("latent_rows: a contiguous bfloat16 cache [pages, ..., page, R + P]")
+    W = cache.shape[-1]
+    out = torch.empty((rows, W), dtype=cache.dtype, device=cache.device)
+    lib, f = _fn("latent_expanded", "dinfer_latent_rows",
+                 [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    check(lib, f(ptr(out), ptr(cache), ptr(block_table), block_table.shape[1], ptr(cu_seqlens), ptr(seq_lens), B, rows, W,
+                 cache.shape[-2], int(window), stream_handle()), "latent_rows")
+    return out
+
+
+def latent_q_turn(q: torch.Tensor, positions: torch.Tensor, cos_sin: Optional[torch.Tensor], num_heads: int, nope_dim: int,
+                  rope_dim: int, halves: bool = False) -> torch.Tensor:
+    """The last ``rope_dim`` elements of every head of ``q`` [T, H * (nope_dim + rope_dim)] rotated in place."""
+    require_cuda(q, positions, cos_sin)
+    _rows_contiguous(q, "latent_q_turn")
+    T = q.shape[0]
+    if q.dtype != torch.bfloat16 or q.shape[1] != num_heads * (nope_dim + rope_dim) or positions.dtype != torch.int32 \
+            or positions.numel() != T:
+        raise KernelError("latent_q_turn: q bfloat16 [T, H (D + P)], positions int32 [T]")
+    if cos_sin is None:
+        return q
+    if cos_sin.dtype != torch.float32 or cos_sin.dim() != 2 or not cos_sin.is_contiguous():
+        raise KernelError("latent_q_turn: angle table must be contiguous float32 [max_pos, rot]")
+    lib, f = _fn("latent_expanded", "dinfer_latent_q_turn",
+                 [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    check(lib, f(ptr(q), q.stride(0), ptr(positions), ptr(cos_sin), cos_sin.shape[1], T, num_heads, nope_dim, rope_dim,
+                 int(bool(halves)), stream_handle()), "latent_q_turn")
+    return q
+
+
+def attention_latent_umma(q: torch.Tensor, out: torch.Tensor, latents: torch.Tensor, expanded: torch.Tensor,
+                          cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, kv_rank: int, rope_dim: int, head_dim: int,
+                          scale: float, window: int = 0, sinks: Optional[torch.Tensor] = None,
+                          pair_bound: int = 0) -> torch.Tensor:
+    """Causal attention of the portions (requests that bring more than one token): ``q`` [T, H * (D + P)] with its last parts
+    turned, ``latents`` [rows, R + P] from ``latent_rows``, ``expanded`` [rows, H * 2 D] the keys and values of every head made
+    from them; ``out`` [T, H, D], the rows of other requests untouched.  ``pair_bound``: at least the sum over the portions of
+    ceil(tokens / 256)."""
+    from . import gemm_ops
+    require_cuda(q, out, latents, expanded, cu_seqlens, seq_lens)
+    B = _check_batch(None, cu_seqlens, seq_lens)
+    T, H = out.shape[0], out.shape[1]
+    rows = latents.shape[0]
+    _rows_contiguous(q, "attention_latent_umma q")
+    _check_sinks(sinks, H)
+    if any(t.dtype != torch.bfloat16 for t in (q, out, latents, expanded)) or out.dim() != 3 or out.shape[2] != head_dim \
+            or out.stride(2) != 1 or out.stride(1) != head_dim or tuple(q.shape) != (T, H * (head_dim + rope_dim)):
+        raise KernelError("attention_latent_umma: bfloat16 q [T, H (D + P)], out [T, H, D] with whole rows")
+    if tuple(latents.shape) != (rows, kv_rank + rope_dim) or tuple(expanded.shape) != (rows, H * 2 * head_dim) \
+            or not latents.is_contiguous() or not expanded.is_contiguous():
+        raise KernelError("attention_latent_umma: latents [rows, R + P] and expanded [rows, H * 2 D], contiguous")
+    if not expanded_supported(q.dtype, kv_rank, rope_dim, head_dim, head_dim):
+        raise KernelError("attention_latent_umma: sizes not supported")
+    status = gemm_ops._state(q.device)["status"]
+    lib, f = _fn("latent_expanded", "dinfer_attention_latent_umma",
+                 [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                  c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p, c_void_p])
+    check(lib, f(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(latents), ptr(expanded), rows, ptr(cu_seqlens), ptr(seq_lens),
+                 T, B, H, kv_rank, rope_dim, head_dim, float(scale), int(window), ptr(sinks), int(pair_bound), ptr(status),
+                 stream_handle()), "attention_latent_umma")
     return out

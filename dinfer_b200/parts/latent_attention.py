@@ -16,6 +16,11 @@ step never expands a cached row into per-head keys and values:
   o[:, h] = o_lat[:, h] W_uv[h]^T          batched product
   y = o W_o^T
 
+Portions of several tokens are worth expanding the rows they see (``LatentAttention._expanded``): from q on
+
+  rows = the cached rows of the portions' requests, gathered;  kv = c [W_uk; W_uv]^T    one product for all heads
+  o[:, h] = softmax((q_h . [k_h | kr]) * scale) v_h
+
 A layer with ``own_kv`` False has no W_dkv: its schedule entry reads another entry's cache (``cache.write`` False)
 with its own W_uk, W_uv and queries.
 """
@@ -109,12 +114,17 @@ class LatentAttention(Mixer):
         # per head: W_uk[h] is [D, R]; the absorbing product wants it as [R, D] (out, in)
         self.uk_t = t["uk"].reshape(self.H, self.D, self.R).transpose(1, 2).contiguous()
         self.uv = t["uv"].reshape(self.H, self.V, self.R).contiguous()
+        # [H (D + V), R]: what makes a row's keys and values of all heads, head after head
+        self.ukv = None
+        if latent_ops.expanded_supported(t["uk"].dtype, self.R, self.P, self.D, self.V) and t["uv"].dtype == t["uk"].dtype:
+            self.ukv = torch.cat([t["uk"].reshape(self.H, self.D, self.R), self.uv], dim=1).reshape(-1, self.R).contiguous()
 
     def cache_need(self):
         return KvCacheNeed(1, self.R + self.P, self.window, int(self.page_size) if self.page_size else None, planes=1)
 
     def kernel_libraries(self):
-        return (["latent_post", "attention_latent", "gemm_f32"] + (["elementwise"] if self.gate_name else []) + self.down.kernel_libraries() + self.uq.kernel_libraries()
+        expanded = ["latent_expanded", "gemm_tc"] if self.ukv is not None and self.env.act_dtype == torch.bfloat16 else []
+        return (["latent_post", "attention_latent", "gemm_f32"] + expanded + (["elementwise"] if self.gate_name else []) + self.down.kernel_libraries() + self.uq.kernel_libraries()
                 + self.o.kernel_libraries())
 
     def forward(self, x, ctx: StepContext, cache: CacheBinding, sink=None):
@@ -131,14 +141,20 @@ class LatentAttention(Mixer):
                                     self.eps, table, cache.kv if write else None, g.slot_mapping if write else None,
                                     halves=self.halves)
         q = self.uq(low[:, :Rq])                                         # [T, H (D + P)]
-        # head-major storage, seen as [T, H, *]: the batched products then write whole matrices per head
-        q_lat = torch.empty((H, T, R + P), dtype=q.dtype, device=q.device).transpose(0, 1)
-        self.absorb(q.view(T, H, D + P)[:, :, :D], self.uk_t, q_lat[:, :, :R])
-        latent_ops.latent_q_rope(q, ctx.positions, table, q_lat, H, D, P, R, halves=self.halves)
-        o_lat = torch.empty((H, T, R), dtype=q.dtype, device=q.device).transpose(0, 1)
-        self.attend(q_lat, o_lat, cache.kv, g, ctx)
-        o = torch.empty((T, H, V), dtype=q.dtype, device=q.device)
-        self.absorb(o_lat, self.uv, o)
+        expanded = self._expanded(ctx, q.dtype)
+        # (a dummy portion of one token in a captured graph belongs to neither way: its row has to hold something finite)
+        make = torch.zeros if expanded is not None and not ctx.any_decode else torch.empty
+        o = make((T, H, V), dtype=q.dtype, device=q.device)
+        if expanded is None or ctx.any_decode:
+            # head-major storage, seen as [T, H, *]: the batched products then write whole matrices per head
+            q_lat = torch.empty((H, T, R + P), dtype=q.dtype, device=q.device).transpose(0, 1)
+            self.absorb(q.view(T, H, D + P)[:, :, :D], self.uk_t, q_lat[:, :, :R])
+            latent_ops.latent_q_rope(q, ctx.positions, table, q_lat, H, D, P, R, halves=self.halves)
+            o_lat = torch.empty((H, T, R), dtype=q.dtype, device=q.device).transpose(0, 1)
+            self.attend(q_lat, o_lat, cache.kv, g, ctx, singles=expanded is not None)
+            self.absorb(o_lat, self.uv, o)
+        if expanded is not None:
+            self.attend_expanded(q, o, cache.kv, g, ctx, table, *expanded)
         o = o.view(T, H * V)
         if self.gate_name:
             ops.sigmoid_gate(o, full[:, self.gate_at:self.gate_at + H * V])
@@ -156,14 +172,72 @@ class LatentAttention(Mixer):
         else:
             ops.gemm_f32_batched(a, w, out)
 
-    def attend(self, q_lat, o_lat, kv, g, ctx: StepContext) -> None:
+    # What the two ways of a portion cost, in flops a second they reach here (the absorbed kernel's mma.sync, the expanding
+    # product, the tcgen05 attention) and seconds (the gather and one more launch).
+    RATES = (150e12, 1000e12, 350e12, 15e-6)
+    # the keys and values of a step's portions, all heads, are expanded at once up to so many bytes
+    EXPANDED_BYTES = 256 << 20
+
+    def _expanded(self, ctx: StepContext, dtype):
+        """Whether the step's portions run over expanded latents: None, or (rows of the gathered latents, row-tile pairs).  The
+        absorbed form needs H (2 R + P) multiply-adds a (token, key) pair, the expanded one H (D + P + V) and R H (D + V) a key.
+        One layer of 16 heads of 128 + 64, R 512, a 2048-token prompt: absorbed @@A@@ us of attention and its two products,
+        expanded @@B@@; a portion of @@C@@.  In a captured graph the lengths are bounds: the tokens spread evenly over the
+        prompt places without a history for what the absorbed form costs at least, every place as long as it may get
+        for what the other one costs at most."""
+        if self.ukv is None or dtype != torch.bfloat16 or not ctx.any_prefill or not ctx.cu_seqlens_host:
+            return None
+        key = ("latent_expanded", self.H, self.D, self.P, self.V, self.R, self.window)
+        if key not in ctx.derived:
+            ctx.derived[key] = self._expanded_shape(ctx)
+        return ctx.derived[key]
+
+    def _expanded_shape(self, ctx: StepContext):
+        cu, window = ctx.cu_seqlens_host, int(self.window or 0)
+        lens = [cu[i + 1] - cu[i] for i in range(len(cu) - 1)]
+        if ctx.decode_splits:                                # captured: any place may hold any of the prompt tokens
+            tokens, places = sum(n for n in lens if n != 1), sum(n != 1 for n in lens)
+            if not tokens:
+                return None
+            longest = ctx.max_prefill_seq_len or ctx.max_seq_len
+            pairs = tokens * tokens / (2.0 * places)
+            bound = [(min(tokens, longest), longest)] * places
+            tiles = tokens // 256 + places
+        else:
+            bound = [(n, s) for n, s in zip(lens, ctx.seq_lens_host) if n > 1]
+            if not bound:
+                return None
+            pairs = float(sum(n * (min(s - n, window) if window else s - n) + n * (n + 1) // 2 for n, s in bound))
+            tiles = sum((n + 255) // 256 for n, _ in bound)
+        if window:
+            pairs = min(pairs, float(window) * sum(n for n, _ in bound))
+        rows = latent_ops.expanded_rows(bound, window)
+        absorbed, expanding, attending, fixed = self.RATES
+        H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
+        pays = (pairs * H * 2 * (2 * R + P) / absorbed
+                > rows * R * H * 2 * (D + V) / expanding + pairs * H * 2 * (D + P + V) / attending + fixed)
+        if not pays or rows * H * (D + V) * 2 > self.EXPANDED_BYTES or tiles > 65535:
+            return None
+        return rows, tiles
+
+    def attend_expanded(self, q, o, kv, g, ctx: StepContext, table, rows: int, tiles: int) -> None:
+        window = int(self.window or 0)
+        latent_ops.latent_q_turn(q, ctx.positions, table, self.H, self.D, self.P, halves=self.halves)
+        latents = latent_ops.latent_rows(kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, rows, window)
+        expanded = torch.empty((rows, self.ukv.shape[0]), dtype=q.dtype, device=q.device)
+        add_launches(1)
+        torch.mm(latents[:, :self.R], self.ukv.t(), out=expanded)
+        latent_ops.attention_latent_umma(q, o, latents, expanded, ctx.cu_seqlens, ctx.seq_lens, self.R, self.P, self.D,
+                                         self.scale, window, sinks=self.sinks, pair_bound=tiles)
+
+    def attend(self, q_lat, o_lat, kv, g, ctx: StepContext, singles: bool = False) -> None:
         window = int(self.window or 0)
         if latent_ops.tc_supported(q_lat.dtype, self.R, self.P, g.block_size):
             # inside a captured graph the longest request is whatever the engine admits
             longest = self.env.max_positions if ctx.decode_splits else ctx.max_seq_len
             latent_ops.attention_latent_tc(q_lat, o_lat, kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, self.R, self.P,
                                            self.scale, window, max_q_len=ctx.max_q_len, max_seq_len=longest,
-                                           sinks=self.sinks)
+                                           sinks=self.sinks, singles=singles)
         else:
             latent_ops.attention_latent_generic(q_lat, o_lat, kv, g.block_table, ctx.cu_seqlens, ctx.positions, self.R,
                                                 self.P, self.scale, window, sinks=self.sinks)
