@@ -252,6 +252,7 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
     bool ok = true;
     for (int j = 0; j < n_w; ++j) {
       if (ok && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&s_full[w]), j & 1))) { *s_abort = 1; atomicExch(p.status, 35); ok = false; }
+      __syncwarp();
       tc_fence_after();
       const int jbase = (tile_first + j) * BN;
       const bool need_mask = (jbase + BN - 1 > hist + row0 + w * BM) || jbase < lo_all;
@@ -339,23 +340,26 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
       if (p.sinks) l += exp2f(sink_log2(p.sinks, head) - m_run);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       __nv_bfloat16* dst = p.out + (int64_t)(t0 + row) * p.ldo + (int64_t)head * D + h * (D / 2);
+      // all of tensor memory is read ahead of the one branch on row_ok: tcgen05.ld is an instruction of the whole warp, and
+      // between two branches on the same lanes' condition the compiler may let the lanes go their ways in between as well
+      uint32_t y[D / 4];
 #pragma unroll
       for (int c = 0; c < D / 64; ++c) {
         float o[32];
+        __syncwarp();
         tmem_ld32(o_addr + c * 32, o);
         tmem_ld_wait();
-        if (row_ok) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint4 v;
-            v.x = pack_bf16(o[q4 * 8] * inv, o[q4 * 8 + 1] * inv); v.y = pack_bf16(o[q4 * 8 + 2] * inv, o[q4 * 8 + 3] * inv);
-            v.z = pack_bf16(o[q4 * 8 + 4] * inv, o[q4 * 8 + 5] * inv); v.w = pack_bf16(o[q4 * 8 + 6] * inv, o[q4 * 8 + 7] * inv);
-            reinterpret_cast<uint4*>(dst + c * 32)[q4] = v;
-          }
-        }
+        for (int i = 0; i < 16; ++i) y[c * 16 + i] = pack_bf16(o[2 * i] * inv, o[2 * i + 1] * inv);
+      }
+      if (row_ok) {
+#pragma unroll
+        for (int i = 0; i < D / 16; ++i)
+          reinterpret_cast<uint4*>(dst)[i] = make_uint4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
       }
     }
   }
+  __syncwarp();                                                // (lanes that had no part in a warp's role wait for the one that did)
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
