@@ -37,7 +37,7 @@ constexpr uint32_t PART = BM * 128;                            // bytes of a 128
 struct Params {
   __nv_bfloat16* out; int64_t ldo;
   const int* cu_seqlens; const int* seq_lens;
-  int B, P, window;
+  int B, window;
   float scale_log2;
   const float* sinks;
   int* status;
@@ -181,16 +181,17 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
       constexpr uint32_t idesc_qk = idesc_bf16(BM, BN, 0), idesc_pv = idesc_bf16(BM, D, 1);
       const uint64_t dq = desc_k_major(sQ), dk = desc_k_major(sK);
       const uint64_t dv = desc_mn_major(sV, PART);
-      const int k_steps = (D + p.P + 15) / 16;
       const int n_of[2] = {n_tiles_a, b_on ? n_tiles : 0};
+      // Every 16 elements of D + 64 are multiplied, zeros behind P included, in one straight run: with a condition on P
+      // around each product the compiled code handed later tiles' products wrong descriptors (sums with parts missing, and
+      // reads outside the block's memory).
       auto issue_qk = [&](int w, int t) {
         const uint64_t dqs = dq + (uint64_t)(w * (S::Q_BYTES >> 4));
         const uint64_t dks = dk + (uint64_t)((t % KS) * (S::K_BYTES >> 4));
 #pragma unroll
         for (int k = 0; k < (NH + 1) * 4; ++k)
-          if (k < k_steps)
-            tc_mma(tmem + w * BN, dqs + (uint64_t)(((k / 4) * PART + (k % 4) * 32) >> 4),
-                   dks + (uint64_t)(((k / 4) * PART + (k % 4) * 32) >> 4), idesc_qk, k > 0 ? 1u : 0u);
+          tc_mma(tmem + w * BN, dqs + (uint64_t)(((k / 4) * PART + (k % 4) * 32) >> 4),
+                 dks + (uint64_t)(((k / 4) * PART + (k % 4) * 32) >> 4), idesc_qk, k > 0 ? 1u : 0u);
         tc_commit(smem_u32(&s_full[w]));
       };
       auto issue_pv = [&](int w, int j) {
@@ -502,13 +503,13 @@ DINFER_API int dinfer_attention_latent_umma(const void* q, int64_t ldq, void* ou
   const cuuint64_t dq[3] = {(cuuint64_t)(D + P), (cuuint64_t)H, (cuuint64_t)T}, sq[2] = {(cuuint64_t)(D + P) * 2, (cuuint64_t)ldq * 2};
   const cuuint64_t dkv[2] = {(cuuint64_t)H * 2 * D, (cuuint64_t)rows}, skv[1] = {(cuuint64_t)H * 2 * D * 2};
   // the rotated part as a tensor of its own, P wide: what a 64-wide box reaches beyond it is zeros.  (With P = 0 the box
-  // begins where a row's latents do; the product skips that part.)
+  // begins where a row's latents do; Q's part is zeros then.)
   const cuuint64_t dr[2] = {(cuuint64_t)(P > 0 ? P : R), (cuuint64_t)rows}, sr[1] = {(cuuint64_t)(R + P) * 2};
   if (!make_map(&mq, q, 3, dq, sq) || !make_map(&mkv, expanded, 2, dkv, skv) ||
       !make_map(&mr, (const __nv_bfloat16*)latents + (P > 0 ? R : 0), 2, dr, sr))
     return refuse(DINFER_BAD_ARGUMENT, "attention_latent_umma: a tensor map could not be made");
   Params p;
-  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.P = P; p.window = window;
+  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.window = window;
   p.scale_log2 = scale * 1.4426950408889634f; p.sinks = sinks; p.status = status;
   const dim3 grid(H, pair_bound);
   return D == 64 ? launch<64>(mq, mkv, mr, p, grid, stream) : launch<128>(mq, mkv, mr, p, grid, stream);
