@@ -43,6 +43,7 @@ LIBRARIES: Dict[str, tuple] = {
     "latent_expanded": ("attention_latent_umma.cu", []),
     "moe": ("moe.cu", []),
     "delta_rule": ("delta_rule.cu", []),
+    "delta_chunks": ("delta_chunks.cu", []),
     "retention": ("retention.cu", []),
     "short_conv": ("short_conv.cu", []),
     "attention_diff": ("attention_diff.cu", []),

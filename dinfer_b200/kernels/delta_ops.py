@@ -61,12 +61,13 @@ def prep(P: torch.Tensor, cols: Tuple[int, int, int, int], A: torch.Tensor, conv
 
 def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor,
                state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, fresh: torch.Tensor,
-               per_channel: bool, widen: int = 0) -> torch.Tensor:
+               per_channel: bool, widen: int = 0, longest: int = 0) -> torch.Tensor:
     """Token by token per request and head: ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q`` (``decay``
     holds ``g - 1``, as ``prep`` makes it), S [dk, dv]
     of head h at ``state[slot, h * dk * dv:]`` (zero for a fresh request), carried in place.  Returns o f32 [T, H, dv].
     ``widen`` (1, 2, 4; 0: the sizes decide): how far a column's rows are spread over more lanes than 16 rows a lane
-    would need, which only changes the order of the sums."""
+    would need, which only changes the order of the sums.  ``longest``: a bound of the tokens a request brings, where the
+    caller knows one; from ``CHUNKS_FROM`` on portions run in chunks (``_chunks``), again another order of the sums."""
     require_cuda(q, k, v, beta, decay, state, cu_seqlens, slots, fresh)
     _ints(cu_seqlens, slots, fresh)
     T, G, dk = q.shape
@@ -79,6 +80,8 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     out = torch.empty((T, H, dv), dtype=torch.float32, device=q.device)
     if T == 0:
         return out
+    if longest >= CHUNKS_FROM and not per_channel and not widen and _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out):
+        return out
     lib, f = _fn("delta_rule", "dinfer_delta_recurrence",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                   c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
@@ -88,6 +91,36 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
                  ptr(slots), ptr(fresh), ptr(out), B, H, G, dk, dv, int(bool(per_channel)),
                  int(widen), int(T > B), stream_handle()), "delta_recurrence")
     return out
+
+
+# Portions from so many tokens on run in chunks of 32: a chunk costs a request's chain about as much as @@N@@ tokens of the token
+# loop, plus the pass that prepares all chunks (2000 tokens of 16 heads of 128: @@C@@ against 501 us; 48 tokens: @@D@@).
+CHUNKS_FROM = 48
+# bytes of workspace (128 KB a chunk of 32 tokens for 4 heads of 128) beyond which a step stays with the token loop
+CHUNKS_BYTES = 1 << 29
+
+
+def _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out) -> bool:
+    """The recurrence with one decay a head in chunks of 32 tokens (``csrc/delta_chunks.cu``); False where the sizes do not
+    allow it (keys of 64 or 128, values in multiples of 16)."""
+    T, G, dk = q.shape
+    _, H, dv = v.shape
+    B = cu_seqlens.numel() - 1
+    if dk not in (64, 128) or dv % 16 or decay.shape[1] != H or any(t.data_ptr() % 16 for t in (q, k, out)):
+        return False
+    lib, floats = _fn("delta_chunks", "dinfer_delta_chunks_floats", [c_int, c_int])
+    floats.restype = c_int64
+    places = T // 32 + B                                     # at most so many chunks, however the tokens are dealt out
+    words = places * H * int(floats(dk, dv))
+    if 4 * words > CHUNKS_BYTES or H > 65535 or B > 65535:
+        return False
+    work = torch.empty(words, dtype=torch.float32, device=q.device)
+    lib, f = _fn("delta_chunks", "dinfer_delta_chunks",
+                 [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    check(lib, f(ptr(q), ptr(k), ptr(v), ptr(beta), ptr(decay), ptr(state), state.stride(0), ptr(cu_seqlens), ptr(slots),
+                 ptr(fresh), ptr(out), ptr(work), places, B, H, G, dk, dv, stream_handle()), "delta_chunks")
+    return True
 
 
 def post(o: torch.Tensor, weight: torch.Tensor, gate: Optional[torch.Tensor], eps: float, sigmoid_gate: bool,

@@ -124,7 +124,7 @@ class GatedDelta(Mixer):
         return StateNeed((self.state_size + (self.taps - 1) * self.channels,), torch.float32)
 
     def kernel_libraries(self):
-        libs = ["delta_rule"] + self.proj.kernel_libraries() + self.o.kernel_libraries()
+        libs = (["delta_rule"] if self.per_channel else ["delta_rule", "delta_chunks"]) + self.proj.kernel_libraries() + self.o.kernel_libraries()
         for l in (self.decay_up, self.gate_up):
             if l is not None:                               # their input is the 32-bit stacked product: the 32-bit product
                 libs += l.kernel_libraries() + ["gemm_f32"]
@@ -148,7 +148,8 @@ class GatedDelta(Mixer):
         q, k, v, beta, decay = delta_ops.prep(P, (cq, ck, cv, cb), A, self.conv_w, self.A_log, self.dt_bias, state,
                                               self.state_size, ctx.cu_seqlens, slots, fresh, self.H, self.G, self.dk,
                                               self.dv, self.taps, self.per_channel)
-        o = delta_ops.recurrence(q, k, v, beta, decay, state, ctx.cu_seqlens, slots, fresh, self.per_channel)
+        o = delta_ops.recurrence(q, k, v, beta, decay, state, ctx.cu_seqlens, slots, fresh, self.per_channel,
+                                 longest=ctx.max_q_len if ctx.any_prefill else 1)
         y = torch.empty((T, self.nv), dtype=x.dtype, device=x.device)
         delta_ops.post(o, self.norm_w, gate, self.eps, self.sigmoid_gate, y)
         return self.o(y, out_dtype=torch.float32 if self.out_float32 else None)

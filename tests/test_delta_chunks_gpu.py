@@ -1,0 +1,89 @@
+"""The delta rule in chunks of 32 tokens against the recurrence in 64-bit, no further off than the token loop."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def plain(q, k, v, beta, g, S):
+    """One request: q, k [n, H, dk], v [n, H, dv], beta, g [n, H], S [H, dk, dv], 64-bit."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S = g[t, :, None, None] * S
+        u = beta[t, :, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S = S + k[t, :, :, None] * u[:, None]
+        out[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return out, S
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+CASES = [  # H, G, dk, dv, tokens of the requests, fresh, decays, keys
+    (2, 1, 128, 128, [200], [1], "mixed", "random"),
+    (4, 2, 64, 64, [1, 31, 32, 33, 64, 7], [1, 0, 1, 0, 0, 1], "mixed", "random"),
+    (3, 3, 128, 16, [65, 2, 97], [0, 1, 0], "slow", "random"),
+    (2, 2, 64, 48, [130], [0], "fast", "random"),
+    (2, 1, 128, 32, [96, 50], [1, 0], "zero", "random"),
+    (2, 1, 64, 32, [150], [0], "slow", "alike"),
+    (2, 2, 128, 256, [40] * 37, [1, 0] * 18 + [1], "mixed", "random"),
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_chunks_against_plain(case):
+    from dinfer_b200.kernels import delta_ops
+    H, G, dk, dv, tokens, fresh, decays, keys = case
+    g_ = torch.Generator().manual_seed(dk + dv + len(tokens))
+    T, B = sum(tokens), len(tokens)
+    rand = lambda *s: torch.randn(*s, generator=g_)
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)
+    q = unit(rand(T, G, dk)) * dk ** -0.5
+    k = unit(rand(T, G, dk) * (0.02 if keys == "alike" else 1.0) + (1.0 if keys == "alike" else 0.0))
+    v, beta = rand(T, H, dv), torch.sigmoid(rand(T, H) + (3.0 if keys == "alike" else 0.0))
+    x = {"slow": 1e-6 * torch.rand(T, H, generator=g_), "fast": 30 * torch.rand(T, H, generator=g_),
+         "mixed": torch.exp(8 * torch.rand(T, H, generator=g_) - 7), "zero": torch.exp(8 * torch.rand(T, H, generator=g_) - 7)}[decays]
+    decay = torch.expm1(-x.double()).float()
+    if decays == "zero":
+        decay[::5] = -1.0                                    # a decay of 0 forgets everything
+    state = rand(B + 2, H * dk * dv + 5)
+    order = torch.randperm(B + 2, generator=g_)[:B].to(torch.int32)
+    cu = torch.tensor([0] + tokens, dtype=torch.int32).cumsum(0).to(torch.int32)
+    fr = torch.tensor(fresh, dtype=torch.int32)
+    c = lambda t: t.cuda()
+    got, states = [], []
+    for longest in (0, 1000):
+        st = c(state).clone()
+        o = delta_ops.recurrence(c(q), c(k), c(v), c(beta), c(decay), st, c(cu), c(order), c(fr), False, longest=longest)
+        got.append(o.cpu())
+        states.append(st.cpu())
+    assert not torch.equal(got[0], got[1])                   # two ways indeed
+    rep = H // G
+    for i in range(B):
+        a, z, slot = int(cu[i]), int(cu[i + 1]), int(order[i])
+        S0 = state[slot, :H * dk * dv].double().reshape(H, dk, dv) * (0.0 if fresh[i] else 1.0)
+        d = lambda t: t[a:z].double()
+        want, S = plain(d(q).repeat_interleave(rep, 1), d(k).repeat_interleave(rep, 1), d(v), d(beta), d(decay) + 1.0, S0)
+        for w, loop, chunks in ((want, got[0][a:z], got[1][a:z]),
+                                (S, states[0][slot, :H * dk * dv].reshape(H, dk, dv), states[1][slot, :H * dk * dv].reshape(H, dk, dv))):
+            # sums of some 200 products in 32-bit: a few 1e-7; the token loop's own error where that is larger
+            assert rel(chunks, w) <= 1.5 * rel(loop, w) + 1e-6, (i, rel(chunks, w), rel(loop, w))
+    used = set(order.tolist())
+    for s in range(B + 2):                                   # other slots and what lies behind S are untouched
+        keep = slice(H * dk * dv, None) if s in used else slice(None)
+        assert torch.equal(states[1][s, keep], state[s, keep])
+
+
+def test_sizes_the_chunks_do_not_take_stay_with_the_token_loop():
+    from dinfer_b200.kernels import delta_ops
+    g = torch.Generator().manual_seed(3)
+    for dk, dv in ((32, 32), (64, 24), (128, 40)):
+        q, k, v = (torch.randn(60, 1, n, generator=g).cuda() for n in (dk, dk, dv))
+        beta, decay = torch.rand(60, 1, generator=g).cuda(), -torch.rand(60, 1, generator=g).cuda()
+        outs = []
+        for longest in (0, 60):
+            st = torch.zeros(1, dk * dv).cuda()
+            i32 = lambda *x: torch.tensor(x, dtype=torch.int32).cuda()
+            outs.append(delta_ops.recurrence(q, k, v, beta, decay, st, i32(0, 60), i32(0), i32(1), False, longest=longest))
+        assert torch.equal(outs[0], outs[1])
