@@ -114,6 +114,103 @@ delta_prep_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv,
   }
 }
 
+// The same for steps of many tokens (four taps; heads of 64 or 128 key channels that fill blocks of 128 channels): a thread
+// owns a channel and walks RUN tokens with the last three inputs in registers, so that an input is read 11 / 8 times
+// instead of four, and the block's eight norms are summed in one exchange.  Bound by the exponentials and divisions of
+// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) @@A@@ us, a block per (token, head) 64.
+constexpr int RUN = 8;
+constexpr int RUN_FROM = 64;                               // tokens of a step from which it is taken (fewer leave SMs idle)
+template <typename TA>
+__global__ void __launch_bounds__(128)
+delta_prep_run_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv, int cb, const TA* __restrict__ A,
+                      int64_t lda, const float* __restrict__ conv_w, const float* __restrict__ A_log,
+                      const float* __restrict__ dt_bias, const float* __restrict__ hist, int64_t hist_stride,
+                      const int* __restrict__ cu, const int* __restrict__ slots, const int* __restrict__ fresh, int B, int T,
+                      float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ beta,
+                      float* __restrict__ decay, int H, int G, int dk, int dv, int per_channel) {
+  constexpr int TAPS = 4;
+  __shared__ float part[4][RUN];
+  pdl_enter();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int t0 = blockIdx.x * RUN, n = min(RUN, T - t0);
+  const int nq = G * dk, nv = H * dv, C = 2 * nq + nv;
+  const int channel_blocks = (C + 127) / 128;
+  if ((int)blockIdx.y >= channel_blocks) {                 // the decays, and the betas with the first of them
+    const int job = blockIdx.y - channel_blocks, nd = per_channel ? H * dk : H;
+    const int c_end = min(nd, (job + 1) * PREP_CHUNK);
+    for (int t = t0; t < t0 + n; ++t) {
+      if (job == 0)
+        for (int h = tid; h < H; h += 128) beta[(int64_t)t * H + h] = sigmoid_f(to_f32<TA>(P[(int64_t)t * ldp + cb + h]));
+      for (int c = job * PREP_CHUNK + tid; c < c_end; c += 128) {
+        const float a = to_f32<TA>(A[(int64_t)t * lda + c]) + dt_bias[c];
+        decay[(int64_t)t * nd + c] = expm1f(-expf(A_log[per_channel ? c / dk : c]) * softplus_f(a));
+      }
+    }
+    return;
+  }
+  const int c = blockIdx.y * 128 + tid;
+  const bool live = c < C;
+  const int col = c < nq ? cq + c : (c < 2 * nq ? ck + c - nq : cv + c - 2 * nq);
+  float w[TAPS], y[RUN];
+#pragma unroll
+  for (int d = 0; d < TAPS; ++d) w[d] = live ? conv_w[c * TAPS + TAPS - 1 - d] : 0.f;    // w[d] weighs the token d back
+  const int b = request_of(cu, B, t0);
+  const int i0 = t0 - cu[b];
+  if (i0 >= TAPS - 1 && t0 + n <= cu[b + 1]) {             // every tap falls into this request's tokens of the step
+    const TA* x = P + (int64_t)(t0 - (TAPS - 1)) * ldp + col;
+    float in[RUN + TAPS - 1];
+#pragma unroll
+    for (int u = 0; u < RUN + TAPS - 1; ++u) in[u] = live && u < n + TAPS - 1 ? to_f32<TA>(x[(int64_t)u * ldp]) : 0.f;
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) {
+      float acc = 0.f;
+#pragma unroll
+      for (int d = 0; d < TAPS; ++d) acc = fmaf(w[d], in[u + TAPS - 1 - d], acc);
+      y[u] = silu_f(acc);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) {
+      y[u] = 0.f;
+      if (u >= n || !live) continue;
+      const int t = t0 + u, bt = request_of(cu, B, t), i = t - cu[bt];
+      const float* hb = hist + (int64_t)slots[bt] * hist_stride;
+      float acc = 0.f;
+      for (int d = 0; d < TAPS; ++d) {
+        float x = 0.f;
+        if (i - d >= 0) x = to_f32<TA>(P[(int64_t)(t - d) * ldp + col]);
+        else if (!fresh[bt]) x = hb[(TAPS - 1 + i - d) * C + c];
+        acc = fmaf(conv_w[c * TAPS + TAPS - 1 - d], x, acc);
+      }
+      y[u] = silu_f(acc);
+    }
+  }
+  if (blockIdx.y * 128 < 2 * nq) {                         // whole heads of q or k: unit vectors
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) {
+      const float ss = warp_sum(y[u] * y[u]);
+      if (lane == 0) part[warp][u] = ss;
+    }
+    __syncthreads();
+    const int warps = dk / 32, w0 = warp / warps * warps;
+    const bool is_q = c < nq;
+    float* o = (is_q ? qn + c : kn + c - nq) + (int64_t)t0 * nq;
+#pragma unroll
+    for (int u = 0; u < RUN; ++u) {
+      float ss = 0.f;
+      for (int k = 0; k < warps; ++k) ss += part[w0 + k][u];
+      float r = 1.f / sqrtf(ss + 1e-6f);
+      if (is_q) r *= 1.f / sqrtf((float)dk);
+      if (u < n) o[(int64_t)u * nq] = y[u] * r;
+    }
+  } else if (live) {
+    float* o = vv + (int64_t)t0 * nv + c - 2 * nq;
+#pragma unroll
+    for (int u = 0; u < RUN; ++u)
+      if (u < n) o[(int64_t)u * nv] = y[u];
+  }
+}
+
 // the step's last (taps - 1) inputs of every channel become the request's history (rows oldest first)
 template <typename TA>
 __global__ void __launch_bounds__(256)
@@ -422,10 +519,17 @@ DINFER_API int dinfer_delta_prep(const void* P, int64_t ldp, int cq, int ck, int
   const int nd = per_channel ? H * dk : H;
   const int jobs = 2 * G + (nv + PREP_CHUNK - 1) / PREP_CHUNK + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
   if (jobs > 65535) return refuse(DINFER_BAD_ARGUMENT, "delta_prep: too many heads for the grid");
+  const int run_jobs = (2 * nq + nv + 127) / 128 + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
+  const bool runs = taps == 4 && (dk == 64 || dk == 128) && (2 * nq) % 128 == 0 && T >= RUN_FROM && run_jobs <= 65535;
   DINFER_DISPATCH_DTYPE(act_dtype, TA, {
-    launch_pdl(delta_prep_kernel<TA>, dim3(T, jobs), dim3(128), smem, stream, (const TA*)P, ldp, cq, ck, cv, cb, (const TA*)A,
-               lda, conv_w, A_log, dt_bias, (const float*)hist, hist_stride, cu, slots, fresh, B, qn, kn, vv, beta,
-               decay, H, G, dk, dv, taps, per_channel);
+    if (runs)
+      launch_pdl(delta_prep_run_kernel<TA>, dim3((T + RUN - 1) / RUN, run_jobs), dim3(128), 0, stream, (const TA*)P, ldp, cq, ck,
+                 cv, cb, (const TA*)A, lda, conv_w, A_log, dt_bias, (const float*)hist, hist_stride, cu, slots, fresh, B, T, qn,
+                 kn, vv, beta, decay, H, G, dk, dv, per_channel);
+    else
+      launch_pdl(delta_prep_kernel<TA>, dim3(T, jobs), dim3(128), smem, stream, (const TA*)P, ldp, cq, ck, cv, cb, (const TA*)A,
+                 lda, conv_w, A_log, dt_bias, (const float*)hist, hist_stride, cu, slots, fresh, B, qn, kn, vv, beta,
+                 decay, H, G, dk, dv, taps, per_channel);
     if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) return refuse((int)e, "delta_prep: %s", cudaGetErrorString(e));
     if (taps > 1) {
       const int C = 2 * nq + nv;

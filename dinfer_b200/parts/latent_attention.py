@@ -143,7 +143,7 @@ class LatentAttention(Mixer):
         q = self.uq(low[:, :Rq])                                         # [T, H (D + P)]
         expanded = self._expanded(ctx, q.dtype)
         # (a dummy portion of one token in a captured graph belongs to neither way: its row has to hold something finite)
-        make = torch.zeros if expanded is not None and not ctx.any_decode else torch.empty
+        make = torch.zeros if expanded is not None and ctx.decode_splits and not ctx.any_decode else torch.empty
         o = make((T, H, V), dtype=q.dtype, device=q.device)
         if expanded is None or ctx.any_decode:
             # head-major storage, seen as [T, H, *]: the batched products then write whole matrices per head

@@ -87,3 +87,47 @@ def test_sizes_the_chunks_do_not_take_stay_with_the_token_loop():
             i32 = lambda *x: torch.tensor(x, dtype=torch.int32).cuda()
             outs.append(delta_ops.recurrence(q, k, v, beta, decay, st, i32(0, 60), i32(0), i32(1), False, longest=longest))
         assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv,per_channel", [(3, 1, 64, 40, False), (3, 3, 64, 16, True), (2, 1, 128, 72, False)])
+def test_preparation_in_runs(dtype, H, G, dk, dv, per_channel):
+    """Steps of 64 tokens and more (a thread walks eight tokens of a channel) against plain formulas and, beside the short
+    steps' kernel, request by request: requests that begin and end anywhere in a run, fresh and carried histories."""
+    from dinfer_b200.kernels import delta_ops
+    F64 = torch.float64
+    g = torch.Generator().manual_seed(dk + dv + H)
+    lens, fresh, taps = [1, 2, 70, 64, 9, 3], [1, 0, 1, 0, 0, 1], 4
+    T, B, nq, nv = sum(lens), len(lens), G * dk, H * dv
+    C, nd = 2 * nq + nv, H * dk if per_channel else H
+    Pm = torch.randn(T, C + H + 5, generator=g).to(dtype)
+    Am = torch.randn(T, nd, generator=g).to(dtype)
+    conv_w, A_log, dt_bias = torch.randn(C, taps, generator=g), torch.randn(H, generator=g), torch.randn(nd, generator=g) - 1.0
+    S0 = H * dk * dv
+    state = torch.randn(B, S0 + (taps - 1) * C, generator=g)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    ints = lambda x: torch.as_tensor(x, dtype=torch.int32).cuda()
+    call = lambda rows, st, cu_, slots, fr: [o.cpu() for o in delta_ops.prep(
+        Pm[rows].cuda(), (0, nq, 2 * nq, C + 5), Am[rows].cuda(), conv_w.cuda(), A_log.cuda(), dt_bias.cuda(), st, S0, ints(cu_),
+        ints(slots), ints(fr), H, G, dk, dv, taps, per_channel)]
+    st = state.clone().cuda()
+    got = call(slice(0, T), st, cu, list(range(B)), fresh)
+    softplus = lambda z: torch.clamp(z, min=0) + torch.log1p(torch.exp(-z.abs()))
+    for i in range(B):
+        a, z = int(cu[i]), int(cu[i + 1])
+        x = Pm[a:z].to(F64)
+        hist = torch.zeros(taps - 1, C, dtype=F64) if fresh[i] else state[i, S0:].to(F64).view(taps - 1, C)
+        full = torch.cat([hist, x[:, :C]])
+        y = sum(full[d:d + z - a] * conv_w[:, d].to(F64) for d in range(taps))
+        y = y * torch.sigmoid(y)
+        unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)
+        decay = torch.expm1(-torch.exp(A_log.to(F64)).repeat_interleave(dk if per_channel else 1) * softplus(Am[a:z].to(F64) + dt_bias.to(F64)))
+        want = [unit(y[:, :nq].view(-1, G, dk)) * dk ** -0.5, unit(y[:, nq:2 * nq].view(-1, G, dk)), y[:, 2 * nq:].view(-1, H, dv),
+                torch.sigmoid(x[:, C + 5:]), decay]
+        for o, w in zip(got, want):
+            assert torch.allclose(o[a:z].to(F64), w, rtol=2e-5, atol=2e-5)
+        assert torch.allclose(st[i, S0:].cpu().to(F64).view(taps - 1, C), full[z - a:], rtol=0, atol=0)
+        if z - a < 64:
+            alone = call(slice(a, z), state.clone().cuda()[i:i + 1], [0, z - a], [0], [fresh[i]])
+            for o, w in zip(got, alone):
+                assert torch.allclose(o[a:z], w, rtol=2e-6, atol=1e-7)
