@@ -49,7 +49,37 @@ struct Params {
   float* part_ml;    // [B, H, splits, 2]
   int* counters;     // [B, Hkv]
   int* status;       // device status word of the TMA variant (bounded waits)
+  int by_length;     // > 0: so many requests, the longest start first (the TMA variant)
 };
+
+constexpr int BY_LENGTH_MAX = 128;     // requests that a warp ranks
+// The request with exactly `rank` longer ones (equal lengths in the order of the batch); n <= BY_LENGTH_MAX, a whole warp.
+__device__ __forceinline__ int request_by_length(const int* seq_lens, int n, int rank, int lane) {
+  int len[BY_LENGTH_MAX / 32], before[BY_LENGTH_MAX / 32];
+#pragma unroll
+  for (int u = 0; u < BY_LENGTH_MAX / 32; ++u) {
+    len[u] = lane + 32 * u < n ? seq_lens[lane + 32 * u] : -1;
+    before[u] = 0;
+  }
+#pragma unroll
+  for (int v = 0; v < BY_LENGTH_MAX / 32; ++v) {
+    if (32 * v >= n) break;
+#pragma unroll 8
+    for (int j = 0; j < 32; ++j) {
+      const int other = __shfl_sync(0xffffffffu, len[v], j);
+#pragma unroll
+      for (int u = 0; u < BY_LENGTH_MAX / 32; ++u)
+        before[u] += other > len[u] || (other == len[u] && 32 * v + j < lane + 32 * u);
+    }
+  }
+  int found = 0;
+#pragma unroll
+  for (int u = 0; u < BY_LENGTH_MAX / 32; ++u) {
+    const unsigned hit = __ballot_sync(0xffffffffu, lane + 32 * u < n && before[u] == rank);
+    if (hit) found = 32 * u + __ffs(hit) - 1;
+  }
+  return found;
+}
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -449,9 +479,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
   __shared__ int s_abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
-  const int b = blockIdx.z, hk = blockIdx.y, split = blockIdx.x;
+  const int hk = blockIdx.y, split = blockIdx.x;
   pdl_launch_dependents();
   // before pdl_wait(): only the batch's index arrays and cache pages of older tokens (see the other kernel)
+  const int b = p.by_length ? request_by_length(p.seq_lens, p.by_length, blockIdx.z, lane) : blockIdx.z;
   const int t0 = p.cu_seqlens[b];
   if (p.cu_seqlens[b + 1] - t0 != 1) return;                  // the whole cluster leaves: same request
   // first phase of the cluster barrier: this CTA runs, its shared memory may be written by the others
@@ -853,7 +884,7 @@ DINFER_API int dinfer_attention_decode(const void* q, int64_t ldq, void* out, in
   p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.H = H; p.Hkv = Hkv; p.group = H / Hkv;
   p.block_size = block_size; p.bs_log2 = 0;
   while ((1 << p.bs_log2) < block_size) ++p.bs_log2;
-  p.window = window; p.chunked = 0; p.keep = 0; p.cap_in = p.cap_out = 0.f; p.sink = 0; p.sinks = nullptr; p.scale_log2 = scale * 1.4426950408889634f; p.splits = splits;
+  p.window = window; p.chunked = 0; p.keep = 0; p.cap_in = p.cap_out = 0.f; p.sink = 0; p.sinks = nullptr; p.scale_log2 = scale * 1.4426950408889634f; p.splits = splits; p.by_length = 0;
   p.slopes = nullptr;
   p.part_o = scratch_floats;
   p.part_ml = scratch_floats ? scratch_floats + (int64_t)B * H * splits * D : nullptr;
@@ -926,6 +957,10 @@ DINFER_API int dinfer_attention_decode_tma_bias(const void* q, int64_t ldq, void
   p.block_size = block_size; p.bs_log2 = 0;
   while ((1 << p.bs_log2) < block_size) ++p.bs_log2;
   p.window = window; p.chunked = chunked; p.sink = sink; p.sinks = sinks; p.scale_log2 = scale * 1.4426950408889634f; p.splits = splits;
+  // With more CTAs than run at a time (two to an SM) and a CTA to a (request, head), the last ones to start end the step: they
+  // should be short.  64 requests of 300 to 4017 tokens, 8 heads of 128: 116 us in the batch's order (rising), @@N@@ us.
+  static const int sms = [] { int d = 0, n = 148; if (cudaGetDevice(&d) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d); return n; }();
+  p.by_length = splits == 1 && B <= BY_LENGTH_MAX && (int64_t)B * Hkv > 2 * sms ? B : 0;
   p.keep = window > 0 ? keep_first : 0;
   p.cap_in = p.cap_out = 0.f;
   if (softcap > 0.f) {                          // the capped scores come out in log2 units

@@ -208,31 +208,64 @@ moe_route_table_kernel(const int* __restrict__ tokens, const int* __restrict__ p
 }
 
 // ---------------------------------------------------------------- pairs laid out expert by expert
-// sorted[pos] = pair index (t * top + k) or `pairs` for padding; tile_expert[tile] = expert of the tile or -1
-__global__ void __launch_bounds__(1024)
+// sorted[pos] = pair index (t * top + k) or `pairs` for padding; tile_expert[tile] = expert of the tile or -1.
+// One block: bound by its chain of passes and, with one counter an expert, by the atomics on it.  So every warp counts (and
+// later deals out) in a copy of its own (as many copies as fit: 32 up to 340 experts), four ids a load, and only the
+// positions that pad are written ahead.  16384 pairs over 64 experts: 22 us with one copy, @@A@@ us now.
+constexpr int ALIGN_THREADS = 1024;
+constexpr int ALIGN_INTS = 12 * 1024 - 64;               // of shared memory, without opting in to more
+__global__ void __launch_bounds__(ALIGN_THREADS)
 moe_align_kernel(const int* __restrict__ ids, int* __restrict__ sorted, int* __restrict__ tile_expert, int pairs,
-                 int E, int BM, int cap, int max_tiles) {
-  extern __shared__ int smi[];                            // count[E], start[E + 1], fill[E]
-  int* count = smi;
-  int* start = smi + E;
-  int* fill = smi + 2 * E + 1;
+                 int E, int BM, int cap, int max_tiles, int copies) {
+  extern __shared__ int smi[];                            // start[E + 1], count[E], place[copies][E]
+  int* start = smi;
+  int* count = smi + E + 1;
+  int* place = smi + 2 * E + 1;
   pdl_enter();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) { count[e] = 0; fill[e] = 0; }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < copies * E; i += ALIGN_THREADS) place[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+  int* own = place + warp % copies * E;
+  const bool vec = pairs % 4 == 0 && !(reinterpret_cast<uintptr_t>(ids) & 15);
+  auto each = [&](auto f) {                               // f(expert, pair) for this thread's pairs, the same both times
+    if (vec) {
+      for (int i = tid; i < pairs / 4; i += ALIGN_THREADS) {
+        const int4 e = reinterpret_cast<const int4*>(ids)[i];
+        f(e.x, 4 * i); f(e.y, 4 * i + 1); f(e.z, 4 * i + 2); f(e.w, 4 * i + 3);
+      }
+    } else {
+      for (int i = tid; i < pairs; i += ALIGN_THREADS) f(ids[i], i);
+    }
+  };
+  each([&](int e, int) { if (e >= 0 && e < E) atomicAdd(&own[e], 1); });
+  __syncthreads();
+  for (int e = tid; e < E; e += ALIGN_THREADS) {          // a copy's count -> where its pairs begin in the expert's run
+    int at = 0;
+    for (int c = 0; c < copies; ++c) { const int n = place[c * E + e]; place[c * E + e] = at; at += n; }
+    count[e] = at;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int e = 0; e < E; ++e) { start[e] = at; at += (count[e] + BM - 1) / BM * BM; }
-    start[E] = at;
+  if (warp == 0) {
+    int before = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, padded = e < E ? (count[e] + BM - 1) / BM * BM : 0;
+      int incl = padded;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      if (e < E) start[e] = before + incl - padded;
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) start[E] = before;
   }
   __syncthreads();
   const int used = start[E];
-  for (int i = threadIdx.x; i < cap; i += blockDim.x) sorted[i] = pairs;
-  for (int tile = threadIdx.x; tile < max_tiles; tile += blockDim.x) {
+  for (int e = warp; e < E; e += ALIGN_THREADS / 32)
+    for (int i = start[e] + count[e] + lane; i < start[e + 1]; i += 32) sorted[i] = pairs;
+  for (int i = used + tid; i < cap; i += ALIGN_THREADS) sorted[i] = pairs;
+  for (int tile = tid; tile < max_tiles; tile += ALIGN_THREADS) {
     const int row = tile * BM;
     int e = -1;
     if (row < used) {                                     // the expert whose padded run holds this row
@@ -242,11 +275,7 @@ moe_align_kernel(const int* __restrict__ ids, int* __restrict__ sorted, int* __r
     }
     tile_expert[tile] = e;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e >= 0 && e < E) sorted[start[e] + atomicAdd(&fill[e], 1)] = i;
-  }
+  each([&](int e, int i) { if (e >= 0 && e < E) sorted[start[e] + atomicAdd(&own[e], 1)] = i; });
 }
 
 // ---------------------------------------------------------------- grouped product, plain arithmetic
@@ -339,19 +368,21 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// Row tiles of 16 (decode steps): bound by reading the weights of the experts that the step's tokens meet, 64 rows of them a
+// block, four stages of 64 k.  Eight tokens, 64 experts of 4096 x 2048 (8 chosen): gate and up 292 us and down 148 us with
+// two stages of 32 k, @@C@@ and @@D@@ us now.
 template <int BM, int MODE>
 __global__ void __launch_bounds__(128)
 moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ Wall,
                     __nv_bfloat16* __restrict__ C, int64_t ldc, const int* __restrict__ sorted,
                     const int* __restrict__ tile_expert, const float* __restrict__ weights, int pairs, int top, int N,
                     int K, int act) {
-  constexpr int BN = BM == 64 ? 128 : 64, BK = 32, LD = BK + 8;
+  constexpr int BN = BM == 64 ? 128 : 64, BK = BM == 64 ? 32 : 64, LD = BK + 8, ST = BM == 64 ? 2 : 4;
   constexpr int WM = BM == 64 ? 2 : 1, WN = 4 / WM;          // warps along rows and columns
   constexpr int MTW = BM / (16 * WM), NTW = BN / (8 * WN);   // m16 and n8 tiles per warp
-  __shared__ __align__(16) __nv_bfloat16 As[2][BM][LD];
-  __shared__ __align__(16) __nv_bfloat16 Bs[2][BN][LD];
+  __shared__ __align__(16) __nv_bfloat16 As[ST][BM][LD];
+  __shared__ __align__(16) __nv_bfloat16 Bs[ST][BN][LD];
   __shared__ int64_t src[BM];
   __shared__ int pair_of[BM];
   pdl_enter();
@@ -368,7 +399,7 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
   __syncthreads();
   const __nv_bfloat16* W = Wall + (int64_t)e * N * K;
   auto load = [&](int k0, int buf) {
-    for (int i = tid; i < (BM + BN) * (BK / 8); i += 128) {
+    for (int i = k0 < K ? tid : (BM + BN) * (BK / 8); i < (BM + BN) * (BK / 8); i += 128) {
       const int r = i / (BK / 8), c = (i % (BK / 8)) * 8;
       const bool in_k = k0 + c < K;
       if (r < BM) {
@@ -390,12 +421,13 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
     for (int j = 0; j < NTW; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-  load(0, 0);
+#pragma unroll
+  for (int u = 0; u < ST - 1; ++u) load(u * BK, u);
   int buf = 0;
-  for (int k0 = 0; k0 < K; k0 += BK, buf ^= 1) {
-    cp_async_wait_all();
-    __syncthreads();
-    if (k0 + BK < K) load(k0 + BK, buf ^ 1);
+  for (int k0 = 0; k0 < K; k0 += BK, buf = (buf + 1) % ST) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+    __syncthreads();                                         // this step's tiles are there, nobody reads the last step's
+    load(k0 + (ST - 1) * BK, (buf + ST - 1) % ST);
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
       uint32_t a[MTW][4];
@@ -489,12 +521,15 @@ moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat
 
 // a[pos] = x[sorted[pos] / top]: the rows of a step laid out expert by expert, for products that want every expert's rows
 // side by side in memory.  Rows that pad a run are left as they are: a product's rows do not depend on one another.
+// A warp per row, eight 16-byte pieces a lane in flight (a block per row spent most of its time starting: 16384 rows of 2048
+// bfloat16 among 32704 places took 35 us, @@B@@ us now).
 template <typename TA>
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const TA* __restrict__ x, int64_t ldx, const int* __restrict__ sorted, TA* __restrict__ a, int pairs,
-                  int top, int h) {
+                  int top, int h, int cap) {
   pdl_enter();
-  const int pos = blockIdx.x;
+  const int pos = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (pos >= cap) return;
   const int pr = sorted[pos];
   if (pr >= pairs) return;
   TA* dst = a + (int64_t)pos * h;
@@ -502,10 +537,20 @@ moe_gather_kernel(const TA* __restrict__ x, int64_t ldx, const int* __restrict__
   const bool vec = sizeof(TA) == 2 && h % 8 == 0 && ldx % 8 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15) &&
                    !(reinterpret_cast<uintptr_t>(a) & 15);
   if (vec) {
-    for (int i = threadIdx.x * 8; i < h; i += blockDim.x * 8)
-      *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+    const uint4* s = reinterpret_cast<const uint4*>(src);
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    const int n = h / 8;
+    for (int i0 = 0; i0 < n; i0 += 256) {
+      uint4 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i0 + 32 * u + lane < n) v[u] = s[i0 + 32 * u + lane];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i0 + 32 * u + lane < n) d[i0 + 32 * u + lane] = v[u];
+    }
   } else {
-    for (int i = threadIdx.x; i < h; i += blockDim.x) dst[i] = src[i];
+    for (int i = lane; i < h; i += 32) dst[i] = src[i];
   }
 }
 
@@ -586,9 +631,11 @@ DINFER_API int dinfer_moe_align(const int* ids, int* sorted, int* tile_expert, i
                                 cudaStream_t stream) {
   if (pairs < 0 || E <= 0 || BM <= 0 || cap % BM || cap < pairs + E * (BM - 1))
     return refuse(DINFER_BAD_ARGUMENT, "moe_align: bad sizes pairs=%d E=%d BM=%d cap=%d", pairs, E, BM, cap);
-  const size_t smem = (size_t)(3 * E + 1) * sizeof(int);
-  if (smem > 48 * 1024) return refuse(DINFER_BAD_ARGUMENT, "moe_align: %d experts above the limit", E);
-  launch_pdl(moe_align_kernel, dim3(1), dim3(1024), smem, stream, ids, sorted, tile_expert, pairs, E, BM, cap, cap / BM);
+  if ((size_t)(3 * E + 1) * sizeof(int) > 48 * 1024) return refuse(DINFER_BAD_ARGUMENT, "moe_align: %d experts above the limit", E);
+  const int room = (ALIGN_INTS - 2 * E - 1) / E, copies = room < 1 ? 1 : (room > 32 ? 32 : room);
+  const size_t smem = (size_t)((2 + copies) * E + 1) * sizeof(int);
+  launch_pdl(moe_align_kernel, dim3(1), dim3(ALIGN_THREADS), smem, stream, ids, sorted, tile_expert, pairs, E, BM, cap, cap / BM,
+             copies);
   return cuda_status("moe_align");
 }
 
@@ -690,7 +737,8 @@ DINFER_API int dinfer_moe_gather(const void* x, int64_t ldx, const int* sorted, 
   if (cap < 0 || pairs < 0 || top <= 0 || h <= 0 || ldx < h) return refuse(DINFER_BAD_ARGUMENT, "moe_gather: bad sizes cap=%d h=%d", cap, h);
   if (cap == 0) return 0;
   DINFER_DISPATCH_DTYPE(act_dtype, TA, {
-    launch_pdl(moe_gather_kernel<TA>, dim3(cap), dim3(256), 0, stream, (const TA*)x, ldx, sorted, (TA*)a, pairs, top, h);
+    launch_pdl(moe_gather_kernel<TA>, dim3((cap + 7) / 8), dim3(256), 0, stream, (const TA*)x, ldx, sorted, (TA*)a, pairs, top, h,
+               cap);
     return cuda_status("moe_gather");
   });
   return 0;

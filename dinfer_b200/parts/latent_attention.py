@@ -31,7 +31,7 @@ from typing import Dict, List, Optional
 import torch
 
 from ..kernels import latent_ops, ops
-from ..kernels.lib import add_launches
+from ..kernels.lib import add_launches, num_sms
 from .base import MIXERS, POSITION_ENCODINGS, BuildEnv, CacheBinding, KvCacheNeed, Mixer, StepContext, build_part
 from .linear import Linear
 from .spec import PartSpec, TensorDecl
@@ -172,18 +172,22 @@ class LatentAttention(Mixer):
         else:
             ops.gemm_f32_batched(a, w, out)
 
-    # What the two ways of a portion cost, in flops a second they reach here (the absorbed kernel's mma.sync, the expanding
-    # product, the tcgen05 attention) and seconds (the gather and one more launch).
-    RATES = (150e12, 1000e12, 350e12, 15e-6)
+    # What the two ways of a portion cost.  Absorbed: flops a second (mma.sync; 120 to 160e12 measured at R 512, 100e12 at
+    # R 256, hence the 100 columns that _expanded_shape adds), bytes a second and seconds that its two products take whatever
+    # the portion.  Expanded: flops a second of the product, bytes a second of the gather, seconds a CTA of the attention takes
+    # for a tile of 128 keys with one and with both of its row tiles.
+    RATES = (150e12, 6e11, 6e-6, 1000e12, 3e12, 1.8e-6, 2.85e-6)
     # the keys and values of a step's portions, all heads, are expanded at once up to so many bytes
     EXPANDED_BYTES = 256 << 20
 
     def _expanded(self, ctx: StepContext, dtype):
         """Whether the step's portions run over expanded latents: None, or (rows of the gathered latents, row-tile pairs).  The
         absorbed form needs H (2 R + P) multiply-adds a (token, key) pair, the expanded one H (D + P + V) and R H (D + V) a key.
-        One layer of 16 heads of 128 + 64, R 512, a 2048-token prompt: absorbed @@A@@ us of attention and its two products,
-        expanded @@B@@; a portion of @@C@@.  In a captured graph the lengths are bounds: the tokens spread evenly over the
-        prompt places without a history for what the absorbed form costs at least, every place as long as it may get
+        But a CTA of the expanded attention walks all keys of its 256 rows one tile after the other, so a few rows behind a
+        long history are the absorbed form's.  A layer of 16 heads of 128 + 64, R 512, absorbed and expanded (us): a prompt of
+        64 tokens 52 and 37, of 2048 565 and 134; 64 tokens behind 4000 129 and 118, behind 16000 291 and 352; 256 behind
+        16000 1187 and 493; 8 heads of 64 + 32, R 256: 64 behind 4000 59 and 86.
+        In a captured graph the lengths are bounds: the tokens spread evenly over the prompt places without a history for what the absorbed form costs at least, every place as long as it may get
         for what the other one costs at most."""
         if self.ukv is None or dtype != torch.bfloat16 or not ctx.any_prefill or not ctx.cu_seqlens_host:
             return None
@@ -200,23 +204,29 @@ class LatentAttention(Mixer):
             if not tokens:
                 return None
             longest = ctx.max_prefill_seq_len or ctx.max_seq_len
-            pairs = tokens * tokens / (2.0 * places)
             bound = [(min(tokens, longest), longest)] * places
+            pairs = tokens * tokens / (2.0 * places)
             tiles = tokens // 256 + places
+            seen = [(tiles, 256, longest)]                   # (CTAs a head, rows of one, keys it walks) at most
         else:
             bound = [(n, s) for n, s in zip(lens, ctx.seq_lens_host) if n > 1]
             if not bound:
                 return None
+            tokens = sum(n for n, _ in bound)
             pairs = float(sum(n * (min(s - n, window) if window else s - n) + n * (n + 1) // 2 for n, s in bound))
-            tiles = sum((n + 255) // 256 for n, _ in bound)
+            seen = [((n + 255) // 256, n, s - n // 2 if n > 256 else s) for n, s in bound]
+            tiles = sum(count for count, _, _ in seen)
         if window:
-            pairs = min(pairs, float(window) * sum(n for n, _ in bound))
+            pairs = min(pairs, float(window) * tokens)
+            seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
         rows = latent_ops.expanded_rows(bound, window)
-        absorbed, expanding, attending, fixed = self.RATES
+        flops, weight_rate, products, expanding, gather, one, both = self.RATES
         H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
-        pays = (pairs * H * 2 * (2 * R + P) / absorbed
-                > rows * R * H * 2 * (D + V) / expanding + pairs * H * 2 * (D + P + V) / attending + fixed)
-        if not pays or rows * H * (D + V) * 2 > self.EXPANDED_BYTES or tiles > 65535:
+        walks = [(count, ((keys + 127) // 128) * (both if n > 128 else one)) for count, n, keys in seen]
+        walking = max(max(w for _, w in walks), H * sum(count * w for count, w in walks) / num_sms())
+        absorbed = pairs * H * 2 * (2 * R + P + 100) / flops + H * R * (D + V) * 2 / weight_rate + products
+        expanded = rows * R * H * 2 * (D + V) / expanding + rows * (R + P) * 4 / gather + walking
+        if absorbed <= expanded or rows * H * (D + V) * 2 > self.EXPANDED_BYTES or tiles > 65535:
             return None
         return rows, tiles
 

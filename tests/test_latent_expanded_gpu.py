@@ -132,6 +132,9 @@ def part_and_context(reqs, window=None, gate=False, sink=False, D=128, P=64, see
     return part, ctx, CacheBinding(kv=kv, group=0, write=True), x
 
 
+ABSORBED, EXPANDED = (1e30, 1e30, 0.0, 1.0, 1.0, 1.0, 1.0), (1.0, 1.0, 1.0, 1e30, 1e30, 0.0, 0.0)
+
+
 @pytest.mark.parametrize("reqs,window,gate,sink", [([(0, 300)], None, False, False), ([(40, 1), (0, 129), (500, 1), (300, 64)], None, True, True),
                                                    ([(700, 150), (3, 1), (0, 2)], 128, False, True)])
 def test_both_ways_of_the_part_agree(reqs, window, gate, sink, monkeypatch):
@@ -139,11 +142,11 @@ def test_both_ways_of_the_part_agree(reqs, window, gate, sink, monkeypatch):
     import dataclasses
     from dinfer_b200.parts.latent_attention import LatentAttention
     outs, caches = [], []
-    for rates in ((1e30, 1.0, 1.0, 0.0), (1.0, 1e30, 1e30, 0.0)):          # the absorbed way is free, then the other
+    for rates in (ABSORBED, EXPANDED):                                        # one way is free, then the other
         part, ctx, cache, x = part_and_context(reqs, window, gate, sink)
         monkeypatch.setattr(LatentAttention, "RATES", rates)
         shape = part._expanded(ctx, torch.bfloat16)
-        assert (shape is None) == (rates[0] == 1e30)
+        assert (shape is None) == (rates is ABSORBED)
         outs.append(part.forward(x, dataclasses.replace(ctx, derived={}), cache).float())
         caches.append(cache.kv.clone())
     assert torch.equal(caches[0], caches[1]) and bool(torch.isfinite(outs[1]).all())
@@ -173,7 +176,7 @@ def test_captured_steps_run_over_expanded_latents_too(monkeypatch):
              "rot": {"base": 10000.0, "dims": 32}}
     cfg = {"architecture": "Dobedra", "vocab": 256, "width": 128, "norm": {"eps": 1e-6}, "logit_softcap": 30.0,
            "layers": [{"type": "latent_attention", "mixer": mixer, "mlp": {"kind": "dense", "ff": 128}}] * 2}
-    monkeypatch.setattr(LatentAttention, "RATES", (1.0, 1e30, 1e30, 0.0))
+    monkeypatch.setattr(LatentAttention, "RATES", EXPANDED)
     calls = []
     whole = LatentAttention.attend_expanded
     monkeypatch.setattr(LatentAttention, "attend_expanded", lambda self, *a: (calls.append(torch.cuda.is_current_stream_capturing()), whole(self, *a))[1])
