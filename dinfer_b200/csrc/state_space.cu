@@ -203,6 +203,47 @@ __global__ void __launch_bounds__(PREP_THREADS) ssm_prep_kernel(const Params p) 
       for (int d = 0; d < TAPS; ++d) w[e][d] = p.conv_w[(int64_t)(c + e) * TAPS + d];
   }
   int start = p.cu[b], end = p.cu[b + 1];
+  if constexpr (TAPS > 0) {
+    // the whole run belongs to one request: its inputs come eight at a time, all asked for before the first is used
+    if (t1 - t0 == PREP_TOKENS && t0 >= start && t1 <= end && end - start > 1) {
+      const float* x = p.P + (int64_t)t0 * p.ldp + inner + c;
+#pragma unroll
+      for (int d = 1; d < TAPS; ++d) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) before[d - 1].x[e] = 0.f;
+        const int i = t0 - start - d;
+        if (i >= 0) before[d - 1] = ldv<V>(x - (int64_t)d * p.ldp);
+        else if (!p.fresh[b]) {
+          const float* hist = p.state + (int64_t)p.slots[b] * p.ld_state + p.hist + (int64_t)(TAPS - 1 + i) * ch + c;
+#pragma unroll
+          for (int e = 0; e < V; ++e) before[d - 1].x[e] = hist[e];
+        }
+      }
+      float* dst = p.xbc + (int64_t)t0 * ch + c;
+      for (int r = 0; r < PREP_TOKENS; r += 8) {
+        Vec<V> in[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) in[u] = ldv<V>(x + (int64_t)(r + u) * p.ldp);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          Vec<V> o;
+#pragma unroll
+          for (int e = 0; e < V; ++e) o.x[e] = bias[e];
+#pragma unroll
+          for (int d = TAPS - 1; d > 0; --d)
+#pragma unroll
+            for (int e = 0; e < V; ++e) o.x[e] = fmaf(w[e][TAPS - 1 - d], before[d - 1].x[e], o.x[e]);
+#pragma unroll
+          for (int e = 0; e < V; ++e) o.x[e] = silu_f(fmaf(w[e][TAPS - 1], in[u].x[e], o.x[e]));
+#pragma unroll
+          for (int d = TAPS - 1; d > 1; --d) before[d - 1] = before[d - 2];
+          if constexpr (TAPS > 1) before[0] = in[u];
+          stv<V>(dst + (int64_t)(r + u) * ch, o);
+        }
+      }
+      return;
+    }
+  }
   bool load = true;                                 // the inputs before the next token are not in registers
   for (int t = t0; t < t1; ++t) {
     while (t >= end && b + 1 < p.B) { ++b; start = end; end = p.cu[b + 1]; load = true; }
@@ -301,15 +342,24 @@ __device__ __forceinline__ void store4(float* p, int left, const float (&v)[4]) 
 __device__ __forceinline__ float4 get4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void put4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
 
-// grid (chunks, H * tiles + G, B): a 64 x 64 tile of U for one (chunk, head), or the scores C_t . B_s of one (chunk, group)
-template <bool VEC>
-__global__ void __launch_bounds__(THREADS) ssm_sums_kernel(const Params p) {
-  __shared__ __align__(16) float a_s[CP][LDT];     // [token][state channel] of B
-  __shared__ __align__(16) float b_s[CP][LDT];     // [token][value column], scaled; or [token][state channel] of C
-  __shared__ double cum[CP];
-  __shared__ float wgt[CP];
+// grid (chunks, H * tiles + G, B): a (64 RN) x 64 tile of U for one (chunk, head), or the scores C_t . B_s of one (chunk,
+// group).  RN = 2 where the state has more than 64 channels: a thread's 8 x 4 elements then take three 16-byte reads of shared
+// memory a token for 32 multiply-adds, 4 x 4 two for 16.  Bound by those multiply-adds (72 TFLOP/s) and by what surrounds them
+// in a block of 2 us, which three blocks to an SM hide: 2047 tokens of 64 heads of 128 x 64 @@A@@ us, with 64 x 64 tiles 87.
+template <int RN> struct SumsTiles {
+  static constexpr int W = TP * RN;                                            // channels of a tile
+  static constexpr int A = CP * (W > LDT ? W : LDT), B = CP * (RN > 1 ? TP : LDT);   // floats; the scores' rows are LDT long
+  static_assert(RN == 1 || CP * W + CP * TP >= 2 * CP * LDT, "the scores' two tiles fit");
+  static constexpr size_t BYTES = (A + B) * sizeof(float) + CP * (sizeof(double) + sizeof(float));
+};
+template <bool VEC, int RN>
+__global__ void __launch_bounds__(THREADS, RN > 1 ? 3 : 0) ssm_sums_kernel(const Params p) {
+  constexpr int W = SumsTiles<RN>::W;
+  extern __shared__ __align__(16) float sums_sm[];
+  double* cum = reinterpret_cast<double*>(sums_sm + SumsTiles<RN>::A + SumsTiles<RN>::B);
+  float* wgt = reinterpret_cast<float*>(cum + CP);
   pdl_enter();
-  const int tiles_n = (p.N + TP - 1) / TP, tiles_v = (p.Pd + TP - 1) / TP;
+  const int tiles_n = (p.N + W - 1) / W, tiles_v = (p.Pd + TP - 1) / TP;
   const int b = blockIdx.z, c = blockIdx.x, tid = threadIdx.x;
   const int t_begin = p.cu[b], t_end = p.cu[b + 1];
   const int t0 = t_begin + c * CP;
@@ -318,12 +368,14 @@ __global__ void __launch_bounds__(THREADS) ssm_sums_kernel(const Params p) {
   const int64_t slot = chunk_slot(t_begin, b, c);
   const int ty = tid >> 4, tx = tid & 15;
   const int ls = tid >> 4, le = (tid & 15) * 4;    // this thread's place in a tile it loads: rows ls + 16 k, columns le ..
-  float acc[4][4] = {};
   const int job = (int)blockIdx.y - p.H * tiles_n * tiles_v;
   if (job >= 0) {
     // ---- scores of group `job`: rows t = 4 ty + i, columns s = tx + 16 j (neighbouring lanes read neighbouring rows)
+    float (*a_s)[LDT] = reinterpret_cast<float (*)[LDT]>(sums_sm);             // [token][state channel] of B
+    float (*b_s)[LDT] = reinterpret_cast<float (*)[LDT]>(sums_sm + CP * LDT);  // [token][state channel] of C
     const float* Bp = p.xbc + (int64_t)t0 * ch + inner + job * p.N;
     const float* Cp = Bp + p.G * p.N;
+    float acc[4][4] = {};
     for (int e0 = 0; e0 < p.N; e0 += CP) {
       __syncthreads();
 #pragma unroll
@@ -356,20 +408,28 @@ __global__ void __launch_bounds__(THREADS) ssm_sums_kernel(const Params p) {
       for (int j = 0; j < 4; ++j) out[(ty * 4 + i) * CP + tx + 16 * j] = acc[i][j];
     return;
   }
+  float (*a_s)[W] = reinterpret_cast<float (*)[W]>(sums_sm);                                  // [token][state channel] of B
+  float (*b_s)[TP] = reinterpret_cast<float (*)[TP]>(sums_sm + SumsTiles<RN>::A);             // [token][value column], scaled
   const int h = blockIdx.y / (tiles_n * tiles_v), tile = blockIdx.y % (tiles_n * tiles_v);
-  const int e0 = (tile / tiles_v) * TP, c0 = (tile % tiles_v) * TP;
+  const int e0 = (tile / tiles_v) * W, c0 = (tile % tiles_v) * TP;
   const int g = h / (p.H / p.G);
-  float4 bv[CP / 16], xv[CP / 16];
+  float4 xv[CP / 16];
   {
     const float* r = p.xbc + (int64_t)t0 * ch;
 #pragma unroll
     for (int k = 0; k < CP / 16; ++k) {
       const int s = ls + 16 * k;
-      bv[k] = load4<VEC>(r + (int64_t)s * ch + inner + g * p.N + e0 + le, s < n ? p.N - e0 - le : 0);
       xv[k] = load4<VEC>(r + (int64_t)s * ch + h * p.Pd + c0 + le, s < n ? p.Pd - c0 - le : 0);
     }
+    if (tid < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
+#pragma unroll
+    for (int u = 0; u < RN; ++u)
+#pragma unroll
+      for (int k = 0; k < CP / 16; ++k) {
+        const int s = ls + 16 * k, e = 64 * u + le;
+        put4(&a_s[s][e], load4<VEC>(r + (int64_t)s * ch + inner + g * p.N + e0 + e, s < n ? p.N - e0 - e : 0));
+      }
   }
-  if (tid < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
   __syncthreads();
   if (tid < CP) wgt[tid] = tid < n ? (float)exp(cum[n - 1] - cum[tid]) * p.dt[(int64_t)(t0 + tid) * p.H + h] : 0.f;
   if (tile == 0 && tid == 0) p.decay[slot * p.H + h] = (float)exp(cum[n - 1]);
@@ -377,25 +437,32 @@ __global__ void __launch_bounds__(THREADS) ssm_sums_kernel(const Params p) {
 #pragma unroll
   for (int k = 0; k < CP / 16; ++k) {
     const float w = wgt[ls + 16 * k];
-    put4(&a_s[ls + 16 * k][le], bv[k]);
     put4(&b_s[ls + 16 * k][le], make_float4(xv[k].x * w, xv[k].y * w, xv[k].z * w, xv[k].w * w));
   }
   __syncthreads();
-#pragma unroll 8
+  float acc[RN][4][4] = {};
+#pragma unroll 4
   for (int s = 0; s < n; ++s) {
-    const float4 a = get4(&a_s[s][ty * 4]), w = get4(&b_s[s][tx * 4]);
-    const float av[4] = {a.x, a.y, a.z, a.w}, wv[4] = {w.x, w.y, w.z, w.w};
+    const float4 w = get4(&b_s[s][tx * 4]);
+    const float wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int u = 0; u < RN; ++u) {
+      const float4 a = get4(&a_s[s][64 * u + ty * 4]);
+      const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[u][i][j] = fmaf(av[i], wv[j], acc[u][i][j]);
+    }
   }
   float* U = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int e = e0 + ty * 4 + i, x = c0 + tx * 4;
-    if (e < p.N) store4<VEC>(U + (int64_t)e * p.Pd + x, p.Pd - x, acc[i]);
-  }
+  for (int u = 0; u < RN; ++u)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = e0 + 64 * u + ty * 4 + i, x = c0 + tx * 4;
+      if (e < p.N) store4<VEC>(U + (int64_t)e * p.Pd + x, p.Pd - x, acc[u][i]);
+    }
 }
 
 // per V neighbouring elements of S: walk the request's chunks and leave in U's place the S that the chunk starts from;
@@ -443,10 +510,14 @@ __global__ void __launch_bounds__(THREADS) ssm_scan_kernel(const Params p) {
 }
 
 // y for one (chunk, head, 64 value columns); grid (chunks, H * column tiles, B).  The passes over the state's channels load
-// the next pass's tiles into registers while they compute.
+// the next pass's tiles into registers while they compute.  A thread has 8 x 4 elements: rows 16 w + (0 or 1) + 2 i of warp w,
+// so that a warp's two rows lie in different banks and it can leave out the tokens behind its last one.  Bound by the
+// multiply-adds and the reads of shared memory that feed them (12 of 16 bytes for 128; 4 x 4 elements: 8 for 64): 2047 tokens
+// of 64 heads of 128 x 64 @@B@@ us, with 4 x 4 elements 109.
+constexpr int OUT_THREADS = 128;
 template <bool VEC>
-__global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p) {
-  constexpr int LDC = KT + 4;
+__global__ void __launch_bounds__(OUT_THREADS, 4) ssm_outputs_kernel(const Params p) {
+  constexpr int LDC = KT + 4, R = 8;
   __shared__ __align__(16) float tiles[CP * LDT];
   static_assert(CP * LDC + KT * TP <= CP * LDT, "a pass's tiles fit where A lies afterwards");
   float (*C_s)[LDC] = reinterpret_cast<float (*)[LDC]>(tiles);                   // [token][state channel]
@@ -462,49 +533,49 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
   const int t0 = t_begin + c * CP;
   if (t_end - t_begin <= 1 || t0 >= t_end) return;
   const int n = min(CP, t_end - t0), tid = threadIdx.x, ch = p.channels(), inner = p.inner();
-  const int ty = tid >> 4, tx = tid & 15, g = h / (p.H / p.G);
+  const int row0 = (tid >> 5) * 16 + ((tid >> 4) & 1), tx = tid & 15, g = h / (p.H / p.G);
   const int64_t slot = chunk_slot(t_begin, b, c);
   const float* S_prev = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd + c0;
   const float* Cp = p.xbc + (int64_t)t0 * ch + inner + (p.G + g) * p.N;
-  // what this thread loads of a pass: C rows ct + 32 k at channels ce .., S rows (channels) sr + 16 k at columns sx ..
+  // what this thread loads of a pass: C rows ct + 16 k at channels ce .., S rows (channels) sr + 8 k at columns sx ..
   const int ct = tid >> 3, ce = (tid & 7) * 4, sr = tid >> 4, sx = (tid & 15) * 4;
-  float4 cv[CP / 32], sv[KT / 16];
+  float4 cv[CP / 16], sv[KT / 8];
   auto fetch = [&](int e0) {
 #pragma unroll
-    for (int k = 0; k < CP / 32; ++k)
-      cv[k] = load4<VEC>(Cp + (int64_t)(ct + 32 * k) * ch + e0 + ce, ct + 32 * k < n ? p.N - e0 - ce : 0);
+    for (int k = 0; k < CP / 16; ++k)
+      cv[k] = load4<VEC>(Cp + (int64_t)(ct + 16 * k) * ch + e0 + ce, ct + 16 * k < n ? p.N - e0 - ce : 0);
 #pragma unroll
-    for (int k = 0; k < KT / 16; ++k)
-      sv[k] = load4<VEC>(S_prev + (int64_t)(e0 + sr + 16 * k) * p.Pd + sx, e0 + sr + 16 * k < p.N ? p.Pd - c0 - sx : 0);
+    for (int k = 0; k < KT / 8; ++k)
+      sv[k] = load4<VEC>(S_prev + (int64_t)(e0 + sr + 8 * k) * p.Pd + sx, e0 + sr + 8 * k < p.N ? p.Pd - c0 - sx : 0);
   };
   fetch(0);
 #pragma unroll
-  for (int k = 0; k < CP / 16; ++k) {
-    const int s = sr + 16 * k;
+  for (int k = 0; k < CP / 8; ++k) {
+    const int s = sr + 8 * k;
     put4(&x_s[s][sx], load4<VEC>(p.xbc + (int64_t)(t0 + s) * ch + h * p.Pd + c0 + sx, s < n ? p.Pd - c0 - sx : 0));
   }
   if (tid < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
   if (tid < CP) dts[tid] = tid < n ? p.dt[(int64_t)(t0 + tid) * p.H + h] : 0.f;
-  float r[4][4] = {};
+  float r[R][4] = {};
   for (int e0 = 0; e0 < p.N; e0 += KT) {
     __syncthreads();                               // the last pass is done with the tiles
 #pragma unroll
-    for (int k = 0; k < CP / 32; ++k) put4(&C_s[ct + 32 * k][ce], cv[k]);
+    for (int k = 0; k < CP / 16; ++k) put4(&C_s[ct + 16 * k][ce], cv[k]);
 #pragma unroll
-    for (int k = 0; k < KT / 16; ++k) put4(&S_s[sr + 16 * k][sx], sv[k]);
+    for (int k = 0; k < KT / 8; ++k) put4(&S_s[sr + 8 * k][sx], sv[k]);
     __syncthreads();
     if (e0 + KT < p.N) fetch(e0 + KT);
-#pragma unroll 2
+#pragma unroll 1
     for (int e = 0; e < KT; e += 4) {
-      float4 q[4];
+      float4 q[R];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = get4(&C_s[ty * 4 + i][e]);
+      for (int i = 0; i < R; ++i) q[i] = get4(&C_s[row0 + 2 * i][e]);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const float4 s4 = get4(&S_s[e + u][tx * 4]);
         const float sw[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < R; ++i) {
           const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
 #pragma unroll
           for (int j = 0; j < 4; ++j) r[i][j] = fmaf(qv, sw[j], r[i][j]);
@@ -516,8 +587,8 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
   // A[t][s] = (C_t . B_s) exp(c_t - c_s) dt_s for s <= t; r <- exp(c_t) r, which the sums over s then join
   const float* cb = p.cb + (slot * p.G + g) * (int64_t)CP * CP;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = ty * 4 + i;
+  for (int i = 0; i < R; ++i) {
+    const int t = row0 + 2 * i;
     const float4 v = get4(cb + t * CP + tx * 4);
     const float vv[4] = {v.x, v.y, v.z, v.w};
     float a[4];
@@ -532,17 +603,18 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
     for (int j = 0; j < 4; ++j) r[i][j] *= d;
   }
   __syncthreads();
-  const int last = min(ty * 4 + 3, n - 1);         // (A is zero beyond t, x_s beyond the chunk's tokens)
+  const int last = min((tid >> 5) * 16 + 15, n - 1);   // (A is zero beyond t, x_s beyond the chunk's tokens)
+#pragma unroll 1
   for (int s = 0; s <= last; s += 4) {
-    float4 q[4];
+    float4 q[R];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) q[i] = get4(&A_s[ty * 4 + i][s]);
+    for (int i = 0; i < R; ++i) q[i] = get4(&A_s[row0 + 2 * i][s]);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const float4 x4 = get4(&x_s[s + u][tx * 4]);
       const float xw[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < R; ++i) {
         const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
 #pragma unroll
         for (int j = 0; j < 4; ++j) r[i][j] = fmaf(qv, xw[j], r[i][j]);
@@ -551,8 +623,8 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
   }
   const float D = p.D[h];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = ty * 4 + i;
+  for (int i = 0; i < R; ++i) {
+    const int t = row0 + 2 * i;
     if (t >= n) continue;
     const float4 x4 = get4(&x_s[t][tx * 4]);
     const float o[4] = {fmaf(D, x4.x, r[i][0]), fmaf(D, x4.y, r[i][1]), fmaf(D, x4.z, r[i][2]), fmaf(D, x4.w, r[i][3])};
@@ -683,6 +755,16 @@ void launch_prep(const Params& p, cudaStream_t stream) {
   }
 }
 
+template <bool VEC, int RN>
+int launch_sums(const Params& p, int chunks, cudaStream_t stream) {
+  constexpr size_t smem = SumsTiles<RN>::BYTES;
+  const cudaError_t e = cudaFuncSetAttribute(ssm_sums_kernel<VEC, RN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return refuse((int)e, "state_space: shared memory opt-in failed: %s", cudaGetErrorString(e));
+  const int tiles = (p.N + SumsTiles<RN>::W - 1) / SumsTiles<RN>::W * ((p.Pd + TP - 1) / TP);
+  launch_pdl(ssm_sums_kernel<VEC, RN>, dim3(chunks, p.H * tiles + p.G, p.B), dim3(THREADS), smem, stream, p);
+  return 0;
+}
+
 bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
 
 }  // namespace
@@ -743,10 +825,12 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
     else launch_prep<1>(p, stream);
     // 16-byte loads of the convolved rows, of the states and of y: every width and base allows them
     const bool vec = P % 4 == 0 && N % 4 == 0 && al16(y);
-    launch_pdl(vec ? ssm_sums_kernel<true> : ssm_sums_kernel<false>, dim3(chunks, H * tiles_n * tiles_v + G, B), dim3(THREADS), 0, stream, p);
+    const int rc = N > TP ? (vec ? launch_sums<true, 2>(p, chunks, stream) : launch_sums<false, 2>(p, chunks, stream))
+                          : (vec ? launch_sums<true, 1>(p, chunks, stream) : launch_sums<false, 1>(p, chunks, stream));
+    if (rc) return rc;
     if (state_vec) launch_pdl(ssm_scan_kernel<4>, dim3((unsigned)((size / 4 + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
     else launch_pdl(ssm_scan_kernel<1>, dim3((unsigned)((size + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
-    launch_pdl(vec ? ssm_outputs_kernel<true> : ssm_outputs_kernel<false>, dim3(chunks, H * tiles_v, B), dim3(THREADS), 0, stream, p);
+    launch_pdl(vec ? ssm_outputs_kernel<true> : ssm_outputs_kernel<false>, dim3(chunks, H * tiles_v, B), dim3(OUT_THREADS), 0, stream, p);
   }
   return cuda_status("state_space");
 }
