@@ -26,9 +26,7 @@ namespace {
 
 constexpr int C = 32;              // tokens of a chunk
 constexpr int BC = 16;             // value columns of a walk's block
-constexpr int THREADS = 256;     // of delta_chunk
-constexpr int WALKERS = 512;     // threads of delta_walk
-constexpr int KG = WALKERS / 64; // parts of the key channels in its first product
+constexpr int THREADS = 256;
 constexpr int LDA = C + 4;         // row stride of the 32 x 32 matrices in shared memory
 constexpr int SMALL = 2 * C + 4;   // per (chunk, head): Gamma [32], exp(c_n - c_s) [32], expm1(c_n)
 constexpr float LOG_FLOOR = -100.f;   // a decay of 0: exp(-100) is 0 beside anything
@@ -215,11 +213,11 @@ template <int DK> struct Walk {
   // one chunk's operands: W_k, Q, K | M | W_v | the small ones
   static constexpr int WK = 0, Q = WK + C * LD, K = Q + C * LD, M = K + C * LD, WV = M + C * LDA, SM = WV + C * BC,
                        STAGE = SM + (SMALL + 3) / 4 * 4;
-  static constexpr int S = 2 * STAGE, PART = S + DK * LDS, U = PART + KG * 2 * C * BC, FLOATS = U + 2 * C * BC;
+  static constexpr int S = 2 * STAGE, PART = S + DK * LDS, U = PART + 4 * 2 * C * BC, FLOATS = U + 2 * C * BC;
 };
 
 template <int DK>
-__global__ void __launch_bounds__(WALKERS)
+__global__ void __launch_bounds__(THREADS)
 delta_walk_kernel(const Args a) {
   using L = Walk<DK>;
   extern __shared__ __align__(16) float sm[];
@@ -234,49 +232,45 @@ delta_walk_kernel(const Args a) {
     float* s = sm + (j & 1) * L::STAGE;
     const int64_t at = (int64_t)(first + j) * a.H + h;
     const int t0 = start + j * C, m = min(C, n - j * C);
-    for (int i = tid; i < C * (DK / 4); i += WALKERS) {
+    for (int i = tid; i < C * (DK / 4); i += THREADS) {
       const int t = i / (DK / 4), e = (i % (DK / 4)) * 4;
       cp_async16(s + L::WK + t * L::LD + e, a.wk + (at * C + t) * DK + e, true);
       const int64_t row = t < m ? (t0 + t) * nq + (int64_t)g * DK + e : 0;
       cp_async16(s + L::Q + t * L::LD + e, a.q + row, t < m);
       cp_async16(s + L::K + t * L::LD + e, a.k + row, t < m);
     }
-    // a piece a thread of the rest
-    constexpr int PM = C * C / 4, PV = C * BC / 4, PS = SMALL / 4;
-    static_assert(PM + PV + PS <= WALKERS, "a piece a thread");
-    if (tid < PM) {
-      const int t = tid / (C / 4), e = (tid % (C / 4)) * 4;
+    {
+      const int t = tid / (C / 4), e = (tid % (C / 4)) * 4;                    // 32 rows of 8 pieces: a piece a thread
       cp_async16(s + L::M + t * LDA + e, a.m + (at * C + t) * C + e, true);
-    } else if (tid < PM + PV) {
-      const int i = tid - PM, t = i / (BC / 4), e = (i % (BC / 4)) * 4;
+    }
+    if (tid < C * BC / 4) {
+      const int t = tid / (BC / 4), e = (tid % (BC / 4)) * 4;
       cp_async16(s + L::WV + t * BC + e, a.wv + (at * C + t) * a.dv + c0 + e, true);
-    } else if (tid < PM + PV + PS) {
-      const int e = (tid - PM - PV) * 4;
+    } else if (tid < C * BC / 4 + SMALL / 4) {
+      const int e = (tid - C * BC / 4) * 4;
       cp_async16(s + L::SM + e, a.small + at * SMALL + e, true);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   stage(0);
-  // S: the first half of the threads own RO x 4 of it each, rows sr .. sr + RO - 1, columns sc .. sc + 3; a copy for all in
+  // S: threads 0 .. DK - 1 (whole warps) own 4 x 4 of it, rows sr .. sr + 3, columns sc .. sc + 3; a copy for all in
   // shared memory
-  constexpr int RO = DK * 4 / (WALKERS / 2);
-  static_assert(RO == 1 || RO == 2, "one or two rows a thread");
-  const bool owner = tid < WALKERS / 2;
-  const int sr = (owner ? tid : 0) / 4 * RO, sc = tid % 4 * 4;
+  const int sr = tid / 4 * 4, sc = tid % 4 * 4;
+  const bool owner = tid < DK;
   float* S_s = sm + L::S;
   float* part = sm + L::PART;
   float* U_s = sm + L::U;                                  // U, then exp(c_n - c_s) U
   float* Sg = a.state + (int64_t)a.slots[b] * a.ld_state + (int64_t)h * DK * a.dv + c0;
-  float S[RO][4];
+  float S[4][4];
   if (owner) {
 #pragma unroll
-    for (int i = 0; i < RO; ++i) {
+    for (int i = 0; i < 4; ++i) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) S[i][j] = a.fresh[b] ? 0.f : Sg[(int64_t)(sr + i) * a.dv + sc + j];
       *reinterpret_cast<float4*>(S_s + (sr + i) * L::LDS + sc) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
     }
   }
-  // the product [W_k; Q] S: an eighth of the key channels to 64 threads, a thread 4 rows (ry + 16 i) by 4 columns
+  // the product [W_k; Q] S: a quarter of the key channels to 64 threads, a thread 4 rows (ry + 16 i) by 4 columns
   const int kg = tid >> 6, ry = (tid & 63) >> 2, cx = (tid & 3) * 4;
   for (int j = 0; j < chunks; ++j) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -289,10 +283,10 @@ delta_walk_kernel(const Args a) {
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
-      const float* rows = s + ry * L::LD + kg * (DK / KG);  // W_k and Q lie one behind the other: rows 0 .. 63
-      const float* sk = S_s + kg * (DK / KG) * L::LDS + cx;
+      const float* rows = s + ry * L::LD + kg * (DK / 4);  // W_k and Q lie one behind the other: rows 0 .. 63
+      const float* sk = S_s + kg * (DK / 4) * L::LDS + cx;
 #pragma unroll 4
-      for (int e = 0; e < DK / KG; e += 4) {
+      for (int e = 0; e < DK / 4; e += 4) {
         float4 r[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(rows + 16 * i * L::LD + e);
@@ -315,43 +309,36 @@ delta_walk_kernel(const Args a) {
             make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     }
     __syncthreads();
-    // thread t: row t / 8 of the stacked 64, two columns: the first half U, the second half O
-    const int t = (tid >> 3) & (C - 1), c2 = (tid & 7) * 2;
-    float2 o = make_float2(0.f, 0.f);
-    const float* mine = part + (tid >> 3) * BC + c2;
+    // thread t: row t / 4 of the stacked 64, four columns
+    const int row = tid >> 2, t = row & (C - 1);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int u = 0; u < KG; ++u) {
-      const float2 p = *reinterpret_cast<const float2*>(mine + u * 2 * C * BC);
-      o.x += p.x; o.y += p.y;
+    for (int u = 0; u < 4; ++u) {
+      const float4 p = *reinterpret_cast<const float4*>(part + (u * 2 * C + row) * BC + cx);
+      o.x += p.x; o.y += p.y; o.z += p.z; o.w += p.w;
     }
-    if (owner) {
-      const float2 w = *reinterpret_cast<const float2*>(s + L::WV + t * BC + c2);
+    if (row < C) {
+      const float4 w = *reinterpret_cast<const float4*>(s + L::WV + t * BC + cx);
       const float rat = s[L::SM + C + t];
-      const float2 u = make_float2(w.x - o.x, w.y - o.y);
-      *reinterpret_cast<float2*>(U_s + t * BC + c2) = u;
-      *reinterpret_cast<float2*>(U_s + (C + t) * BC + c2) = make_float2(rat * u.x, rat * u.y);
+      const float4 u = make_float4(w.x - o.x, w.y - o.y, w.z - o.z, w.w - o.w);
+      *reinterpret_cast<float4*>(U_s + t * BC + cx) = u;
+      *reinterpret_cast<float4*>(U_s + (C + t) * BC + cx) = make_float4(rat * u.x, rat * u.y, rat * u.z, rat * u.w);
     }
     __syncthreads();
     if (owner) {
       // S <- exp(c_n) S + K^T (exp(c_n - c_s) U)
       const float gm1 = s[L::SM + 2 * C];
 #pragma unroll
-      for (int i = 0; i < RO; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int c = 0; c < 4; ++c) S[i][c] = fmaf(S[i][c], gm1, S[i][c]);
-#pragma unroll 16
+#pragma unroll 8
       for (int u = 0; u < C; ++u) {
-        const float* k = s + L::K + u * L::LD + sr;
+        const float4 k = *reinterpret_cast<const float4*>(s + L::K + u * L::LD + sr);
         const float4 x = *reinterpret_cast<const float4*>(U_s + (C + u) * BC + sc);
-        float kk[RO];
-        if constexpr (RO == 2) {
-          const float2 k2 = *reinterpret_cast<const float2*>(k);
-          kk[0] = k2.x; kk[RO - 1] = k2.y;
-        } else {
-          kk[0] = k[0];
-        }
+        const float kk[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-        for (int i = 0; i < RO; ++i) {
+        for (int i = 0; i < 4; ++i) {
           S[i][0] = fmaf(kk[i], x.x, S[i][0]);
           S[i][1] = fmaf(kk[i], x.y, S[i][1]);
           S[i][2] = fmaf(kk[i], x.z, S[i][2]);
@@ -359,30 +346,33 @@ delta_walk_kernel(const Args a) {
         }
       }
 #pragma unroll
-      for (int i = 0; i < RO; ++i)
+      for (int i = 0; i < 4; ++i)
         *reinterpret_cast<float4*>(S_s + (sr + i) * L::LDS + sc) = make_float4(S[i][0], S[i][1], S[i][2], S[i][3]);
-    } else {
+    }
+    if (row >= C) {
       // o_t = Gamma_t (q_t S) + sum_(s <= t) M[t, s] u_s
       const float gam = s[L::SM + t];
-      o.x *= gam; o.y *= gam;
-#pragma unroll
+      o.x *= gam; o.y *= gam; o.z *= gam; o.w *= gam;
+#pragma unroll 4
       for (int u = 0; u < C; u += 4) {
         const float4 m = *reinterpret_cast<const float4*>(s + L::M + t * LDA + u);
         const float mm[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float2 x = *reinterpret_cast<const float2*>(U_s + (u + e) * BC + c2);
+          const float4 x = *reinterpret_cast<const float4*>(U_s + (u + e) * BC + cx);
           o.x = fmaf(mm[e], x.x, o.x);
           o.y = fmaf(mm[e], x.y, o.y);
+          o.z = fmaf(mm[e], x.z, o.z);
+          o.w = fmaf(mm[e], x.w, o.w);
         }
       }
       if (j * C + t < n)
-        *reinterpret_cast<float2*>(a.out + ((int64_t)(start + j * C + t) * a.H + h) * a.dv + c0 + c2) = o;
+        *reinterpret_cast<float4*>(a.out + ((int64_t)(start + j * C + t) * a.H + h) * a.dv + c0 + cx) = o;
     }
   }
   if (owner) {
 #pragma unroll
-    for (int i = 0; i < RO; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) Sg[(int64_t)(sr + i) * a.dv + sc + j] = S[i][j];
   }
@@ -397,7 +387,7 @@ int launch(const Args& a, int places, cudaStream_t stream) {
   launch_pdl(delta_chunk_kernel<DK>, dim3(places, a.H), dim3(THREADS), 0, stream, a);
   if ((e = cudaGetLastError()) != cudaSuccess) return refuse((int)e, "delta_chunks: %s", cudaGetErrorString(e));
   // a plain launch: its blocks are a chain of chunks each and have to be spread evenly over the SMs
-  delta_walk_kernel<DK><<<dim3(a.dv / BC, a.H, a.B), dim3(WALKERS), smem, stream>>>(a);
+  delta_walk_kernel<DK><<<dim3(a.dv / BC, a.H, a.B), dim3(THREADS), smem, stream>>>(a);
   return cuda_status("delta_chunks");
 }
 
