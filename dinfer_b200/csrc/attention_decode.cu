@@ -958,7 +958,7 @@ DINFER_API int dinfer_attention_decode_tma_bias(const void* q, int64_t ldq, void
   while ((1 << p.bs_log2) < block_size) ++p.bs_log2;
   p.window = window; p.chunked = chunked; p.sink = sink; p.sinks = sinks; p.scale_log2 = scale * 1.4426950408889634f; p.splits = splits;
   // With more CTAs than run at a time (two to an SM) and a CTA to a (request, head), the last ones to start end the step: they
-  // should be short.  64 requests of 300 to 4017 tokens, 8 heads of 128: 116 us in the batch's order (rising), @@N@@ us.
+  // should be short.  64 requests of 300 to 4017 tokens, 8 heads of 128: 116 us in the batch's order (rising), 96 us.
   static const int sms = [] { int d = 0, n = 148; if (cudaGetDevice(&d) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d); return n; }();
   p.by_length = splits == 1 && B <= BY_LENGTH_MAX && (int64_t)B * Hkv > 2 * sms ? B : 0;
   p.keep = window > 0 ? keep_first : 0;

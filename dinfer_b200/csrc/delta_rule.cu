@@ -117,7 +117,7 @@ delta_prep_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv,
 // The same for steps of many tokens (four taps; heads of 64 or 128 key channels that fill blocks of 128 channels): a thread
 // owns a channel and walks RUN tokens with the last three inputs in registers, so that an input is read 11 / 8 times
 // instead of four, and the block's eight norms are summed in one exchange.  Bound by the exponentials and divisions of
-// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) @@A@@ us, a block per (token, head) 64.
+// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) 41 us, a block per (token, head) 64.
 constexpr int RUN = 8;
 constexpr int RUN_FROM = 64;                               // tokens of a step from which it is taken (fewer leave SMs idle)
 template <typename TA>
