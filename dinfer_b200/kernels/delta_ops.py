@@ -6,7 +6,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from .lib import KernelError, check, dtype_code, ptr, require_cuda, stream_handle
+from .lib import KernelError, check, dtype_code, num_sms, ptr, require_cuda, stream_handle
 from .ops import _fn, _rows_contiguous
 
 
@@ -67,7 +67,7 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     of head h at ``state[slot, h * dk * dv:]`` (zero for a fresh request), carried in place.  Returns o f32 [T, H, dv].
     ``widen`` (1, 2, 4; 0: the sizes decide): how far a column's rows are spread over more lanes than 16 rows a lane
     would need, which only changes the order of the sums.  ``longest``: a bound of the tokens a request brings, where the
-    caller knows one; from ``CHUNKS_FROM`` on portions run in chunks (``_chunks``), again another order of the sums."""
+    caller knows one; long portions then run in chunks (``CHUNKS_FROM``, ``_chunks``), again another order of the sums."""
     require_cuda(q, k, v, beta, decay, state, cu_seqlens, slots, fresh)
     _ints(cu_seqlens, slots, fresh)
     T, G, dk = q.shape
@@ -80,7 +80,7 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     out = torch.empty((T, H, dv), dtype=torch.float32, device=q.device)
     if T == 0:
         return out
-    if longest >= CHUNKS_FROM and not per_channel and not widen and _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out):
+    if longest and not per_channel and not widen and _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest):
         return out
     lib, f = _fn("delta_rule", "dinfer_delta_recurrence",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
@@ -93,19 +93,26 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     return out
 
 
-# Portions from so many tokens on run in chunks of 32: a chunk costs a request's chain about as much as @@N@@ tokens of the token
-# loop, plus the pass that prepares all chunks (2000 tokens of 16 heads of 128: @@C@@ against 501 us; 48 tokens: @@D@@).
-CHUNKS_FROM = 48
+# Chunks of 32 are worth it where the token loop is bound by its chain (0.25 us a token) and not by its work: the walk over the
+# chunks runs a block per (request, head, 16 value columns), about one to an SM, and with more blocks than SMs takes as many
+# rounds.  So for one, two and three blocks an SM from so many tokens of the longest portion on, never beyond.  Keys and values
+# of 128, token loop and chunks (us), 16 heads, one portion: of 48 tokens 15 and 18, of 64 19 and 18, of 2000 502 and 220; two:
+# 64 22 and 25, 96 31 and 31, 2000 585 and 436; three: 96 38 and 44, 256 94 and 91, 2000 710 and 649; four: 256 114 and 118,
+# 2000 857 and 860.
+CHUNKS_FROM = (64, 96, 256)
 # bytes of workspace (128 KB a chunk of 32 tokens for 4 heads of 128) beyond which a step stays with the token loop
 CHUNKS_BYTES = 1 << 29
 
 
-def _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out) -> bool:
+def _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest: int) -> bool:
     """The recurrence with one decay a head in chunks of 32 tokens (``csrc/delta_chunks.cu``); False where the sizes do not
-    allow it (keys of 64 or 128, values in multiples of 16)."""
+    allow it (keys of 64 or 128, values in multiples of 16) or the token loop is as good."""
     T, G, dk = q.shape
     _, H, dv = v.shape
     B = cu_seqlens.numel() - 1
+    rounds = -(-(B * H * (dv // 16)) // num_sms())
+    if rounds > len(CHUNKS_FROM) or longest < CHUNKS_FROM[rounds - 1]:
+        return False
     if dk not in (64, 128) or dv % 16 or decay.shape[1] != H or any(t.data_ptr() % 16 for t in (q, k, out)):
         return False
     lib, floats = _fn("delta_chunks", "dinfer_delta_chunks_floats", [c_int, c_int])

@@ -27,7 +27,7 @@ CASES = [  # H, G, dk, dv, tokens of the requests, fresh, decays, keys
     (2, 2, 64, 48, [130], [0], "fast", "random"),
     (2, 1, 128, 32, [96, 50], [1, 0], "zero", "random"),
     (2, 1, 64, 32, [150], [0], "slow", "alike"),
-    (2, 2, 128, 256, [40] * 37, [1, 0] * 18 + [1], "mixed", "random"),
+    (2, 2, 128, 256, [40] * 13, [1, 0] * 6 + [1], "mixed", "random"),
 ]
 
 
@@ -82,7 +82,7 @@ def test_sizes_the_chunks_do_not_take_stay_with_the_token_loop():
         q, k, v = (torch.randn(60, 1, n, generator=g).cuda() for n in (dk, dk, dv))
         beta, decay = torch.rand(60, 1, generator=g).cuda(), -torch.rand(60, 1, generator=g).cuda()
         outs = []
-        for longest in (0, 60):
+        for longest in (0, 1000):
             st = torch.zeros(1, dk * dv).cuda()
             i32 = lambda *x: torch.tensor(x, dtype=torch.int32).cuda()
             outs.append(delta_ops.recurrence(q, k, v, beta, decay, st, i32(0, 60), i32(0), i32(1), False, longest=longest))
@@ -131,3 +131,17 @@ def test_preparation_in_runs(dtype, H, G, dk, dv, per_channel):
             alone = call(slice(a, z), state.clone().cuda()[i:i + 1], [0, z - a], [0], [fresh[i]])
             for o, w in zip(got, alone):
                 assert torch.allclose(o[a:z], w, rtol=2e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("B,H,longest,chunks", [(1, 16, 63, False), (1, 16, 64, True), (2, 16, 95, False), (2, 16, 96, True), (3, 16, 255, False),
+                                                (3, 16, 256, True), (4, 16, 4000, False)])
+def test_which_portions_run_in_chunks(B, H, longest, chunks, monkeypatch):
+    from dinfer_b200.kernels import delta_ops
+    monkeypatch.setattr(delta_ops, "num_sms", lambda: 148)
+    z = lambda *s: torch.zeros(*s, device="cuda")
+    i = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    q, v, beta = z(2 * B, 8, 128), z(2 * B, H, 128), z(2 * B, H)
+    took = delta_ops._chunks(q, q, v, beta, beta, z(B, H * 128 * 128), i(*range(0, 2 * B + 1, 2)), i(*range(B)), i(*[1] * B),
+                             torch.empty_like(v), longest)
+    torch.cuda.synchronize()
+    assert took is chunks
