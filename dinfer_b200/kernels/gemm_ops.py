@@ -105,7 +105,8 @@ def supported(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 def decode_splits(tokens: int, N: int, K: int) -> int:
     """K splits of the decode orientation: one wave of CTAs (three fit an SM up to 16 tokens, two
-    beyond), at least eight 64-wide K blocks per CTA, at most ``MAX_SPLITS`` (the CTAs of a tile are
+    beyond), at least four 64-wide K blocks per CTA (at eight, one row of 1024 x 2048 took 4.8 us, now 3.9;
+    4096 x 1024 5.1 and 4.2, 6144 x 1024 5.6 and 4.9, 1024 x 3072 4.9 and 4.6), at most ``MAX_SPLITS`` (the CTAs of a tile are
     one thread-block cluster)."""
     tiles = (N + 127) // 128
     k_blocks = (K + 63) // 64
