@@ -20,18 +20,18 @@ def tc_supported(dtype: torch.dtype, head_dim: int, group: int) -> bool:
     return dtype == torch.bfloat16 and head_dim in (32, 64, 128) and 1 <= group <= 16
 
 
-def decode_splits(num_reqs: int, num_kv_heads: int, max_seq_len: int, ctas_per_sm: int = 2) -> int:
+def decode_splits(num_reqs: int, num_kv_heads: int, max_seq_len: int, ctas_per_sm: int = 2, lone: bool = True) -> int:
     """Key splits of the decode shape.  ``ctas_per_sm`` CTAs fit an SM (two of the attention kernels; the differential kernel says how many of its own):
     with few (request, kv head) pairs the
     splits fill those slots in one wave; with as many pairs as slots or more, splitting only adds
-    partial sums to fold, so there is none.  Never more than a quarter of the 64-key tiles (half of them
-    for at most eight splits of one CTA an SM: 1000 keys of one request's 8 heads 4.4 us with 8 splits, 4.75
+    partial sums to fold, so there is none.  Never more than a quarter of the 64-key tiles (half of them,
+    with ``lone``, for at most eight splits of one CTA an SM: 1000 keys of one request's 8 heads 4.4 us with 8 splits, 4.75
     with 4; 3 or fewer tiles a split lose where two CTAs share an SM), at most 16 (the largest cluster)."""
     slots = ctas_per_sm * num_sms()
     base = max(1, num_reqs * num_kv_heads)
     want = slots // base if base <= slots else 1
     tiles = max(1, (max_seq_len + 63) // 64)
-    alone = min(num_sms() // base, tiles // 2, 8) if tiles >= 8 else 1
+    alone = min(num_sms() // base, tiles // 2, 8) if lone and tiles >= 8 else 1
     return max(1, min(want, max(1, tiles // 4), MAX_CLUSTER_SPLITS), alone)
 
 

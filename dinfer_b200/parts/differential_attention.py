@@ -105,7 +105,7 @@ class DifferentialAttention(Mixer):
             longest = self.env.max_positions if ctx.decode_splits else ctx.max_seq_len
             seen = min(longest, window + self.keep_first) if window else longest
             splits = self.force_splits or attention_ops.decode_splits(ctx.num_reqs, G, seen,
-                                                                      attention_ops.diff_tc_decode_ctas_per_sm(D, Dv))
+                                                                      attention_ops.diff_tc_decode_ctas_per_sm(D, Dv), lone=False)
             attention_ops.attention_diff_tc(q, out, gate, cache.kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, H, G, D, Dv,
                                             self.scale, window, self.keep_first, self.lam, self.eps, 1.0 - self.diff,
                                             ctx.max_q_len, ctx.any_decode, ctx.any_prefill, splits)
