@@ -85,7 +85,9 @@ def logprobs(logits: torch.Tensor, chosen: torch.Tensor, k: int):
     return ids, lp, rank
 
 
-_MASK = 0xFFFFFFFFFFFFFFFF          # seeds and counts as their 64 bits
+def _u64(x: int) -> int:
+    x &= 0xFFFFFFFFFFFFFFFF
+    return x - (1 << 64) if x >= (1 << 63) else x
 
 
 class Sampler:
@@ -115,8 +117,8 @@ class Sampler:
                 base = dev.data_ptr()
                 self._slots.append(dict(
                     host=host, dev=dev, event=None,
-                    # columns: seeds, offsets (uint64), temperature, top_p, min_p (float32), top_k (int32)
-                    u64=h[:16 * cap].view(np.uint64).reshape(2, cap),
+                    # columns: seeds, offsets (int64), temperature, top_p, min_p (float32), top_k (int32)
+                    i64=h[:16 * cap].view(np.int64).reshape(2, cap),
                     f32=h[16 * cap:28 * cap].view(np.float32).reshape(3, cap),
                     i32=h[28 * cap:32 * cap].view(np.int32),
                     seeds=base, offsets=base + 8 * cap, temperature=base + 16 * cap, top_p=base + 20 * cap,
@@ -180,15 +182,11 @@ class Sampler:
         if logits.dtype != torch.float32 or logits.stride(1) != 1:
             raise ValueError("sample: logits must be float32 with a contiguous last axis")
         slot = self._staging(R)
-        u64, f32, i32 = slot["u64"], slot["f32"], slot["i32"]
-        # a column at a time: element by element, 64 rows took 60 us of the host, as long as the kernel; now 28
-        n = len(params)
-        f32[0, :n] = np.fromiter([p.temperature for p in params], np.float32, n)
-        f32[1, :n] = np.fromiter([p.top_p for p in params], np.float32, n)
-        f32[2, :n] = np.fromiter([p.min_p for p in params], np.float32, n)
-        i32[:n] = np.fromiter([p.top_k for p in params], np.int32, n)
-        u64[0, :n] = np.fromiter([seeds[i] & _MASK for i in range(n)], np.uint64, n)
-        u64[1, :n] = np.fromiter([num_generated[i] & _MASK for i in range(n)], np.uint64, n)
+        i64, f32, i32 = slot["i64"], slot["f32"], slot["i32"]
+        for i, p in enumerate(params):
+            f32[0, i], f32[1, i], f32[2, i] = p.temperature, p.top_p, p.min_p
+            i32[i] = p.top_k
+            i64[0, i], i64[1, i] = _u64(seeds[i]), _u64(num_generated[i])
         slot["dev"].copy_(slot["host"], non_blocking=True)
         if slot["dev"].is_cuda:
             ev = slot["event"] or torch.cuda.Event()
