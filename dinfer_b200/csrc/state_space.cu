@@ -558,13 +558,14 @@ __global__ void __launch_bounds__(OutTiles<HEADS>::THREADS, HEADS == 2 ? 3 : 6) 
   const int64_t slot = chunk_slot(t_begin, b, c);
   const float* S_prev = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd + c0;
   const float* Cp = p.xbc + (int64_t)t0 * ch + inner + (p.G + g) * p.N;
-  // what this thread loads of a pass: C rows ct + (NT / 8) k at channels ce .., its head's S rows (channels) sr + 4 k at columns sx ..
-  const int ct = tid >> 3, ce = (tid & 7) * 4, sr = mine >> 4, sx = (mine & 15) * 4;
+  // what this thread loads of a pass: C rows ct + CR k at channels ce .., its head's S rows (channels) sr + 4 k at columns sx ..
+  constexpr int CR = NT / (KT / 4);
+  const int ct = tid / (KT / 4), ce = tid % (KT / 4) * 4, sr = mine >> 4, sx = (mine & 15) * 4;
   float4 cv[CV], sv[SV];
   auto fetch = [&](int e0) {
 #pragma unroll
     for (int k = 0; k < CV; ++k) {
-      const int t = ct + NT / 8 * k;
+      const int t = ct + CR * k;
       cv[k] = load4<VEC>(Cp + (int64_t)t * ch + e0 + ce, t < n ? p.N - e0 - ce : 0);
     }
 #pragma unroll
@@ -600,7 +601,7 @@ __global__ void __launch_bounds__(OutTiles<HEADS>::THREADS, HEADS == 2 ? 3 : 6) 
   for (int e0 = 0; e0 < p.N; e0 += KT) {
     __syncthreads();                               // the last pass is done with the tiles
 #pragma unroll
-    for (int k = 0; k < CV; ++k) put4(&C_s[ct + NT / 8 * k][ce], cv[k]);
+    for (int k = 0; k < CV; ++k) put4(&C_s[ct + CR * k][ce], cv[k]);
 #pragma unroll
     for (int k = 0; k < SV; ++k) put4(&S_s[sr + 4 * k][sx], sv[k]);
     __syncthreads();
