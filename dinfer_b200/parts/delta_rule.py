@@ -13,7 +13,7 @@ Data flow of one step (prompt portions and decoded tokens alike):
   P = x [W_q; W_k; W_v; W_b; W_a | W_a1; W_g | W_g1]^T      one stacked product
   a, gate = thin second products where the design has them
   q, k, v, beta, g = delta_prep(P, a, convolution history)    32-bit; the history then moves on
-  o = delta_recurrence(q, k, v, beta, g, S)                    32-bit, S in place
+  o = delta_recurrence(q, k, v, beta, g, S)                    32-bit, S in place; token by token, long portions in chunks
   y = delta_post(o, w, gate);  out = y W_o^T
 What a request keeps is one row of a fixed-size state: S of every head, then the last ``taps - 1`` inputs of the
 convolutions.  Everything reads the step's slots and fresh flags from the device, so steps replay as CUDA graphs.
