@@ -82,14 +82,17 @@ __device__ __forceinline__ float dot4(const float4& a, const float4& b, float c)
   return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
 }
 
+// Bound by the reads of shared memory that feed its multiply-adds (a warp's 16-byte read takes four passes whatever its lanes
+// share): 4 x 4 sums a thread for the products, 4 x 8 for the columns, which take beta and Gamma with the inverse's columns.
 template <int DK>
 __global__ void __launch_bounds__(THREADS, 2)
 delta_chunk_kernel(const Args a) {
-  constexpr int LD = DK + 4;
-  __shared__ __align__(16) float KQ[2 * C][LD];          // keys, then queries
-  __shared__ __align__(16) float As[C][LDA], Ts[C][LDA]; // A; the inverse, transposed: Ts[s][t]
+  constexpr int LD = DK + 4, CW = DK / 16;               // columns of a thread
+  __shared__ __align__(16) float KQ[2 * C][LD];          // keys, then queries, later values
+  __shared__ __align__(16) float As[C][LDA];             // A
+  __shared__ __align__(16) float Ts[2][C][LDA];          // the inverse, transposed: Ts[.][s][t], times beta_s; times beta_s Gamma_s
   __shared__ double c_s[C];
-  __shared__ float beta_s[C], gam_s[C];
+  __shared__ float beta_s[C];
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int place = blockIdx.x, h = blockIdx.y, g = h / (a.H / a.G);
@@ -106,10 +109,10 @@ delta_chunk_kernel(const Args a) {
     cp_async16(&KQ[r][e], src, t < n);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
+  float gam = 0.f, be = 0.f;                             // of token `lane`, in warp 0
   if (warp == 0) {
     // the decays' logarithms (0 behind the portion's end), their running sums in 64-bit
     double l = 0.0;
-    float be = 0.f;
     if (lane < n) {
       l = fmax(log1p((double)a.decay[(int64_t)(t0 + lane) * a.H + h]), (double)LOG_FLOOR);
       be = a.beta[(int64_t)(t0 + lane) * a.H + h];
@@ -122,46 +125,63 @@ delta_chunk_kernel(const Args a) {
     const double last = __shfl_sync(0xffffffffu, l, 31);
     c_s[lane] = l;
     beta_s[lane] = be;
-    const float gam = expf((float)l);
-    gam_s[lane] = gam;
+    gam = expf((float)l);
     float* sm = a.small + at * SMALL;
     sm[lane] = gam;
     sm[C + lane] = expf((float)(last - l));
     if (lane == 0) sm[2 * C] = expm1f((float)last);
   }
-  // this thread's column of the right-hand side, where that is a value column
-  const int cols = a.dv + DK;
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   {
-    // k_t . k_s and q_t . k_s: rows ty + 16 i of the stacked 64, columns tx + 16 j
-    const int ty = tid >> 4, tx = tid & 15;
-    float acc[4][2];
+    // k_t . k_s and q_t . k_s: rows ty + 16 i of the stacked 64, columns tx + 8 j; half of the key channels to 128 threads.
+    // Then the first half of the threads completes the rows of A, the second those of M.
+    const int kh = tid >> 7, ty = (tid & 127) >> 3, tx = tid & 7;
+    float acc[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.f;
-#pragma unroll 4
-    for (int e = 0; e < DK; e += 4) {
-      float4 r[4], s[2];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+    for (int e = kh * (DK / 2); e < (kh + 1) * (DK / 2); e += 4) {
+      float4 r[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[i] = *reinterpret_cast<const float4*>(&KQ[ty + 16 * i][e]);
 #pragma unroll
-      for (int j = 0; j < 2; ++j) s[j] = *reinterpret_cast<const float4*>(&KQ[tx + 16 * j][e]);
+      for (int j = 0; j < 4; ++j) {
+        const float4 s = *reinterpret_cast<const float4*>(&KQ[tx + 8 * j][e]);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j] = dot4(r[i], s[j], acc[i][j]);
+        for (int i = 0; i < 4; ++i) acc[i][j] = dot4(r[i], s, acc[i][j]);
+      }
     }
+    float (*other)[LDA] = Ts[kh];                          // what the other half of the threads lacks
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) other[ty + 16 * i][tx + 8 * j] = kh ? acc[i][j] : acc[i + 2][j];
+    __syncthreads();
     float* m = a.m + at * C * C;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int t = ty + 16 * i, s = tx + 16 * j;
+      for (int j = 0; j < 4; ++j) {
+        const int t = ty + 16 * i, s = tx + 8 * j;
         const float e = s <= t ? expf((float)(c_s[t] - c_s[s])) : 0.f;
-        As[t][s] = s < t ? beta_s[t] * e * acc[i][j] : 0.f;
-        m[t * C + s] = e * acc[i + 2][j];
+        const float dot = (kh ? acc[i + 2][j] : acc[i][j]) + Ts[kh ^ 1][t][s];
+        if (kh == 0) As[t][s] = s < t ? beta_s[t] * e * dot : 0.f;
+        else m[t * C + s] = e * dot;
       }
   }
+  // nobody reads the queries any more: DK value columns take their place (zeros behind the portion's end)
+  auto values = [&](int c0) {
+    for (int i = tid; i < C * (DK / 4); i += THREADS) {
+      const int t = i / (DK / 4), e = (i % (DK / 4)) * 4;
+      const bool live = t < n && c0 + e < a.dv;
+      cp_async16(&KQ[C + t][e], a.v + (live ? ((int64_t)(t0 + t) * a.H + h) * a.dv + c0 + e : 0), live);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  values(0);
   __syncthreads();
   if (warp == 0) {
     // column `lane` of (I + A)^-1 by substitution: x_t = [t = lane] - sum_(s < t) A[t, s] x_s
@@ -170,41 +190,67 @@ delta_chunk_kernel(const Args a) {
     for (int t = 0; t < C; ++t) {
       float p[4] = {t == lane ? 1.f : 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int s = 0; s < t; ++s) p[s & 3] = fmaf(-As[t][s], x[s], p[s & 3]);
+      for (int s = 0; s < t; s += 4) {
+        const float4 r = *reinterpret_cast<const float4*>(&As[t][s]);
+        p[0] = fmaf(-r.x, x[s], p[0]);
+        if (s + 1 < t) p[1] = fmaf(-r.y, x[s + 1], p[1]);
+        if (s + 2 < t) p[2] = fmaf(-r.z, x[s + 2], p[2]);
+        if (s + 3 < t) p[3] = fmaf(-r.w, x[s + 3], p[3]);
+      }
       x[t] = (p[0] + p[1]) + (p[2] + p[3]);
     }
 #pragma unroll
-    for (int t = 0; t < C; t += 4) *reinterpret_cast<float4*>(&Ts[lane][t]) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
-  }
-  __syncthreads();
-  // a thread per column of [beta V | beta Gamma K]
-  for (int col = tid; col < cols; col += THREADS) {
-    float r[C], acc[C];
-    if (col < a.dv) {
-      const float* v = a.v + ((int64_t)t0 * a.H + h) * a.dv + col;
-#pragma unroll
-      for (int s = 0; s < C; ++s) r[s] = s < n ? beta_s[s] * v[(int64_t)s * a.H * a.dv] : 0.f;
-    } else {
-#pragma unroll
-      for (int s = 0; s < C; ++s) r[s] = beta_s[s] * gam_s[s] * KQ[s][col - a.dv];
+    for (int t = 0; t < C; t += 4) {
+      const float4 v = make_float4(be * x[t], be * x[t + 1], be * x[t + 2], be * x[t + 3]);
+      *reinterpret_cast<float4*>(&Ts[0][lane][t]) = v;
+      *reinterpret_cast<float4*>(&Ts[1][lane][t]) = make_float4(gam * v.x, gam * v.y, gam * v.z, gam * v.w);
     }
+  }
+  // [W_v | W_k]: a half of the threads has DK columns, a thread rows rt .. rt + 3 of columns cx + 64 j ..
+  const bool keys = tid < 128;
+  const int rt = ((tid & 127) >> 4) * 4, cx = (tid & 15) * 4, s_end = (((tid & 127) >> 5) * 2 + 1) * 4 + 4;   // (a warp's last row)
+  for (int c0 = 0; c0 < a.dv; c0 += DK) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (!keys || c0 == 0) {
+      const float (*right)[LD] = keys ? KQ : KQ + C;
+      const float (*T)[LDA] = Ts[keys];
+      float acc[4][CW];
 #pragma unroll
-    for (int t = 0; t < C; ++t) acc[t] = 0.f;
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int s = 0; s < C; ++s) {
+        for (int j = 0; j < CW; ++j) acc[i][j] = 0.f;
+#pragma unroll 4
+      for (int s = 0; s < s_end; ++s) {
+        const float4 t4 = *reinterpret_cast<const float4*>(&T[s][rt]);
+        const float t[4] = {t4.x, t4.y, t4.z, t4.w};
 #pragma unroll
-      for (int t = s & ~3; t < C; t += 4) {
-        const float4 w = *reinterpret_cast<const float4*>(&Ts[s][t]);
-        acc[t] = fmaf(w.x, r[s], acc[t]);
-        acc[t + 1] = fmaf(w.y, r[s], acc[t + 1]);
-        acc[t + 2] = fmaf(w.z, r[s], acc[t + 2]);
-        acc[t + 3] = fmaf(w.w, r[s], acc[t + 3]);
+        for (int j = 0; j < CW; j += 4) {
+          const float4 r = *reinterpret_cast<const float4*>(&right[s][cx + 16 * j]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            acc[i][j] = fmaf(t[i], r.x, acc[i][j]);
+            acc[i][j + 1] = fmaf(t[i], r.y, acc[i][j + 1]);
+            acc[i][j + 2] = fmaf(t[i], r.z, acc[i][j + 2]);
+            acc[i][j + 3] = fmaf(t[i], r.w, acc[i][j + 3]);
+          }
+        }
+      }
+      float* w = keys ? a.wk + at * C * DK : a.wv + at * C * a.dv + c0;
+      const int ld = keys ? DK : a.dv;
+#pragma unroll
+      for (int j = 0; j < CW; j += 4) {
+        const int c = cx + 16 * j;
+        if (!keys && c0 + c >= a.dv) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float4*>(w + (int64_t)(rt + i) * ld + c) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
       }
     }
-    float* w = col < a.dv ? a.wv + at * C * a.dv + col : a.wk + at * C * DK + col - a.dv;
-    const int ld = col < a.dv ? a.dv : DK;
-#pragma unroll
-    for (int t = 0; t < C; ++t) w[t * ld] = acc[t];
+    if (c0 + DK < a.dv) {
+      __syncthreads();
+      values(c0 + DK);
+    }
   }
 }
 
@@ -409,7 +455,7 @@ DINFER_API int dinfer_delta_chunks(const float* q, const float* k, const float* 
                                    float* work, int places, int B, int H, int G, int dk, int dv, cudaStream_t stream) {
   if (B <= 0 || H <= 0 || G <= 0 || H % G || places < 0 || H > 65535 || B > 65535 || !dinfer_delta_chunks_supports(dk, dv))
     return refuse(DINFER_BAD_ARGUMENT, "delta_chunks: bad sizes B=%d H=%d G=%d dk=%d dv=%d", B, H, G, dk, dv);
-  if (!aligned16(q) || !aligned16(k) || !aligned16(out) || !aligned16(work))
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(work))
     return refuse(DINFER_BAD_ARGUMENT, "delta_chunks: 16-byte aligned rows");
   if (places == 0) return 0;
   Args a;

@@ -113,7 +113,7 @@ def _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest:
     rounds = -(-(B * H * (dv // 16)) // num_sms())
     if rounds > len(CHUNKS_FROM) or longest < CHUNKS_FROM[rounds - 1]:
         return False
-    if dk not in (64, 128) or dv % 16 or decay.shape[1] != H or any(t.data_ptr() % 16 for t in (q, k, out)):
+    if dk not in (64, 128) or dv % 16 or decay.shape[1] != H or any(t.data_ptr() % 16 for t in (q, k, v, out)):
         return False
     lib, floats = _fn("delta_chunks", "dinfer_delta_chunks_floats", [c_int, c_int])
     floats.restype = c_int64
