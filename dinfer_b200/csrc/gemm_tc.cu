@@ -473,27 +473,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-// ---- prompts, two SMs on one tile: the CTAs of a cluster of two share a tile of 256 weight rows x up to 256 tokens
-// (tcgen05.mma.cta_group::2).  Each CTA stages its own 128 of the 256 weight rows (the MMA's rows) and its own half of the
-// tokens (its columns), so every byte of either operand is fetched by one SM of the pair only; the leader (cluster rank 0)
-// issues the MMAs for both, which leave the sums of 128 weight rows in each CTA's tensor memory.  TMA completions of both CTAs
-// count on the leader's barrier; tcgen05.commit hands stages and accumulators back to both CTAs at once.  No load is multicast.
-// Tokens are the columns because their number may be any multiple of 16: the last tile of a step's tokens, or of an expert's
-// run, is as wide as it has rows (in steps of 64, so that a CTA loads boxes of 32 rows) instead of 256.  A tile of 64 tokens is
-// bound by its weights' way through L2 and still takes @@S@@ of a full one's time: 2048 tokens of top 8 of 64 experts (about
-// 256 rows an expert, half of them one row tile and a little) @@A@@ us for both products where full tiles took 340.
+// ---- prompts, two SMs on one tile: the CTAs of a cluster of two share a 256 x 256 output tile
+// (tcgen05.mma.cta_group::2).  Each CTA stages its own 128 token rows and its own 128 of the 256 weight rows,
+// so a stage is 32 KB instead of 48 and every byte of the weight tile is fetched by one SM of the pair only;
+// the leader (cluster rank 0) issues the MMAs for both, which leave 128 accumulator rows in each CTA's tensor
+// memory.  TMA completions of both CTAs count on the leader's barrier; tcgen05.commit hands stages and
+// accumulators back to both CTAs at once.  No load is multicast.
 // CTAs are persistent: a pair walks over tiles (token tile fastest, so that pairs running at the same time read the
 // same few weight tiles from L2), the shared-memory ring runs on across tiles, and the accumulator is double-buffered
-// in tensor memory (2 x 256 columns): the epilogue warps drain tile i while the MMAs of tile i + 1 run.  A lane of them
-// has one weight row; two neighbours exchange a token each, so that a lane stores two neighbouring columns of one token.  With
+// in tensor memory (2 x 256 columns): the epilogue warps drain tile i while the MMAs of tile i + 1 run.  With
 // EPI_GATED the weight rows are (gate, up) pairs and the epilogue writes silu(gate) * up, half as wide, with EPI_CLAMPED
 // the clamped gate; with EPI_ACT it
 // applies the activation grp_act, with EPI_XIELU that one.
+// (Narrower tiles, chosen so that the last round of tiles leaves fewer SMs idle, were measured and are slower at
+// every shape.)
 constexpr int EPI_PLAIN = 0, EPI_GATED = 1, EPI_ACT = 2, EPI_XIELU = 3, EPI_CLAMPED = 4;
-constexpr int NT = 256;                                                       // weight rows of the pair's tile, and its most tokens
-constexpr int X_BOX = 32;                                                     // token rows of a load where a tile is narrower
+constexpr int NT = 256;                                                       // columns of the pair's tile
 constexpr int C_STAGES = 6, C_ACC_BUFS = 2, C_TMEM_COLS = NT * C_ACC_BUFS;
-constexpr uint32_t C_A_BYTES = TILE_M * BLOCK_K * 2, C_B_BYTES = (NT / 2) * BLOCK_K * 2;   // this CTA's rows of both operands (at most)
+constexpr uint32_t C_A_BYTES = TILE_M * BLOCK_K * 2, C_B_BYTES = (NT / 2) * BLOCK_K * 2;   // this CTA's rows of both operands
 constexpr size_t C_SMEM_BYTES = (size_t)C_STAGES * (C_A_BYTES + C_B_BYTES) + 1024;
 
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
@@ -529,33 +526,9 @@ __device__ __forceinline__ void tcgen05_mma_f16_pair(uint32_t d_tmem, uint64_t a
                ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// two neighbouring results of one token: columns n, n + 1 of its row
-template <typename OutT>
-__device__ __forceinline__ void store2(OutT* dst, float lo, float hi, int left, bool vec) {
-  if (vec && left >= 2) {
-    if constexpr (sizeof(OutT) == 2) *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(lo, hi);
-    else *reinterpret_cast<float2*>(dst) = make_float2(lo, hi);
-  } else {
-    if (left > 0) dst[0] = out_cast<OutT>(lo);
-    if (left > 1) dst[1] = out_cast<OutT>(hi);
-  }
-}
-
-// Rows of row tile m (0: none), by a whole warp.  An expert's run has its pairs in front and padding behind them.
-__device__ __forceinline__ int rows_of_tile(const GemmParams& p, int m, int lane) {
-  if (!p.tile_expert) return min(256, p.tokens - m * 256);
-  if (p.tile_expert[m] < 0) return 0;
-  if (!p.sorted) return 256;
-  int rows = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) rows += __popc(__ballot_sync(0xffffffffu, p.sorted[m * 256 + 32 * i + lane] < p.pairs));
-  return rows;
-}
-
 template <typename OutT, int EPI>
 __global__ void __launch_bounds__(NTHREADS)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                    const __grid_constant__ CUtensorMap map_x_box, const GemmParams p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   extern __shared__ unsigned char smem_dyn[];
   __shared__ __align__(8) uint64_t full_bar[C_STAGES], empty_bar[C_STAGES], acc_full_bar[C_ACC_BUFS], acc_empty_bar[C_ACC_BUFS];
   __shared__ uint32_t s_tmem_base;
@@ -565,20 +538,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const uint32_t rank = cluster_ctarank();                      // 0 = leader
   const int m_tiles = (p.tokens + 255) / 256, n_tiles = (p.N + NT - 1) / NT;
   const int tiles = m_tiles * n_tiles;
-  // the order of the tiles: token tile fastest, so that pairs running at the same time read the same few weight tiles, and a
-  // narrower last token tile's after all others; in grouped mode weight tile fastest, because a row tile has an expert's
-  // weights to itself and its rows are what is shared
-  const int whole = p.tokens / 256;
-  const auto m_of = [&](int tile) { return p.tile_expert ? tile / n_tiles : (tile < whole * n_tiles ? tile % whole : whole); };
-  const auto n_of = [&](int tile) { return p.tile_expert ? tile % n_tiles : (tile < whole * n_tiles ? tile / whole : tile - whole * n_tiles); };
+  // the order of the tiles: token tile fastest, so that pairs running at the same time read the same few weight tiles; in
+  // grouped mode weight tile fastest, because a row tile has an expert's weights to itself and its rows are what is shared
+  const auto m_of = [&](int tile) { return p.tile_expert ? tile / n_tiles : tile % m_tiles; };
+  const auto n_of = [&](int tile) { return p.tile_expert ? tile % n_tiles : tile / m_tiles; };
   const int total_kb = (p.K + BLOCK_K - 1) / BLOCK_K;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   pdl_enter();
 
   if (threadIdx.x == 0) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x_box) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     for (int s = 0; s < C_STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
     for (int b = 0; b < C_ACC_BUFS; ++b) { mbar_init(smem_u32(&acc_full_bar[b]), 1); mbar_init(smem_u32(&acc_empty_bar[b]), 8); }
     s_abort = 0;
@@ -595,74 +565,62 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   tcgen05_fence_after();
   const uint32_t tmem = s_tmem_base;
 
-  if (warp == 0) {                                              // ---- TMA producer (both CTAs; lane 0, the others count rows)
-    uint32_t it = 0;
-    bool ok = true;
-    for (int tile = pair; tile < tiles && ok; tile += pairs) {
-      const int rows = rows_of_tile(p, m_of(tile), lane);
-      if (rows == 0) continue;
-      if (lane == 0) {
-        const int nt = (rows + 2 * X_BOX - 1) / (2 * X_BOX) * (2 * X_BOX);     // the tile's tokens, half of them this CTA's
-        const int m0 = m_of(tile) * 256 + (int)rank * (nt / 2);
-        const int n0 = (p.tile_expert ? p.tile_expert[m_of(tile)] * p.N : 0) + n_of(tile) * NT + (int)rank * 128;
+  if (warp == 0) {
+    if (lane == 0) {                                            // ---- TMA producer (both CTAs)
+      uint32_t it = 0;
+      bool ok = true;
+      for (int tile = pair; tile < tiles && ok; tile += pairs) {
+        int expert = 0;
+        if (p.tile_expert) { expert = p.tile_expert[m_of(tile)]; if (expert < 0) continue; }
+        const int m0 = m_of(tile) * 256 + (int)rank * 128;
+        const int n0 = expert * p.N + n_of(tile) * NT + (int)rank * (NT / 2);
         for (int kb = 0; kb < total_kb; ++kb, ++it) {
           const uint32_t s = it % C_STAGES;
           if (!mbar_wait(smem_u32(&empty_bar[s]), ((it / C_STAGES) & 1) ^ 1)) { s_abort = 1; atomicExch(p.status, 1); ok = false; break; }
-          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * C_A_BYTES + (uint32_t)nt * BLOCK_K * 2);
+          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * (C_A_BYTES + C_B_BYTES));
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);
-          const uint32_t sa = smem_base + s * (C_A_BYTES + C_B_BYTES), sb = sa + C_A_BYTES;
-          tma_load_2d_pair(sa, &map_w, kb * BLOCK_K, n0, bar);
-          if (nt == NT) {
-            tma_load_2d_pair(sb, &map_x, kb * BLOCK_K, m0, bar);
-          } else {
-            for (int i = 0; i < nt / 2; i += X_BOX) tma_load_2d_pair(sb + i * BLOCK_K * 2, &map_x_box, kb * BLOCK_K, m0 + i, bar);
-          }
+          const uint32_t sa = smem_base + s * (C_A_BYTES + C_B_BYTES);
+          tma_load_2d_pair(sa, &map_a, kb * BLOCK_K, m0, bar);
+          tma_load_2d_pair(sa + C_A_BYTES, &map_b, kb * BLOCK_K, n0, bar);
         }
       }
-      ok = __shfl_sync(0xffffffffu, (int)ok, 0);
     }
   } else if (warp == 1) {
-    if (rank == 0) {                                            // ---- MMA issue (the leader, for both CTAs; lane 0)
+    if (lane == 0 && rank == 0) {                               // ---- MMA issue (the leader, for both CTAs)
+      constexpr uint32_t idesc = instr_desc_bf16(256, NT);
       uint32_t it = 0, lt = 0;
       bool ok = true;
-      for (int tile = pair; tile < tiles && ok; tile += pairs) {
-        const int rows = rows_of_tile(p, m_of(tile), lane);
-        if (rows == 0) continue;                                // a tile without rows
-        if (lane == 0) {
-          const uint32_t idesc = instr_desc_bf16(256, (rows + 2 * X_BOX - 1) / (2 * X_BOX) * (2 * X_BOX));
-          const uint32_t b = lt % C_ACC_BUFS;
-          if (!mbar_wait_cluster(smem_u32(&acc_empty_bar[b]), ((lt / C_ACC_BUFS) & 1) ^ 1)) { s_abort = 1; atomicExch(p.status, 2); ok = false; }
+      for (int tile = pair; tile < tiles && ok; tile += pairs, ++lt) {
+        if (p.tile_expert && p.tile_expert[m_of(tile)] < 0) { --lt; continue; }       // a tile without rows
+        const uint32_t b = lt % C_ACC_BUFS;
+        if (!mbar_wait_cluster(smem_u32(&acc_empty_bar[b]), ((lt / C_ACC_BUFS) & 1) ^ 1)) { s_abort = 1; atomicExch(p.status, 2); break; }
+        tcgen05_fence_after();
+        const uint32_t acc = tmem + b * NT;
+        for (int kb = 0; kb < total_kb; ++kb, ++it) {
+          const uint32_t s = it % C_STAGES;
+          if (!mbar_wait_cluster(smem_u32(&full_bar[s]), (it / C_STAGES) & 1)) { s_abort = 1; atomicExch(p.status, 2); ok = false; break; }
           tcgen05_fence_after();
-          const uint32_t acc = tmem + b * NT;
-          for (int kb = 0; kb < total_kb && ok; ++kb, ++it) {
-            const uint32_t s = it % C_STAGES;
-            if (!mbar_wait_cluster(smem_u32(&full_bar[s]), (it / C_STAGES) & 1)) { s_abort = 1; atomicExch(p.status, 2); ok = false; break; }
-            tcgen05_fence_after();
-            const uint32_t sa = smem_base + s * (C_A_BYTES + C_B_BYTES);
-            const uint64_t da = smem_desc_k_sw128(sa), db = smem_desc_k_sw128(sa + C_A_BYTES);
+          const uint32_t sa = smem_base + s * (C_A_BYTES + C_B_BYTES);
+          const uint64_t da = smem_desc_k_sw128(sa), db = smem_desc_k_sw128(sa + C_A_BYTES);
 #pragma unroll
-            for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
-              tcgen05_mma_f16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            tcgen05_commit_pair(smem_u32(&empty_bar[s]));
-          }
-          if (ok) tcgen05_commit_pair(smem_u32(&acc_full_bar[b]));
+          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+            tcgen05_mma_f16_pair(acc, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          tcgen05_commit_pair(smem_u32(&empty_bar[s]));
         }
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0);
-        ++lt;
+        if (ok) tcgen05_commit_pair(smem_u32(&acc_full_bar[b]));
       }
     }
-  } else {                                                      // ---- epilogue (both CTAs, 128 weight rows each)
+  } else {                                                      // ---- epilogue (both CTAs, 128 rows each)
     const int quarter = warp & 3;
-    const bool odd = lane & 1;
+    const int r = quarter * 32 + lane;
     OutT* out = reinterpret_cast<OutT*>(p.out);
-    const bool vec = p.ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(p.out) & (2 * sizeof(OutT) - 1)) == 0;
-    constexpr bool GATED = EPI == EPI_GATED || EPI == EPI_CLAMPED;
-    const bool scatter = p.tile_expert && p.grp_epi == 1;       // the rows go to their pairs' places, weighed
+    const bool vec = sizeof(OutT) == 2 && (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    const int n_out = EPI == EPI_GATED || EPI == EPI_CLAMPED ? p.N / 2 : p.N;
     uint32_t lt = 0;
-    for (int tile = pair; tile < tiles; tile += pairs) {
-      const int m = m_of(tile), rows = rows_of_tile(p, m, lane);
-      if (rows == 0) continue;                                  // a tile without rows
+    for (int tile = pair; tile < tiles; tile += pairs, ++lt) {
+      if (p.tile_expert && p.tile_expert[m_of(tile)] < 0) { --lt; continue; }         // a tile without rows
       const uint32_t b = lt % C_ACC_BUFS;
+      const int m0 = m_of(tile) * 256 + (int)rank * 128, n0 = n_of(tile) * NT;
       if (total_kb > 0) {
         if (!mbar_wait(smem_u32(&acc_full_bar[b]), (lt / C_ACC_BUFS) & 1)) {
           if (lane == 0) { s_abort = 1; atomicExch(p.status, 3); }
@@ -670,10 +628,18 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
         tcgen05_fence_after();
       }
-      const int n = n_of(tile) * NT + (int)rank * 128 + quarter * 32 + (lane & ~1);    // this lane's columns n, n + 1
+      const int t = m0 + r;
+      int64_t t_out = t;                                        // the output row of this thread's accumulator row
+      float row_scale = 1.f;
+      bool skip_row = false;
+      if (p.tile_expert && p.grp_epi == 1 && t < p.tokens) {
+        const int pr = p.sorted[t];
+        skip_row = pr >= p.pairs;
+        if (!skip_row) { t_out = pr; row_scale = p.row_w[pr]; }
+      }
       const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + b * NT;
 #pragma unroll 1
-      for (int c0 = 0; c0 < rows; c0 += 32) {
+      for (int c0 = 0; c0 < NT; c0 += 32) {
         uint32_t v[2][16];
         if (total_kb > 0) {
           tmem_ld_32x32b_x16(acc + c0, v[0]);
@@ -683,33 +649,62 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 16; ++j) { v[0][j] = 0u; v[1][j] = 0u; }
         }
-        int place = 0;                                          // of token c0 + lane
-        float weight = 1.f;
-        if (scatter && c0 + lane < rows) { place = p.sorted[m * 256 + c0 + lane]; weight = p.row_w[place]; }
+        if (t >= p.tokens || skip_row) continue;
+        if constexpr (EPI == EPI_ACT || EPI == EPI_XIELU) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const uint32_t v0 = v[j >> 4][j & 15], v1 = v[j >> 4][(j & 15) + 1];
-          const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-          float lo = __uint_as_float(odd ? got : v0), hi = __uint_as_float(odd ? v1 : got);
-          const int c = c0 + j + odd;                           // this lane's token
-          int64_t row = m * 256 + c;
-          if (scatter) {
-            row = __shfl_sync(0xffffffffu, place, j + odd);
-            const float w = __shfl_sync(0xffffffffu, weight, j + odd);
-            lo *= w;
-            hi *= w;
-          }
-          if (c < rows && n < p.N) {
-            if constexpr (GATED) {
-              const float y = EPI == EPI_CLAMPED ? clamped_swish_fast(lo, hi, p.a_pos, p.a_neg)
-                              : p.act == 2 ? gelu_tanh_mul(lo, hi) : silu_mul_fast(lo, hi);
-              out[row * p.ldc + (n >> 1)] = out_cast<OutT>(y);
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float x = __uint_as_float(v[h][j]);
+              v[h][j] = __float_as_uint(EPI == EPI_XIELU ? xielu_fast(x, p.a_pos, p.a_neg) : grouped_act(x, p));
+            }
+        }
+        if (EPI == EPI_PLAIN && p.row_w) {                      // grouped, second product: times the row's weight
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[h][j] = __float_as_uint(__uint_as_float(v[h][j]) * row_scale);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (EPI == EPI_GATED || EPI == EPI_CLAMPED) {
+            const int o0 = (n0 + c0 + h * 16) >> 1;
+            OutT* dst = out + (int64_t)t * p.ldc + o0;
+            float y[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              y[j] = EPI == EPI_CLAMPED ? clamped_swish_fast(__uint_as_float(v[h][2 * j]), __uint_as_float(v[h][2 * j + 1]), p.a_pos, p.a_neg)
+                     : p.act == 2 ? gelu_tanh_mul(__uint_as_float(v[h][2 * j]), __uint_as_float(v[h][2 * j + 1]))
+                                  : silu_mul_fast(__uint_as_float(v[h][2 * j]), __uint_as_float(v[h][2 * j + 1]));
+            if (vec && o0 + 8 <= n_out) {
+              uint4 w0;
+              __nv_bfloat162* h0 = reinterpret_cast<__nv_bfloat162*>(&w0);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) h0[j] = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
+              *reinterpret_cast<uint4*>(dst) = w0;
             } else {
-              if constexpr (EPI == EPI_ACT || EPI == EPI_XIELU) {
-                lo = EPI == EPI_XIELU ? xielu_fast(lo, p.a_pos, p.a_neg) : grouped_act(lo, p);
-                hi = EPI == EPI_XIELU ? xielu_fast(hi, p.a_pos, p.a_neg) : grouped_act(hi, p);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if (o0 + j < n_out) dst[j] = out_cast<OutT>(y[j]);
+            }
+          } else {
+            const int o0 = n0 + c0 + h * 16;
+            OutT* dst = out + t_out * p.ldc + o0;
+            if (vec && o0 + 16 <= n_out) {
+              uint4 w0, w1;
+              __nv_bfloat162* h0 = reinterpret_cast<__nv_bfloat162*>(&w0);
+              __nv_bfloat162* h1 = reinterpret_cast<__nv_bfloat162*>(&w1);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                h0[j] = __floats2bfloat162_rn(__uint_as_float(v[h][2 * j]), __uint_as_float(v[h][2 * j + 1]));
+                h1[j] = __floats2bfloat162_rn(__uint_as_float(v[h][8 + 2 * j]), __uint_as_float(v[h][8 + 2 * j + 1]));
               }
-              store2<OutT>(out + row * p.ldc + n, lo, hi, p.N - n, vec);
+              reinterpret_cast<uint4*>(dst)[0] = w0;
+              reinterpret_cast<uint4*>(dst)[1] = w1;
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j)
+                if (o0 + j < n_out) dst[j] = out_cast<OutT>(__uint_as_float(v[h][j]));
             }
           }
         }
@@ -718,7 +713,6 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&acc_empty_bar[b]), 0));
-      ++lt;
     }
   }
 
@@ -833,7 +827,7 @@ int cluster_pairs_resident(const void* kernel, size_t smem) {
 }
 
 template <typename OutT, int EPI>
-int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxb, const GemmParams& p, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t stream) {
   auto k = gemm_tc_pair_kernel<OutT, EPI>;
   static int max_pairs = 0;
   if (!max_pairs) {
@@ -845,7 +839,7 @@ int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
   }
   const int tiles = ((p.tokens + 255) / 256) * ((p.N + NT - 1) / NT);
   dim3 grid(2 * (tiles < max_pairs ? tiles : max_pairs));
-  cudaError_t e = launch_pdl_cluster(k, grid, dim3(NTHREADS), dim3(2, 1, 1), C_SMEM_BYTES, stream, mw, mx, mxb, p);
+  cudaError_t e = launch_pdl_cluster(k, grid, dim3(NTHREADS), dim3(2, 1, 1), C_SMEM_BYTES, stream, ma, mb, p);
   if (e != cudaSuccess) return refuse((int)e, "gemm_tc: launch failed: %s", cudaGetErrorString(e));
   return cuda_status("gemm_tc");
 }
@@ -927,11 +921,9 @@ DINFER_API int dinfer_gemm_tc_all(const void* x, int64_t ldx, const void* w, int
   }
   p.k_blocks_per_split = total_kb;
   p.splits = 1;
-  CUtensorMap mc;
-  if ((rc = make_map(&ma, w, N, K, ldw, TILE_M))) return rc;
-  if ((rc = make_map(&mb, x, tokens, K, ldx, NT / 2))) return rc;
-  if ((rc = make_map(&mc, x, tokens, K, ldx, X_BOX))) return rc;
-#define GO(EPI) (out_f32 ? launch_pair<float, EPI>(ma, mb, mc, p, stream) : launch_pair<__nv_bfloat16, EPI>(ma, mb, mc, p, stream))
+  if ((rc = make_map(&ma, x, tokens, K, ldx, TILE_M))) return rc;
+  if ((rc = make_map(&mb, w, N, K, ldw, NT / 2))) return rc;
+#define GO(EPI) (out_f32 ? launch_pair<float, EPI>(ma, mb, p, stream) : launch_pair<__nv_bfloat16, EPI>(ma, mb, p, stream))
   if (act) return act == 3 ? GO(EPI_CLAMPED) : GO(EPI_GATED);
   if (unary == 5) return GO(EPI_XIELU);
   return unary ? GO(EPI_ACT) : GO(EPI_PLAIN);
@@ -968,13 +960,12 @@ DINFER_API int dinfer_gemm_tc_grouped(const void* x, int64_t ldx, const void* w,
   p.k_blocks_per_split = (K + BLOCK_K - 1) / BLOCK_K; p.splits = 1;
   p.tile_expert = tile_expert; p.sorted = sorted; p.row_w = epi == 1 ? row_w : nullptr; p.pairs = pairs; p.grp_epi = epi; p.grp_act = act;
   p.act = gate; p.a_pos = gate_a; p.a_neg = gate_b;
-  CUtensorMap ma, mb, mc;
+  CUtensorMap ma, mb;
   int rc;
-  if ((rc = make_map(&ma, w, (int64_t)E * N, K, K, TILE_M))) return rc;
-  if ((rc = make_map(&mb, x, cap, K, ldx, NT / 2))) return rc;
-  if ((rc = make_map(&mc, x, cap, K, ldx, X_BOX))) return rc;
-  if (gate) return gate == 3 ? launch_pair<__nv_bfloat16, EPI_CLAMPED>(ma, mb, mc, p, stream) : launch_pair<__nv_bfloat16, EPI_GATED>(ma, mb, mc, p, stream);
-  return act ? launch_pair<__nv_bfloat16, EPI_ACT>(ma, mb, mc, p, stream) : launch_pair<__nv_bfloat16, EPI_PLAIN>(ma, mb, mc, p, stream);
+  if ((rc = make_map(&ma, x, cap, K, ldx, TILE_M))) return rc;
+  if ((rc = make_map(&mb, w, (int64_t)E * N, K, K, NT / 2))) return rc;
+  if (gate) return gate == 3 ? launch_pair<__nv_bfloat16, EPI_CLAMPED>(ma, mb, p, stream) : launch_pair<__nv_bfloat16, EPI_GATED>(ma, mb, p, stream);
+  return act ? launch_pair<__nv_bfloat16, EPI_ACT>(ma, mb, p, stream) : launch_pair<__nv_bfloat16, EPI_PLAIN>(ma, mb, p, stream);
 }
 
 DINFER_API int dinfer_gemm_tc(const void* x, int64_t ldx, const void* w, int64_t ldw, void* out, int64_t ldc,
