@@ -34,7 +34,7 @@ namespace {
 constexpr int THREADS = 256;
 constexpr int CP = 64;           // tokens per chunk
 constexpr int TP = 64;           // tile edge: state channels x value columns (sums), tokens x value columns (outputs)
-constexpr int KT = 16;           // state channels per pass of the outputs kernel
+constexpr int KT = 32;           // state channels per pass of the outputs kernel
 constexpr int LDT = TP + 4;      // row stride of the transposed tiles (rows stay 16-byte aligned)
 
 struct Params {
@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(PREP_THREADS) ssm_prep_kernel(const Params p) 
   }
   int start = p.cu[b], end = p.cu[b + 1];
   if constexpr (TAPS > 0) {
-    // the whole run belongs to one request: its inputs come eight at a time, all asked for before the first is used
+    // the whole run belongs to one request: its inputs come eight at a time, all asked for before the first is used (2047
+    // tokens of 6144 channels 37 us one at a time, 31 so)
     if (t1 - t0 == PREP_TOKENS && t0 >= start && t1 <= end && end - start > 1) {
       const float* x = p.P + (int64_t)t0 * p.ldp + inner + c;
 #pragma unroll
@@ -343,11 +344,10 @@ __device__ __forceinline__ float4 get4(const float* p) { return *reinterpret_cas
 __device__ __forceinline__ void put4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
 
 // grid (chunks, H * tiles + G, B): a (64 RN) x 64 tile of U for one (chunk, head), or the scores C_t . B_s of one (chunk,
-// group).  RN = 2 where the state has more than 64 channels: a thread's 8 x 8 elements then take four 16-byte reads of shared
-// memory a token for 64 multiply-adds, 4 x 4 two for 16.  Bound by those reads (a warp's takes four passes) and by what
-// surrounds them in a block of some us, which four blocks to an SM hide: 2047 tokens of 64 heads of 128 x 64 @@A@@ us, with
-// 8 x 4 elements 75, with 64 x 64 tiles of 4 x 4 87.
-constexpr int SUMS_THREADS = 128;
+// group).  RN = 2 where the state has more than 64 channels: a thread's 8 x 4 elements then take three 16-byte reads of shared
+// memory a token for 32 multiply-adds, 4 x 4 two for 16.  Bound by those multiply-adds (72 TFLOP/s) and by what surrounds them
+// in a block of 2 us, which three blocks to an SM hide: 2047 tokens of 64 heads of 128 x 64 75 us, with 64 x 64 tiles 87.
+// (8 x 8 elements, 128 threads: 74.)
 template <int RN> struct SumsTiles {
   static constexpr int W = TP * RN;                                            // channels of a tile
   static constexpr int A = CP * (W > LDT ? W : LDT), B = CP * (RN > 1 ? TP : LDT);   // floats; the scores' rows are LDT long
@@ -355,7 +355,7 @@ template <int RN> struct SumsTiles {
   static constexpr size_t BYTES = (A + B) * sizeof(float) + CP * (sizeof(double) + sizeof(float));
 };
 template <bool VEC, int RN>
-__global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params p) {
+__global__ void __launch_bounds__(THREADS, RN > 1 ? 3 : 0) ssm_sums_kernel(const Params p) {
   constexpr int W = SumsTiles<RN>::W;
   extern __shared__ __align__(16) float sums_sm[];
   double* cum = reinterpret_cast<double*>(sums_sm + SumsTiles<RN>::A + SumsTiles<RN>::B);
@@ -368,48 +368,46 @@ __global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params 
   if (t_end - t_begin <= 1 || t0 >= t_end) return;
   const int n = min(CP, t_end - t0), ch = p.channels(), inner = p.inner();
   const int64_t slot = chunk_slot(t_begin, b, c);
-  const int ty = tid >> 3, tx = tid & 7;
-  const int ls = tid >> 4, le = (tid & 15) * 4;    // this thread's place in a tile it loads: rows ls + 8 k, columns le ..
+  const int ty = tid >> 4, tx = tid & 15;
+  const int ls = tid >> 4, le = (tid & 15) * 4;    // this thread's place in a tile it loads: rows ls + 16 k, columns le ..
   const int job = (int)blockIdx.y - p.H * tiles_n * tiles_v;
   if (job >= 0) {
-    // ---- scores of group `job`: rows t = 4 ty + i, columns s = tx + 8 j (neighbouring lanes read neighbouring rows)
+    // ---- scores of group `job`: rows t = 4 ty + i, columns s = tx + 16 j (neighbouring lanes read neighbouring rows)
     float (*a_s)[LDT] = reinterpret_cast<float (*)[LDT]>(sums_sm);             // [token][state channel] of B
     float (*b_s)[LDT] = reinterpret_cast<float (*)[LDT]>(sums_sm + CP * LDT);  // [token][state channel] of C
     const float* Bp = p.xbc + (int64_t)t0 * ch + inner + job * p.N;
     const float* Cp = Bp + p.G * p.N;
-    float acc[4][8] = {};
+    float acc[4][4] = {};
     for (int e0 = 0; e0 < p.N; e0 += CP) {
       __syncthreads();
 #pragma unroll
-      for (int k = 0; k < CP / 8; ++k) {
-        const int s = ls + 8 * k, left = s < n ? p.N - e0 - le : 0;
+      for (int k = 0; k < CP / 16; ++k) {
+        const int s = ls + 16 * k, left = s < n ? p.N - e0 - le : 0;
         put4(&a_s[s][le], load4<VEC>(Bp + (int64_t)s * ch + e0 + le, left));
         put4(&b_s[s][le], load4<VEC>(Cp + (int64_t)s * ch + e0 + le, left));
       }
       __syncthreads();
       const int ne = min(CP, p.N - e0);
       for (int e = 0; e < ne; e += 4) {
-        float4 q[4];
+        float4 q[4], k4[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) q[i] = get4(&b_s[ty * 4 + i][e]);
+        for (int i = 0; i < 4; ++i) { q[i] = get4(&b_s[ty * 4 + i][e]); k4[i] = get4(&a_s[tx + 16 * i][e]); }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float4 k4 = get4(&a_s[tx + 8 * j][e]);
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            acc[i][j] = fmaf(q[i].x, k4.x, acc[i][j]);
-            acc[i][j] = fmaf(q[i].y, k4.y, acc[i][j]);
-            acc[i][j] = fmaf(q[i].z, k4.z, acc[i][j]);
-            acc[i][j] = fmaf(q[i].w, k4.w, acc[i][j]);
+          for (int j = 0; j < 4; ++j) {
+            acc[i][j] = fmaf(q[i].x, k4[j].x, acc[i][j]);
+            acc[i][j] = fmaf(q[i].y, k4[j].y, acc[i][j]);
+            acc[i][j] = fmaf(q[i].z, k4[j].z, acc[i][j]);
+            acc[i][j] = fmaf(q[i].w, k4[j].w, acc[i][j]);
           }
-        }
       }
     }
     float* out = p.cb + (slot * p.G + job) * (int64_t)CP * CP;      // [t][s]
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) out[(ty * 4 + i) * CP + tx + 8 * j] = acc[i][j];
+      for (int j = 0; j < 4; ++j) out[(ty * 4 + i) * CP + tx + 16 * j] = acc[i][j];
     return;
   }
   float (*a_s)[W] = reinterpret_cast<float (*)[W]>(sums_sm);                                  // [token][state channel] of B
@@ -417,20 +415,20 @@ __global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params 
   const int h = blockIdx.y / (tiles_n * tiles_v), tile = blockIdx.y % (tiles_n * tiles_v);
   const int e0 = (tile / tiles_v) * W, c0 = (tile % tiles_v) * TP;
   const int g = h / (p.H / p.G);
-  float4 xv[CP / 8];
+  float4 xv[CP / 16];
   {
     const float* r = p.xbc + (int64_t)t0 * ch;
 #pragma unroll
-    for (int k = 0; k < CP / 8; ++k) {
-      const int s = ls + 8 * k;
+    for (int k = 0; k < CP / 16; ++k) {
+      const int s = ls + 16 * k;
       xv[k] = load4<VEC>(r + (int64_t)s * ch + h * p.Pd + c0 + le, s < n ? p.Pd - c0 - le : 0);
     }
     if (tid < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
 #pragma unroll
     for (int u = 0; u < RN; ++u)
 #pragma unroll
-      for (int k = 0; k < CP / 8; ++k) {
-        const int s = ls + 8 * k, e = 64 * u + le;
+      for (int k = 0; k < CP / 16; ++k) {
+        const int s = ls + 16 * k, e = 64 * u + le;
         put4(&a_s[s][e], load4<VEC>(r + (int64_t)s * ch + inner + g * p.N + e0 + e, s < n ? p.N - e0 - e : 0));
       }
   }
@@ -439,16 +437,16 @@ __global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params 
   if (tile == 0 && tid == 0) p.decay[slot * p.H + h] = (float)exp(cum[n - 1]);
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < CP / 8; ++k) {
-    const float w = wgt[ls + 8 * k];
-    put4(&b_s[ls + 8 * k][le], make_float4(xv[k].x * w, xv[k].y * w, xv[k].z * w, xv[k].w * w));
+  for (int k = 0; k < CP / 16; ++k) {
+    const float w = wgt[ls + 16 * k];
+    put4(&b_s[ls + 16 * k][le], make_float4(xv[k].x * w, xv[k].y * w, xv[k].z * w, xv[k].w * w));
   }
   __syncthreads();
-  float acc[RN][4][8] = {};
+  float acc[RN][4][4] = {};
 #pragma unroll 4
   for (int s = 0; s < n; ++s) {
-    const float4 lo = get4(&b_s[s][tx * 4]), hi = get4(&b_s[s][32 + tx * 4]);
-    const float wv[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    const float4 w = get4(&b_s[s][tx * 4]);
+    const float wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int u = 0; u < RN; ++u) {
       const float4 a = get4(&a_s[s][64 * u + ty * 4]);
@@ -456,7 +454,7 @@ __global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params 
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[u][i][j] = fmaf(av[i], wv[j], acc[u][i][j]);
+        for (int j = 0; j < 4; ++j) acc[u][i][j] = fmaf(av[i], wv[j], acc[u][i][j]);
     }
   }
   float* U = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd;
@@ -464,14 +462,8 @@ __global__ void __launch_bounds__(SUMS_THREADS, 4) ssm_sums_kernel(const Params 
   for (int u = 0; u < RN; ++u)
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int e = e0 + 64 * u + ty * 4 + i;
-      if (e >= p.N) continue;
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int x = c0 + 32 * v + tx * 4;
-        const float o[4] = {acc[u][i][4 * v], acc[u][i][4 * v + 1], acc[u][i][4 * v + 2], acc[u][i][4 * v + 3]};
-        store4<VEC>(U + (int64_t)e * p.Pd + x, p.Pd - x, o);
-      }
+      const int e = e0 + 64 * u + ty * 4 + i, x = c0 + tx * 4;
+      if (e < p.N) store4<VEC>(U + (int64_t)e * p.Pd + x, p.Pd - x, acc[u][i]);
     }
 }
 
@@ -519,137 +511,121 @@ __global__ void __launch_bounds__(THREADS) ssm_scan_kernel(const Params p) {
   stv<V>(S_g, S);
 }
 
-// y for one chunk and HEADS neighbours among a group's (head, 64 value columns), which share C; grid (chunks, runs of HEADS of
-// them, B).  The passes over the state's channels load the next pass's tiles into registers while they compute.  64 threads
-// have a head's 64 x 64 values, 8 x 8 each: rows 32 w + (0 .. 3) + 4 i of the head's warp w (a warp can then leave out the
-// tokens behind its last one), columns 4 x and 32 + 4 x.  Bound by the reads of shared memory that feed the multiply-adds (a
-// 16-byte read of a warp takes four passes, and 8 x 8 elements need 16 of them for 256 multiply-adds): 2047 tokens of 64 heads
-// of 128 x 64 @@B@@ us; with 8 x 4 elements and one head a block 112, with 4 x 4 109.
-template <int HEADS> struct OutTiles {
-  static constexpr int THREADS = 64 * HEADS, LDC = KT + 4;
-  static constexpr int PASS = CP * LDC + HEADS * KT * TP, A = HEADS * CP * LDT;    // floats: a pass's tiles, later A
-  static constexpr int X = PASS > A ? PASS : A;
-  static constexpr size_t BYTES = (X + HEADS * CP * TP) * sizeof(float) + HEADS * CP * (sizeof(double) + sizeof(float));
-};
-template <bool VEC, int HEADS>
-__global__ void __launch_bounds__(OutTiles<HEADS>::THREADS, HEADS == 2 ? 3 : 6) ssm_outputs_kernel(const Params p) {
-  using O = OutTiles<HEADS>;
-  constexpr int R = 8, NT = O::THREADS, CV = CP * KT / 4 / NT, SV = KT * TP / 4 / 64;
-  extern __shared__ __align__(16) float outs_sm[];
-  float (*C_s)[O::LDC] = reinterpret_cast<float (*)[O::LDC]>(outs_sm);            // [token][state channel]
-  double* cum_all = reinterpret_cast<double*>(outs_sm + O::X + HEADS * CP * TP);
-  float* dts_all = reinterpret_cast<float*>(cum_all + HEADS * CP);
+// y for one (chunk, head, 64 value columns); grid (chunks, H * column tiles, B).  The passes over the state's channels load
+// the next pass's tiles into registers while they compute.
+template <bool VEC>
+__global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p) {
+  constexpr int LDC = KT + 4;
+  __shared__ __align__(16) float tiles[CP * LDT];
+  static_assert(CP * LDC + KT * TP <= CP * LDT, "a pass's tiles fit where A lies afterwards");
+  float (*C_s)[LDC] = reinterpret_cast<float (*)[LDC]>(tiles);                   // [token][state channel]
+  float (*S_s)[TP] = reinterpret_cast<float (*)[TP]>(tiles + CP * LDC);          // [state channel][value column]
+  float (*A_s)[LDT] = reinterpret_cast<float (*)[LDT]>(tiles);                   // [token t][token s], after the passes
+  __shared__ __align__(16) float x_s[CP][TP];      // [token s][value column]
+  __shared__ double cum[CP];
+  __shared__ float dts[CP];
   pdl_enter();
-  const int tiles_v = (p.Pd + TP - 1) / TP, per_group = p.H / p.G * tiles_v, runs = (per_group + HEADS - 1) / HEADS;
-  const int b = blockIdx.z, c = blockIdx.x, g = blockIdx.y / runs;
+  const int tiles_v = (p.Pd + TP - 1) / TP;
+  const int b = blockIdx.z, c = blockIdx.x, h = blockIdx.y / tiles_v, c0 = (blockIdx.y % tiles_v) * TP;
   const int t_begin = p.cu[b], t_end = p.cu[b + 1];
   const int t0 = t_begin + c * CP;
   if (t_end - t_begin <= 1 || t0 >= t_end) return;
-  const int tid = threadIdx.x, lane = tid & 31, half = tid >> 6, mine = tid & 63;   // this thread's head among the HEADS
-  const int job = g * per_group + blockIdx.y % runs * HEADS + half;                 // (launched only where runs divide the group)
-  const int h = job / tiles_v, c0 = job % tiles_v * TP;
-  const int n = min(CP, t_end - t0), ch = p.channels(), inner = p.inner();
-  float (*S_s)[TP] = reinterpret_cast<float (*)[TP]>(outs_sm + CP * O::LDC + half * KT * TP);   // [state channel][value column]
-  float (*A_s)[LDT] = reinterpret_cast<float (*)[LDT]>(outs_sm + half * CP * LDT);              // [token t][token s], after the passes
-  float (*x_s)[TP] = reinterpret_cast<float (*)[TP]>(outs_sm + O::X + half * CP * TP);          // [token s][value column]
-  double* cum = cum_all + half * CP;
-  float* dts = dts_all + half * CP;
-  const int row0 = (mine >> 5) * 32 + (lane >> 3), x0 = (lane & 7) * 4;
+  const int n = min(CP, t_end - t0), tid = threadIdx.x, ch = p.channels(), inner = p.inner();
+  const int ty = tid >> 4, tx = tid & 15, g = h / (p.H / p.G);
   const int64_t slot = chunk_slot(t_begin, b, c);
   const float* S_prev = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd + c0;
   const float* Cp = p.xbc + (int64_t)t0 * ch + inner + (p.G + g) * p.N;
-  // what this thread loads of a pass: C rows ct + CR k at channels ce .., its head's S rows (channels) sr + 4 k at columns sx ..
-  constexpr int CR = NT / (KT / 4);
-  const int ct = tid / (KT / 4), ce = tid % (KT / 4) * 4, sr = mine >> 4, sx = (mine & 15) * 4;
-  float4 cv[CV], sv[SV];
+  // what this thread loads of a pass: C rows ct + 32 k at channels ce .., S rows (channels) sr + 16 k at columns sx ..
+  const int ct = tid >> 3, ce = (tid & 7) * 4, sr = tid >> 4, sx = (tid & 15) * 4;
+  float4 cv[CP / 32], sv[KT / 16];
   auto fetch = [&](int e0) {
 #pragma unroll
-    for (int k = 0; k < CV; ++k) {
-      const int t = ct + CR * k;
-      cv[k] = load4<VEC>(Cp + (int64_t)t * ch + e0 + ce, t < n ? p.N - e0 - ce : 0);
-    }
+    for (int k = 0; k < CP / 32; ++k)
+      cv[k] = load4<VEC>(Cp + (int64_t)(ct + 32 * k) * ch + e0 + ce, ct + 32 * k < n ? p.N - e0 - ce : 0);
 #pragma unroll
-    for (int k = 0; k < SV; ++k)
-      sv[k] = load4<VEC>(S_prev + (int64_t)(e0 + sr + 4 * k) * p.Pd + sx, e0 + sr + 4 * k < p.N ? p.Pd - c0 - sx : 0);
+    for (int k = 0; k < KT / 16; ++k)
+      sv[k] = load4<VEC>(S_prev + (int64_t)(e0 + sr + 16 * k) * p.Pd + sx, e0 + sr + 16 * k < p.N ? p.Pd - c0 - sx : 0);
   };
   fetch(0);
 #pragma unroll
-  for (int k = 0; k < CP / 4; ++k) {
-    const int s = sr + 4 * k;
+  for (int k = 0; k < CP / 16; ++k) {
+    const int s = sr + 16 * k;
     put4(&x_s[s][sx], load4<VEC>(p.xbc + (int64_t)(t0 + s) * ch + h * p.Pd + c0 + sx, s < n ? p.Pd - c0 - sx : 0));
   }
-  if (mine < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
-  dts[mine] = mine < n ? p.dt[(int64_t)(t0 + mine) * p.H + h] : 0.f;
-  float r[R][8] = {};
-  // r += rows of a [.][k] (stride lda) times columns of b [k][TP], four k
-  auto step = [&](const float* a, int lda, const float (*bt)[TP]) {
-    float4 q[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) q[i] = get4(a + 4 * i * lda);
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float4 lo = get4(&bt[u][x0]), hi = get4(&bt[u][32 + x0]);
-      const float w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) r[i][j] = fmaf(qv, w[j], r[i][j]);
-      }
-    }
-  };
+  if (tid < 32) chunk_log_decay(p.la + (int64_t)t0 * p.H + h, p.H, n, cum);
+  if (tid < CP) dts[tid] = tid < n ? p.dt[(int64_t)(t0 + tid) * p.H + h] : 0.f;
+  float r[4][4] = {};
   for (int e0 = 0; e0 < p.N; e0 += KT) {
     __syncthreads();                               // the last pass is done with the tiles
 #pragma unroll
-    for (int k = 0; k < CV; ++k) put4(&C_s[ct + CR * k][ce], cv[k]);
+    for (int k = 0; k < CP / 32; ++k) put4(&C_s[ct + 32 * k][ce], cv[k]);
 #pragma unroll
-    for (int k = 0; k < SV; ++k) put4(&S_s[sr + 4 * k][sx], sv[k]);
+    for (int k = 0; k < KT / 16; ++k) put4(&S_s[sr + 16 * k][sx], sv[k]);
     __syncthreads();
     if (e0 + KT < p.N) fetch(e0 + KT);
-#pragma unroll 1
-    for (int e = 0; e < KT; e += 4) step(&C_s[row0][e], O::LDC, &S_s[e]);
+#pragma unroll 2
+    for (int e = 0; e < KT; e += 4) {
+      float4 q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = get4(&C_s[ty * 4 + i][e]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 s4 = get4(&S_s[e + u][tx * 4]);
+        const float sw[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) r[i][j] = fmaf(qv, sw[j], r[i][j]);
+        }
+      }
+    }
   }
   __syncthreads();
   // A[t][s] = (C_t . B_s) exp(c_t - c_s) dt_s for s <= t; r <- exp(c_t) r, which the sums over s then join
   const float* cb = p.cb + (slot * p.G + g) * (int64_t)CP * CP;
-  {
-    const int s0 = (lane & 15) * 4;
-#pragma unroll 4
-    for (int t = (mine >> 4); t < CP; t += 4) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (s0 <= t) v = get4(cb + t * CP + s0);
-      const float vv[4] = {v.x, v.y, v.z, v.w};
-      float a[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int s = s0 + j;
-        a[j] = (s <= t && t < n) ? vv[j] * expf((float)(cum[t] - cum[s])) * dts[s] : 0.f;
-      }
-      put4(&A_s[t][s0], make_float4(a[0], a[1], a[2], a[3]));
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty * 4 + i;
+    const float4 v = get4(cb + t * CP + tx * 4);
+    const float vv[4] = {v.x, v.y, v.z, v.w};
+    float a[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int s = tx * 4 + j;
+      a[j] = (s <= t && t < n) ? vv[j] * expf((float)(cum[t] - cum[s])) * dts[s] : 0.f;
     }
-  }
+    put4(&A_s[t][tx * 4], make_float4(a[0], a[1], a[2], a[3]));
+    const float d = expf((float)cum[t]);
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const float d = expf((float)cum[row0 + 4 * i]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) r[i][j] *= d;
+    for (int j = 0; j < 4; ++j) r[i][j] *= d;
   }
   __syncthreads();
-  const int last = min((mine >> 5) * 32 + 31, n - 1);   // (A is zero beyond t, x_s beyond the chunk's tokens)
-#pragma unroll 1
-  for (int s = 0; s <= last; s += 4) step(&A_s[row0][s], LDT, &x_s[s]);
+  const int last = min(ty * 4 + 3, n - 1);         // (A is zero beyond t, x_s beyond the chunk's tokens)
+  for (int s = 0; s <= last; s += 4) {
+    float4 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = get4(&A_s[ty * 4 + i][s]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 x4 = get4(&x_s[s + u][tx * 4]);
+      const float xw[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[i][j] = fmaf(qv, xw[j], r[i][j]);
+      }
+    }
+  }
   const float D = p.D[h];
 #pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const int t = row0 + 4 * i;
+  for (int i = 0; i < 4; ++i) {
+    const int t = ty * 4 + i;
     if (t >= n) continue;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int x = 32 * u + x0;
-      const float4 x4 = get4(&x_s[t][x]);
-      const float o[4] = {fmaf(D, x4.x, r[i][4 * u]), fmaf(D, x4.y, r[i][4 * u + 1]), fmaf(D, x4.z, r[i][4 * u + 2]), fmaf(D, x4.w, r[i][4 * u + 3])};
-      store4<VEC>(p.y + (int64_t)(t0 + t) * inner + (int64_t)h * p.Pd + c0 + x, p.Pd - c0 - x, o);
-    }
+    const float4 x4 = get4(&x_s[t][tx * 4]);
+    const float o[4] = {fmaf(D, x4.x, r[i][0]), fmaf(D, x4.y, r[i][1]), fmaf(D, x4.z, r[i][2]), fmaf(D, x4.w, r[i][3])};
+    store4<VEC>(p.y + (int64_t)(t0 + t) * inner + (int64_t)h * p.Pd + c0 + tx * 4, p.Pd - c0 - tx * 4, o);
   }
 }
 
@@ -782,17 +758,7 @@ int launch_sums(const Params& p, int chunks, cudaStream_t stream) {
   const cudaError_t e = cudaFuncSetAttribute(ssm_sums_kernel<VEC, RN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return refuse((int)e, "state_space: shared memory opt-in failed: %s", cudaGetErrorString(e));
   const int tiles = (p.N + SumsTiles<RN>::W - 1) / SumsTiles<RN>::W * ((p.Pd + TP - 1) / TP);
-  launch_pdl(ssm_sums_kernel<VEC, RN>, dim3(chunks, p.H * tiles + p.G, p.B), dim3(SUMS_THREADS), smem, stream, p);
-  return 0;
-}
-
-template <bool VEC, int HEADS>
-int launch_outputs(const Params& p, int chunks, cudaStream_t stream) {
-  constexpr size_t smem = OutTiles<HEADS>::BYTES;
-  const cudaError_t e = cudaFuncSetAttribute(ssm_outputs_kernel<VEC, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return refuse((int)e, "state_space: shared memory opt-in failed: %s", cudaGetErrorString(e));
-  const int jobs = p.H * ((p.Pd + TP - 1) / TP);
-  launch_pdl(ssm_outputs_kernel<VEC, HEADS>, dim3(chunks, jobs / HEADS, p.B), dim3(OutTiles<HEADS>::THREADS), smem, stream, p);
+  launch_pdl(ssm_sums_kernel<VEC, RN>, dim3(chunks, p.H * tiles + p.G, p.B), dim3(THREADS), smem, stream, p);
   return 0;
 }
 
@@ -861,10 +827,7 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
     if (rc) return rc;
     if (state_vec) launch_pdl(ssm_scan_kernel<4>, dim3((unsigned)((size / 4 + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
     else launch_pdl(ssm_scan_kernel<1>, dim3((unsigned)((size + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
-    // two neighbours to a block where a group's can be dealt out in twos
-    const int rc2 = H / G * tiles_v % 2 == 0 ? (vec ? launch_outputs<true, 2>(p, chunks, stream) : launch_outputs<false, 2>(p, chunks, stream))
-                                             : (vec ? launch_outputs<true, 1>(p, chunks, stream) : launch_outputs<false, 1>(p, chunks, stream));
-    if (rc2) return rc2;
+    launch_pdl(vec ? ssm_outputs_kernel<true> : ssm_outputs_kernel<false>, dim3(chunks, H * tiles_v, B), dim3(THREADS), 0, stream, p);
   }
   return cuda_status("state_space");
 }
