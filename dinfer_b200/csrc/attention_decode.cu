@@ -548,7 +548,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int c) {
 // SORT: the longest requests start first (a variant of its own: the switch at run time cost a step of eight requests 0.6 %)
 // RAW: the q/k kernel's work is done here, one launch less a layer (a layer of a decode step has seven short ones in a row; 2.2
 // us each): every CTA norms and turns its own q heads on their way to the operand, and the CTA that visits the newest tile
-// puts the token's key and value into that tile (fetched ahead of the wait, like all) and into the cache.  @@R@@
+// writes the token's key and value to their page ahead of that tile's copies.  @@R@@
 template <int D, int NH8, bool CAP, bool SORT, bool RAW>
 __global__ void __launch_bounds__(NT_TMA, 2)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
@@ -558,7 +558,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
   extern __shared__ __align__(128) unsigned char smem_raw[];   // aligned to 1024 by hand below
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ int s_table[TABLE_SLOTS];
-  __shared__ __align__(8) uint64_t new_bar;                   // RAW: the newest token is in its tile
   __shared__ int s_abort;
   __shared__ __align__(16) __nv_bfloat16 s_q[RAW ? 8 : 1][RAW ? D + 8 : 8];
   static_assert(!RAW || (D == 128 && NH8 == 1 && !CAP), "RAW");
@@ -573,7 +572,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
   // first phase of the cluster barrier: this CTA runs, its shared memory may be written by the others
   if (p.splits > 1) cluster_arrive_relaxed();
   const int seq_len = p.seq_lens[b];
-  const int position = RAW ? p.positions[t0] : 0;
   const int pos = seq_len - 1;
   const int lo = first_key(pos, p.window, p.chunked), hi = seq_len;
   const int* table = p.block_table + (int64_t)b * p.max_blocks;
@@ -596,7 +594,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
     for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 4); }
-    if (RAW) mbar_init(smem_u32(&new_bar), 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -623,7 +620,29 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
     for (int t = 0; t < n_tiles && alive; ++t) {
       const int s = t % STAGES;
       const int j0 = tile_of(v0 + t, kept, tile_first) * BN;
-      if (!RAW && !waited && j0 + BN > pos) { pdl_wait(); waited = true; }        // the newest token's page
+      if (!waited && j0 + BN > pos) {                                     // the newest token's page
+        if constexpr (RAW) {
+          // lanes 0-15 its key, 16-31 its value
+          const int l = lane & 15, slot = p.slots[t0];
+          const RawHead head(p, p.k_weight, p.positions[t0], l);
+          pdl_wait();
+          const __nv_bfloat16* row = p.q + (int64_t)t0 * p.ldq + (int64_t)(p.H + (lane < 16 ? 0 : p.Hkv) + hk) * D + 4 * l;
+          uint2 x = *reinterpret_cast<const uint2*>(row), y = *reinterpret_cast<const uint2*>(row + D / 2);
+          head.apply(p, x, y, lane < 16);
+          if (slot >= 0) {
+            __nv_bfloat16* dst = p.cache_new + ((((int64_t)(slot >> p.bs_log2) * 2 + (lane >> 4)) * p.Hkv + hk) * p.block_size +
+                                                (slot & (p.block_size - 1))) * D + 4 * l;
+            *reinterpret_cast<uint2*>(dst) = x;
+            *reinterpret_cast<uint2*>(dst + D / 2) = y;
+          }
+          __threadfence();
+          asm volatile("fence.proxy.async;" ::: "memory");                // the copies below read it through the other proxy
+          __syncwarp();
+        } else {
+          pdl_wait();
+        }
+        waited = true;
+      }
       bool ok = true;
       if (lane == 0) ok = mbar_wait(smem_u32(&empty_bar[s]), ((t / STAGES) & 1) ^ 1);
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -662,35 +681,11 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
         if (valid[u]) tma_load_2d(dst[u], &map_kv, col[u], row[u], bar);
     }
     if (!waited) pdl_wait();
-    if constexpr (RAW) {
-      // The newest token's row (lanes 0-15 its key, 16-31 its value) takes its place in the last tile, which was fetched ahead
-      // of the wait like the others, and in the cache.
-      const int slot = p.slots[t0];
-      if (alive && n_tiles > 0 && v0 + n_tiles == visits) {
-        const int l = lane & 15, t = n_tiles - 1, r = pos - tile_of(v0 + t, kept, tile_first) * BN;
-        const RawHead head(p, p.k_weight, position, l);
-        const __nv_bfloat16* row = p.q + (int64_t)t0 * p.ldq + (int64_t)(p.H + (lane < 16 ? 0 : p.Hkv) + hk) * D + 4 * l;
-        uint2 x = *reinterpret_cast<const uint2*>(row), y = *reinterpret_cast<const uint2*>(row + D / 2);
-        head.apply(p, x, y, lane < 16);
-        if (!mbar_wait(smem_u32(&full_bar[t % STAGES]), (t / STAGES) & 1)) { s_abort = 1; if (lane == 0) atomicExch(p.status, 22); }
-        else if (slot >= 0) {
-          unsigned char* tile = gbase + (t % STAGES) * 2 * KV_BYTES + (lane >> 4) * KV_BYTES + (l & 1) * 8;
-          *reinterpret_cast<uint2*>(tile + sw128(r, l >> 1)) = x;
-          *reinterpret_cast<uint2*>(tile + sw128(r, 8 + (l >> 1))) = y;
-          __nv_bfloat16* dst = p.cache_new + ((((int64_t)(slot >> p.bs_log2) * 2 + (lane >> 4)) * p.Hkv + hk) * p.block_size +
-                                              (slot & (p.block_size - 1))) * D + 4 * l;
-          *reinterpret_cast<uint2*>(dst) = x;
-          *reinterpret_cast<uint2*>(dst + D / 2) = y;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&new_bar));
-      }
-    }
   } else {                                                    // ---- four compute warps, 16 keys of every tile each
     unsigned qb[D / 16][NH8][2];
     if constexpr (RAW) {
       const int l = lane & 15, mine = warp * 2 + (lane >> 4);  // a head to 16 lanes
-      const RawHead head(p, p.q_weight, position, l);
+      const RawHead head(p, p.q_weight, p.positions[t0], l);
       pdl_wait();                                             // q comes from the kernel before this one
       uint2 x = make_uint2(0u, 0u), y = x;
       if (mine < p.group) {
@@ -732,8 +727,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
     bool ok = true;
     for (int t = 0; t < n_tiles && ok; ++t) {
       const int s = t % STAGES;
-      if (!mbar_wait(smem_u32(&full_bar[s]), (t / STAGES) & 1) ||
-          (RAW && v0 + t + 1 == visits && !mbar_wait(smem_u32(&new_bar), 0))) { s_abort = 1; atomicExch(p.status, 22); ok = false; break; }
+      if (!mbar_wait(smem_u32(&full_bar[s]), (t / STAGES) & 1)) { s_abort = 1; atomicExch(p.status, 22); ok = false; break; }
       const unsigned char* kt = gbase + s * 2 * KV_BYTES;
       const unsigned char* vt = kt + KV_BYTES;
       const int jbase = tile_of(v0 + t, kept, tile_first) * BN + key_off;
