@@ -49,85 +49,6 @@ struct Params {
   float* part_ml;    // [B, H, splits, 2]
   int* counters;     // [B, Hkv]
   int* status;       // device status word of the TMA variant (bounded waits)
-  // RAW: q is the first of the rows [q | k | v] as the projection left them; see the TMA variant
-  const int* positions; const int* slots;
-  const void *q_weight, *k_weight; int weights_f32;
-  float eps;
-  const float* cos_sin;
-  __nv_bfloat16* cache_new;
-};
-
-// RAW: the norms and the rotation of one head of 128, 16 lanes a head (lane l: elements 4 l .. and 64 + 4 l ..), to the bit
-// what the q/k kernel (qk_post.cu) makes of it.  The weights and the angles are fetched while the kernel in front may run.
-struct RawHead {
-  float w[2][4], c[4], s[4];
-  bool norm, turn;
-  __device__ __forceinline__ RawHead(const Params& p, const void* weight, int position, int l) {
-    norm = weight != nullptr;
-    turn = p.cos_sin != nullptr;
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[u][j] = 1.f;
-    if (norm && p.weights_f32) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const float4 x = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(weight) + 64 * u + 4 * l);
-        w[u][0] = x.x; w[u][1] = x.y; w[u][2] = x.z; w[u][3] = x.w;
-      }
-    } else if (norm) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) unpack(*reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(weight) + 64 * u + 4 * l), w[u]);
-    }
-    float4 cc = make_float4(1.f, 1.f, 1.f, 1.f), ss = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (turn) {
-      cc = *reinterpret_cast<const float4*>(p.cos_sin + (int64_t)position * 128 + 4 * l);
-      ss = *reinterpret_cast<const float4*>(p.cos_sin + (int64_t)position * 128 + 64 + 4 * l);
-    }
-    c[0] = cc.x; c[1] = cc.y; c[2] = cc.z; c[3] = cc.w;
-    s[0] = ss.x; s[1] = ss.y; s[2] = ss.z; s[3] = ss.w;
-  }
-  static __device__ __forceinline__ void unpack(uint2 x, float (&v)[4]) {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&x);
-    const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-  }
-  static __device__ __forceinline__ uint2 pack(const float (&v)[4]) {
-    uint2 x;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&x);
-    h[0] = __floats2bfloat162_rn(v[0], v[1]);
-    h[1] = __floats2bfloat162_rn(v[2], v[3]);
-    return x;
-  }
-  // a whole warp; lanes with `live` false keep what they hold
-  __device__ __forceinline__ void apply(const Params& p, uint2& lo, uint2& hi, bool live) const {
-    float a[4], b[4], ss = 0.f;
-    unpack(lo, a);
-    unpack(hi, b);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) ss += a[j] * a[j] + b[j] * b[j];
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (!live) return;
-    if (norm) {
-      const float rinv = rsqrtf(ss / 128.f + p.eps);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        a[j] = a[j] * rinv * w[0][j];
-        b[j] = b[j] * rinv * w[1][j];
-      }
-    }
-    if (turn) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float x = a[j], y = b[j];
-        a[j] = x * c[j] - y * s[j];
-        b[j] = y * c[j] + x * s[j];
-      }
-    }
-    lo = pack(a);
-    hi = pack(b);
-  }
 };
 
 constexpr int BY_LENGTH_MAX = 128;     // requests that a warp ranks
@@ -546,10 +467,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int c) {
 }
 
 // SORT: the longest requests start first (a variant of its own: the switch at run time cost a step of eight requests 0.6 %)
-// RAW: the q/k kernel's work is done here, one launch less a layer (a layer of a decode step has seven short ones in a row; 2.2
-// us each): every CTA norms and turns its own q heads on their way to the operand, and the CTA that visits the newest tile
-// writes the token's key and value to their page ahead of that tile's copies.  @@R@@
-template <int D, int NH8, bool CAP, bool SORT, bool RAW>
+template <int D, int NH8, bool CAP, bool SORT>
 __global__ void __launch_bounds__(NT_TMA, 2)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Params p) {
   constexpr int NHF = D / 64;                                 // 64-wide halves of the head
@@ -559,8 +477,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ int s_table[TABLE_SLOTS];
   __shared__ int s_abort;
-  __shared__ __align__(16) __nv_bfloat16 s_q[RAW ? 8 : 1][RAW ? D + 8 : 8];
-  static_assert(!RAW || (D == 128 && NH8 == 1 && !CAP), "RAW");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;
   const int hk = blockIdx.y, split = blockIdx.x;
@@ -620,29 +536,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
     for (int t = 0; t < n_tiles && alive; ++t) {
       const int s = t % STAGES;
       const int j0 = tile_of(v0 + t, kept, tile_first) * BN;
-      if (!waited && j0 + BN > pos) {                                     // the newest token's page
-        if constexpr (RAW) {
-          // lanes 0-15 its key, 16-31 its value
-          const int l = lane & 15, slot = p.slots[t0];
-          const RawHead head(p, p.k_weight, p.positions[t0], l);
-          pdl_wait();
-          const __nv_bfloat16* row = p.q + (int64_t)t0 * p.ldq + (int64_t)(p.H + (lane < 16 ? 0 : p.Hkv) + hk) * D + 4 * l;
-          uint2 x = *reinterpret_cast<const uint2*>(row), y = *reinterpret_cast<const uint2*>(row + D / 2);
-          head.apply(p, x, y, lane < 16);
-          if (slot >= 0) {
-            __nv_bfloat16* dst = p.cache_new + ((((int64_t)(slot >> p.bs_log2) * 2 + (lane >> 4)) * p.Hkv + hk) * p.block_size +
-                                                (slot & (p.block_size - 1))) * D + 4 * l;
-            *reinterpret_cast<uint2*>(dst) = x;
-            *reinterpret_cast<uint2*>(dst + D / 2) = y;
-          }
-          __threadfence();
-          asm volatile("fence.proxy.async;" ::: "memory");                // the copies below read it through the other proxy
-          __syncwarp();
-        } else {
-          pdl_wait();
-        }
-        waited = true;
-      }
+      if (!waited && j0 + BN > pos) { pdl_wait(); waited = true; }        // the newest token's page
       bool ok = true;
       if (lane == 0) ok = mbar_wait(smem_u32(&empty_bar[s]), ((t / STAGES) & 1) ^ 1);
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -682,37 +576,16 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Pa
     }
     if (!waited) pdl_wait();
   } else {                                                    // ---- four compute warps, 16 keys of every tile each
+    pdl_wait();                                               // q comes from the kernel before this one
     unsigned qb[D / 16][NH8][2];
-    if constexpr (RAW) {
-      const int l = lane & 15, mine = warp * 2 + (lane >> 4);  // a head to 16 lanes
-      const RawHead head(p, p.q_weight, p.positions[t0], l);
-      pdl_wait();                                             // q comes from the kernel before this one
-      uint2 x = make_uint2(0u, 0u), y = x;
-      if (mine < p.group) {
-        const __nv_bfloat16* row = p.q + (int64_t)t0 * p.ldq + (int64_t)(hk * p.group + mine) * D + 4 * l;
-        x = *reinterpret_cast<const uint2*>(row);
-        y = *reinterpret_cast<const uint2*>(row + D / 2);
-      }
-      head.apply(p, x, y, mine < p.group);
-      *reinterpret_cast<uint2*>(&s_q[mine][4 * l]) = x;
-      *reinterpret_cast<uint2*>(&s_q[mine][D / 2 + 4 * l]) = y;
-      asm volatile("bar.sync 1, 128;" ::: "memory");          // the four compute warps
+#pragma unroll
+    for (int nt = 0; nt < NH8; ++nt) {
+      const int head = nt * 8 + g;
+      const __nv_bfloat16* qrow = p.q + (int64_t)t0 * p.ldq + (int64_t)(hk * p.group + head) * D;
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
-        qb[ks][0][0] = *reinterpret_cast<const unsigned*>(&s_q[g][ks * 16 + 2 * tq]);
-        qb[ks][0][1] = *reinterpret_cast<const unsigned*>(&s_q[g][ks * 16 + 8 + 2 * tq]);
-      }
-    } else {
-      pdl_wait();                                             // q comes from the kernel before this one
-#pragma unroll
-      for (int nt = 0; nt < NH8; ++nt) {
-        const int head = nt * 8 + g;
-        const __nv_bfloat16* qrow = p.q + (int64_t)t0 * p.ldq + (int64_t)(hk * p.group + head) * D;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          qb[ks][nt][0] = head < p.group ? *reinterpret_cast<const unsigned*>(qrow + ks * 16 + 2 * tq) : 0u;
-          qb[ks][nt][1] = head < p.group ? *reinterpret_cast<const unsigned*>(qrow + ks * 16 + 8 + 2 * tq) : 0u;
-        }
+        qb[ks][nt][0] = head < p.group ? *reinterpret_cast<const unsigned*>(qrow + ks * 16 + 2 * tq) : 0u;
+        qb[ks][nt][1] = head < p.group ? *reinterpret_cast<const unsigned*>(qrow + ks * 16 + 8 + 2 * tq) : 0u;
       }
     }
     const int key_off = warp * 16;
@@ -910,9 +783,9 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int D, int NH8, bool CAP, bool SORT, bool RAW = false>
+template <int D, int NH8, bool CAP, bool SORT>
 int launch_tma(const CUtensorMap& map, const Params& p, int B, cudaStream_t stream) {
-  auto k = attention_decode_tma_kernel<D, NH8, CAP, SORT, RAW>;
+  auto k = attention_decode_tma_kernel<D, NH8, CAP, SORT>;
   // tiles (the four warps' fold reuses them: it is smaller), then the cluster's receive buffer
   static_assert((size_t)(4 * NH8 * 8 * D + 2 * 4 * NH8 * 8) * sizeof(float) <= (size_t)2 * STAGES * (D / 64) * BN * 128,
                 "the fold of the four warps fits the tiles");
@@ -1043,11 +916,11 @@ DINFER_API int dinfer_attention_decode_tma_sink(const void* q, int64_t ldq, void
                                           B, H, Hkv, D, block_size, scale, window, 0, 0, 0.f, sink, nullptr, nullptr, splits, status, stream);
 }
 
-static int decode_tma(const void* q, int64_t ldq, void* out, int64_t ldo, const void* cache,
+DINFER_API int dinfer_attention_decode_tma_bias(const void* q, int64_t ldq, void* out, int64_t ldo, const void* cache,
                                                 int64_t num_blocks, const int* block_table, int max_blocks,
                                                 const int* cu_seqlens, const int* seq_lens, int B, int H, int Hkv, int D,
                                                 int block_size, float scale, int window, int chunked, int keep_first, float softcap, int sink, const float* sinks, const float* slopes,
-                                                int splits, int* status, const Params* raw, cudaStream_t stream) {
+                                                int splits, int* status, cudaStream_t stream) {
   if (B <= 0 || H <= 0 || Hkv <= 0 || H % Hkv || max_blocks <= 0 || num_blocks <= 0)
     return refuse(DINFER_BAD_ARGUMENT, "attention_decode_tma: bad sizes B=%d H=%d Hkv=%d", B, H, Hkv);
   if (keep_first < 0 || (keep_first > 0 && chunked) || !(softcap >= 0.f))
@@ -1096,47 +969,10 @@ static int decode_tma(const void* q, int64_t ldq, void* out, int64_t ldo, const 
   p.slopes = slopes;
   p.part_o = nullptr; p.part_ml = nullptr; p.counters = nullptr; p.status = status;
   const int nh8 = (p.group + 7) / 8;
-  if (raw) {
-    p.positions = raw->positions; p.slots = raw->slots; p.q_weight = raw->q_weight; p.k_weight = raw->k_weight;
-    p.weights_f32 = raw->weights_f32; p.eps = raw->eps; p.cos_sin = raw->cos_sin;
-    p.cache_new = (__nv_bfloat16*)const_cast<void*>(cache);
-    return sort ? launch_tma<128, 1, false, true, true>(map, p, B, stream) : launch_tma<128, 1, false, false, true>(map, p, B, stream);
-  }
 #define GO(CAP, SORT) (D == 64 ? (nh8 == 1 ? launch_tma<64, 1, CAP, SORT>(map, p, B, stream) : launch_tma<64, 2, CAP, SORT>(map, p, B, stream)) \
                                : (nh8 == 1 ? launch_tma<128, 1, CAP, SORT>(map, p, B, stream) : launch_tma<128, 2, CAP, SORT>(map, p, B, stream)))
   return softcap > 0.f ? (sort ? GO(true, true) : GO(true, false)) : (sort ? GO(false, true) : GO(false, false));
 #undef GO
-}
-
-DINFER_API int dinfer_attention_decode_tma_bias(const void* q, int64_t ldq, void* out, int64_t ldo, const void* cache,
-                                                int64_t num_blocks, const int* block_table, int max_blocks,
-                                                const int* cu_seqlens, const int* seq_lens, int B, int H, int Hkv, int D,
-                                                int block_size, float scale, int window, int chunked, int keep_first, float softcap, int sink, const float* sinks, const float* slopes,
-                                                int splits, int* status, cudaStream_t stream) {
-  return decode_tma(q, ldq, out, ldo, cache, num_blocks, block_table, max_blocks, cu_seqlens, seq_lens, B, H, Hkv, D, block_size,
-                    scale, window, chunked, keep_first, softcap, sink, sinks, slopes, splits, status, nullptr, stream);
-}
-
-// The same from the projection's rows [q: H | k: Hkv | v: Hkv heads of 128] of one token a request (at most 8 q heads a k head):
-// the q and k heads are divided by their root mean square and multiplied by the weights [128] (f32 or bf16; null: no norm),
-// turned by row positions[t] of cos_sin [positions, 128] f32 (64 cosines, 64 sines; elements i and i + 64 are a pair; null: not
-// turned), and k and v go to place slots[t] of the cache (below 0: nowhere) before the token sees them.  The rows are not written.
-DINFER_API int dinfer_attention_decode_tma_raw(const void* qkv, int64_t ldq, void* out, int64_t ldo, void* cache, int64_t num_blocks,
-                                               const int* block_table, int max_blocks, const int* cu_seqlens, const int* seq_lens,
-                                               int B, int H, int Hkv, int block_size, float scale, int window, int chunked,
-                                               int keep_first, int sink, const float* sinks, const float* slopes, int splits,
-                                               const int* positions, const int* slots, const void* q_weight, const void* k_weight,
-                                               int weights_f32, float eps, const float* cos_sin, int* status, cudaStream_t stream) {
-  if (!positions || !slots || Hkv <= 0 || H <= 0 || H % Hkv || H / Hkv > 8 || ldq < (int64_t)(H + 2 * Hkv) * 128 || ldq % 4 ||
-      (reinterpret_cast<uintptr_t>(qkv) & 7) || (reinterpret_cast<uintptr_t>(q_weight) & 15) ||
-      (reinterpret_cast<uintptr_t>(k_weight) & 15) || (reinterpret_cast<uintptr_t>(cos_sin) & 15) || !q_weight != !k_weight)
-    return refuse(DINFER_BAD_ARGUMENT, "attention_decode_tma_raw: H=%d Hkv=%d ldq=%lld, rows of 8-byte and weights of 16-byte aligned "
-                  "pieces, both norms or none", H, Hkv, (long long)ldq);
-  Params raw{};
-  raw.positions = positions; raw.slots = slots; raw.q_weight = q_weight; raw.k_weight = k_weight; raw.weights_f32 = weights_f32;
-  raw.eps = eps; raw.cos_sin = cos_sin;
-  return decode_tma(qkv, ldq, out, ldo, cache, num_blocks, block_table, max_blocks, cu_seqlens, seq_lens, B, H, Hkv, 128, block_size,
-                    scale, window, chunked, keep_first, 0.f, sink, sinks, slopes, splits, status, &raw, stream);
 }
 
 DINFER_API int dinfer_attention_decode_tma(const void* q, int64_t ldq, void* out, int64_t ldo, const void* cache,

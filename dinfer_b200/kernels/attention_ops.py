@@ -40,54 +40,6 @@ def decode_supported(dtype: torch.dtype, head_dim: int, group: int, block_size: 
             and block_size > 0 and block_size & (block_size - 1) == 0)
 
 
-def decode_raw_supported(qkv: torch.Tensor, head_dim: int, group: int, block_size: int, rot: int, interleaved: bool, softcap: float) -> bool:
-    """Whether ``attention_decode_raw`` takes these rows: heads of 128 turned whole (or not at all), pages that TMA fetches."""
-    return (head_dim == 128 and group <= 8 and block_size >= 8 and decode_supported(qkv.dtype, head_dim, group, block_size)
-            and not interleaved and rot in (0, 128) and not softcap and qkv.stride(1) == 1 and qkv.stride(0) % 4 == 0
-            and qkv.data_ptr() % 8 == 0)
-
-
-def attention_decode_raw(qkv: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
-                         cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, num_heads: int, num_kv_heads: int, scale: float,
-                         window: int, splits: int, positions: torch.Tensor, slots: torch.Tensor, eps: float,
-                         q_weight: Optional[torch.Tensor], k_weight: Optional[torch.Tensor], cos_sin: Optional[torch.Tensor],
-                         sink: bool = False, slopes: Optional[torch.Tensor] = None, chunked: bool = False,
-                         sinks: Optional[torch.Tensor] = None, keep_first: int = 0, softcap: float = 0.0) -> torch.Tensor:
-    """``ops.qk_post`` and ``attention_decode`` in one kernel, for steps that bring one token a request: from the projection's
-    rows ``qkv`` [T, >= (H + 2 Hkv) 128] (left as they are), where ``decode_raw_supported``."""
-    require_cuda(qkv, out, cache, block_table, cu_seqlens, seq_lens, positions, slots, q_weight, k_weight, cos_sin, slopes, sinks)
-    sink = _check_heads(num_heads, slopes, sinks) or sink
-    rot = 0 if cos_sin is None else cos_sin.shape[1]
-    T = qkv.shape[0]
-    if cache.dim() != 5 or cache.dtype != torch.bfloat16 or not cache.is_contiguous() or out.dtype != torch.bfloat16 or out.stride(-1) != 1 \
-            or tuple(cache.shape[1:3]) != (2, num_kv_heads) \
-            or not decode_raw_supported(qkv, cache.shape[4], num_heads // num_kv_heads, cache.shape[3], rot, False, softcap):
-        raise KernelError("attention_decode_raw: bfloat16 rows of heads of 128, a contiguous cache [blocks, 2, Hkv, block >= 8, 128]")
-    for t, n in ((block_table, "block_table"), (cu_seqlens, "cu_seqlens"), (seq_lens, "seq_lens"), (positions, "positions"), (slots, "slots")):
-        if t.dtype != torch.int32 or not t.is_contiguous():
-            raise KernelError(f"attention_decode_raw: {n} must be contiguous int32")
-    if positions.numel() != T or slots.numel() != T:
-        raise KernelError("attention_decode_raw: positions and slots [T]")
-    if cos_sin is not None and (cos_sin.dtype != torch.float32 or not cos_sin.is_contiguous()):
-        raise KernelError("attention_decode_raw: angle table contiguous float32")
-    if (q_weight is None) != (k_weight is None) or (q_weight is not None and (
-            q_weight.numel() != 128 or k_weight.numel() != 128 or k_weight.dtype != q_weight.dtype
-            or q_weight.dtype not in (torch.float32, torch.bfloat16) or not (q_weight.is_contiguous() and k_weight.is_contiguous()))):
-        raise KernelError("attention_decode_raw: norm weights [128] of one dtype, both or none")
-    from . import gemm_ops
-    lib, f = _fn("attention_decode", "dinfer_attention_decode_tma_raw",
-                 [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_void_p,
-                  c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
-                  c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p, c_void_p])
-    check(lib, f(ptr(qkv), qkv.stride(0), ptr(out), out.stride(0), ptr(cache), cache.shape[0], ptr(block_table), block_table.shape[1],
-                 ptr(cu_seqlens), ptr(seq_lens), cu_seqlens.numel() - 1, num_heads, num_kv_heads, cache.shape[3], float(scale),
-                 int(window), int(bool(chunked)), int(keep_first or 0), int(bool(sink)), ptr(sinks), ptr(slopes),
-                 min(int(splits), MAX_CLUSTER_SPLITS), ptr(positions), ptr(slots), ptr(q_weight), ptr(k_weight),
-                 int(q_weight is not None and q_weight.dtype == torch.float32), float(eps), ptr(cos_sin),
-                 ptr(gemm_ops._state(qkv.device)["status"]), stream_handle()), "attention_decode_tma_raw")
-    return out
-
-
 # Scratch of the split-key decode kernel, per device: f32 partial sums and a block of counters that
 # every launch leaves at zero.  Buffers are only ever replaced by larger ones and the old ones are
 # kept alive, because a captured CUDA graph holds their addresses.  All launches that use it run on

@@ -258,7 +258,7 @@ class GQAttention(Mixer):
         interleaved = getattr(self.position, "interleaved", False)
         if self.value_turn and self.v_table is None:
             self.v_table = rope_table(self.Dv, self.value_turn, int(self.env.max_positions), self.env.device)
-        v_table, out = self.v_table, None
+        v_table = self.v_table
         if self.general:
             if not self.position.fused:
                 raise NotImplementedError("attention: a head norm behind the rotation, or values of another width, "
@@ -277,12 +277,6 @@ class GQAttention(Mixer):
                                  interleaved=interleaved, bias=self.qkv_bias32,
                                  q_temperature=self.q_temperature, v_first=v_first, v_lambda=self.v_lambda,
                                  v_cos_sin=v_table)
-        elif self.decodes_raw(qkv, table, kv, g, ctx):
-            # one token a request: the attention kernel norms, turns and caches on its way
-            out = torch.empty((qkv.shape[0], H * self.Dv), dtype=qkv.dtype, device=qkv.device)
-            attention_ops.attention_decode_raw(qkv, out, kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, H, Hkv, self.scale,
-                                               int(self.window or 0), self.decode_key_splits(ctx), ctx.positions, g.slot_mapping,
-                                               self.eps, self.q_norm_w, self.k_norm_w, table, **self.seen())
         elif self.position.fused:
             ops.qk_post(qkv, ctx.positions, H, Hkv, D, self.eps, self.q_norm_w, self.k_norm_w, table,
                         kv, g.slot_mapping, g.block_size, interleaved=interleaved)
@@ -296,9 +290,8 @@ class GQAttention(Mixer):
             if kv is not None:
                 ops.qk_post(qkv, ctx.positions, H, Hkv, D, self.eps, None, None, None, kv,
                             g.slot_mapping, g.block_size)
-        if out is None:
-            out = torch.empty((qkv.shape[0], H * self.Dv), dtype=qkv.dtype, device=qkv.device)
-            self.attend(qkv[:, :H * D], out, cache.kv, g, ctx)
+        out = torch.empty((qkv.shape[0], H * self.Dv), dtype=qkv.dtype, device=qkv.device)
+        self.attend(qkv[:, :H * D], out, cache.kv, g, ctx)
         if v_table is not None or (self.gate_name and self.gate_per_head):
             gate = qkv[:, self.gate_col:self.gate_col + H] if self.gate_name and self.gate_per_head else None
             ops.heads_out(out, ctx.positions, H, self.Dv, v_table, gate, interleaved=interleaved)
@@ -308,30 +301,17 @@ class GQAttention(Mixer):
             return self.o.into_residual(out, sink[0], sink[1])
         return self.o(out, out_dtype=torch.float32 if self.out_float32 else None)
 
-    def seen(self) -> dict:
-        return dict(sink=self.sink, slopes=self.slopes, chunked=self.chunked, sinks=self.sinks, keep_first=self.keep_first,
-                    softcap=self.softcap)
-
-    def decode_key_splits(self, ctx: StepContext) -> int:
-        splits = ctx.decode_splits or attention_ops.decode_splits(ctx.num_reqs, self.Hkv, ctx.max_seq_len)
-        if self.chunked or self.keep_first:                 # a decoded token sees its chunk, or the window and the kept tokens, at most
-            longest = int(self.env.max_positions) if ctx.decode_splits else ctx.max_seq_len        # (a captured graph's bound)
-            splits = min(splits, attention_ops.decode_splits(ctx.num_reqs, self.Hkv, min(int(self.window or 0) + self.keep_first, longest)))
-        return splits
-
-    def decodes_raw(self, qkv, table, kv, g, ctx: StepContext) -> bool:
-        """Whether the step is decoded tokens alone, in sizes whose q/k work the decode attention does itself.  With a history
-        that another layer wrote (``kv`` None) there is nothing to cache, and q alone is not worth a variant."""
-        return (kv is not None and ctx.any_decode and not ctx.any_prefill and self.position.fused and self._fast(qkv.dtype)
-                and attention_ops.decode_raw_supported(qkv, self.D, self.H // self.Hkv, g.block_size, 0 if table is None else table.shape[1],
-                                                       getattr(self.position, "interleaved", False), self.softcap))
-
     def attend(self, q, out, kv, g, ctx: StepContext) -> None:
         """Tensor-core kernels where they take the head size (bfloat16; 32, 64, 128), else the
         plain-arithmetic kernel, which takes every size."""
-        window, seen = int(self.window or 0), self.seen()
+        window = int(self.window or 0)
+        seen = dict(sink=self.sink, slopes=self.slopes, chunked=self.chunked, sinks=self.sinks, keep_first=self.keep_first,
+                    softcap=self.softcap)
         if self._fast(q.dtype):
-            splits = self.decode_key_splits(ctx)
+            splits = ctx.decode_splits or attention_ops.decode_splits(ctx.num_reqs, self.Hkv, ctx.max_seq_len)
+            if self.chunked or self.keep_first:             # a decoded token sees its chunk, or the window and the kept tokens, at most
+                longest = int(self.env.max_positions) if ctx.decode_splits else ctx.max_seq_len    # (a captured graph's bound)
+                splits = min(splits, attention_ops.decode_splits(ctx.num_reqs, self.Hkv, min(window + self.keep_first, longest)))
             tc_decode = ctx.any_decode
             if ctx.any_decode and attention_ops.decode_supported(q.dtype, self.D, self.H // self.Hkv, g.block_size) \
                     and (g.block_size >= 8 or not (self.sink or self.slopes is not None or self.chunked or self.keep_first or self.softcap)):
