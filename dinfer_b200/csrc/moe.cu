@@ -367,6 +367,10 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
+// the same, and the 256 bytes around it come into L2: a row's next 128 bytes are the next step's
+__device__ __forceinline__ void cp_async16_ahead(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 // Row tiles of 16 (decode steps): bound by reading the weights of the experts that the step's tokens meet, 64 rows of them a
@@ -407,7 +411,10 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
         else *reinterpret_cast<uint4*>(&As[buf][r][c]) = make_uint4(0, 0, 0, 0);
       } else {
         const int n = r - BM;
-        if (n0 + n < N && in_k) cp_async16(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
+        if (n0 + n < N && in_k) {
+          if (BM == 16) cp_async16_ahead(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
+          else cp_async16(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
+        }
         else *reinterpret_cast<uint4*>(&Bs[buf][n][c]) = make_uint4(0, 0, 0, 0);
       }
     }
