@@ -96,7 +96,7 @@ def test_gemm_f32(M, N, K, adt, wdt, cdt):
 
 
 @pytest.mark.parametrize("M,N,K", [(9, 129, 16), (64, 128, 132), (65, 127, 260), (128, 256, 1024), (333, 1024, 3072), (64, 8, 2050),
-                                   (40, 20, 4)])
+                                   (40, 20, 4), (9, 48, 48), (25, 5, 129), (32, 2049, 128), (31, 2048, 128), (17, 33, 1)])
 @pytest.mark.parametrize("adt,wdt,cdt", [(torch.float32,) * 3, (torch.bfloat16, torch.float32, torch.bfloat16),
                                          (torch.float32, torch.bfloat16, torch.float32)])
 def test_gemm_f32_tiles_and_splits(M, N, K, adt, wdt, cdt):
