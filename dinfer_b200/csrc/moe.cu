@@ -375,7 +375,7 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 
 // Row tiles of 16 (decode steps): bound by reading the weights of the experts that the step's tokens meet, 64 rows of them a
 // block, four stages of 64 k.  Eight tokens, 64 experts of 4096 x 2048 (8 chosen): gate and up 292 us and down 148 us with
-// two stages of 32 k, 265 and 131 us now (5.3 TB/s).
+// two stages of 32 k, 244 and 126 us now (5.7 TB/s; 265 and 131 without the 256-byte fetch into L2).
 template <int BM, int MODE>
 __global__ void __launch_bounds__(128)
 moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ Wall,
