@@ -445,11 +445,9 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 DINFER_DEFINE_LAST_ERROR()
 
 DINFER_API int dinfer_delta_chunks_tokens() { return C; }
-// floats of the workspace a (chunk, head) takes
-DINFER_API int64_t dinfer_delta_chunks_floats(int dk, int dv) { return (int64_t)C * (dk + dv) + C * C + SMALL; }
 DINFER_API int dinfer_delta_chunks_supports(int dk, int dv) { return (dk == 64 || dk == 128) && dv > 0 && dv % BC == 0; }
 
-// As dinfer_delta_recurrence with one decay a head.  work: places * H * dinfer_delta_chunks_floats(dk, dv) floats, places >=
+// As dinfer_delta_recurrence with one decay a head.  work: places * H * (32 (dk + dv) + 32 * 32 + 68) floats, places >=
 // the sum over the requests of ceil(tokens / 32).
 DINFER_API int dinfer_delta_chunks(const float* q, const float* k, const float* v, const float* beta, const float* decay,
                                    float* state, int64_t ld_state, const int* cu, const int* slots, const int* fresh, float* out,

@@ -80,7 +80,7 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
     out = torch.empty((T, H, dv), dtype=torch.float32, device=q.device)
     if T == 0:
         return out
-    if longest and not per_channel and not widen and _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest):
+    if longest >= CHUNKS_FROM[0] and not per_channel and not widen and _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest):
         return out
     lib, f = _fn("delta_rule", "dinfer_delta_recurrence",
                  [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
@@ -98,8 +98,9 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
 # rounds.  So for one, two and three blocks an SM from so many tokens of the longest portion on, never beyond.  Keys and values
 # of 128, token loop and chunks (us), 16 heads, one portion: of 48 tokens 15 and 18, of 64 19 and 18, of 2000 502 and 220; two:
 # 64 22 and 25, 96 31 and 31, 2000 585 and 436; three: 96 38 and 44, 256 94 and 91, 2000 710 and 649; four: 256 114 and 118,
-# 2000 857 and 860.
-CHUNKS_FROM = (64, 96, 256)
+# 2000 857 and 860.  The lines lie where the chunks also make up for one more launch and a workspace where the host is what a
+# step waits for (one portion of 109 tokens, 32 heads: a step of 111 us took 124).
+CHUNKS_FROM = (128, 256, 512)
 # bytes of workspace (128 KB a chunk of 32 tokens for 4 heads of 128) beyond which a step stays with the token loop
 CHUNKS_BYTES = 1 << 29
 
@@ -115,10 +116,8 @@ def _chunks(q, k, v, beta, decay, state, cu_seqlens, slots, fresh, out, longest:
         return False
     if dk not in (64, 128) or dv % 16 or decay.shape[1] != H or any(t.data_ptr() % 16 for t in (q, k, v, out)):
         return False
-    lib, floats = _fn("delta_chunks", "dinfer_delta_chunks_floats", [c_int, c_int])
-    floats.restype = c_int64
     places = T // 32 + B                                     # at most so many chunks, however the tokens are dealt out
-    words = places * H * int(floats(dk, dv))
+    words = places * H * (32 * (dk + dv) + 32 * 32 + 68)       # as dinfer_delta_chunks lays them out
     if 4 * words > CHUNKS_BYTES or H > 65535 or B > 65535:
         return False
     work = torch.empty(words, dtype=torch.float32, device=q.device)

@@ -133,8 +133,8 @@ def test_preparation_in_runs(dtype, H, G, dk, dv, per_channel):
                 assert torch.allclose(o[a:z], w, rtol=2e-6, atol=1e-7)
 
 
-@pytest.mark.parametrize("B,H,longest,chunks", [(1, 16, 63, False), (1, 16, 64, True), (2, 16, 95, False), (2, 16, 96, True), (3, 16, 255, False),
-                                                (3, 16, 256, True), (4, 16, 4000, False)])
+@pytest.mark.parametrize("B,H,longest,chunks", [(1, 16, 127, False), (1, 16, 128, True), (2, 16, 255, False), (2, 16, 256, True), (3, 16, 511, False),
+                                                (3, 16, 512, True), (4, 16, 4000, False)])
 def test_which_portions_run_in_chunks(B, H, longest, chunks, monkeypatch):
     from dinfer_b200.kernels import delta_ops
     monkeypatch.setattr(delta_ops, "num_sms", lambda: 148)
