@@ -444,7 +444,6 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 DINFER_DEFINE_LAST_ERROR()
 
-DINFER_API int dinfer_delta_chunks_tokens() { return C; }
 DINFER_API int dinfer_delta_chunks_supports(int dk, int dv) { return (dk == 64 || dk == 128) && dv > 0 && dv % BC == 0; }
 
 // As dinfer_delta_recurrence with one decay a head.  work: places * H * (32 (dk + dv) + 32 * 32 + 68) floats, places >=
