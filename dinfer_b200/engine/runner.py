@@ -75,14 +75,18 @@ def graph_shape(prompt_lens: Sequence[int], num_decodes: int, budget: int, bucke
 
 def capture_places(total: int, n_places: int, bucket: int, longest: int):
     """The dummy batch a graph of this shape is captured on, as (-1, tokens) per place: ``total`` prompt tokens
-    spread over the prompt places, none longer than ``longest``, then the bucket's one-token places.  None when
-    the places cannot hold them."""
+    spread over the prompt places, none longer than ``longest``, then the bucket's one-token places.  No prompt
+    place holds a single token: the parts take a place of one token for a decoded one, and the bounds they derive
+    from the dummy batch (row tiles, gathered rows) have to count every prompt place and token, since a replay
+    may put any portion there.  None when the places cannot hold them so."""
     places, rest = [], total
     for _ in range(n_places):
         n = min(rest, longest)
+        if rest - n == 1:
+            n -= 1                                           # two for the next place
         places.append((-1, n))
         rest -= n
-    if rest > 0:
+    if rest > 0 or any(n == 1 for _, n in places):
         return None
     return places + [(-1, 1)] * bucket
 
@@ -446,6 +450,7 @@ class ModelRunner:
         ids, rows, ctx = self.plan.build([], [], table_width=width, dev=dev, slots=places)
         hkv = max([kv.num_kv_heads for kv, _ in map(split_needs, self.model.cache_needs()) if kv is not None] or [1])
         ctx.decode_splits = attention_ops.decode_splits(max(1, bucket), hkv, self.engine.max_model_len)
+        ctx.max_q_len = min(total, self.engine.max_model_len)   # of any replay (a dummy place may hold one token less)
         ctx.max_seq_len = self.engine.max_model_len
         ctx.max_prefill_seq_len = min(self.SHORT_CONTEXT, self.engine.max_model_len) if short else self.engine.max_model_len
         ctx.split_norms = False

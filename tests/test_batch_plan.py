@@ -128,6 +128,49 @@ def test_dummy_places_of_a_captured_graph_stay_inside_the_tables_and_the_positio
         B.VALIDATE_PLANS = old
 
 
+@pytest.mark.parametrize("longest,extra", [(512, 1), (512, 0), (512, 2), (96, 1), (128, 127), (3, 1)])
+@pytest.mark.parametrize("n_places,bucket", [(4, 0), (4, 2), (16, 1)])
+def test_bounds_of_a_captured_graph_hold_for_every_replay(longest, extra, n_places, bucket):
+    """Prompt tokens that are one more than whole longest requests (and others beside them): what the parts derive from the
+    dummy batch covers any way of dealing the same tokens out over the prompt places, each request as long as it may get."""
+    from types import SimpleNamespace
+    from dinfer_b200.engine.runner import ModelRunner
+    from dinfer_b200.kernels import attention_ops, latent_ops
+    from dinfer_b200.parts.latent_attention import LatentAttention
+    part = LatentAttention.__new__(LatentAttention)
+    part.H, part.D, part.P, part.V, part.R, part.window = 16, 128, 64, 128, 512, None
+    part.RATES = (1.0, 1.0, 1.0, 1e30, 1e30, 0.0, 0.0)                         # the expanded way, whatever the sizes
+    part.EXPANDED_BYTES = 1 << 60
+    for full in range(1, n_places):
+        total = full * longest + extra
+        seen = []
+        runner = SimpleNamespace(
+            max_blocks_per_seq=(longest + 3) // 4, device=torch.device("cpu"), SHORT_CONTEXT=512, sampled=None, _graphs={},
+            engine=SimpleNamespace(max_model_len=longest), model=SimpleNamespace(cache_needs=lambda: []),
+            plan=PlanBuilder(CacheManager([GroupSpec()], 4, 8, max_num_seqs=32), "cpu", total + bucket, n_places + bucket, (longest + 3) // 4),
+            _capture_one=lambda ids, rows, ctx: (seen.append(ctx), {})[1])
+        ModelRunner._capture_mixed(runner, ("mixed", total, n_places, bucket, False))
+        ctx, = seen
+        cu = ctx.cu_seqlens_host
+        lens = [cu[i + 1] - cu[i] for i in range(len(cu) - 1)]
+        assert sum(lens[:n_places]) == total and max(lens) <= longest and lens[n_places:] == [1] * bucket
+        assert ctx.max_q_len == min(total, longest)
+        rows, pairs = part._expanded_shape(ctx)
+        rng = random.Random(total)
+        for trial in range(40):
+            # portions of two tokens and more: a few cuts through the tokens, or as many places as there are
+            count = rng.randint(-(-total // longest), min(n_places, total // 2))
+            portions, rest = [], total
+            for k in range(count, 0, -1):
+                lo, hi = max(2, rest - (k - 1) * longest), min(longest, rest - 2 * (k - 1))
+                portions.append(rng.choice([lo, hi, rng.randint(lo, hi)]))
+                rest -= portions[-1]
+            assert rest == 0
+            assert latent_ops.expanded_rows([(n, longest) for n in portions]) <= rows
+            assert sum((n + 255) // 256 for n in portions) <= pairs
+            for group in (1, 4):
+                assert sum((n * group + 255) // 256 for n in portions) <= attention_ops.umma_pair_bound(lens, group)
+
 def test_slots_and_tables_of_groups_with_page_sizes_of_their_own():
     """A token's slot in a group is page * (the group's page size) + offset, and every group's table is as wide as
     the plan says (the unused entries -1)."""
