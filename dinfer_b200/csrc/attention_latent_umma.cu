@@ -19,7 +19,7 @@
 // a stage is three (two) boxes; the 64-wide rotated part is a third part of Q and K (a narrower one is filled up with
 // zeros by TMA, beyond the row's end); shared memory holds Q (96 KB), two stages of K (96 KB) and one of V (32 KB) at
 // D = 128, so its small arrays share a row.
-// Bounded waits; status codes 31-36.
+// Bounded waits; status codes 31-36, and 37 for a step whose portions pass the bounds of its launch (rows, row-tile pairs).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -37,7 +37,7 @@ constexpr uint32_t PART = BM * 128;                            // bytes of a 128
 struct Params {
   __nv_bfloat16* out; int64_t ldo;
   const int* cu_seqlens; const int* seq_lens;
-  int B, window;
+  int B, window, rows;
   float scale_log2;
   const float* sinks;
   int* status;
@@ -87,30 +87,38 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x;
   pdl_enter();
-  // which request's pair this is, and where its keys begin: every warp adds the requests up for itself
-  int b = -1, pair = 0, pairs_b = 0, key0 = 0;
+  // which request's pair this is, and where its keys begin: every warp adds the requests up for itself (the last block's all of
+  // them: a captured graph may be replayed on any lengths, and pairs beyond the grid would go unnoticed)
+  int b = -1, pair = 0, pairs_b = 0, key0 = 0, key_end = 0;
   {
     const int y = blockIdx.y;
+    const bool all = y == (int)gridDim.y - 1 && head == 0;
     int before = 0, keys_before = 0;
     for (int i0 = 0; i0 < p.B; i0 += 32) {
       const int i = i0 + lane;
       const Share sh = i < p.B ? share_of(p.cu_seqlens, p.seq_lens, i, p.window) : Share{0, 0, 0, 0};
       const int incl = warp_inclusive(sh.pairs, lane), kincl = warp_inclusive(sh.rows, lane);
       const int chunk = __shfl_sync(0xffffffffu, incl, 31);
-      if (y < before + chunk) {
+      if (b < 0 && y < before + chunk) {
         const unsigned hit = __ballot_sync(0xffffffffu, y >= before + incl - sh.pairs && y < before + incl);
         const int src = __ffs(hit) - 1;
         b = i0 + src;
         pair = y - before - __shfl_sync(0xffffffffu, incl - sh.pairs, src);
         pairs_b = __shfl_sync(0xffffffffu, sh.pairs, src);
         key0 = keys_before + __shfl_sync(0xffffffffu, kincl - sh.rows, src);
-        break;
+        key_end = keys_before + __shfl_sync(0xffffffffu, kincl, src);
+        if (!all) break;
       }
       before += chunk;
       keys_before += __shfl_sync(0xffffffffu, kincl, 31);
     }
+    if (all && before > (int)gridDim.y && threadIdx.x == 0) atomicExch(p.status, 37);
   }
   if (b < 0) return;                                           // beyond the batch's pairs
+  if (key_end > p.rows) {                                      // keys that were not gathered
+    if (threadIdx.x == 0) atomicExch(p.status, 37);
+    return;
+  }
   const int t0 = p.cu_seqlens[b];
   const int rows_total = p.cu_seqlens[b + 1] - t0;
   const int row0 = (pairs_b - 1 - pair) * 2 * BM;              // the latest rows, which see the most keys, start first
@@ -509,7 +517,7 @@ DINFER_API int dinfer_attention_latent_umma(const void* q, int64_t ldq, void* ou
       !make_map(&mr, (const __nv_bfloat16*)latents + (P > 0 ? R : 0), 2, dr, sr))
     return refuse(DINFER_BAD_ARGUMENT, "attention_latent_umma: a tensor map could not be made");
   Params p;
-  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.window = window;
+  p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.window = window; p.rows = rows;
   p.scale_log2 = scale * 1.4426950408889634f; p.sinks = sinks; p.status = status;
   const dim3 grid(H, pair_bound);
   return D == 64 ? launch<64>(mq, mkv, mr, p, grid, stream) : launch<128>(mq, mkv, mr, p, grid, stream);

@@ -56,6 +56,7 @@ STATUS_MEANING = {
     34: "attention over expanded latents: the MMA thread waited for a K or V tile",
     35: "attention over expanded latents: the softmax warps waited for a score tile",
     36: "attention over expanded latents: the softmax warps waited for the last P V before writing the output",
+    37: "attention over expanded latents: the step's portions pass the rows or row tiles its launch was made for",
 }
 
 
@@ -64,11 +65,12 @@ def describe_status(code: int) -> str:
 
 
 def check_status(device=None) -> None:
-    """Raise if a kernel gave up one of its bounded waits.  The word stays set (every later check raises too)
+    """Raise if a kernel gave up one of its bounded waits, or met a step beyond its launch's bounds.  The word stays set (every later check raises too)
     until ``reset_status``: after such a fault the step's results are not to be trusted."""
     code = device_status(device)
     if code:
-        raise KernelError(f"a kernel gave up a bounded wait and returned early (status {code}: "
+        what = "met a step beyond its launch's bounds" if code == 37 else "gave up a bounded wait and returned early"
+        raise KernelError(f"a kernel {what} (status {code}: "
                           f"{describe_status(code)}); the results of that step are invalid")
 
 

@@ -84,6 +84,29 @@ def test_rows_and_attention_against_plain(case):
     assert bool((lat[at:] == 0).all())
 
 
+@pytest.mark.parametrize("rows,pairs,bad", [(512, 3, False), (511, 3, True), (256, 3, True), (512, 2, True), (600, 7, False)])
+def test_portions_beyond_the_launch_leave_a_status(rows, pairs, bad):
+    """Portions that need 512 gathered rows and three row-tile pairs: a launch made for fewer says so."""
+    from dinfer_b200.kernels import gemm_ops, latent_ops as L
+    from dinfer_b200.kernels.lib import KernelError
+    D, P, R, H = 64, 32, 64, 2
+    # 256, 128 and 128 gathered rows, a pair each; behind 40 single tokens the scan takes a second turn
+    reqs = [(100, 150)] + [(5, 1)] * 40 + [(0, 120), (0, 9)]
+    cu, seq, table, pages = batch(reqs, 16, 2)
+    c = lambda t: t.cuda()
+    cache = torch.randn(pages, 1, 1, 16, R + P).to(torch.bfloat16).cuda()
+    q = torch.randn(int(cu[-1]), H * (D + P)).to(torch.bfloat16).cuda()
+    w = torch.randn(H * 2 * D, R).to(torch.bfloat16).cuda()
+    out = torch.zeros(int(cu[-1]), H, D, dtype=torch.bfloat16, device="cuda")
+    lat = L.latent_rows(cache, c(table), c(cu), c(seq), rows, 0)
+    L.attention_latent_umma(q, out, lat, lat[:, :R] @ w.T, c(cu), c(seq), R, P, D, 0.1, 0, pair_bound=pairs)
+    if bad:
+        with pytest.raises(KernelError, match="status 37"):
+            gemm_ops.check_status()
+        assert gemm_ops.reset_status() == 37
+    gemm_ops.check_status()
+
+
 @pytest.mark.parametrize("P,rot,halves", [(64, 64, False), (32, 20, False), (64, 64, True), (16, 8, True)])
 def test_rotation_in_place(P, rot, halves):
     from dinfer_b200.kernels import latent_ops as L
