@@ -115,7 +115,8 @@ delta_chunk_kernel(const Args a) {
     // the decays' logarithms (0 behind the portion's end), their running sums in 64-bit
     double l = 0.0;
     if (lane < n) {
-      l = fmax(log1p((double)a.decay[(int64_t)(t0 + lane) * a.H + h]), (double)LOG_FLOOR);
+      l = log1p((double)a.decay[(int64_t)(t0 + lane) * a.H + h]);
+      if (l < (double)LOG_FLOOR) l = LOG_FLOOR;            // (not fmax: a NaN stays one, as token by token)
       be = a.beta[(int64_t)(t0 + lane) * a.H + h];
     }
 #pragma unroll

@@ -75,6 +75,35 @@ def test_chunks_against_plain(case):
         assert torch.equal(states[1][s, keep], state[s, keep])
 
 
+def loop_and_chunks(where, value, at):
+    """Outputs and states of both ways, one request behind another, with ``value`` in one element of one input at token
+    ``at`` of the first request."""
+    from dinfer_b200.kernels import delta_ops
+    H, G, dk, dv, tokens = 4, 2, 64, 32, [150, 40]
+    g = torch.Generator().manual_seed(at + dk)
+    T = sum(tokens)
+    rand = lambda *s: torch.randn(*s, generator=g)
+    x = {"q": rand(T, G, dk) / dk, "k": rand(T, G, dk) * dk ** -0.5, "v": rand(T, H, dv), "beta": torch.sigmoid(rand(T, H)),
+         "decay": torch.expm1(-0.1 * torch.rand(T, H, generator=g))}
+    x[where].view(T, -1)[at, 1] = value
+    state, cu = rand(2, H * dk * dv), torch.tensor([0] + tokens, dtype=torch.int32).cumsum(0).to(torch.int32).cuda()
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32).cuda()
+    out = []
+    for longest in (0, 1000):
+        st = state.clone().cuda()
+        o = delta_ops.recurrence(*[x[n].cuda() for n in ("q", "k", "v", "beta", "decay")], st, cu, i32(0, 1), i32(0, 0), False,
+                                 longest=longest)
+        out.append((o.cpu(), st.cpu().view(2, H, dk, dv)))
+    return out
+
+
+@pytest.mark.parametrize("at", [0, 21, 95, 149])
+def test_a_decay_that_is_not_a_number_stays_one(at):
+    (loop, loop_state), (chunks, state) = loop_and_chunks("decay", float("nan"), at)
+    assert not bool(torch.isfinite(loop[at:150, 1]).any()) and not bool(torch.isfinite(loop_state[0, 1]).any())
+    assert not bool(torch.isfinite(chunks[at:150, 1]).any()) and not bool(torch.isfinite(state[0, 1]).any())
+
+
 def test_sizes_the_chunks_do_not_take_stay_with_the_token_loop():
     from dinfer_b200.kernels import delta_ops
     g = torch.Generator().manual_seed(3)
