@@ -12,13 +12,18 @@
 //   delta_chunk   everything that needs no state, all (chunk, head) side by side, into a workspace
 //   delta_walk    per (request, head, 16 value columns) the chunks in order; S in registers and shared memory
 //
+// What a token's output and what it adds to the state are made of are sums over the tokens up to it and nothing else: an
+// infinity or NaN at one token leaves the outputs before it alone, as token by token, where a zero of the triangular matrices
+// times it would not.
+//
 // All arithmetic is 32-bit; the running sums are 64-bit, so that a difference of two large ones is exact; the state's decay is
 // S + S expm1(c_n).  An update of the state rounds once a chunk where the token loop rounds 32 times.
 //
 // What bounds it: the walk, 32-bit multiply-adds on small tiles with every operand from shared memory (1.5 loads of 16 bytes
-// for every eight), and the chain of chunks.  2000 tokens of 16 heads of 128 x 128: the token loop 501 us (a chain of 250 ns
-// a token), delta_chunk 41 us (46 with 4 x 2 sums a thread and a thread a
-// column) and delta_walk 170 us.
+// for every eight), and the chain of chunks.  2000 tokens of 16 heads of 128 x 128: the token loop 502 us (a chain of 250 ns
+// a token), both kernels 199 us (220 with the products of the upper triangles), delta_chunk 44 us of it, delta_walk the rest.
+#include <type_traits>
+
 #include "common.cuh"
 
 using namespace dinfer;
@@ -210,7 +215,7 @@ delta_chunk_kernel(const Args a) {
   }
   // [W_v | W_k]: a half of the threads has DK columns, a thread rows rt .. rt + 3 of columns cx + 64 j ..
   const bool keys = tid < 128;
-  const int rt = ((tid & 127) >> 4) * 4, cx = (tid & 15) * 4, s_end = (((tid & 127) >> 5) * 2 + 1) * 4 + 4;   // (a warp's last row)
+  const int rt = ((tid & 127) >> 4) * 4, cx = (tid & 15) * 4, w0 = (tid & 127) >> 5 << 3;   // (a warp has rows w0 .. w0 + 7)
   for (int c0 = 0; c0 < a.dv; c0 += DK) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -222,8 +227,7 @@ delta_chunk_kernel(const Args a) {
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < CW; ++j) acc[i][j] = 0.f;
-#pragma unroll 4
-      for (int s = 0; s < s_end; ++s) {
+      auto add = [&](int s, auto diagonal) {
         const float4 t4 = *reinterpret_cast<const float4*>(&T[s][rt]);
         const float t[4] = {t4.x, t4.y, t4.z, t4.w};
 #pragma unroll
@@ -231,13 +235,18 @@ delta_chunk_kernel(const Args a) {
           const float4 r = *reinterpret_cast<const float4*>(&right[s][cx + 16 * j]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
+            if (diagonal && s > rt + i) continue;          // a later token's value, which may not be finite
             acc[i][j] = fmaf(t[i], r.x, acc[i][j]);
             acc[i][j + 1] = fmaf(t[i], r.y, acc[i][j + 1]);
             acc[i][j + 2] = fmaf(t[i], r.z, acc[i][j + 2]);
             acc[i][j + 3] = fmaf(t[i], r.w, acc[i][j + 3]);
           }
         }
-      }
+      };
+#pragma unroll 4
+      for (int s = 0; s < w0; ++s) add(s, std::false_type());
+#pragma unroll 4
+      for (int u = 0; u < 8; ++u) add(w0 + u, std::true_type());
       float* w = keys ? a.wk + at * C * DK : a.wv + at * C * a.dv + c0;
       const int ld = keys ? DK : a.dv;
 #pragma unroll
@@ -401,19 +410,24 @@ delta_walk_kernel(const Args a) {
       // o_t = Gamma_t (q_t S) + sum_(s <= t) M[t, s] u_s
       const float gam = s[L::SM + t];
       o.x *= gam; o.y *= gam; o.z *= gam; o.w *= gam;
-#pragma unroll 4
-      for (int u = 0; u < C; u += 4) {
+      auto add = [&](int u, auto diagonal) {
         const float4 m = *reinterpret_cast<const float4*>(s + L::M + t * LDA + u);
         const float mm[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
+          if (diagonal && u + e > t) continue;             // a later token's update, which may not be finite
           const float4 x = *reinterpret_cast<const float4*>(U_s + (u + e) * BC + cx);
           o.x = fmaf(mm[e], x.x, o.x);
           o.y = fmaf(mm[e], x.y, o.y);
           o.z = fmaf(mm[e], x.z, o.z);
           o.w = fmaf(mm[e], x.w, o.w);
         }
-      }
+      };
+      const int w0 = t & ~7;                               // (a warp has rows w0 .. w0 + 7)
+#pragma unroll 4
+      for (int u = 0; u < w0; u += 4) add(u, std::false_type());
+#pragma unroll
+      for (int u = 0; u < 8; u += 4) add(w0 + u, std::true_type());
       if (j * C + t < n)
         *reinterpret_cast<float4*>(a.out + ((int64_t)(start + j * C + t) * a.H + h) * a.dv + c0 + cx) = o;
     }

@@ -96,9 +96,9 @@ def recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, beta: torch.Te
 # Chunks of 32 are worth it where the token loop is bound by its chain (0.25 us a token) and not by its work: the walk over the
 # chunks runs a block per (request, head, 16 value columns), about one to an SM, and with more blocks than SMs takes as many
 # rounds.  So for one, two and three blocks an SM from so many tokens of the longest portion on, never beyond.  Keys and values
-# of 128, token loop and chunks (us), 16 heads, one portion: of 48 tokens 15 and 18, of 64 19 and 18, of 2000 502 and 220; two:
-# 64 22 and 25, 96 31 and 31, 2000 585 and 436; three: 96 38 and 44, 256 94 and 91, 2000 710 and 649; four: 256 114 and 118,
-# 2000 857 and 860.  The lines lie where the chunks also make up for one more launch and a workspace where the host is what a
+# of 128, token loop and chunks (us), 16 heads, one portion: of 48 tokens 15 and 17, of 64 19 and 17, of 2000 502 and 199; two:
+# 64 22 and 24, 96 31 and 29, 2000 586 and 396; three: 96 38 and 42, 256 94 and 86, 2000 710 and 593; four, with the chunks'
+# kernels a tenth slower than now: 256 114 and 118, 2000 857 and 860.  The lines lie where the chunks also make up for one more launch and a workspace where the host is what a
 # step waits for (one portion of 109 tokens, 32 heads: a step of 111 us took 124).
 CHUNKS_FROM = (128, 256, 512)
 # bytes of workspace (128 KB a chunk of 32 tokens for 4 heads of 128) beyond which a step stays with the token loop
