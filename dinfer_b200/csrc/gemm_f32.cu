@@ -23,6 +23,8 @@ constexpr int TILE_SMEM = STAGES * STAGE_FLOATS * 4;
 static_assert(BM * LDC_S <= STAGES * STAGE_FLOATS, "the partial tile takes the stages' place");
 static_assert(TILE_SMEM <= 48 * 1024, "no opt-in");
 constexpr int MAX_SPLITS = 8;                  // CTAs that may share a tile's K (a portable cluster)
+constexpr int GRID_ROWS = 65535 * BM;          // rows of one launch (row tiles are the grid's y)
+constexpr int MAX_ROWS = 65535 * 128;          // rows of one product
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // 16 bytes, or zeros where `live` is false (nothing is read then)
@@ -313,21 +315,24 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
     while (splits < MAX_SPLITS && tiles * (splits + 1) <= num_sms() * 5 / 3 && k_tiles / (splits + 1) >= 8 &&
            (int64_t)batch * (splits + 1) <= 65535)
       ++splits;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch * splits);
-    if (grid.y > 65535) return refuse(DINFER_BAD_ARGUMENT, "gemm_f32: M=%d too large", M);
+    if (M > MAX_ROWS) return refuse(DINFER_BAD_ARGUMENT, "gemm_f32: M=%d too large", M);
     const auto fast = [](const void* q, size_t size, int64_t ld, int64_t stride) {
       return (int)((reinterpret_cast<uintptr_t>(q) % (4 * size)) == 0 && ld % 4 == 0 && stride % 4 == 0);
     };
     const int a_fast = fast(A, sizeof(TA), lda, sa) && K % 4 == 0, w_fast = fast(W, sizeof(TW), ldw, sw) && K % 4 == 0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = dim3(TILE_THREADS); cfg.dynamicSmemBytes = TILE_SMEM; cfg.stream = stream;
+    cfg.blockDim = dim3(TILE_THREADS); cfg.dynamicSmemBytes = TILE_SMEM; cfg.stream = stream;
     cudaLaunchAttribute cluster;
     cluster.id = cudaLaunchAttributeClusterDimension;
     cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
     cluster.val.clusterDim.z = splits;
     cfg.attrs = &cluster; cfg.numAttrs = splits > 1 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, gemm_tile_kernel<TA, TW, TC>, (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw,
-                       sc, splits, a_fast, w_fast, fast(C, sizeof(TC), ldc, sc));
+    for (int r = 0; r < M; r += GRID_ROWS) {                // (one launch up to 4.19 million rows)
+      const int rows = M - r < GRID_ROWS ? M - r : GRID_ROWS;
+      cfg.gridDim = dim3((N + BN - 1) / BN, (rows + BM - 1) / BM, batch * splits);
+      cudaLaunchKernelEx(&cfg, gemm_tile_kernel<TA, TW, TC>, (const TA*)A + r * lda, lda, (const TW*)W, ldw, (TC*)C + r * ldc, ldc,
+                         rows, N, K, sa, sw, sc, splits, a_fast, w_fast, fast(C, sizeof(TC), ldc, sc));
+    }
   }
   return cuda_status("gemm_f32");
 }

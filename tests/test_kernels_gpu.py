@@ -129,6 +129,23 @@ def test_gemm_f32_tiles_and_splits(M, N, K, adt, wdt, cdt):
     assert bool(((out.double().cpu() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("M", [65535 * 64, 65535 * 64 + 1, 65535 * 128])
+def test_gemm_f32_of_millions_of_rows(M):
+    """As many row tiles as a grid has, one more, and the most rows a product may have; one more is refused."""
+    from dinfer_b200.kernels import ops
+    from dinfer_b200.kernels.lib import KernelError
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, w = torch.randn(M, 4, generator=g, device="cuda"), torch.randn(5, 4, generator=g, device="cuda")
+    out = torch.full((M + 1, 5), 7.0, device="cuda")
+    ops.gemm_f32(a, w, out[:M])
+    # four products of a few units and their sum in 32-bit: 5 roundings of 2^-24
+    assert float((out[:M].double() - a.double() @ w.double().T).abs().max()) <= 5 * 2.0 ** -24 * float(a.abs().max() * w.abs().max()) * 4
+    assert bool((out[M] == 7.0).all())
+    if M == 65535 * 128:
+        with pytest.raises(KernelError, match="too large"):
+            ops.gemm_f32(torch.zeros(M + 1, 1, device="cuda"), w[:, :1].contiguous(), torch.empty(M + 1, 5, device="cuda"))
+
+
 def test_gemm_f32_strided_operands():
     from dinfer_b200.kernels import ops
     g = torch.Generator().manual_seed(3)
