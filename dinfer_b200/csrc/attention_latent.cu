@@ -206,8 +206,8 @@ struct LatentTcParams {
   int num_reqs, H, R, P, block_size, window, splits;
   int singles;                   // only the requests that bring one token (the portions are somebody else's)
   float scale_log2;
-  float* part;                   // [T * H, splits, R] unnormalised sums (splits > 1)
-  float* ml;                     // [T * H, splits, 2] maximum (log2 domain) and sum
+  float* part;                   // [T * H, splits, R] unnormalised sums (splits > 1); with singles [B * H, splits, R], by request
+  float* ml;                     // [T * H or B * H, splits, 2] maximum (log2 domain) and sum
   const float* sinks;            // [H] or null: one more term exp(sinks[h]) in head h's denominator, without a value
 };
 
@@ -430,7 +430,7 @@ attention_latent_tc_kernel(const LatentTcParams p) {
             *reinterpret_cast<__nv_bfloat162*>(dst + col) = __floats2bfloat162_rn(o[mt][nt][half * 2] * inv, o[mt][nt][half * 2 + 1] * inv);
         }
       } else {
-        const int64_t slot = (tok * p.H + head) * p.splits + blockIdx.y;
+        const int64_t slot = ((p.singles ? b : tok) * p.H + head) * p.splits + blockIdx.y;
         float* dst = p.part + slot * p.R;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -442,15 +442,22 @@ attention_latent_tc_kernel(const LatentTcParams p) {
     }
 }
 
-// out[row] = sum_s 2^(m_s - M) part[row, s] / sum_s 2^(m_s - M) l_s, in split order; one block per (token, head)
+// out[row] = sum_s 2^(m_s - M) part[row, s] / sum_s 2^(m_s - M) l_s, in split order; one block per (token, head), or with
+// singles (cu: the requests' offsets) per (request, head), nothing for a request that brings more than one token or none
 __global__ void __launch_bounds__(128)
 attention_latent_fold_kernel(const float* __restrict__ part, const float* __restrict__ ml, __nv_bfloat16* __restrict__ out,
-                             int64_t ldo_t, int64_t ldo_h, int rows, int H, int R, int splits,
-                             const float* __restrict__ sinks) {
+                             int64_t ldo_t, int64_t ldo_h, int H, int R, int splits,
+                             const float* __restrict__ sinks, const int* __restrict__ cu) {
   __shared__ float w_s[64];
   __shared__ float inv_s;
   pdl_enter();
   const int row = blockIdx.x;
+  int tok = row / H;
+  if (cu) {
+    const int b = tok;
+    tok = cu[b];
+    if (cu[b + 1] - tok != 1) return;
+  }
   const float* mlr = ml + (int64_t)row * splits * 2;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -467,7 +474,7 @@ attention_latent_fold_kernel(const float* __restrict__ part, const float* __rest
     }
   }
   __syncthreads();
-  __nv_bfloat16* dst = out + (int64_t)(row / H) * ldo_t + (int64_t)(row % H) * ldo_h;
+  __nv_bfloat16* dst = out + (int64_t)tok * ldo_t + (int64_t)(row % H) * ldo_h;
   const float* pr = part + (int64_t)row * splits * R;
   for (int c = threadIdx.x; c < R; c += blockDim.x) {
     float a = 0.f;
@@ -503,9 +510,10 @@ DINFER_API int dinfer_attention_latent_tc_rows(int R, int max_rows_per_req) {
 }
 
 // bfloat16 only.  q [T, H, R + P] (ldq_t, ldq_h), out [T, H, R] (ldo_t, ldo_h), cache [pages, block_size, R + P];
-// singles: requests that bring more than one token are left out (their rows of out hold nothing afterwards).
+// singles: requests that bring more than one token are left out (their rows of out are as they were).
 // seq_lens [B]: tokens of each request after the step; row_tiles >= sum_b ceil(n_q(b) * H / BM) with BM from
-// dinfer_attention_latent_tc_rows(R, max_q_len * H); splits > 1 needs part [T * H * splits * R] and ml [T * H * splits * 2].
+// dinfer_attention_latent_tc_rows(R, max_q_len * H); splits > 1 needs part [T * H * splits * R] and ml [T * H * splits * 2]
+// (with singles B in the place of T: a few decoded tokens beside a long prompt share their keys many ways).
 DINFER_API int dinfer_attention_latent_tc(const void* q, int64_t ldq_t, int64_t ldq_h, void* out, int64_t ldo_t,
                                           int64_t ldo_h, const void* cache, const int* block_table, int max_blocks,
                                           const int* cu_seqlens, const int* seq_lens, int T, int B, int H, int R, int P,
@@ -535,7 +543,7 @@ DINFER_API int dinfer_attention_latent_tc(const void* q, int64_t ldq_t, int64_t 
   else { if (nt <= 1) GO(4, 1); else if (nt <= 2) GO(4, 2); else if (nt <= 4) GO(4, 4); else rc = launch_tc<4, 8, 1>(p, row_tiles, stream); }
 #undef GO
   if (rc != 0 || splits == 1) return rc;
-  launch_pdl(attention_latent_fold_kernel, dim3(T * H), dim3(128), 0, stream, (const float*)part, (const float*)ml,
-             (__nv_bfloat16*)out, ldo_t, ldo_h, T * H, H, R, splits, sinks);
+  launch_pdl(attention_latent_fold_kernel, dim3((singles ? B : T) * H), dim3(128), 0, stream, (const float*)part, (const float*)ml,
+             (__nv_bfloat16*)out, ldo_t, ldo_h, H, R, splits, sinks, singles ? cu_seqlens : (const int*)nullptr);
   return cuda_status("attention_latent_fold");
 }

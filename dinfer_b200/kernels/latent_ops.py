@@ -142,8 +142,8 @@ def attention_latent_tc(q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Ten
     """The same attention on tensor cores (bfloat16): prompt portions and decoded tokens in one launch.  ``seq_lens`` [B]:
     tokens of each request after the step (a token's position follows from it); ``max_q_len``: the longest portion of
     the batch (chooses the row tile); ``max_seq_len``: the longest request (chooses how many CTAs share a row tile's keys
-    unless ``splits`` says).  ``singles``: only for the requests that bring one token; the rows of the others hold
-    nothing afterwards."""
+    unless ``splits`` says).  ``singles``: only for the requests that bring one token; the rows of the others are
+    left as they are."""
     T, H = _check_attention(q_lat, out, cache, block_table, cu_seqlens, kv_rank, rope_dim)
     require_cuda(seq_lens)
     _check_sinks(sinks, H)
@@ -159,8 +159,9 @@ def attention_latent_tc(q_lat: torch.Tensor, out: torch.Tensor, cache: torch.Ten
         splits = tc_splits(row_tiles, max_seq_len)
     part = ml = None
     if splits > 1:
-        part = torch.empty((T * H * splits * kv_rank,), dtype=torch.float32, device=q_lat.device)
-        ml = torch.empty((T * H * splits * 2,), dtype=torch.float32, device=q_lat.device)
+        n = (B if singles else T) * H
+        part = torch.empty((n * splits * kv_rank,), dtype=torch.float32, device=q_lat.device)
+        ml = torch.empty((n * splits * 2,), dtype=torch.float32, device=q_lat.device)
     lib, f = _fn("attention_latent", "dinfer_attention_latent_tc",
                  [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                   c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,

@@ -187,6 +187,40 @@ def test_both_ways_of_the_part_agree(reqs, window, gate, sink, monkeypatch):
         assert torch.equal(got[a:z], outs[1][a:z])
 
 
+@pytest.mark.parametrize("order", [(0, 1, 2), (1, 0, 2), (1, 2, 0)])
+def test_few_single_tokens_beside_a_long_portion(order):
+    """Decoded tokens beside a portion share their keys many ways: the workspace follows their number, not the portion's, and
+    the portion's rows stay as they are.  Against plain 64-bit formulas."""
+    from dinfer_b200.kernels import latent_ops as L
+    R, P, H, page, scale = 128, 32, 4, 16, 0.1
+    reqs = [[(0, 3000), (3999, 1), (130, 1)][i] for i in order]
+    cu, seq, table, pages = batch(reqs, page, 5)
+    T = int(cu[-1])
+    g = torch.Generator().manual_seed(9)
+    cache = torch.randn(pages, 1, 1, page, R + P, generator=g).to(torch.bfloat16)
+    q = torch.randn(T, H, R + P, generator=g).to(torch.bfloat16)
+    out = torch.full((T, H, R), 7.0, dtype=torch.bfloat16, device="cuda")
+    args = (q.cuda(), out, cache.cuda(), table.cuda(), cu.cuda(), seq.cuda())
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    L.attention_latent_tc(*args, R, P, scale, max_q_len=3000, max_seq_len=4000, singles=True)
+    # at most 64 ways: sums of R and two numbers for each of 3 requests' heads
+    assert torch.cuda.max_memory_allocated() - held <= 2 * 3 * H * 64 * (R + 2) * 4 + 4096
+    out = out.cpu()
+    for i, (h, n) in enumerate(reqs):
+        t0 = int(cu[i])
+        if n > 1:
+            assert bool((out[t0:t0 + n] == 7.0).all())
+            continue
+        j = torch.arange(h + 1)
+        rows = cache[table[i].long()[j // page], 0, 0, j % page].double()
+        p = torch.softmax(q[t0].double() @ rows.T * scale, dim=1)
+        o = p @ rows[:, :R]
+        # weights rounded to bfloat16 (2^-9 each, against sums that are not), the result (2^-9), scores in 32-bit
+        assert bool(((out[t0].double() - o).abs() <= 2.0 ** -8 * (p @ rows[:, :R].abs()) + 2.0 ** -8 * o.abs() + 1e-5).all())
+
+
 def test_captured_steps_run_over_expanded_latents_too(monkeypatch):
     """Prompts taken in portions of the whole budget beside decoded tokens, kernel by kernel and as graphs: the same logits
     up to rounding, and the graph's bounds hold prompts of other lengths than it was captured on."""
