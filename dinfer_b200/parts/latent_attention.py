@@ -143,22 +143,37 @@ class LatentAttention(Mixer):
         q = self.uq(low[:, :Rq])                                         # [T, H (D + P)]
         expanded = self._expanded(ctx, q.dtype)
         # (a dummy portion of one token in a captured graph belongs to neither way: its row has to hold something finite)
-        make = torch.zeros if expanded is not None and ctx.decode_splits and not ctx.any_decode else torch.empty
+        make = torch.zeros if expanded is not None and ctx.decode_splits else torch.empty
         o = make((T, H, V), dtype=q.dtype, device=q.device)
         if expanded is None or ctx.any_decode:
             # head-major storage, seen as [T, H, *]: the batched products then write whole matrices per head
             q_lat = torch.empty((H, T, R + P), dtype=q.dtype, device=q.device).transpose(0, 1)
-            self.absorb(q.view(T, H, D + P)[:, :, :D], self.uk_t, q_lat[:, :, :R])
-            latent_ops.latent_q_rope(q, ctx.positions, table, q_lat, H, D, P, R, halves=self.halves)
             o_lat = torch.empty((H, T, R), dtype=q.dtype, device=q.device).transpose(0, 1)
+            rows = (q, ctx.positions, q_lat, o_lat, o)
+            if expanded is not None:                         # the rows from the first single token to the last
+                a, z = self._single_rows(ctx)
+                rows = tuple(t[a:z] for t in rows)
+            q_, positions, q_lat_, o_lat_, o_ = rows
+            self.absorb(q_.view(-1, H, D + P)[:, :, :D], self.uk_t, q_lat_[:, :, :R])
+            latent_ops.latent_q_rope(q_, positions, table, q_lat_, H, D, P, R, halves=self.halves)
             self.attend(q_lat, o_lat, cache.kv, g, ctx, singles=expanded is not None)
-            self.absorb(o_lat, self.uv, o)
+            self.absorb(o_lat_, self.uv, o_)
         if expanded is not None:
             self.attend_expanded(q, o, cache.kv, g, ctx, table, *expanded)
         o = o.view(T, H * V)
         if self.gate_name:
             ops.sigmoid_gate(o, full[:, self.gate_at:self.gate_at + H * V])
         return self.o(o, out_dtype=torch.float32 if self.out_float32 else None)
+
+    @staticmethod
+    def _single_rows(ctx: StepContext):
+        """(first row, end) of the requests that bring one token, with what lies between them.  (In a captured graph they are the
+        batch's last places.)"""
+        if "single_rows" not in ctx.derived:
+            cu = ctx.cu_seqlens_host
+            rows = [cu[i] for i in range(len(cu) - 1) if cu[i + 1] - cu[i] == 1]
+            ctx.derived["single_rows"] = (rows[0], rows[-1] + 1)
+        return ctx.derived["single_rows"]
 
     # rows up to which the per-head products run on this package's own kernel (each weight read once, 32-bit
     # multiply-adds); beyond, bfloat16 goes to the library's batched product like the other prompt-sized products

@@ -187,6 +187,19 @@ def test_both_ways_of_the_part_agree(reqs, window, gate, sink, monkeypatch):
         assert torch.equal(got[a:z], outs[1][a:z])
 
 
+@pytest.mark.parametrize("reqs,rows", [([(0, 129), (500, 1), (40, 1)], 2), ([(500, 1), (0, 129), (0, 2), (40, 1), (3, 7)], 133), ([(9, 1), (0, 300)], 1)])
+def test_the_absorbing_products_see_the_single_tokens_only(reqs, rows, monkeypatch):
+    """Beside portions over expanded latents: the rows from the first single token to the last."""
+    from dinfer_b200.parts.latent_attention import LatentAttention
+    monkeypatch.setattr(LatentAttention, "RATES", EXPANDED)
+    monkeypatch.setattr(LatentAttention, "MIXED_HOST", 0.0, raising=False)
+    seen, absorb = [], LatentAttention.absorb
+    monkeypatch.setattr(LatentAttention, "absorb", lambda self, a, w, out: (seen.append((a.shape[0], out.shape[0])), absorb(self, a, w, out))[1])
+    part, ctx, cache, x = part_and_context(reqs)
+    y = part.forward(x, ctx, cache)
+    assert seen == [(rows, rows)] * 2 and bool(torch.isfinite(y.float()).all())
+
+
 @pytest.mark.parametrize("order", [(0, 1, 2), (1, 0, 2), (1, 2, 0)])
 def test_few_single_tokens_beside_a_long_portion(order):
     """Decoded tokens beside a portion share their keys many ways: the workspace follows their number, not the portion's, and
