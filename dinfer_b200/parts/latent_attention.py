@@ -192,6 +192,9 @@ class LatentAttention(Mixer):
     # the portion.  Expanded: flops a second of the product, bytes a second of the gather, seconds a CTA of the attention takes
     # for a tile of 128 keys with one and with both of its row tiles.
     RATES = (150e12, 6e11, 6e-6, 1000e12, 3e12, 1.8e-6, 2.85e-6)
+    # Beside decoded tokens the expanded way's launches come on top of the absorbed one's.  Kernel by kernel that is so much more
+    # of the host (s), which such a step is waiting for: 200 us a layer and 258 on the machine that was measured.
+    MIXED_HOST = 76e-6
     # the keys and values of a step's portions, all heads, are expanded at once up to so many bytes
     EXPANDED_BYTES = 256 << 20
 
@@ -202,10 +205,17 @@ class LatentAttention(Mixer):
         long history are the absorbed form's.  A layer of 16 heads of 128 + 64, R 512, absorbed and expanded (us): a prompt of
         64 tokens 52 and 37, of 2048 565 and 134; 64 tokens behind 4000 129 and 118, behind 16000 291 and 352; 256 behind
         16000 1187 and 493; 8 heads of 64 + 32, R 256: 64 behind 4000 59 and 86.
-        In a captured graph the lengths are bounds: the tokens spread evenly over the prompt places without a history for what the absorbed form costs at least, every place as long as it may get
-        for what the other one costs at most."""
+        With decoded tokens in the step the absorbing products run for them all the same, and its launches too: nothing but the
+        portions' attention is saved.  Eight tokens at 1000 beside a prompt, the same layer, as a graph and kernel by kernel:
+        128 tokens 90 and 71, 200 and 258; 600 199 and 92, 216 and 265; 1024 299 and 118, 318 and 263; 2048 670 and 170, 683
+        and 262; 64 behind 4000 160 and 165, 203 and 258; 256 behind 2000 210 and 136, 224 and 259; behind 4000 323 and 200, 337
+        and 264.
+        In a captured graph the lengths are bounds: the tokens spread evenly over the prompt places without a history for what
+        the absorbed form costs at least, every place as long as it may get for what the other one costs at most."""
         if self.ukv is None or dtype != torch.bfloat16 or not ctx.any_prefill or not ctx.cu_seqlens_host:
             return None
+        if ctx.any_decode and not latent_ops.tc_supported(dtype, self.R, self.P):
+            return None                                      # the plain kernel for the single tokens does all rows at once
         key = ("latent_expanded", self.H, self.D, self.P, self.V, self.R, self.window)
         if key not in ctx.derived:
             ctx.derived[key] = self._expanded_shape(ctx)
@@ -234,12 +244,18 @@ class LatentAttention(Mixer):
         if window:
             pairs = min(pairs, float(window) * tokens)
             seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
-        rows = latent_ops.expanded_rows(bound, window)
         flops, weight_rate, products, expanding, gather, one, both = self.RATES
         H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
+        absorbed = pairs * H * 2 * (2 * R + P + 100) / flops
+        if not ctx.any_decode:
+            absorbed += H * R * (D + V) * 2 / weight_rate + products
+        elif not ctx.decode_splits:
+            absorbed -= self.MIXED_HOST
+        if absorbed <= 0.0:
+            return None
+        rows = latent_ops.expanded_rows(bound, window)
         walks = [(count, ((keys + 127) // 128) * (both if n > 128 else one)) for count, n, keys in seen]
         walking = max(max(w for _, w in walks), H * sum(count * w for count, w in walks) / num_sms())
-        absorbed = pairs * H * 2 * (2 * R + P + 100) / flops + H * R * (D + V) * 2 / weight_rate + products
         expanded = rows * R * H * 2 * (D + V) / expanding + rows * (R + P) * 4 / gather + walking
         if absorbed <= expanded or rows * H * (D + V) * 2 > self.EXPANDED_BYTES or tiles > 65535:
             return None
