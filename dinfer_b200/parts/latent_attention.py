@@ -117,13 +117,13 @@ class LatentAttention(Mixer):
         # [H (D + V), R]: what makes a row's keys and values of all heads, head after head
         self.ukv = None
         if latent_ops.expanded_supported(t["uk"].dtype, self.R, self.P, self.D, self.V) and t["uv"].dtype == t["uk"].dtype:
-            self.ukv = torch.cat([t["uk"].reshape(self.H, self.D, self.R), self.uv], dim=1).reshape(-1, self.R).contiguous()
+            self.ukv = Linear(torch.cat([t["uk"].reshape(self.H, self.D, self.R), self.uv], dim=1).reshape(-1, self.R))
 
     def cache_need(self):
         return KvCacheNeed(1, self.R + self.P, self.window, int(self.page_size) if self.page_size else None, planes=1)
 
     def kernel_libraries(self):
-        expanded = ["latent_expanded", "gemm_tc"] if self.ukv is not None and self.env.act_dtype == torch.bfloat16 else []
+        expanded = ["latent_expanded"] + self.ukv.kernel_libraries() if self.ukv is not None and self.env.act_dtype == torch.bfloat16 else []
         return (["latent_post", "attention_latent", "gemm_f32"] + expanded + (["elementwise"] if self.gate_name else []) + self.down.kernel_libraries() + self.uq.kernel_libraries()
                 + self.o.kernel_libraries())
 
@@ -265,9 +265,7 @@ class LatentAttention(Mixer):
         window = int(self.window or 0)
         latent_ops.latent_q_turn(q, ctx.positions, table, self.H, self.D, self.P, halves=self.halves)
         latents = latent_ops.latent_rows(kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, rows, window)
-        expanded = torch.empty((rows, self.ukv.shape[0]), dtype=q.dtype, device=q.device)
-        add_launches(1)
-        torch.mm(latents[:, :self.R], self.ukv.t(), out=expanded)
+        expanded = self.ukv(latents[:, :self.R])
         latent_ops.attention_latent_umma(q, o, latents, expanded, ctx.cu_seqlens, ctx.seq_lens, self.R, self.P, self.D,
                                          self.scale, window, sinks=self.sinks, pair_bound=tiles)
 
