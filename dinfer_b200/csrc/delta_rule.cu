@@ -117,9 +117,15 @@ delta_prep_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv,
 // The same for steps of many tokens (four taps; heads of 64 or 128 key channels that fill blocks of 128 channels): a thread
 // owns a channel and walks RUN tokens with the last three inputs in registers, so that an input is read 11 / 8 times
 // instead of four, and the block's eight norms are summed in one exchange.  Bound by the exponentials and divisions of
-// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) 41 us, a block per (token, head) 64.
+// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) 40.5 us, a block per (token, head) 59.
+// Tokens of a run that spans requests (or begins a portion) go one after the other, with a search and loads of their own, so
+// it is taken for portions: from RUN_FROM tokens and RUN_PORTION tokens a request on (256 for a request alone).  us, a block
+// per (token, head) and in runs, 16 heads of 128: 128 tokens 10.2 and 10.6, 256 13.4 and 12.9, 512 19.6 and 16.3; 32 requests of
+// 16 25.0 and 23.5, 64 of 8 27.3 and 31.0, 64 of 16 43.8 and 39.1; 64 single tokens and 64 of a portion 14.5 and 24.0, 16 and
+// 240 16.2 and 21.6, 16 and 496 23.8 and 22.8; 512 single tokens 45.7 and 51.8.  (16 heads of 64: 256 tokens 12.0 and 10.8, 32
+// of 16 20.9 and 18.6, 16 and 496 20.1 and 20.4.)
 constexpr int RUN = 8;
-constexpr int RUN_FROM = 64;                               // tokens of a step from which it is taken (fewer leave SMs idle)
+constexpr int RUN_FROM = 512, RUN_FROM_ALONE = 256, RUN_PORTION = 16;
 template <typename TA>
 __global__ void __launch_bounds__(128)
 delta_prep_run_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv, int cb, const TA* __restrict__ A,
@@ -505,6 +511,12 @@ delta_post_kernel(const float* __restrict__ o, const float* __restrict__ w, cons
 
 DINFER_DEFINE_LAST_ERROR()
 
+// Whether the preparation of a step of T tokens and B requests walks runs of tokens.
+DINFER_API int dinfer_delta_prep_runs(int T, int B, int G, int dk, int taps) {
+  return taps == 4 && (dk == 64 || dk == 128) && (2 * G * dk) % 128 == 0 && T >= (B == 1 ? RUN_FROM_ALONE : RUN_FROM) &&
+         (int64_t)B * RUN_PORTION <= T;
+}
+
 DINFER_API int dinfer_delta_prep(const void* P, int64_t ldp, int cq, int ck, int cv, int cb, const void* A, int64_t lda,
                                  const float* conv_w, const float* A_log, const float* dt_bias, float* hist,
                                  int64_t hist_stride, const int* cu, const int* slots, const int* fresh, int B,
@@ -520,7 +532,7 @@ DINFER_API int dinfer_delta_prep(const void* P, int64_t ldp, int cq, int ck, int
   const int jobs = 2 * G + (nv + PREP_CHUNK - 1) / PREP_CHUNK + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
   if (jobs > 65535) return refuse(DINFER_BAD_ARGUMENT, "delta_prep: too many heads for the grid");
   const int run_jobs = (2 * nq + nv + 127) / 128 + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
-  const bool runs = taps == 4 && (dk == 64 || dk == 128) && (2 * nq) % 128 == 0 && T >= RUN_FROM && run_jobs <= 65535;
+  const bool runs = dinfer_delta_prep_runs(T, B, G, dk, taps) && run_jobs <= 65535;
   DINFER_DISPATCH_DTYPE(act_dtype, TA, {
     if (runs)
       launch_pdl(delta_prep_run_kernel<TA>, dim3((T + RUN - 1) / RUN, run_jobs), dim3(128), 0, stream, (const TA*)P, ldp, cq, ck,

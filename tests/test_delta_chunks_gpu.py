@@ -129,15 +129,26 @@ def test_sizes_the_chunks_do_not_take_stay_with_the_token_loop():
         assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("lens,runs", [([1] * 64, False), ([1] * 512, False), ([64], False), ([255], False), ([256], True), ([8] * 64, False),
+                                       ([16] * 32, True), ([1] * 16 + [240], False), ([1] * 31 + [481], True), ([100, 411], False),
+                                       ([1, 2, 470, 64, 9, 3], True)])
+def test_which_steps_are_prepared_in_runs(lens, runs):
+    """Portions of many tokens; decoded tokens and short portions keep a block per (token, head)."""
+    from dinfer_b200.kernels.lib import library
+    takes = library("delta_rule").dinfer_delta_prep_runs
+    assert bool(takes(sum(lens), len(lens), 8, 128, 4)) is runs
+    assert not takes(sum(lens), len(lens), 8, 128, 3) and not takes(sum(lens), len(lens), 8, 32, 4) and not takes(sum(lens), len(lens), 3, 96, 4)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,dk,dv,per_channel", [(3, 1, 64, 40, False), (3, 3, 64, 16, True), (2, 1, 128, 72, False)])
 def test_preparation_in_runs(dtype, H, G, dk, dv, per_channel):
-    """Steps of 64 tokens and more (a thread walks eight tokens of a channel) against plain formulas and, beside the short
+    """Steps of many tokens (a thread walks eight tokens of a channel) against plain formulas and, beside the short
     steps' kernel, request by request: requests that begin and end anywhere in a run, fresh and carried histories."""
     from dinfer_b200.kernels import delta_ops
     F64 = torch.float64
     g = torch.Generator().manual_seed(dk + dv + H)
-    lens, fresh, taps = [1, 2, 70, 64, 9, 3], [1, 0, 1, 0, 0, 1], 4
+    lens, fresh, taps = [1, 2, 470, 64, 9, 3], [1, 0, 1, 0, 0, 1], 4
     T, B, nq, nv = sum(lens), len(lens), G * dk, H * dv
     C, nd = 2 * nq + nv, H * dk if per_channel else H
     Pm = torch.randn(T, C + H + 5, generator=g).to(dtype)
