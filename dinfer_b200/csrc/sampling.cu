@@ -1,5 +1,5 @@
-// Sampling on f32 logits.  A row is shared by a thread-block cluster of ROW_CTAS CTAs of 1024 threads:
-// every CTA keeps its contiguous slice of the row (scaled by 1/temperature) in shared memory, so the
+// Sampling on f32 logits.  A row is shared by a thread-block cluster of ROW_CTAS CTAs (of 512 threads in the sampler, of 1024
+// in argmax): every CTA keeps its contiguous slice of the row (scaled by 1/temperature) in shared memory, so the
 // row is read from memory once, and the CTAs exchange their partial results through each other's
 // shared memory (st.shared::cluster + one cluster barrier per exchange).
 //
@@ -15,14 +15,14 @@
 //
 // Same contract as the reference (crates/kernels/cuda/sampling.cu:13-56,60-133,143-157,196-283,
 // 322-349; order of operations models/qwen3/src/executor.rs:552-605).  Unlike it the logits are not
-// rewritten: the three filters reduce to one keep-threshold on the scaled logits.  The top-k and the
-// top-p threshold are each found by a radix-16 descent over the order-preserving 32-bit image of a
-// float (eight rounds, every round one pass over shared memory): the largest value t such that the
-// kept entries >= t number at least k (have at least the share p of the mass).  Where at most CAND_MAX
-// entries decide (nearly always) both take a short way instead: one pass counts (and weighs) the
-// entries above a few cuts below the maximum, the entries above the first cut that is enough are
-// collected in every CTA, sorted, and both thresholds read off.  All sums are taken in a fixed order
-// (segment, warp of segments, CTA rank), so the same logits, seed and count give the same token.
+// rewritten: the three filters reduce to one keep-threshold on the scaled logits, the largest value t such that the kept entries
+// >= t number at least k (have at least the share p of the mass).  A pass over the row in shared memory counts (and weighs)
+// the entries above a few cuts below the maximum; further ones cut up the gap that holds the threshold, until at most
+// CAND_MAX entries are left in it (the first pass, nearly always).  Those are collected in every CTA and sorted, and the
+// threshold is read off; for a small k the whole top of the row is collected, so that top-p is read off it too.  Where more
+// entries than that crowd the gap to the end, a radix-16 descent over the order-preserving 32-bit image of a float goes on
+// inside it.  All sums are taken in a fixed order (segment, warp of segments, CTA rank), so the same logits, seed and count
+// give the same token.
 #include "common.cuh"
 
 using namespace dinfer;
@@ -41,6 +41,10 @@ constexpr int VT = 2;
 constexpr int NT = SEGMENTS / VT;           // threads of the sampling kernel
 constexpr int ROW_CTAS = 8;                 // cluster size: CTAs that share a row
 constexpr int MAX_SLICE = 48 * 1024;        // floats of a row slice that shared memory holds (192 KB)
+// Dynamic shared memory that keeps a second CTA of the sampling kernel off an SM.  With as few rows as find an SM for every CTA
+// two of them share one all the same otherwise: 8 rows without likely tokens, top-p 0.9 42 us on shared SMs and 37 apart, top-k
+// 1000 35 and 31.
+constexpr size_t LONE_SMEM = 110 * 1024;
 constexpr int XCH = 16;                     // floats a CTA hands to the others per exchange
 constexpr int ARGMAX_MANY_ROWS = 40;        // from so many rows on the argmax runs a CTA per row
 
@@ -200,23 +204,31 @@ struct Slice {
   __device__ __forceinline__ int end(int u) const { return min(n_mine, (u + 1) * seg); }
 };
 
-// The largest value t such that the entries x >= max(t, floor_) weigh at least `target`, where an
-// entry weighs 1 (MASS = false) or exp(x - m) (MASS = true).  Radix-16 descent over float_key:
-// `above` is the weight of the entries beyond the digits fixed so far.
-template <bool MASS>
-__device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, float m, float floor_, float target) {
-  uint32_t prefix = 0;
+// Where a threshold is known to lie: the float_key from `base` on, `width` more at most, and the weight of the entries beyond.
+struct Bracket {
+  uint32_t base = 0, width = 0xffffffffu;
   float above = 0.f;
+};
+
+// The largest value t of the bracket such that the entries x >= max(t, floor_) weigh at least `target`, where an
+// entry weighs 1 (MASS = false) or exp(x - m) (MASS = true).  Radix-16 descent over float_key - base: `above` is the
+// weight of the entries beyond the digits fixed so far.  Eight passes over the row for all floats, fewer for a bracket.
+template <bool MASS>
+__device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, float m, float floor_, float target,
+                                 const Bracket& where) {
+  uint32_t prefix = 0;
+  float above = where.above;
+  const int first = where.width ? (31 - __clz(where.width)) & ~3 : 0;
 #pragma unroll 1
-  for (int shift = 28; shift >= 0; shift -= 4) {
+  for (int shift = first; shift >= 0; shift -= 4) {
     float tot[16];
     row_sum<16>(sh, rank, tot, [&](int u, float (&h)[16]) {
       const int i1 = sl.end(u);
       for (int i = sl.begin(u); i < i1; ++i) {
         const float x = sl.at(i);
         if (!(x >= floor_)) continue;
-        const uint32_t k = float_key(x);
-        if (shift < 28 && (k >> (shift + 4)) != (prefix >> (shift + 4))) continue;
+        const uint32_t k = float_key(x) - where.base;      // (a key below the base wraps beyond the width)
+        if (k > where.width || (shift < first && (k >> (shift + 4)) != (prefix >> (shift + 4)))) continue;
         const float w = MASS ? expf(x - m) : 1.f;
         const int dgt = (k >> shift) & 15;
 #pragma unroll
@@ -237,13 +249,13 @@ __device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, flo
     above = run;
     prefix |= (uint32_t)chosen << shift;
   }
-  return key_float(prefix);
+  return key_float(where.base + prefix);
 }
 
 // ---- the short way to the two thresholds: where at most CAND_MAX entries hold the k largest, or the share p of the mass
 constexpr int CAND_MAX = 1024;
 constexpr int CUTS = 8;                       // cuts a pass counts at, the last one the floor
-constexpr int CUT_ROUNDS = 3;
+constexpr int CUT_ROUNDS = 4;
 static_assert(CAND_MAX <= SEGMENTS && 2 * CUTS <= XCH, "a candidate per segment; counts and masses in one exchange");
 
 struct Candidates {
@@ -282,15 +294,19 @@ __device__ __forceinline__ void segment_scan(int (&v)[VT], int* warp_tot, int& t
 
 // The highest of a few cuts c such that the kept entries (x >= floor_) with x >= c are enough: at least k of them (MASS
 // false), or at least the share p of the mass of all kept ones (true; `denom` is then that mass).  The first pass cuts at
-// fixed distances below the maximum (x is in units of the softmax's exponent), further ones inside the gap where the count
-// goes from too few to more than CAND_MAX.  Returns whether a cut with at most CAND_MAX entries was found.
+// fixed distances below the maximum (x is in units of the softmax's exponent), further ones inside the gap between the lowest
+// cut that is not enough and the highest that is.  Returns whether at most CAND_MAX entries are left to look through: with
+// `whole` those from the cut up, else those of the gap, from the cut up to `below` (gap.above is what lies beyond weighs).
+// Where there are more after CUT_ROUNDS passes, or equal ones crowd a gap of few floats, a descent inside the gap finds the
+// threshold.
 template <bool MASS>
-__device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, float lo, float floor_, float need, float& cut,
-                         float& denom) {
+__device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, float lo, float floor_, float need, bool whole,
+                         float& cut, float& below, float& denom, Bracket& gap) {
   float c[CUTS] = {m - 1.f, m - 2.f, m - 4.f, m - 6.f, m - 9.f, m - 13.f, m - 18.f, floor_};
 #pragma unroll
   for (int j = 0; j < CUTS; ++j) c[j] = fmaxf(c[j], floor_);
-  float target = need;
+  float target = need, hi = m, n_above = 0.f;
+  below = INFINITY;                                        // (no cut that is not enough was met yet)
 #pragma unroll 1
   for (int round = 0; round < CUT_ROUNDS; ++round) {
     float tot[MASS ? 2 * CUTS : CUTS];
@@ -298,7 +314,7 @@ __device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, fl
       const int i1 = sl.end(u);
       for (int i = sl.begin(u); i < i1; ++i) {
         const float x = sl.at(i);
-        const float w = MASS ? (x >= floor_ ? expf(x - m) : 0.f) : 0.f;
+        const float w = MASS ? (x >= c[CUTS - 1] ? expf(x - m) : 0.f) : 0.f;
 #pragma unroll
         for (int j = 0; j < CUTS; ++j) {
           h[j] += x >= c[j] ? 1.f : 0.f;
@@ -307,36 +323,46 @@ __device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, fl
       }
     });
     if (MASS && round == 0) { denom = tot[(MASS ? CUTS : 0) + CUTS - 1]; target = need * denom; }
-    float hi = m, low = c[CUTS - 1], n_above = 0.f, n = tot[CUTS - 1];
+    float n = tot[CUTS - 1];
     bool reached = false;
+    cut = c[CUTS - 1];
 #pragma unroll
     for (int j = 0; j < CUTS; ++j) {
       const float have = MASS ? tot[(MASS ? CUTS : 0) + j] : tot[j];
       if (!reached) {
-        if (have >= target || j == CUTS - 1) { reached = true; low = c[j]; n = tot[j]; }
-        else { hi = c[j]; n_above = tot[j]; }
+        if (have >= target || j == CUTS - 1) { reached = true; cut = c[j]; n = tot[j]; }
+        else { hi = below = c[j]; n_above = tot[j]; gap.above = have; }
       }
     }
-    cut = low;
-    if (n <= (float)CAND_MAX) return true;
-    if (n_above >= (float)CAND_MAX) return false;          // even what is not enough is too many
-    low = fmaxf(low, lo);                                  // (the floor may be -inf)
+    if (whole && n <= (float)CAND_MAX) { below = INFINITY; return true; }
+    if (!whole && n - n_above <= (float)CAND_MAX) return true;
+    const float low = fmaxf(cut, lo);                      // (the floor may be -inf, and masked entries with it)
+    gap.base = float_key(MASS ? low : cut);                // (masked entries have no mass, but they count)
+    gap.width = hi <= lo ? 0u : float_key(hi) - (below < INFINITY ? 1u : 0u) - gap.base;
+    if (gap.width < 256u || (whole && n_above >= (float)CAND_MAX)) return false;
+    const bool masked = low > cut;                         // then the lowest cut but one is the smallest finite entry
+    const float step = (hi - low) * (masked ? 1.f / (CUTS - 1) : 1.f / CUTS);
 #pragma unroll
-    for (int j = 0; j < CUTS - 1; ++j) c[j] = hi - (hi - low) * ((float)(j + 1) * (1.f / CUTS));
+    for (int j = 0; j < CUTS - 1; ++j) c[j] = hi - (float)(j + 1) * step;
+    if (masked) c[CUTS - 2] = low;
     c[CUTS - 1] = cut;
   }
   return false;
 }
 
-// Fills cd.x with the entries from `cut` up (at most CAND_MAX), in vocabulary order, and cd.s with the same from the
-// largest down; returns their number.
-__device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32_t rank, float cut) {
+// Fills cd.x with the entries from `cut` up and below `below` (at most CAND_MAX), in vocabulary order, and cd.s with the same
+// from the largest down; returns their number.
+template <bool GAP>
+__device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32_t rank, float cut, float below) {
   int cnt[VT], end[VT], cta_total;
 #pragma unroll
   for (int vt = 0; vt < VT; ++vt) {
     const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
     int n = 0;
-    for (int i = sl.begin(u); i < i1; ++i) n += sl.at(i) >= cut;
+    for (int i = sl.begin(u); i < i1; ++i) {
+      const float xv = sl.at(i);
+      n += xv >= cut && (!GAP || xv < below);
+    }
     cnt[vt] = end[vt] = n;
   }
   segment_scan(end, cd.warp_tot, cta_total);
@@ -353,7 +379,7 @@ __device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32
     int at = base + end[vt] - cnt[vt];
     for (int i = sl.begin(u); i < i1 && cnt[vt] > 0; ++i) {
       const float xv = sl.at(i);
-      if (xv >= cut && at < CAND_MAX) {
+      if (xv >= cut && (!GAP || xv < below) && at < CAND_MAX) {
         const uint32_t dst = smem_u32(&cd.x[at]);
 #pragma unroll
         for (uint32_t r = 0; r < ROW_CTAS; ++r) st_cluster_f32(dst, r, xv);
@@ -385,9 +411,9 @@ __device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32
   return n;
 }
 
-// The largest of the sorted candidates v >= floor_ such that those >= v hold at least the share p of `denom` (of the mass
-// of the candidates >= floor_ where denom < 0).
-__device__ float topp_of_sorted(Candidates& cd, int n, float m, float floor_, float p, float denom) {
+// The largest of the sorted candidates v >= floor_ such that those >= v and what weighs `above` beyond them hold at least the
+// share p of `denom` (of the mass of the candidates >= floor_ where denom < 0).
+__device__ float topp_of_sorted(Candidates& cd, int n, float m, float floor_, float p, float denom, float above) {
   const int lane = threadIdx.x & 31;
   float cum[VT];
   if (threadIdx.x == 0) cd.found = n;
@@ -405,7 +431,7 @@ __device__ float topp_of_sorted(Candidates& cd, int n, float m, float floor_, fl
   __syncthreads();
   float before[VT], all = 0.f;
 #pragma unroll
-  for (int vt = 0; vt < VT; ++vt) before[vt] = 0.f;
+  for (int vt = 0; vt < VT; ++vt) before[vt] = above;
 #pragma unroll 8
   for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) {
     const float t = cd.warp_mass[w];
@@ -485,8 +511,10 @@ argmax_many_kernel(const float* __restrict__ logits, int64_t ld, int* __restrict
 // What bounds it: the instructions of its passes over the row in shared memory and the cluster barriers between them, not
 // the one read of the row (39 MB for 64 rows of 151936: 6 us).  64 rows, greedy / temperature / top-k 20 + top-p 0.95 /
 // top-p 0.9 in turn, took 165 us with eight radix rounds for the top-p threshold, a shared-memory histogram for the top-k
-// one and one block of 1024 threads to an SM; 58 us now.  Alone, at 8 and 64 rows: top-k 20 + top-p 24 and 118 -> 23 and
-// 57 us, top-p 0.9 72 and 359 -> 29 and 77 us.
+// one and one block of 1024 threads to an SM; 58 us now.  Alone, at 8 and 64 rows: top-k 20 + top-p 24 and 118 -> 22 and
+// 57 us, top-p 0.9 72 and 359 -> 26 and 77 us.  Rows without likely tokens (normal, sigma 1.4 and 4.3), top-p 0.95: 80 and 397,
+// 77 and 381 -> 60 and 204, 46 to 62 and 164 us (90 and 298, 101 and 318 where only whole rows' candidates and a descent over
+// all floats were known); top-k 1000 70 and 344 -> 31 to 45 and 115 to 136.
 __global__ void __launch_bounds__(NT, 2)
 sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
@@ -554,32 +582,31 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   const int k = top_k ? top_k[b] : -1;
   const bool finite = m < INFINITY && m > -INFINITY;      // else nothing is kept, whatever the thresholds
   int n_cand = -1;                                       // >= 0: cand holds every entry from the top-k threshold up
-  float cut, denom = -1.f;
+  float cut, below, denom = -1.f;
+  Bracket gap;                                           // (all floats where no cut is looked for)
   if (k > 0 && k < vocab) {
-    if (k <= CAND_MAX / 2 && finite && find_cut<false>(sh, sl, rank, m, lo, thr, (float)k, cut, denom)) {
-      n_cand = gather_sorted(sh, cand, sl, rank, cut);
-      if (k <= n_cand) thr = fmaxf(thr, cand.s[k - 1]);  // else all of them are kept
+    const bool whole = k <= CAND_MAX / 2;                // a small k leaves the candidates to top-p
+    if (finite && find_cut<false>(sh, sl, rank, m, lo, thr, (float)k, whole, cut, below, denom, gap)) {
+      const int n = whole ? gather_sorted<false>(sh, cand, sl, rank, cut, below) : gather_sorted<true>(sh, cand, sl, rank, cut, below);
+      const int place = whole ? k : k - (int)gap.above;
+      if (place <= n) thr = fmaxf(thr, cand.s[place - 1]);   // else all of them are kept
+      if (whole) n_cand = n;
     } else {
-      thr = fmaxf(thr, radix_threshold<false>(sh, sl, rank, m, thr, (float)k));
+      thr = fmaxf(thr, radix_threshold<false>(sh, sl, rank, m, thr, (float)k, gap));
     }
   }
   const float p = top_p ? top_p[b] : 1.f;
   if (p < 1.f && p > 0.f) {
     if (n_cand >= 0) {
-      thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, -1.f));
-    } else if (finite && find_cut<true>(sh, sl, rank, m, lo, thr, p, cut, denom)) {
-      n_cand = gather_sorted(sh, cand, sl, rank, cut);
-      thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, denom));
-    } else {
-      float all[1];
-      row_sum<1>(sh, rank, all, [&](int u, float (&v)[1]) {
-        const int i1 = sl.end(u);
-        for (int i = sl.begin(u); i < i1; ++i) {
-          const float x = sl.at(i);
-          if (x >= thr) v[0] += expf(x - m);
-        }
-      });
-      thr = fmaxf(thr, radix_threshold<true>(sh, sl, rank, m, thr, p * all[0]));
+      thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, -1.f, 0.f));
+    } else if (finite) {
+      gap = Bracket();
+      if (find_cut<true>(sh, sl, rank, m, lo, thr, p, false, cut, below, denom, gap)) {
+        const int n = gather_sorted<true>(sh, cand, sl, rank, cut, below);
+        thr = fmaxf(thr, topp_of_sorted(cand, n, m, thr, p, denom, gap.above));
+      } else {
+        thr = fmaxf(thr, radix_threshold<true>(sh, sl, rank, m, thr, p * denom, gap));
+      }
     }
   }
 
@@ -831,13 +858,23 @@ DINFER_API int dinfer_sample(const float* logits, int64_t ld, const float* tempe
   // a row slice that fits shared memory is kept there (read once); a longer one is read again every pass
   const int per = (vocab + ROW_CTAS - 1) / ROW_CTAS;
   const int cache_slice = per <= MAX_SLICE ? 1 : 0;
-  const size_t smem = cache_slice ? (size_t)per * sizeof(float) : 0;
+  size_t smem = cache_slice ? (size_t)per * sizeof(float) : 0;
   static bool opted = false;
+  static int lone_rows = 0;                              // rows whose CTAs all run at once with an SM each
   if (!opted) {
     cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SLICE * (int)sizeof(float));
     if (e != cudaSuccess) return refuse((int)e, "sample: shared memory opt-in failed: %s", cudaGetErrorString(e));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(64 * ROW_CTAS); cfg.blockDim = dim3(NT); cfg.dynamicSmemBytes = LONE_SMEM;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = ROW_CTAS; cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.attrs = &cluster; cfg.numAttrs = 1;
+    e = cudaOccupancyMaxActiveClusters(&lone_rows, sample_kernel, &cfg);
+    if (e != cudaSuccess) return refuse((int)e, "sample: cluster occupancy query failed: %s", cudaGetErrorString(e));
     opted = true;
   }
+  if (rows <= lone_rows && smem < LONE_SMEM) smem = LONE_SMEM;
   return launch_rows(sample_kernel, rows, NT, smem, stream, "sample", logits, ld, temperature, top_k, top_p, min_p, seeds,
                      offsets, out, vocab, cache_slice);
 }

@@ -489,6 +489,45 @@ def test_sampling_cuts_and_many_rows(V):
             assert upto >= target - near and upto - float(w[t]) <= target + near, (i, off)
 
 
+@pytest.mark.parametrize("V", [3001, 50001, 151936])
+def test_sampling_thresholds_far_down_a_row(V):
+    """Thresholds below more entries than the short way collects: flat rows (around zero, where floats crowd), rows of few
+    distinct values, one value, masked rows with fewer entries than k; nine rows at once and one at a time.  The draw falls
+    into the token's share of the plain sampler's mass."""
+    from dinfer_b200.sampling import sampler as S
+    g = torch.Generator().manual_seed(V + 1)
+    base = torch.randn(V, generator=g)
+    rounded = (base * 3).bfloat16().float()
+    masked = base.clone()
+    masked[torch.randperm(V, generator=g)[:V - 1500]] = float("-inf")
+    asks = [(-1, 0.5, 0.0), (-1, 0.9, 0.0), (-1, 0.99, 0.0), (-1, 0.999, 1e-3), (1000, 1.0, 0.0), (1000, 0.9, 0.0), (2000, 1.0, 0.0),
+            (2000, 0.95, 0.0), (513, 1.0, 0.2)]
+    R = len(asks)
+    temps, seeds = torch.full((R,), 0.7), torch.arange(R, dtype=torch.int64) + 5
+    topk = torch.tensor([a[0] for a in asks], dtype=torch.int32)
+    topp, minp = torch.tensor([a[1] for a in asks]), torch.tensor([a[2] for a in asks])
+    cols = [dev(t) for t in (temps, seeds, topk, topp, minp)]
+    for row in (base, base * 3, rounded, masked, base + 20.0, torch.zeros(V)):
+        d = dev(row)[None].expand(R, V).contiguous()
+        scaled = row.double() / 0.7
+        weights = []
+        for a in asks:                                        # (a sort cuts through equal values; the kernel keeps all of them)
+            x = P.filter_logits(scaled, *a)
+            weights.append(torch.where(scaled >= x[x > float("-inf")].min(), torch.exp(scaled - scaled.max()), torch.zeros(())))
+        for off in range(4):
+            offs = dev(torch.full((R,), off, dtype=torch.int64))
+            got = S.sample(d, cols[0], cols[1], offs, top_k=cols[2], top_p=cols[3], min_p=cols[4])
+            alone = torch.cat([S.sample(d[i:i + 1], cols[0][i:i + 1], cols[1][i:i + 1], offs[i:i + 1], top_k=cols[2][i:i + 1],
+                                        top_p=cols[3][i:i + 1], min_p=cols[4][i:i + 1]) for i in range(R)])
+            assert torch.equal(got, alone)
+            for i, w in enumerate(weights):
+                # as above: sums off by at most (seg + 5 + 32 + 8) 2^-24 of the total, a threshold by an entry at most
+                t = int(got[i])
+                near = float(w.sum()) * 64 * 2.0 ** -24 + 2 * float(w[w > 0].min())
+                target, upto = P.philox_uniform(int(seeds[i]), off) * float(w.sum()), float(w[:t + 1].sum())
+                assert upto >= target - near and upto - float(w[t]) <= target + near, (i, off)
+
+
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 def test_attention_generic_without_pages(dt):
     """A request whose table holds no page (a dummy row of a captured graph) has no keys: its output is zero and
