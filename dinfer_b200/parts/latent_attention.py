@@ -223,7 +223,7 @@ class LatentAttention(Mixer):
 
     def _expanded_shape(self, ctx: StepContext):
         cu, window = ctx.cu_seqlens_host, int(self.window or 0)
-        lens = [cu[i + 1] - cu[i] for i in range(len(cu) - 1)]
+        lens = [b - a for a, b in zip(cu, cu[1:])]
         if ctx.decode_splits:                                # captured: any place may hold any of the prompt tokens
             tokens, places = sum(n for n in lens if n != 1), sum(n != 1 for n in lens)
             if not tokens:
@@ -231,19 +231,14 @@ class LatentAttention(Mixer):
             longest = ctx.max_prefill_seq_len or ctx.max_seq_len
             bound = [(min(tokens, longest), longest)] * places
             pairs = tokens * tokens / (2.0 * places)
-            tiles = tokens // 256 + places
-            seen = [(tiles, 256, longest)]                   # (CTAs a head, rows of one, keys it walks) at most
         else:
             bound = [(n, s) for n, s in zip(lens, ctx.seq_lens_host) if n > 1]
             if not bound:
                 return None
             tokens = sum(n for n, _ in bound)
             pairs = float(sum(n * (min(s - n, window) if window else s - n) + n * (n + 1) // 2 for n, s in bound))
-            seen = [((n + 255) // 256, n, s - n // 2 if n > 256 else s) for n, s in bound]
-            tiles = sum(count for count, _, _ in seen)
         if window:
             pairs = min(pairs, float(window) * tokens)
-            seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
         flops, weight_rate, products, expanding, gather, one, both = self.RATES
         H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
         absorbed = pairs * H * 2 * (2 * R + P + 100) / flops
@@ -253,6 +248,15 @@ class LatentAttention(Mixer):
             absorbed -= self.MIXED_HOST
         if absorbed <= 0.0:
             return None
+        # (CTAs a head, rows of one, keys it walks), at most
+        if ctx.decode_splits:
+            tiles = tokens // 256 + places
+            seen = [(tiles, 256, longest)]
+        else:
+            seen = [((n + 255) // 256, n, s - n // 2 if n > 256 else s) for n, s in bound]
+            tiles = sum(count for count, _, _ in seen)
+        if window:
+            seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
         rows = latent_ops.expanded_rows(bound, window)
         walks = [(count, ((keys + 127) // 128) * (both if n > 128 else one)) for count, n, keys in seen]
         walking = max(max(w for _, w in walks), H * sum(count * w for count, w in walks) / num_sms())
