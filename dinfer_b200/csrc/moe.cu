@@ -210,7 +210,7 @@ moe_route_table_kernel(const int* __restrict__ tokens, const int* __restrict__ p
 // ---------------------------------------------------------------- pairs laid out expert by expert
 // sorted[pos] = pair index (t * top + k) or `pairs` for padding; tile_expert[tile] = expert of the tile or -1.
 // One block: bound by its chain of passes and, with one counter an expert, by the atomics on it.  So every warp counts (and
-// later deals out) in a copy of its own (as many copies as fit: 32 up to 340 experts), four ids a load, and only the
+// later deals out) in a copy of its own (as many copies as fit: 32 up to 359 experts), four ids a load, and only the
 // positions that pad are written ahead.  16384 pairs over 64 experts: 22 us with one copy, 15 us now.
 constexpr int ALIGN_THREADS = 1024;
 constexpr int ALIGN_INTS = 12 * 1024 - 64;               // of shared memory, without opting in to more

@@ -6,7 +6,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("E,pairs,tile,shift", [(1, 5, 16, 0), (64, 16384, 256, 0), (64, 4095, 64, 0), (33, 4096, 16, 1),
-                                                (340, 8192, 16, 0), (341, 8190, 64, 0), (4095, 9000, 16, 0), (7, 0, 16, 0)])
+                                                (340, 8192, 16, 0), (341, 8190, 64, 0), (359, 8192, 16, 0), (360, 8190, 64, 0),
+                                                (4095, 9000, 16, 0), (7, 0, 16, 0)])
 def test_align_deals_every_pair_once(E, pairs, tile, shift):
     """Pairs of ids outside [0, E) are left out; every expert's run holds its pairs, then padding; nothing else is written."""
     from dinfer_b200.kernels import moe_ops
