@@ -190,9 +190,10 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
       const uint64_t dq = desc_k_major(sQ), dk = desc_k_major(sK);
       const uint64_t dv = desc_mn_major(sV, PART);
       const int n_of[2] = {n_tiles_a, b_on ? n_tiles : 0};
-      // Every 16 elements of D + 64 are multiplied, zeros behind P included, in one straight run: with a condition on P
-      // around each product the compiled code handed later tiles' products wrong descriptors (sums with parts missing, and
-      // reads outside the block's memory).
+      // Every 16 elements of D + 64 are multiplied, zeros behind P included, in one straight run.  (With a run-time bound on the
+      // run, k < (D + P + 15) / 16, sums came out with parts missing and memory outside the block was read.  Why is not known:
+      // nothing documented asks for more than one issuing thread, and the conditions on the step around these runs, here and
+      // in attention_umma.cu, are borne out by every test.  The zeros cost at most four products a tile.)
       auto issue_qk = [&](int w, int t) {
         const uint64_t dqs = dq + (uint64_t)(w * (S::Q_BYTES >> 4));
         const uint64_t dks = dk + (uint64_t)((t % KS) * (S::K_BYTES >> 4));

@@ -264,9 +264,11 @@ gemm_rows_bf16x8_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const 
   store_rows<TC, ROWS>(acc, C + n, ldc, M, lane);
 }
 
-// A matrix up to which 9 to 32 rows go a warp per output column: of 128 x 128, 9 rows 7.9 us and 11.1 on a tile, 32 rows 10.2
-// and 11.5; of 48 x 48, 6.1 and 5.8, 7.8 and 6.2, with 0.7 of the tile's rounding error (lanes sum apart); at K 256 a tile is
-// as fast, at 512 it takes 12 us and a warp a column 19 to 25.
+// A matrix up to which 9 to 32 rows go a warp per output column.  Two reasons: lanes sum apart, which is 0.7 of a tile's
+// rounding error (a model of small 32-bit products amplifies it), and one tile or a few leave the SMs idle.  us on a tile and
+// so, 9 and 32 rows in 32-bit: N 48 K 48 6.1 and 3.5, 6.6 and 4.5; N 128 K 128 11.7 and 5.5, 11.9 and 6.8; N 2048 K 128 11.7 and
+// 6.1, 12.1 and 7.6; N 2048 K 16 4.5 and 3.7, 4.7 and 4.3 (back to back in a graph; every N and K measured between them alike,
+// bfloat16 further apart).  At K 256 a tile is as fast, at 512 it takes 12 us and a warp a column 19 to 25.
 constexpr int FEW_ROWS_K = 128, FEW_ROWS_N = 2048;
 
 int num_sms() {                                             // of the current device, asked once
