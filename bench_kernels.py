@@ -259,7 +259,7 @@ def sampling(vocab, rows_list):
                  ("temperature", lambda i: S.sample(logits, temp, seeds, offs, ints(-1), one, zero, out)),
                  ("top-k 20 + top-p 0.95", lambda i: S.sample(logits, temp, seeds, offs, ints(20), one * 0.95, zero, out)),
                  ("top-p 0.95 alone", lambda i: S.sample(logits, temp, seeds, offs, ints(-1), one * 0.95, zero, out)),
-                 ("top-k 1000 (radix descent)", lambda i: S.sample(logits, temp, seeds, offs, ints(1000), one, zero, out))]
+                 ("top-k 1000", lambda i: S.sample(logits, temp, seeds, offs, ints(1000), one, zero, out))]
         cells = [f"{name} {graph_time_us(fn, 8):6.1f}" for name, fn in cases]
         print(f"rows {R:3d} | " + " | ".join(cells), flush=True)
 
