@@ -197,6 +197,7 @@ class LatentAttention(Mixer):
     MIXED_HOST = 76e-6
     # the keys and values of a step's portions, all heads, are expanded at once up to so many bytes
     EXPANDED_BYTES = 256 << 20
+    _sms = 0                                                # of the device, asked at the first step that weighs the two
 
     def _expanded(self, ctx: StepContext, dtype):
         """Whether the step's portions run over expanded latents: None, or (rows of the gathered latents, row-tile pairs).  The
@@ -223,44 +224,51 @@ class LatentAttention(Mixer):
 
     def _expanded_shape(self, ctx: StepContext):
         cu, window = ctx.cu_seqlens_host, int(self.window or 0)
-        lens = [b - a for a, b in zip(cu, cu[1:])]
+        flops, weight_rate, products, expanding, gather, one, both = self.RATES
+        H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
         if ctx.decode_splits:                                # captured: any place may hold any of the prompt tokens
+            lens = [b - a for a, b in zip(cu, cu[1:])]
             tokens, places = sum(n for n in lens if n != 1), sum(n != 1 for n in lens)
             if not tokens:
                 return None
             longest = ctx.max_prefill_seq_len or ctx.max_seq_len
             bound = [(min(tokens, longest), longest)] * places
             pairs = tokens * tokens / (2.0 * places)
+            tiles = tokens // 256 + places
+            seen = [(tiles, 256, longest)]                   # (CTAs a head, rows of one, keys it walks) at most
         else:
-            bound = [(n, s) for n, s in zip(lens, ctx.seq_lens_host) if n > 1]
+            tokens, pairs, tiles, bound, seen, start = 0, 0, 0, [], [], 0
+            for end, s in zip(cu[1:], ctx.seq_lens_host):    # (one turn over the requests: the host waits for it)
+                n = end - start
+                start = end
+                if n <= 1:
+                    continue
+                count = (n + 255) // 256
+                tokens += n
+                pairs += n * (min(s - n, window) if window else s - n) + n * (n + 1) // 2
+                tiles += count
+                bound.append((n, s))
+                seen.append((count, n, s - n // 2 if n > 256 else s))
             if not bound:
                 return None
-            tokens = sum(n for n, _ in bound)
-            pairs = float(sum(n * (min(s - n, window) if window else s - n) + n * (n + 1) // 2 for n, s in bound))
         if window:
             pairs = min(pairs, float(window) * tokens)
-        flops, weight_rate, products, expanding, gather, one, both = self.RATES
-        H, D, P, V, R = self.H, self.D, self.P, self.V, self.R
+            seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
         absorbed = pairs * H * 2 * (2 * R + P + 100) / flops
         if not ctx.any_decode:
             absorbed += H * R * (D + V) * 2 / weight_rate + products
         elif not ctx.decode_splits:
             absorbed -= self.MIXED_HOST
-        if absorbed <= 0.0:
+        longest_walk = walked = 0.0
+        for count, n, keys in seen:
+            walk = (keys + 127) // 128 * (both if n > 128 else one)
+            longest_walk = max(longest_walk, walk)
+            walked += count * walk
+        if absorbed <= longest_walk:
             return None
-        # (CTAs a head, rows of one, keys it walks), at most
-        if ctx.decode_splits:
-            tiles = tokens // 256 + places
-            seen = [(tiles, 256, longest)]
-        else:
-            seen = [((n + 255) // 256, n, s - n // 2 if n > 256 else s) for n, s in bound]
-            tiles = sum(count for count, _, _ in seen)
-        if window:
-            seen = [(count, n, min(keys, window + 256)) for count, n, keys in seen]
+        self._sms = self._sms or num_sms()
         rows = latent_ops.expanded_rows(bound, window)
-        walks = [(count, ((keys + 127) // 128) * (both if n > 128 else one)) for count, n, keys in seen]
-        walking = max(max(w for _, w in walks), H * sum(count * w for count, w in walks) / num_sms())
-        expanded = rows * R * H * 2 * (D + V) / expanding + rows * (R + P) * 4 / gather + walking
+        expanded = rows * R * H * 2 * (D + V) / expanding + rows * (R + P) * 4 / gather + max(longest_walk, H * walked / self._sms)
         if absorbed <= expanded or rows * H * (D + V) * 2 > self.EXPANDED_BYTES or tiles > 65535:
             return None
         return rows, tiles
