@@ -1,0 +1,79 @@
+// 32-bit operands on the tensor cores: an element x is the sum of three bfloat16 numbers h + m + l (each the rest rounded
+// to nearest; 3 x 8 bits hold the 24 of a 32-bit number), and a product of two such elements is taken as
+// h h' + h m' + m h' + m m' + h l' + l h', every one of them exact, summed in 32-bit.  What is left out (m l', l m', l l')
+// is at most 2^-23 of the product and 2^-26 on average, less than one rounding of a 32-bit sum.
+//
+// Limits: an element of more than 3.39e38 rounds to an infinite h, and an infinite or undefined element has parts that are
+// not numbers, so whatever such an element meets comes out as not a number: a kernel looks at its results and sums those
+// that are not finite again with plain multiply-adds.  An element below 2^-110 (7e-34) keeps its digits down to 2^-133 only.
+#pragma once
+#include "umma_attention.cuh"
+
+namespace dinfer_split {
+
+constexpr int PARTS = 3;
+// the six products, the smallest first: their sums are small while they are added
+constexpr int PRODUCTS = 6;
+__host__ __device__ constexpr int part_a(int i) { constexpr int t[PRODUCTS] = {1, 2, 0, 1, 0, 0}; return t[i]; }
+__host__ __device__ constexpr int part_b(int i) { constexpr int t[PRODUCTS] = {1, 0, 2, 0, 1, 0}; return t[i]; }
+
+// two independent 32-bit sums, each rounded once, in one instruction
+__device__ __forceinline__ uint64_t pair(float a, float b) { return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t c;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  return c;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {     // a - b (the product by -1 is exact)
+  uint64_t c;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(c) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+  return c;
+}
+
+// two elements: their parts packed, the first in the lower half
+__device__ __forceinline__ void split2(float a, float b, uint32_t (&p)[PARTS]) {
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) {
+    p[i] = dinfer_umma::pack_bf16(a, b);
+    if (i + 1 < PARTS) {
+      const uint64_t rest = sub2(pair(a, b), pair(__uint_as_float(p[i] << 16), __uint_as_float(p[i] & 0xffff0000u)));
+      a = __uint_as_float((uint32_t)rest);
+      b = __uint_as_float((uint32_t)(rest >> 32));
+    }
+  }
+}
+// eight elements to the 16 bytes of each part
+__device__ __forceinline__ void split8(const float (&x)[8], uint4 (&p)[PARTS]) {
+  uint32_t q[4][PARTS];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], q[i]);
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) p[i] = make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
+}
+
+// where the 16-byte piece c of row r lies in a tile of 128-byte rows with the 128-byte swizzle (c 0..7), and in one of
+// 64-byte rows with the 64-byte swizzle (c 0..3)
+__device__ __forceinline__ uint32_t swizzled128(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
+__device__ __forceinline__ uint32_t swizzled64(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
+// K-major operand tile with 64-byte rows, 64-byte swizzle: stride between 8-row groups 512 B
+__device__ __forceinline__ uint64_t desc_k_major64(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) |
+         ((uint64_t)4 << 61);
+}
+__device__ __forceinline__ uint4 ld_shared16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared16(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// eight columns of tensor memory, one lane a thread
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& a, const uint4& b) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+}
+// what this thread has written to shared memory is seen by MMAs that start after the barrier it arrives at next
+__device__ __forceinline__ void fence_to_mma() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+}  // namespace dinfer_split

@@ -57,6 +57,11 @@ STATUS_MEANING = {
     35: "attention over expanded latents: the softmax warps waited for a score tile",
     36: "attention over expanded latents: the softmax warps waited for the last P V before writing the output",
     37: "attention over expanded latents: the step's portions pass the rows or row tiles its launch was made for",
+    41: "32-bit product: the splitting warps waited for a free stage",
+    42: "32-bit product: an MMA thread waited for a split stage or a free accumulator",
+    43: "32-bit product: the summing warps waited for a stage's sums",
+    44: "32-bit product: the TMA producer waited for a free stage",
+    45: "32-bit product: the splitting warps waited for an operand tile",
 }
 
 

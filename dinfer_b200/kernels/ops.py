@@ -203,8 +203,15 @@ def cast(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
     return dst
 
 
+def _status(device) -> int:
+    """The device's status word (see gemm_ops), for kernels with bounded waits."""
+    from . import gemm_ops
+    return ptr(gemm_ops._state(device)["status"])
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T, 32-bit multiply-adds on the CUDA cores; each operand f32 or bf16."""
+    """out[M, N] = a[M, K] @ w[N, K]^T to 32-bit accuracy (32-bit elements as three bfloat16 parts on the tensor cores, or
+    32-bit multiply-adds where rows are few); each operand f32 or bf16."""
     require_cuda(a, w, out)
     for t, n in ((a, "a"), (w, "w"), (out, "out")):
         if t.dim() != 2:
@@ -216,9 +223,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tenso
         raise KernelError(f"gemm_f32: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not agree")
     lib, f = _fn("gemm_f32", "dinfer_gemm_f32",
                  [c_void_p, c_int64, c_int, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int,
-                  c_int, c_int, c_int, c_void_p])
+                  c_int, c_int, c_int, c_void_p, c_void_p])
     check(lib, f(ptr(a), a.stride(0), dtype_code(a.dtype), ptr(w), w.stride(0), dtype_code(w.dtype),
-                 ptr(out), out.stride(0), dtype_code(out.dtype), M, N, K, stream_handle()), "gemm_f32")
+                 ptr(out), out.stride(0), dtype_code(out.dtype), M, N, K, _status(a.device), stream_handle()), "gemm_f32")
     return out
 
 
@@ -582,7 +589,7 @@ def gated_act_scaled(x: torch.Tensor, out: torch.Tensor, scale: torch.Tensor, in
 
 def gemm_f32_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """out[:, b, :] = a[:, b, :] @ w[b]^T for every b: a [M, B, K], w [B, N, K], out [M, B, N] (any views whose last
-    axis is contiguous, e.g. the heads of a row); 32-bit multiply-adds on the CUDA cores, operands f32 or bf16."""
+    axis is contiguous, e.g. the heads of a row); as ``gemm_f32``, operands f32 or bf16."""
     require_cuda(a, w, out)
     if a.dim() != 3 or w.dim() != 3 or out.dim() != 3:
         raise KernelError("gemm_f32_batched: a [M, B, K], w [B, N, K], out [M, B, N]")
@@ -594,10 +601,10 @@ def gemm_f32_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> tor
         _rows_contiguous(t, "gemm_f32_batched")
     lib, f = _fn("gemm_f32", "dinfer_gemm_f32_batched",
                  [c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_int64, c_int,
-                  c_int, c_int, c_int, c_int, c_void_p])
+                  c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     check(lib, f(ptr(a), a.stride(0), a.stride(1), dtype_code(a.dtype), ptr(w), w.stride(1), w.stride(0),
                  dtype_code(w.dtype), ptr(out), out.stride(0), out.stride(1), dtype_code(out.dtype), M, N, K, B,
-                 stream_handle()), "gemm_f32_batched")
+                 _status(a.device), stream_handle()), "gemm_f32_batched")
     return out
 
 

@@ -129,6 +129,49 @@ def test_gemm_f32_tiles_and_splits(M, N, K, adt, wdt, cdt):
     assert bool(((out.double().cpu() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(112, 128, 32), (113, 129, 33), (111, 127, 31), (224, 136, 68), (1, 200, 64), (33, 8, 4096), (256, 2048, 96)])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_gemm_f32_extreme_values(M, N, K, batch):
+    """Infinities, values that are not numbers and the largest ones give what plain 32-bit sums give; rows of tiny values keep
+    their digits down to 2^-133 (what a split element keeps), rows with large and small values side by side theirs."""
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, batch, K, generator=g), torch.randn(batch, N, K, generator=g)
+    a *= torch.exp(torch.randn(M, batch, 1, generator=g) * 6)            # rows of all sizes
+    a[M // 2] *= torch.exp(torch.randn(batch, K, generator=g) * 4)
+    a[M // 3] *= 2.0 ** -100
+    plain = torch.einsum("mbk,bnk->mbn", a.double(), w.double())
+    size = torch.einsum("mbk,bnk->mbn", a.double().abs(), w.double().abs())
+    weight = w.double().abs().sum(2)                                      # [batch, N]
+    bound = (K + 1) * 2.0 ** -24 * size + 2.0 ** -133 * weight[None]
+    out = torch.full((M, batch, N), 7.0, device="cuda")
+    ops.gemm_f32_batched(dev(a), dev(w), out)
+    assert bool(((out.double().cpu() - plain).abs() <= bound).all())
+    # one element of a row, one of a weight row: everything they do not meet is as before, bit for bit
+    row, col, k = M - 1, N // 2, K - 1
+    for bad in (math.inf, -math.inf, math.nan, 3.4028234e38):
+        b = a.clone()
+        b[row, batch - 1, k] = bad
+        v = w.clone()
+        v[0, col, k] = -bad
+        got = torch.full((M, batch, N), 7.0, device="cuda")
+        ops.gemm_f32_batched(dev(b), dev(v), got)
+        want = torch.einsum("mbk,bnk->mbn", b.double(), v.double())
+        rest = torch.ones(M, batch, N, dtype=torch.bool)
+        rest[row, batch - 1] = False
+        rest[:, 0, col] = False
+        assert torch.equal(got.cpu()[rest], out.cpu()[rest])
+        hit, want = got.cpu()[~rest], want[~rest]
+        if math.isinf(bad) or math.isnan(bad):
+            assert torch.equal(torch.isnan(hit), torch.isnan(want)) and torch.equal(hit[torch.isinf(hit)].double(), want[torch.isinf(hit)])
+            assert bool((torch.isfinite(hit) == torch.isfinite(want)).all())
+        else:                                                             # beyond 32-bit: infinite; else one large product
+            big = want.abs() > 3.5e38
+            assert bool((torch.isinf(hit[big])).all()) and torch.equal(torch.sign(hit[big]).double(), torch.sign(want[big]))
+            fine = want.abs() < 3.3e38
+            assert bool(((hit.double() - want).abs()[fine] <= (K + 1) * 2.0 ** -24 * 4 * 3.4028234e38).all())
+
+
 @pytest.mark.parametrize("M", [65535 * 64, 65535 * 64 + 1, 65535 * 128])
 def test_gemm_f32_of_millions_of_rows(M):
     """As many row tiles as a grid has, one more, and the most rows a product may have; one more is refused."""
