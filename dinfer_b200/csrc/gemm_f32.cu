@@ -6,8 +6,6 @@
 // (split_umma.cuh; its results are closer to 64-bit ones than those of 32-bit multiply-adds in order), and a
 // warp-per-output-column one for the few rows of a decode step, with plain 32-bit multiply-adds.  The reference has no 32-bit
 // path (its weights are bf16 and its products cuBLASLt: crates/kernels/src/gemm.rs:649-690).
-#include <atomic>
-
 #include "split_umma.cuh"
 
 using namespace dinfer;
@@ -86,6 +84,7 @@ __device__ __noinline__ float plain_sum(const TA* __restrict__ a, const TW* __re
 }
 __device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
 
+constexpr size_t MAX_SMEM = 227 * 1024 - 256;               // (the barriers are static)
 struct TileParams {
   int64_t lda, ldw, ldc, sa, sw, sc;
   int M, N, K, bt, splits, c_fast;
@@ -214,32 +213,30 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
   } else if (warp >= MMA_WARP) {
-    if (lane == 0) {                                            // ---- MMA issue
-      // Two warps take turns, so that one waits (some 300 cycles a barrier, met or not) while the other's MMAs run: one warp
-      // took 1450 cycles a stage whose MMAs take 670.
-      const uint32_t idesc = idesc_bf16(BN, bt, 0);
-      const uint64_t da0 = desc_k_major64(base);
-      for (int j = warp - MMA_WARP; j < n_st; j += MMA_WARPS) {
-        const int s = j % STAGES;
-        if (!mbar_spin(smem_u32(&read_bar[s]), ((j / STAGES) & 1) ^ 1) || !mbar_spin(smem_u32(&full_bar[s]), (j / STAGES) & 1)) {
-          s_abort = 1; atomicExch(p.status, 42);
-          break;
-        }
-        tc_fence_after();
-        const uint64_t da = da0 + s * (st_bytes >> 4);
-        const uint32_t tw = tmem + STAGES * BT + s * W_COLS;
-        uint32_t accumulate = 0;
-#pragma unroll
-        for (int i = 0; i < PRODUCTS; ++i) {
-          if (part_a(i) >= parts_of<TW>() || part_b(i) >= parts_of<TA>()) continue;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {                   // 16 k: eight columns, 32 bytes (in 16-byte units)
-            tc_mma_ts(tmem + s * BT, tw + part_a(i) * (BK / 2) + 8 * k, da + part_b(i) * (a_part >> 4) + 2 * k, idesc, accumulate);
-            accumulate = 1;
-          }
-        }
-        tc_commit(smem_u32(&free_bar[s]));                      // the stage is free, its sums are there
+    // ---- MMA issue.  Two warps take turns, so that one waits (some 300 cycles a barrier, met or not) while the other's MMAs
+    // run: one warp took 1450 cycles a stage whose MMAs take 670.
+    const uint32_t idesc = idesc_bf16(BN, bt, 0), lead = elect_lane(), tm = uniform(tmem);
+    const uint64_t da0 = desc_k_major64(base);
+    for (int j = (int)uniform(warp) - MMA_WARP; j < n_st; j += MMA_WARPS) {
+      const int s = j % STAGES;
+      if (!mbar_spin(smem_u32(&read_bar[s]), ((j / STAGES) & 1) ^ 1) || !mbar_spin(smem_u32(&full_bar[s]), (j / STAGES) & 1)) {
+        s_abort = 1; atomicExch(p.status, 42);
+        break;
       }
+      tc_fence_after();
+      const uint64_t da = da0 + s * (st_bytes >> 4);
+      const uint32_t tw = tm + STAGES * BT + s * W_COLS;
+      uint32_t accumulate = 0;
+#pragma unroll
+      for (int i = 0; i < PRODUCTS; ++i) {
+        if (part_a(i) >= parts_of<TW>() || part_b(i) >= parts_of<TA>()) continue;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) {                     // 16 k: eight columns, 32 bytes (in 16-byte units)
+          mma_ts_if(lead, tm + s * BT, tw + part_a(i) * (BK / 2) + 8 * k, da + part_b(i) * (a_part >> 4) + 2 * k, idesc, accumulate);
+          accumulate = 1;
+        }
+      }
+      commit_if(lead, smem_u32(&free_bar[s]));                  // the stage is free, its sums are there
     }
   } else {                                                      // ---- a stage's sums leave tensor memory
     // warps 0-3 and 4-7 have half of the tile's columns each; TMEM lanes by warp mod 4
@@ -545,7 +542,8 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
     auto k = whole ? gemm_tile_kernel<TA, TW, TC, true> : gemm_tile_kernel<TA, TW, TC, false>;
     const size_t stages = (size_t)STAGES * stage_bytes<TA>(bt) + RAW_STAGES * raw_bytes<TA, TW>(bt), part = (size_t)bt * LDC_S * 4;
     const size_t smem = (stages > part ? stages : part) + 1024;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<uint64_t> done[2];
+    cudaError_t e = allow_shared(k, MAX_SMEM, done[whole]);
     if (e != cudaSuccess) return refuse((int)e, "gemm_f32: shared memory opt-in failed: %s", cudaGetErrorString(e));
     e = launch_pdl_cluster(k, dim3((unsigned)(tiles / batch), 1, batch * splits), dim3(TILE_THREADS), dim3(1, 1, splits), smem, stream,
                            ma, mw, (const TA*)A, (const TW*)W, (TC*)C, p);

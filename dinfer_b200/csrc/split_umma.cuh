@@ -7,9 +7,25 @@
 // not numbers, so whatever such an element meets comes out as not a number: a kernel looks at its results and sums those
 // that are not finite again with plain multiply-adds.  An element below 2^-110 (7e-34) keeps its digits down to 2^-133 only.
 #pragma once
+#include <atomic>
+
 #include "umma_attention.cuh"
 
 namespace dinfer_split {
+
+// Lets a kernel take `bytes` of dynamic shared memory on the current device, once a device (the call costs the host a
+// microsecond a launch); `done` has a bit a device.
+template <typename K>
+inline cudaError_t allow_shared(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 constexpr int PARTS = 3;
 // the six products, the smallest first: their sums are small while they are added
@@ -30,13 +46,16 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {     // a - b 
   return c;
 }
 
-// two elements: their parts packed, the first in the lower half
-__device__ __forceinline__ void split2(float a, float b, uint32_t (&p)[PARTS]) {
+// two elements: their parts packed, the first in the lower half.  LOW: what was rounded off the elements joins the rest behind
+// their first part.
+template <bool LOW = false>
+__device__ __forceinline__ void split2(float a, float b, uint32_t (&p)[PARTS], float a_low = 0.f, float b_low = 0.f) {
 #pragma unroll
   for (int i = 0; i < PARTS; ++i) {
     p[i] = dinfer_umma::pack_bf16(a, b);
     if (i + 1 < PARTS) {
-      const uint64_t rest = sub2(pair(a, b), pair(__uint_as_float(p[i] << 16), __uint_as_float(p[i] & 0xffff0000u)));
+      uint64_t rest = sub2(pair(a, b), pair(__uint_as_float(p[i] << 16), __uint_as_float(p[i] & 0xffff0000u)));
+      if (LOW && i == 0) rest = add2(rest, pair(a_low, b_low));
       a = __uint_as_float((uint32_t)rest);
       b = __uint_as_float((uint32_t)(rest >> 32));
     }
@@ -49,6 +68,36 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4 (&p)[PARTS]) {
   for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], q[i]);
 #pragma unroll
   for (int i = 0; i < PARTS; ++i) p[i] = make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
+}
+
+// the same of x[i] * w, the products' rounding kept
+__device__ __forceinline__ void split8_times(const float (&x)[8], float w, uint4 (&p)[PARTS]) {
+  uint32_t q[4][PARTS];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float a = x[2 * i] * w, b = x[2 * i + 1] * w;
+    split2<true>(a, b, q[i], fmaf(x[2 * i], w, -a), fmaf(x[2 * i + 1], w, -b));
+  }
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) p[i] = make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
+}
+
+// A whole warp walks the MMAs and one lane issues them, so that descriptors and addresses, the same in all lanes, stay in the
+// warp's uniform registers (a branch for one lane alone moves them there for every MMA, 60 to 90 cycles each).
+__device__ __forceinline__ uint32_t elect_lane() {
+  uint32_t lead;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
+  return lead;
+}
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ void mma_ts_if(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+               "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+               ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void commit_if(uint32_t lead, uint32_t bar) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+               "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(lead) : "memory");
 }
 
 // where the 16-byte piece c of row r lies in a tile of 128-byte rows with the 128-byte swizzle (c 0..7), and in one of

@@ -13,7 +13,8 @@
 //                 front of it its convolution's inputs), each element is read and written once.  The decay is applied as S + S * expm1(..), which keeps the digits of a decay just below one.
 //   ssm_prep      requests that bring more: convolution and silu of x, B, C; dt and the decay's logarithm
 //   ssm_sums, ssm_scan, ssm_outputs
-//                 their chunks of 64 tokens side by side.  With c_t the running sum of the decays' logarithms inside a
+//                 their chunks of 64 tokens side by side (of 128 on the tensor cores where the sizes allow it:
+//                 state_space_chunks.cuh).  With c_t the running sum of the decays' logarithms inside a
 //                 chunk, n its tokens and S the state before it:
 //                     U    = sum_s exp(c_n - c_s) dt_s B_s x_s^T              per (chunk, head): needs no state
 //                     S   <- exp(c_n) S + U                                   a walk over the chunks per element of S
@@ -25,7 +26,7 @@
 //
 // A request whose `fresh` flag is set starts from zeros whatever its slot holds.  What a token gets depends on how a
 // request is cut into steps through the order of sums only.
-#include "common.cuh"
+#include "split_umma.cuh"
 
 using namespace dinfer;
 
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(THREADS, RN > 1 ? 3 : 0) ssm_sums_kernel(const
 
 // per V neighbouring elements of S: walk the request's chunks and leave in U's place the S that the chunk starts from;
 // grid (elements / V / THREADS, B).  Eight chunks' loads are in flight, the next eight ahead of the last ones' stores.
-template <int V>
+template <int V, int TOKENS>
 __global__ void __launch_bounds__(THREADS) ssm_scan_kernel(const Params p) {
   constexpr int DEPTH = 8;
   pdl_enter();
@@ -484,10 +485,10 @@ __global__ void __launch_bounds__(THREADS) ssm_scan_kernel(const Params p) {
 #pragma unroll
   for (int e = 0; e < V; ++e) S.x[e] = 0.f;
   if (!p.fresh[b]) S = ldv<V>(S_g);
-  const int64_t slot0 = chunk_slot(t_begin, b, 0);
+  const int64_t slot0 = t_begin / TOKENS + b;
   float* U = p.U + slot0 * total + i;
   const float* dec = p.decay + slot0 * p.H + h;
-  const int chunks = (len + CP - 1) / CP;
+  const int chunks = (len + TOKENS - 1) / TOKENS;
   Vec<V> u[DEPTH], nxt[DEPTH];
 #pragma unroll
   for (int j = 0; j < DEPTH; ++j)
@@ -629,6 +630,8 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
   }
 }
 
+#include "state_space_chunks.cuh"
+
 // ---------------------------------------------------------------- gate, norm, the convolution's inputs
 constexpr int POST_THREADS = 128;
 constexpr int HOLD = 4;                             // runs a thread holds in registers (longer parts read theirs again)
@@ -762,6 +765,24 @@ int launch_sums(const Params& p, int chunks, cudaStream_t stream) {
   return 0;
 }
 
+template <int V>
+void launch_scan(const Params& p, int64_t size, bool wide, cudaStream_t stream) {
+  const dim3 grid((unsigned)((size / V + THREADS - 1) / THREADS), p.B);
+  launch_pdl(wide ? ssm_scan_kernel<V, CU> : ssm_scan_kernel<V, CP>, grid, dim3(THREADS), 0, stream, p);
+}
+
+int num_sms() {                                             // of the current device, asked once
+  static const int n = [] {
+    int dev = 0, v = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
+// chunks on the tensor cores: whole column tiles and 16-byte rows, a state that fits an MMA's rows
+bool umma_takes(int N, int P) { return P % VT == 0 && N % 16 == 0 && N <= CU; }
+
 bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
 
 }  // namespace
@@ -772,7 +793,9 @@ DINFER_DEFINE_LAST_ERROR()
 DINFER_API int64_t dinfer_state_space_work_floats(int64_t T, int B, int H, int G, int N, int P) {
   const int64_t slots = T / CP + B, channels = (int64_t)H * P + 2 * (int64_t)G * N;
   auto r4 = [](int64_t n) { return (n + 3) / 4 * 4; };
-  return r4(T * channels) + 2 * r4(T * H) + slots * H * (int64_t)N * P + r4(slots * H) + slots * G * CP * CP + 4;
+  const int64_t wide = T / CU + B;
+  const int64_t scores = umma_takes(N, P) && wide * CU * CU > slots * CP * CP ? wide * CU * CU : slots * CP * CP;
+  return r4(T * channels) + 2 * r4(T * H) + slots * H * (int64_t)N * P + r4(slots * H) + scores * G + 4;
 }
 
 // The recurrence of a step.  proj: f32 rows [z | x | B | C | dt] of stride ldp; conv_w [channels, taps], conv_b [channels],
@@ -784,7 +807,7 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
                                   const float* dt_bias, const float* A_log, const float* D, float* state, int64_t ld_state,
                                   int hist, const int* cu, const int* slots, const int* fresh, float* y, float* work, int T,
                                   int B, int H, int G, int N, int P, int taps, int single, int portions, int max_q_len,
-                                  cudaStream_t stream) {
+                                  int* status, cudaStream_t stream) {
   if (T < 0 || B <= 0 || H <= 0 || G <= 0 || H % G || N <= 0 || P <= 0 || taps <= 0 || B > 65535)
     return refuse(DINFER_BAD_ARGUMENT, "state_space: bad sizes T=%d B=%d H=%d G=%d N=%d P=%d taps=%d", T, B, H, G, N, P, taps);
   Params p{};
@@ -808,25 +831,39 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
   }
   if (portions) {
     if (!work || !al16(work) || max_q_len <= 0) return refuse(DINFER_BAD_ARGUMENT, "state_space: portions need work space and their longest");
-    const int chunks = (max_q_len + CP - 1) / CP;
-    const int64_t chunk_slots = (int64_t)T / CP + B;
+    // 16-byte loads of the convolved rows, of the states and of y: every width and base allows them
+    const bool vec = P % 4 == 0 && N % 4 == 0 && al16(y);
+    const bool wide = vec && umma_takes(N, P) && status != nullptr;
+    const int tokens = wide ? CU : CP, chunks = (max_q_len + tokens - 1) / tokens;
+    const int64_t chunk_slots = (int64_t)T / tokens + B;
     auto r4 = [](int64_t n) { return (n + 3) / 4 * 4; };
     p.U = work;
     p.cb = p.U + chunk_slots * size;
     if ((chunk_slots * size) % 4) p.cb += 4 - (chunk_slots * size) % 4;
-    p.xbc = p.cb + chunk_slots * G * CP * CP;
+    p.xbc = p.cb + chunk_slots * G * tokens * tokens;
     p.dt = p.xbc + r4((int64_t)T * ch);
     p.la = p.dt + r4((int64_t)T * H);
     p.decay = p.la + r4((int64_t)T * H);
     if (ch % 4 == 0 && ldp % 4 == 0 && inner % 4 == 0 && al16(proj)) launch_prep<4>(p, stream);
     else launch_prep<1>(p, stream);
-    // 16-byte loads of the convolved rows, of the states and of y: every width and base allows them
-    const bool vec = P % 4 == 0 && N % 4 == 0 && al16(y);
+    if (wide) {
+      // 2047 tokens of 64 heads of 128 x 64: sums 75 -> 22 us, walk 30 -> 17, outputs 109 -> 45 (the mixer 434 -> 350); 1024 tokens
+      // of 32 heads 113 -> 96.  Portions of 64 tokens and less take as long as they did.
+      const int per_group = H / G * (P / VT), units = units_of(T / CU + 1, G, per_group, num_sms()), runs = (per_group + units - 1) / units;
+      static std::atomic<uint64_t> sums_done, outputs_done;
+      cudaError_t e = dinfer_split::allow_shared(ssm_sums_umma_kernel, SUMS_SMEM, sums_done);
+      if (e == cudaSuccess) e = dinfer_split::allow_shared(ssm_outputs_umma_kernel, OUTPUTS_SMEM, outputs_done);
+      if (e != cudaSuccess) return refuse((int)e, "state_space: shared memory opt-in failed: %s", cudaGetErrorString(e));
+      const unsigned places = (unsigned)(T / CU + B < (int64_t)chunks * B ? T / CU + B : chunks * B);
+      launch_pdl(ssm_sums_umma_kernel, dim3(places, G * runs + G), dim3(UMMA_THREADS), SUMS_SMEM, stream, p, units, status);
+      if (state_vec) launch_scan<4>(p, size, true, stream); else launch_scan<1>(p, size, true, stream);
+      launch_pdl(ssm_outputs_umma_kernel, dim3(places, G * runs), dim3(UMMA_THREADS), OUTPUTS_SMEM, stream, p, units, status);
+      return cuda_status("state_space");
+    }
     const int rc = N > TP ? (vec ? launch_sums<true, 2>(p, chunks, stream) : launch_sums<false, 2>(p, chunks, stream))
                           : (vec ? launch_sums<true, 1>(p, chunks, stream) : launch_sums<false, 1>(p, chunks, stream));
     if (rc) return rc;
-    if (state_vec) launch_pdl(ssm_scan_kernel<4>, dim3((unsigned)((size / 4 + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
-    else launch_pdl(ssm_scan_kernel<1>, dim3((unsigned)((size + THREADS - 1) / THREADS), B), dim3(THREADS), 0, stream, p);
+    if (state_vec) launch_scan<4>(p, size, false, stream); else launch_scan<1>(p, size, false, stream);
     launch_pdl(vec ? ssm_outputs_kernel<true> : ssm_outputs_kernel<false>, dim3(chunks, H * tiles_v, B), dim3(THREADS), 0, stream, p);
   }
   return cuda_status("state_space");

@@ -203,10 +203,15 @@ def cast(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
     return dst
 
 
-def _status(device) -> int:
+_status_of = None
+
+
+def _status(device):
     """The device's status word (see gemm_ops), for kernels with bounded waits."""
-    from . import gemm_ops
-    return ptr(gemm_ops._state(device)["status"])
+    global _status_of
+    if _status_of is None:                                  # (gemm_ops needs this module first)
+        from .gemm_ops import _state as _status_of
+    return ptr(_status_of(device)["status"])
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:

@@ -9,7 +9,7 @@ from typing import Optional, Tuple
 import torch
 
 from .lib import KernelError, add_launches, check, dtype_code, ptr, require_cuda, stream_handle
-from .ops import _fn
+from .ops import _fn, _status
 
 
 def _rows(t: torch.Tensor, n: int, T: int, what: str) -> None:
@@ -136,7 +136,7 @@ def state_space(P: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_
     ``dt = softplus(dt + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + dt B x^T``, ``y = S^T C + D x`` per request and head, S
     [N, P] carried in the first ``H N P`` floats of row ``slots[b]`` of ``state`` (zero for a fresh request); the
     convolution's earlier inputs are read from behind them and moved on by ``state_space_post``.  Requests that bring one
-    token go through one kernel, the others' chunks of 64 tokens side by side through four; ``any_single`` /
+    token go through one kernel, the others' chunks of 64 or 128 tokens side by side through four; ``any_single`` /
     ``any_portion`` say which there are, ``max_q_len`` (0: not known) bounds the longest portion.  Returns y f32 [T, H * P]."""
     require_cuda(P, conv_w, conv_b, dt_bias, A_log, D, state, cu_seqlens, slots, fresh)
     H, G, N, dv = num_heads, groups, state_dim, value_dim
@@ -154,12 +154,13 @@ def state_space(P: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_
     work = None
     if any_portion:
         size = lib.dinfer_state_space_work_floats
-        size.restype, size.argtypes = c_int64, [c_int64, c_int, c_int, c_int, c_int, c_int]
+        if size.restype is not c_int64:
+            size.restype, size.argtypes = c_int64, [c_int64, c_int, c_int, c_int, c_int, c_int]
         work = torch.empty(size(T, B, H, G, N, dv), dtype=torch.float32, device=P.device)
     check(lib, f(ptr(P), P.stride(0), ptr(conv_w), ptr(conv_b), ptr(dt_bias), ptr(A_log), ptr(D), ptr(state),
                  state.stride(0), hist, ptr(cu_seqlens), ptr(slots), ptr(fresh), ptr(y), ptr(work), T, B, H, G, N, dv, taps,
-                 int(bool(any_single)), int(bool(any_portion)), int(max_q_len) if max_q_len > 0 else T, stream_handle()),
-          "state_space")
+                 int(bool(any_single)), int(bool(any_portion)), int(max_q_len) if max_q_len > 0 else T,
+                 _status(P.device), stream_handle()), "state_space")
     add_launches((1 if any_single else 0) + (4 if any_portion else 0) - 1)
     return y
 

@@ -2,6 +2,7 @@
 that differ in every size replayed whole / with a decoded tail / in portions down to two tokens / mixed on a pool that only
 holds the most demanding step, the trace runner as a process, and greedy generation through ``LLM``."""
 import json
+import math
 import os
 import random
 
@@ -338,6 +339,76 @@ def test_state_space_decays_that_change():
     err = (y.double().cpu().reshape(T, H_, V) - want).abs().amax(dim=2) / want.abs().amax(dim=2).clamp(min=1e-6)
     assert float(err.max()) < 2e-5, float(err.max())
     assert torch.allclose(state[0, :H_ * N * V].double().cpu().reshape(H_, N, V), S, rtol=2e-5, atol=1e-6)
+
+
+def recurrence(proj, A_log, dt_bias, conv_b, H_, G, N, V, S):
+    """The recurrence of one request's projected rows (one tap, weights one) in 64 bits: (y [T, H, V] without D, S at the end)."""
+    inner = H_ * V
+    act = P.silu(proj[:, inner:2 * inner + 2 * G * N].double() + conv_b.double())
+    x, B, Cc = act[:, :inner].reshape(-1, H_, V), act[:, inner:inner + G * N].reshape(-1, G, N), act[:, inner + G * N:].reshape(-1, G, N)
+    dt = P.softplus(proj[:, -H_:].double() + dt_bias.double())
+    g = torch.exp(-torch.exp(A_log.double()) * dt)
+    ys, rep = [], H_ // G
+    for t in range(proj.shape[0]):
+        b, c = B[t].repeat_interleave(rep, 0), Cc[t].repeat_interleave(rep, 0)
+        S = g[t, :, None, None] * S + dt[t, :, None, None] * b[:, :, None] * x[t][:, None, :]
+        ys.append(torch.einsum("hn,hnv->hv", c, S))
+    return torch.stack(ys), x, S
+
+
+def run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V):
+    from dinfer_b200.kernels import gemm_ops, state_ops
+    ch, B = H_ * V + 2 * G * N, len(cu) - 1
+    lens = [cu[i + 1] - cu[i] for i in range(B)]
+    y = state_ops.state_space(dev(proj), torch.ones(ch, 1, device="cuda"), dev(conv_b), dev(dt_bias), dev(A_log), dev(D), state, i32(cu),
+                              i32(list(range(B))), i32(fresh), H_, G, N, V, 1, any_single=1 in lens, any_portion=max(lens) > 1, max_q_len=max(lens))
+    assert gemm_ops.device_status(y.device) == 0
+    return y.double().cpu().reshape(-1, H_, V)
+
+
+@pytest.mark.parametrize("H_, G, N, V", [(4, 2, 16, 64), (2, 1, 128, 128), (6, 2, 48, 64), (16, 1, 64, 64), (9, 1, 112, 64), (3, 3, 80, 192)])
+@pytest.mark.parametrize("lens", [[2, 1, 15, 16, 17], [127, 128, 129], [1, 256, 300], [64, 400]])
+def test_state_space_wide_chunks(H_, G, N, V, lens):
+    """The sizes whose chunks go through the tensor cores: edges of a chunk and of its runs of sixteen tokens, runs of heads that
+    do not divide a group, several column tiles, requests that start from a state and requests that do not, single tokens
+    between them; outputs and states against 64 bits, to 2e-5 of the largest (some 300 roundings of 2^-24)."""
+    g = torch.Generator().manual_seed(H_ * N + len(lens))
+    cu = [0] + list(torch.tensor(lens).cumsum(0))
+    cu = [int(c) for c in cu]
+    T, B = cu[-1], len(lens)
+    proj = torch.randn(T, 2 * H_ * V + 2 * G * N + H_, generator=g)
+    A_log, dt_bias = torch.linspace(-5.0, 1.5, H_), torch.linspace(-1.0, 1.0, H_)
+    conv_b, D = torch.randn(H_ * V + 2 * G * N, generator=g) * 0.3, torch.randn(H_, generator=g)
+    start = torch.randn(B, H_, N, V, generator=g)
+    fresh = [i % 2 for i in range(B)]
+    state = dev(start.reshape(B, -1).clone())
+    got = run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V)
+    for i in range(B):
+        y, x, S = recurrence(proj[cu[i]:cu[i + 1]], A_log, dt_bias, conv_b, H_, G, N, V, torch.zeros_like(start[i]).double() if fresh[i] else start[i].double())
+        want = y + D.double()[None, :, None] * x
+        assert float((got[cu[i]:cu[i + 1]] - want).abs().max() / want.abs().max()) < 2e-5, i
+        assert float((state[i].double().cpu().reshape(H_, N, V) - S).abs().max() / S.abs().max()) < 2e-5, i
+
+
+@pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt"])
+def test_state_space_wide_chunks_keep_the_past_clean(where, bad):
+    """A value that is not finite at one token reaches no earlier one, and no other head (or group) than its own."""
+    H_, G, N, V, T, t = 4, 2, 32, 64, 200, 77
+    g = torch.Generator().manual_seed(1)
+    proj = torch.randn(T, 2 * H_ * V + 2 * G * N + H_, generator=g)
+    A_log, dt_bias, conv_b, D = torch.linspace(-4.0, 1.0, H_), torch.zeros(H_), torch.zeros(H_ * V + 2 * G * N), torch.ones(H_)
+    clean = run_recurrence(proj, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V)
+    broken = proj.clone()
+    broken[t, {"x": H_ * V + 1, "B": 2 * H_ * V + 3, "C": 2 * H_ * V + G * N + 3, "dt": 2 * H_ * V + 2 * G * N}[where]] = bad
+    got = run_recurrence(broken, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V)
+    assert bool(torch.isfinite(got[:t]).all()) and bool(torch.isfinite(got[:, 2:]).all())
+    scale = float(clean.abs().max())
+    assert float((got[:t] - clean[:t]).abs().max()) < 1e-5 * scale and float((got[:, 2:] - clean[:, 2:]).abs().max()) < 1e-5 * scale
+    if math.isnan(bad):
+        assert bool(torch.isnan(got[t]).any())
+    if where == "C":                                          # a token's read-out alone
+        assert bool(torch.isfinite(got[t + 1:]).all())
 
 
 @pytest.mark.parametrize("T, parts, inner_vdim", [(1, 1, 40), (700, 8, 64), (3, 2, 1300), (650, 1, 9)])
