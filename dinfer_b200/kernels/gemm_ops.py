@@ -203,6 +203,48 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: Optiona
     return out
 
 
+# the longest input of a lone token's product (shared memory)
+GEMV_MAX_K = 12 * 1024 - 16
+
+
+def gemv_supported(w: torch.Tensor) -> bool:
+    """A matrix whose product with one bfloat16 row ``gemv`` takes."""
+    return (w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[1] % 8 == 0 and w.shape[1] <= GEMV_MAX_K and w.stride(1) == 1
+            and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemv(x: Optional[torch.Tensor], w: torch.Tensor, out: torch.Tensor, gated: bool = False, norm=None) -> torch.Tensor:
+    """out[1, N] = x[1, K] @ w[N, K]^T for one row in bfloat16; ``gated``: the rows of w are (gate, up) pairs and out [1, N / 2]
+    gets silu(gate) * up.  With ``norm = (residual [1, K] f32, delta [1, K] bfloat16 or None, residual_out [1, K] f32 or None,
+    weight [K], eps)`` the input is the RMSNorm of residual + delta (rounded to bfloat16), and residual_out, another buffer
+    than residual, gets the sum."""
+    require_cuda(w, out)
+    K, N = w.shape[1], w.shape[0]
+    if not gemv_supported(w) or tuple(out.shape) != (1, N // 2 if gated else N) or out.stride(1) != 1 or (gated and N % 2) \
+            or out.dtype not in (torch.bfloat16, torch.float32):
+        raise KernelError(f"gemv: w{tuple(w.shape)} bfloat16 rows of 16-byte pieces, out{tuple(out.shape)} bfloat16 or float32")
+    residual = delta = residual_out = weight = None
+    eps = 0.0
+    if norm is None:
+        if x.dtype != torch.bfloat16 or tuple(x.shape) != (1, K) or x.stride(1) != 1 or x.data_ptr() % 16:
+            raise KernelError("gemv: x bfloat16 [1, K], 16-byte aligned")
+    else:
+        residual, delta, residual_out, weight, eps = norm
+        x = None
+        for t, dt in ((residual, torch.float32), (delta, torch.bfloat16), (residual_out, torch.float32)):
+            if t is not None and (t.dtype != dt or tuple(t.shape) != (1, K) or t.stride(1) != 1 or t.data_ptr() % 16):
+                raise KernelError("gemv: residual and residual_out float32 [1, K], delta bfloat16 [1, K], 16-byte aligned")
+        if weight.dtype not in (torch.bfloat16, torch.float32) or weight.numel() != K or not weight.is_contiguous() or weight.data_ptr() % 16 \
+                or (delta is not None and (residual_out is None or residual_out.data_ptr() == residual.data_ptr())):
+            raise KernelError("gemv: the norm's weight [K], and with a delta another buffer for the new residual")
+    lib, f = _fn("gemv", "dinfer_gemv", [c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                         c_void_p, c_void_p, c_int, c_float, c_void_p])
+    check(lib, f(ptr(x), ptr(w), w.stride(0), ptr(out), int(out.dtype == torch.float32), N, K, int(bool(gated)), ptr(residual),
+                 ptr(delta), ptr(residual_out), ptr(weight), int(weight is not None and weight.dtype == torch.float32), float(eps),
+                 stream_handle()), "gemv")
+    return out
+
+
 def residual_parts(tokens: int, N: int, K: int, splits: Optional[int] = None) -> int:
     """Rows of the ``sums`` the residual epilogue writes for these sizes."""
     if splits is None:

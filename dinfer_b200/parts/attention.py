@@ -240,6 +240,9 @@ class GQAttention(Mixer):
     def takes_half_normed(self, rows: int) -> bool:
         return self.qkv.fuses_norm(rows, self.env.act_dtype)
 
+    def makes_norm(self, rows: int) -> bool:
+        return self.qkv.makes_norm(rows, self.env.act_dtype)
+
     def adds_into_residual(self, rows: int) -> bool:
         return self.o.fuses_norm(rows, self.env.act_dtype)
 

@@ -148,12 +148,38 @@ class HalfNormed:
         return self.xw.shape
 
 
+@dataclass
+class Unnormed:
+    """A lone token's row ahead of an RMSNorm that the product behind it makes for itself (``Linear.makes_norm``): ``norm`` of the
+    stream's residual plus ``delta``.  ``take`` hands out what that product needs and leaves the sum, which it writes, as the
+    stream's residual: a new buffer, since every block of the product reads the old one."""
+    stream: "ResidualStream"
+    delta: Optional[torch.Tensor]
+    norm: "Norm"
+
+    @property
+    def shape(self):
+        return self.stream.x.shape
+
+    @property
+    def device(self):
+        return self.stream.x.device
+
+    def take(self):
+        old = self.stream.x
+        new = None
+        if self.delta is not None:
+            self.stream.x = new = torch.empty_like(old)
+        return old, self.delta, new, self.norm.weight, self.norm.eps
+
+
 class Mixer(Part):
     """Optional beside ``forward``, for parts whose first and last operation can take an RMSNorm apart (see
     ``HalfNormed``): ``takes_half_normed(rows) -> bool`` says that ``forward`` accepts a ``HalfNormed`` as
     ``x`` for this many rows; ``adds_into_residual(rows) -> bool`` says that ``forward(..., sink=(residual,
     norm))`` adds the part's output into the residual itself and returns the ``HalfNormed`` input of the
-    next part instead of the output.  A part without them always gets and gives plain tensors."""
+    next part instead of the output; ``makes_norm(rows) -> bool`` says that ``forward`` accepts an ``Unnormed`` as
+    ``x``.  A part without them always gets and gives plain tensors."""
 
     # A mixer with open ends can be run between two products that are not its own (a pair of mixers then shares one
     # product in front and one behind): ``open_ends()`` is then (columns of the projected rows, columns of the result
@@ -190,7 +216,7 @@ def split_needs(need):
 
 
 class FeedForward(Part):
-    """The optional ``takes_half_normed`` / ``adds_into_residual`` of a ``Mixer`` hold here too."""
+    """The optional ``takes_half_normed`` / ``adds_into_residual`` / ``makes_norm`` of a ``Mixer`` hold here too."""
 
     def forward(self, x: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         raise NotImplementedError

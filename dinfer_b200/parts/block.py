@@ -3,7 +3,7 @@ from __future__ import annotations
 
 from typing import Optional
 
-from .base import BLOCKS, Block, CacheBinding, ResidualStream, StepContext
+from .base import BLOCKS, Block, CacheBinding, ResidualStream, StepContext, Unnormed
 import torch
 
 from .norm import RMSNorm
@@ -18,6 +18,18 @@ def norm_comes_apart(producer, norm, consumer, rows: int) -> bool:
             and give(rows) and take(rows))
 
 
+def normed(stream: ResidualStream, norm, delta, consumer):
+    """The input of ``consumer`` (None: of whoever) behind ``norm`` of the stream plus ``delta``: the rows, or what ``consumer``
+    makes them of."""
+    takes = getattr(consumer, "makes_norm", None)
+    x = stream.x
+    if takes is not None and x.shape[0] == 1 and takes(1) and isinstance(norm, RMSNorm) and norm.weight is not None \
+            and (delta is None or (isinstance(delta, torch.Tensor) and delta.dtype == torch.bfloat16)) \
+            and x.dtype == torch.float32 and stream.results is None:
+        return Unnormed(stream, delta, norm)
+    return norm.forward(x, delta=delta)
+
+
 @BLOCKS.register("prenorm_residual")
 class PreNormResidual(Block):
     """``x += mixer(norm1(x)); x += ffn(norm2(x))`` (a layer may have no feed-forward, kind "none").
@@ -25,6 +37,8 @@ class PreNormResidual(Block):
     Each add is done inside the norm that follows it, and the feed-forward's output stays pending
     until the next layer's (or the model's final) norm picks it up, as the reference defers its MLP
     residual (models/qwen3/src/model.rs:700-743,772-813).  The stream itself stays 32-bit.
+
+    A lone token's norms are made by the products behind them where those can (``normed``).
 
     Where the step asks for it (``ctx.split_norms``) and the parts on both sides of a norm can (few rows,
     bfloat16: decode steps), the norm has no kernel of its own: the part before it adds into the residual and
@@ -36,14 +50,14 @@ class PreNormResidual(Block):
     def forward(self, stream: ResidualStream, ctx: StepContext, cache: CacheBinding,
                 next_block: Optional[Block] = None) -> None:
         rows = stream.x.shape[0]
+        split = bool(getattr(ctx, "split_norms", False))
         if stream.half is not None:
             if stream.half_norm is not self.mixer_norm:
                 raise RuntimeError("half-normed rows were made for another norm than this block's first")
             h, stream.half, stream.half_norm = stream.half, None, None
         else:
-            h = self.mixer_norm.forward(stream.x, delta=stream.pending)
+            h = normed(stream, self.mixer_norm, stream.pending, None if split else self.mixer)
             stream.pending = None
-        split = bool(getattr(ctx, "split_norms", False))
         if getattr(self.feed_forward, "absent", False):     # a layer that is a mixer alone
             stream.pending = self.mixer.forward(h, ctx, cache)
             return
@@ -51,7 +65,7 @@ class PreNormResidual(Block):
             h = self.mixer.forward(h, ctx, cache, sink=(stream.x, self.feed_forward_norm))
         else:
             a = self.mixer.forward(h, ctx, cache)
-            h = self.feed_forward_norm.forward(stream.x, delta=a)
+            h = normed(stream, self.feed_forward_norm, a, None if split else self.feed_forward)
         if split and next_block is not None and norm_comes_apart(self.feed_forward, next_block.mixer_norm, next_block.mixer, rows):
             stream.half = self.feed_forward.forward(h, ctx, sink=(stream.x, next_block.mixer_norm))
             stream.half_norm = next_block.mixer_norm

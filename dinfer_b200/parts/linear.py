@@ -4,6 +4,8 @@ Which product runs follows from the dtypes and the number of rows at hand:
   * float32 activations (the true 32-bit engine): 32-bit multiply-adds on the CUDA cores;
   * bfloat16 activations and a weight the file stores in 32-bit: the same 32-bit product, the
     activations widened on the fly;
+  * bfloat16 activations and weight, one row (a single chat's decode step) and a matrix of at most ``GEMV_MAX_BYTES``: a
+    warp per few weight rows, which can also make the RMSNorm in front of the product (``Unnormed``);
   * bfloat16 activations and weight, up to ``TC_MAX_DECODE_TOKENS`` rows (decode steps): this
     package's tcgen05 / TMA kernel with the operands swapped, so that the weight is streamed from
     memory exactly once (where the reference uses its own small-M kernels,
@@ -21,7 +23,7 @@ import torch
 
 from ..kernels import gemm_ops, ops
 from ..kernels.lib import add_launches
-from .base import HalfNormed
+from .base import HalfNormed, Unnormed
 
 # rows up to which a bfloat16 product takes the swapped-operand tcgen05 kernel
 TC_MAX_DECODE_TOKENS = 32
@@ -31,6 +33,13 @@ PROMPT_BACKEND = "library"
 # the two thresholds the library product followed by the gate kernel is faster (measured at the 0.6B, 8B and 32B
 # shapes: 38.7 against 42.7 us at 33 rows, 43.4 against 55.4 at 128, even at 512, 280 against 300 at 2048)
 TC_MIN_GATED_PROMPT_TOKENS = 512
+
+
+# A lone row's product goes a warp per few weight rows up to this matrix (bytes): beyond, both kernels wait for memory alone, and
+# the tcgen05 one reads faster.  us in a graph, on tensor cores and so, the norm in front included where there is one (*): 4096 x
+# 1024* 5.4 and 3.5, 1024 x 2048 3.9 and 2.9, 6144 x 1024* gated 6.2 and 4.4, 1024 x 3072 4.5 and 3.8, 2048 x 2048 4.3 and 3.5; in a
+# model of 5 layers with matrices of 8 to 63 MB a step took 296 with none of them so, 293 with those up to 13 MB, 303 up to 33 MB.
+GEMV_MAX_BYTES = 13 << 20
 
 
 class Linear:
@@ -44,9 +53,10 @@ class Linear:
         if bias is not None and tuple(bias.shape) != (self.out_features,):
             raise ValueError(f"a bias of {tuple(bias.shape)} does not fit {self.out_features} outputs")
         self.bias = None if bias is None else bias.contiguous()
+        self.lone_row = gemm_ops.gemv_supported(self.weight) and self.weight.numel() * 2 <= GEMV_MAX_BYTES
 
     def kernel_libraries(self):
-        return (["gemm_f32"] if self.weight.dtype == torch.float32 else ["gemm_tc"]) + (["elementwise"] if self.bias is not None else [])
+        return (["gemm_f32"] if self.weight.dtype == torch.float32 else ["gemm_tc"]) + (["gemv"] if self.lone_row else []) + (["elementwise"] if self.bias is not None else [])
 
     def fuses_gate(self, x: torch.Tensor) -> bool:
         """Whether ``gated_pairs`` runs as one kernel for these rows: the tcgen05 product with the gate in its
@@ -63,6 +73,10 @@ class Linear:
         return (self.bias is None and act_dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and 0 < rows <= TC_MAX_DECODE_TOKENS
                 and self.in_features % 8 == 0 and self.out_features % 8 == 0 and w.data_ptr() % 16 == 0)
 
+    def makes_norm(self, rows: int, act_dtype: torch.dtype) -> bool:
+        """Whether this product can make the RMSNorm of its rows itself (``Unnormed``)."""
+        return rows == 1 and self.lone_row and self.bias is None and act_dtype == torch.bfloat16
+
     def gated_pairs(self, x, activation: str = "silu") -> torch.Tensor:
         """For a weight whose rows are (gate, up) pairs: ``act(x gate_j^T) * (x up_j^T)``, [rows, out/2].
         One kernel where ``fuses_gate`` (the silu gate), else the product followed by the gate kernel."""
@@ -71,11 +85,16 @@ class Linear:
             if (activation[0] if isinstance(activation, tuple) else activation) in gemm_ops.GATES and self.fuses_gate(x):
                 return gemm_ops.gemm_tc(x, self.weight, act, gated=activation)
             return ops.gated_act(self(x), act, activation, pairs=True)
+        if isinstance(x, Unnormed):
+            act = torch.empty((1, self.out_features // 2), dtype=torch.bfloat16, device=x.device)
+            return gemm_ops.gemv(None, self.weight, act, gated=True, norm=x.take())
         if isinstance(x, HalfNormed):
             act = torch.empty((x.shape[0], self.out_features // 2), dtype=x.xw.dtype, device=x.xw.device)
             return gemm_ops.gemm_tc(x.xw, self.weight, act, gated=True, row_scale=(x.sums, x.parts, x.size, x.eps))
         act = torch.empty((x.shape[0], self.out_features // 2), dtype=x.dtype, device=x.device)
         if self.fuses_gate(x):
+            if self.lone_row and x.shape[0] == 1:
+                return gemm_ops.gemv(x, self.weight, act, gated=True)
             return gemm_ops.gemm_tc(x, self.weight, act, gated=True)
         return ops.silu_mul(self(x), act, pairs=True)
 
@@ -105,6 +124,10 @@ class Linear:
 
     def __call__(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                  out: Optional[torch.Tensor] = None) -> torch.Tensor:
+        if isinstance(x, Unnormed):                        # the product makes the norm
+            if out is None:
+                out = torch.empty((1, self.out_features), dtype=out_dtype or torch.bfloat16, device=x.device)
+            return gemm_ops.gemv(None, self.weight, out, norm=x.take())
         if isinstance(x, HalfNormed):                      # the product finishes the norm (see HalfNormed)
             if out is None:
                 out = torch.empty((x.shape[0], self.out_features), dtype=out_dtype or x.xw.dtype, device=x.xw.device)
@@ -123,6 +146,8 @@ class Linear:
         rows = x.shape[0]
         use_tc = rows <= TC_MAX_DECODE_TOKENS or PROMPT_BACKEND == "tc"
         if use_tc and gemm_ops.supported(x, w):
+            if rows == 1 and self.lone_row:
+                return gemm_ops.gemv(x, w, out)
             return gemm_ops.gemm_tc(x, w, out)
         add_launches(1)
         if out.dtype == torch.bfloat16:

@@ -67,6 +67,9 @@ class SwiGLU(FeedForward):
         return (self.activation == "silu" and self.gate_up.fuses_norm(rows, self.env.act_dtype)
                 and self.gate_up.out_features % 2 == 0)
 
+    def makes_norm(self, rows: int) -> bool:
+        return self.activation == "silu" and self.gate_up.out_features % 2 == 0 and self.gate_up.makes_norm(rows, self.env.act_dtype)
+
     def adds_into_residual(self, rows: int) -> bool:
         return self.down.fuses_norm(rows, self.env.act_dtype)
 

@@ -91,6 +91,9 @@ class ParallelMixers(Mixer):
     def takes_half_normed(self, rows: int) -> bool:
         return self.scales is not None and self.proj.fuses_norm(rows, self.env.act_dtype)
 
+    def makes_norm(self, rows: int) -> bool:
+        return self.scales is not None and self.proj.makes_norm(rows, self.env.act_dtype)
+
     def adds_into_residual(self, rows: int) -> bool:
         return self.scales is not None and self.o.fuses_norm(rows, self.env.act_dtype)
 

@@ -161,3 +161,61 @@ def test_norm_taken_apart_between_two_products(tokens, N, K, N2):
         want_act = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
         assert float((act.float() - want_act).abs().max()) < 2e-2 * max(1.0, float(want_act.abs().max()))
     G.check_status()
+
+
+@pytest.mark.parametrize("N,K", [(1, 8), (2, 1016), (130, 1024), (2046, 1032), (2048, 264), (4094, 2048), (4096, 1024), (4102, 1032),
+                                 (6144, 256), (1024, 3072), (20000, 520), (66, 12240)])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("f32_out", [False, True])
+def test_lone_row(N, K, gated, f32_out):
+    """A lone token's product with one to four weight rows a warp, ragged batches and pieces, with a plain input, and with the norm of
+    a residual alone and of a residual and a delta made inside.  K products summed in any order in 32-bit are off by at most (K + 1)
+    2^-24 of the sum of their sizes; a made input may differ by a rounding to bfloat16 (2^-8 of it) where the norm's own
+    32-bit roundings decide it, a few elements of a thousand."""
+    from dinfer_b200.kernels import gemm_ops as G, ops
+    if gated and N % 2:
+        pytest.skip("pairs of rows")
+    g = torch.Generator().manual_seed(N + K)
+    w = (torch.randn(N, K + 8, generator=g) / math.sqrt(K)).bfloat16().cuda()[:, :K]
+    dt = torch.float32 if f32_out else torch.bfloat16
+
+    def hold(out, h, slack):
+        z, size = (h.double() @ w.double().T)[0], (h.double().abs() @ w.double().abs().T)[0]
+        err = (K + 1) * 2.0 ** -24 * size + slack * z.abs().mean()
+        if gated:
+            a, u = z[0::2], z[1::2]
+            want = a * torch.sigmoid(a) * u
+            err = err[0::2] * 1.1 * u.abs() + err[1::2] * a.abs() + err[0::2] * err[1::2] + 2.0 ** -20 * want.abs()
+        else:
+            want = z
+        bound = err + (0 if f32_out else 2.0 ** -8 * want.abs())
+        assert bool(((out[0].double() - want).abs() <= bound + 1e-30).all()), float(((out[0].double() - want).abs() / (bound + 1e-30)).max())
+
+    def fresh():
+        return torch.full((1, N // 2 if gated else N), float("nan"), dtype=dt, device="cuda")
+    x = torch.randn(1, K, generator=g).bfloat16().cuda()
+    hold(G.gemv(x, w, fresh(), gated=gated), x, 0.0)
+    residual = torch.randn(1, K, generator=g).cuda()
+    delta = torch.randn(1, K, generator=g).bfloat16().cuda()
+    for weight in ((1 + 0.1 * torch.randn(K, generator=g)).cuda(), (1 + 0.1 * torch.randn(K, generator=g)).bfloat16().cuda()):
+        for d in (None, delta):
+            old, new = residual.clone(), torch.full((1, K), float("nan"), device="cuda")
+            got = G.gemv(None, w, fresh(), gated=gated, norm=(old, d, new if d is not None else None, weight, 1e-6))
+            v = residual if d is None else residual + d.float()
+            assert torch.equal(old, residual) and (d is None or torch.equal(new, v))
+            h = torch.empty(1, K, dtype=torch.bfloat16, device="cuda")
+            ops.rmsnorm(v.clone(), weight, 1e-6, h)
+            hold(got, h, 0.02)
+
+
+def test_lone_row_refusals():
+    from dinfer_b200.kernels import gemm_ops as G
+    from dinfer_b200.kernels.lib import KernelError
+    w, x = torch.zeros(16, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 64, dtype=torch.bfloat16, device="cuda")
+    out, r = torch.zeros(1, 16, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 64, device="cuda")
+    assert not G.gemv_supported(w[:, :60]) and not G.gemv_supported(w.float()) and not G.gemv_supported(w[:, 4:])
+    for bad in (lambda: G.gemv(x.expand(2, -1), w, out), lambda: G.gemv(x[:, :32], w, out), lambda: G.gemv(x, w, out[:, :8]),
+                lambda: G.gemv(x, w[:15], out[:, :7], gated=True), lambda: G.gemv(None, w, out, norm=(r, x, None, x[0], 1e-6)),
+                lambda: G.gemv(None, w, out, norm=(r, x, r, x[0], 1e-6)), lambda: G.gemv(None, w, out, norm=(r, None, None, x[0, :32], 1e-6))):
+        with pytest.raises(KernelError):
+            bad()
