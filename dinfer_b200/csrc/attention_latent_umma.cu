@@ -31,6 +31,7 @@ using namespace dinfer_umma;
 namespace {
 
 constexpr int BM = 128, BN = 128, NTHREADS = 608;              // rows per row tile (two per CTA), keys per tile
+constexpr int MIN_SHARED = 6, LONG_WALK = 16;                  // key tiles of a pair that two CTAs share; of a long one
 constexpr int V_WARP = 18;
 constexpr uint32_t PART = BM * 128;                            // bytes of a 128 x 64 part of a tile
 
@@ -70,7 +71,12 @@ template <int D> struct Shape {
   static_assert(SMEM <= 227 * 1024, "fits a CTA");
 };
 
-template <int D>
+// SPLIT: a cluster of two CTAs to a row-tile pair, half of its keys each where it has MIN_SHARED key tiles or more (else the
+// second has nothing to do).  Each then writes out one of the two row tiles and sends what it has of the other (unnormalised
+// sums, reference maximum, sum of exponentials) through distributed shared memory, where Q lay, behind two cluster barriers.  A
+// prompt's last pair walks all its key tiles, its first one two: 2048 tokens of 16 heads are 128 CTAs whose longest takes 16 tiles
+// of 2.85 us where the mean is 8.5.
+template <int D, bool SPLIT>
 __global__ void __maxnreg__(96)
 attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                              const __grid_constant__ CUtensorMap map_r, const Params p) {
@@ -85,14 +91,14 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
   volatile uint32_t* s_tmem_base = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* s_abort = reinterpret_cast<int*>(bars + 17);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int head = blockIdx.x;
-  pdl_enter();
+  const int head = SPLIT ? blockIdx.x >> 1 : blockIdx.x, rank = SPLIT ? blockIdx.x & 1 : 0;
+  pdl_wait();
   // which request's pair this is, and where its keys begin: every warp adds the requests up for itself (the last block's all of
   // them: a captured graph may be replayed on any lengths, and pairs beyond the grid would go unnoticed)
   int b = -1, pair = 0, pairs_b = 0, key0 = 0, key_end = 0;
   {
     const int y = blockIdx.y;
-    const bool all = y == (int)gridDim.y - 1 && head == 0;
+    const bool all = y == (int)gridDim.y - 1 && blockIdx.x == 0;
     int before = 0, keys_before = 0;
     for (int i0 = 0; i0 < p.B; i0 += 32) {
       const int i = i0 + lane;
@@ -127,9 +133,15 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
   const bool b_on = row0 + BM < rows_total;                    // the second row tile exists
   const int last_a = min(row0 + BM, rows_total) - 1, last = min(row0 + 2 * BM, rows_total) - 1;
   const int hi = hist + last + 1, hi_a = hist + last_a + 1;
-  const int tile_first = first_key(hist + row0, p.window, 0) / BN;
-  const int n_tiles = (hi + BN - 1) / BN - tile_first;         // tiles of B (or of A when B does not exist)
-  const int n_tiles_a = (hi_a + BN - 1) / BN - tile_first;
+  const int tile0 = first_key(hist + row0, p.window, 0) / BN;
+  const int n_all = (hi + BN - 1) / BN - tile0;                // tiles of B (or of A when B does not exist)
+  const int n_all_a = (hi_a + BN - 1) / BN - tile0;
+  const bool shared = SPLIT && n_all >= MIN_SHARED;
+  if (SPLIT && rank == 1 && !shared) return;
+  const int per = shared ? (n_all + 1) / 2 : n_all;            // this CTA's: the first ones, or the rest
+  const int tile_first = tile0 + rank * per;
+  const int n_tiles = min(per, n_all - rank * per);
+  const int n_tiles_a = max(0, min(per, n_all_a - rank * per));
 
   const uint32_t base = smem_u32(smem);
   const uint32_t sQ = base, sK = sQ + 2 * S::Q_BYTES, sV = sK + KS * S::K_BYTES;
@@ -157,6 +169,7 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();                                     // (now that the tensor memory is ours)
   const uint32_t tmem = *s_tmem_base;
 
   if (warp == 0 || warp == V_WARP) {
@@ -345,29 +358,98 @@ attention_latent_umma_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
     s_max[w][h][r] = l_run;                                    // (every thread of the row tile is past its last maximum)
     asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
-    if (ok && n_w > 0) {
-      float l = s_max[w][0][r] + s_max[w][1][r];
-      if (p.sinks) l += exp2f(sink_log2(p.sinks, head) - m_run);
-      const float inv = l > 0.f ? 1.f / l : 0.f;
-      __nv_bfloat16* dst = p.out + (int64_t)(t0 + row) * p.ldo + (int64_t)head * D + h * (D / 2);
-      // all of tensor memory is read ahead of the one branch on row_ok: tcgen05.ld is an instruction of the whole warp, and
-      // between two branches on the same lanes' condition the compiler may let the lanes go their ways in between as well
-      uint32_t y[D / 4];
+    const bool have = ok && n_w > 0;                           // O holds something (the same for a whole warp)
+    const float l_own = have ? s_max[w][0][r] + s_max[w][1][r] : 0.f;
+    const float m_own = have ? m_run : -INFINITY;
+    __nv_bfloat16* dst = p.out + (int64_t)(t0 + row) * p.ldo + (int64_t)head * D + h * (D / 2);
+    if (!shared) {
+      if (have) {
+        float l = l_own;
+        if (p.sinks) l += exp2f(sink_log2(p.sinks, head) - m_run);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        // all of tensor memory is read ahead of the one branch on row_ok: tcgen05.ld is an instruction of the whole warp, and
+        // between two branches on the same lanes' condition the compiler may let the lanes go their ways in between as well
+        uint32_t y[D / 4];
 #pragma unroll
-      for (int c = 0; c < D / 64; ++c) {
-        float o[32];
-        __syncwarp();
-        tmem_ld32(o_addr + c * 32, o);
-        tmem_ld_wait();
+        for (int c = 0; c < D / 64; ++c) {
+          float o[32];
+          __syncwarp();
+          tmem_ld32(o_addr + c * 32, o);
+          tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) y[c * 16 + i] = pack_bf16(o[2 * i] * inv, o[2 * i + 1] * inv);
+          for (int i = 0; i < 16; ++i) y[c * 16 + i] = pack_bf16(o[2 * i] * inv, o[2 * i + 1] * inv);
+        }
+        if (row_ok) {
+#pragma unroll
+          for (int i = 0; i < D / 16; ++i)
+            reinterpret_cast<uint4*>(dst)[i] = make_uint4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+        }
       }
-      if (row_ok) {
+    } else if constexpr (SPLIT) {
+      // what a CTA receives: [4-column group][row] float4 where Q lay, and [row] maxima and sums where the row tiles' were
+      float* x_max = &s_max[0][0][0];
+      float* x_sum = &s_max[0][1][0];
+      cluster_sync_all();                                      // both CTAs' products have completed, their maxima are read
+      if (w != rank) {
+        const uint32_t peer = 1 - rank;
+        const uint32_t remote = map_to_rank(sQ, peer) + (uint32_t)((h * (D / 8) * BM + r) * 16);
 #pragma unroll
-        for (int i = 0; i < D / 16; ++i)
-          reinterpret_cast<uint4*>(dst)[i] = make_uint4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+        for (int c = 0; c < D / 64; ++c) {
+          float o[32];
+          __syncwarp();
+          tmem_ld32(o_addr + c * 32, o);                       // (anything where this CTA has no keys for the tile: its sum says so)
+          tmem_ld_wait();
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            st_cluster_f32x4(remote + (uint32_t)((c * 8 + q4) * BM * 16), o[q4 * 4], o[q4 * 4 + 1], o[q4 * 4 + 2], o[q4 * 4 + 3]);
+        }
+        if (h == 0) {
+          st_cluster_f32(map_to_rank(smem_u32(&x_max[r]), peer), m_own);
+          st_cluster_f32(map_to_rank(smem_u32(&x_sum[r]), peer), l_own);
+        }
+      }
+      cluster_sync_all();
+      if (w == rank && ok) {
+        const float m_x = x_max[r], l_x = x_sum[r], m = fmaxf(m_own, m_x);
+        const float a_own = l_own > 0.f ? fast_exp2(m_own - m) : 0.f, a_x = l_x > 0.f ? fast_exp2(m_x - m) : 0.f;
+        float l = l_own * a_own + l_x * a_x;
+        if (l_own != l_own || l_x != l_x) l = l_own + l_x;     // (not a number: stays one)
+        if (p.sinks) l += exp2f(sink_log2(p.sinks, head) - m);
+        const float inv = l > 0.f ? 1.f / l : (l != l ? l : 0.f);
+        const float4* recv = reinterpret_cast<const float4*>(smem) + h * (D / 8) * BM + r;
+        uint32_t y[D / 4];
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) {
+          float o[32];
+          __syncwarp();
+          tmem_ld32(o_addr + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4) {
+            const float4 v = recv[(c * 8 + q4) * BM];
+            const float x[4] = {v.x, v.y, v.z, v.w};
+            float z[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                      // (a side without keys holds anything)
+              z[i] = a_own != 0.f ? o[q4 * 4 + i] * a_own : 0.f;
+              if (a_x != 0.f) z[i] = fmaf(a_x, x[i], z[i]);
+              z[i] *= inv;
+            }
+            y[c * 16 + q4 * 2] = pack_bf16(z[0], z[1]);
+            y[c * 16 + q4 * 2 + 1] = pack_bf16(z[2], z[3]);
+          }
+        }
+        if (row_ok) {
+#pragma unroll
+          for (int i = 0; i < D / 16; ++i)
+            reinterpret_cast<uint4*>(dst)[i] = make_uint4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+        }
       }
     }
+  }
+  if (SPLIT && shared && (warp < 2 || warp == V_WARP)) {       // the other warps pass the cluster's two barriers too
+    cluster_sync_all();
+    cluster_sync_all();
   }
   __syncwarp();                                                // (lanes that had no part in a warp's role wait for the one that did)
   tc_fence_before();
@@ -452,12 +534,22 @@ bool make_map(CUtensorMap* m, const void* base, int n, const cuuint64_t* dims, c
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int D>
-int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, const Params& p, dim3 grid, cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(attention_latent_umma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)Shape<D>::SMEM);
+int num_sms() {                                             // of the current device, asked once
+  static const int n = [] {
+    int dev = 0, v = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  }();
+  return n;
+}
+
+template <int D, bool SPLIT>
+int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtensorMap& mr, const Params& p, int H, int pairs, cudaStream_t stream) {
+  auto k = attention_latent_umma_kernel<D, SPLIT>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<D>::SMEM);
   if (e != cudaSuccess) return refuse((int)e, "attention_latent_umma: shared memory opt-in failed: %s", cudaGetErrorString(e));
-  launch_pdl(attention_latent_umma_kernel<D>, grid, dim3(NTHREADS), Shape<D>::SMEM, stream, mq, mkv, mr, p);
+  e = launch_pdl_cluster(k, dim3(SPLIT ? 2 * H : H, pairs), dim3(NTHREADS), dim3(SPLIT ? 2 : 1, 1, 1), Shape<D>::SMEM, stream, mq, mkv, mr, p);
+  if (e != cudaSuccess) return refuse((int)e, "attention_latent_umma: launch failed: %s", cudaGetErrorString(e));
   return cuda_status("attention_latent_umma");
 }
 
@@ -497,11 +589,11 @@ DINFER_API int dinfer_attention_latent_umma_supports(int R, int P, int D, int V)
 
 // Portions (more than one token) only.  q [T, H, D + P] rows of stride ldq (turned), out [T, H, D] rows of stride ldo;
 // latents [rows, R + P] as dinfer_latent_rows leaves them, expanded [rows, H, 2 D] with a head's key, then its value.
-// pair_bound >= the sum over the portions of ceil(tokens / 256).  sinks [H] f32 or null.  window <= 0: all keys.
+// pair_bound >= the sum over the portions of ceil(tokens / 256); max_keys: about the keys of the longest request (0: not known).  sinks [H] f32 or null.  window <= 0: all keys.
 DINFER_API int dinfer_attention_latent_umma(const void* q, int64_t ldq, void* out, int64_t ldo, const void* latents,
                                             const void* expanded, int rows, const int* cu_seqlens, const int* seq_lens, int T,
                                             int B, int H, int R, int P, int D, float scale, int window, const float* sinks,
-                                            int pair_bound, int* status, cudaStream_t stream) {
+                                            int pair_bound, int max_keys, int* status, cudaStream_t stream) {
   if (T <= 0 || B <= 0 || H <= 0 || rows <= 0 || pair_bound <= 0 || pair_bound > 65535)
     return refuse(DINFER_BAD_ARGUMENT, "attention_latent_umma: bad sizes T=%d B=%d H=%d rows=%d pairs=%d", T, B, H, rows, pair_bound);
   if (!dinfer_attention_latent_umma_supports(R, P, D, D))
@@ -517,9 +609,16 @@ DINFER_API int dinfer_attention_latent_umma(const void* q, int64_t ldq, void* ou
   if (!make_map(&mq, q, 3, dq, sq) || !make_map(&mkv, expanded, 2, dkv, skv) ||
       !make_map(&mr, (const __nv_bfloat16*)latents + (P > 0 ? R : 0), 2, dr, sr))
     return refuse(DINFER_BAD_ARGUMENT, "attention_latent_umma: a tensor map could not be made");
-  Params p;
+  Params p{};
   p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.window = window; p.rows = rows;
   p.scale_log2 = scale * 1.4426950408889634f; p.sinks = sinks; p.status = status;
-  const dim3 grid(H, pair_bound);
-  return D == 64 ? launch<64>(mq, mkv, mr, p, grid, stream) : launch<128>(mq, mkv, mr, p, grid, stream);
+  // Two CTAs to a pair where those of all pairs run at once, or where the longest pair's walk is what a single round of CTAs waits
+  // for (a cluster waits for two SMs, and a shared pair takes some 4 us more).  us alone and shared, 128 wide: 8 heads, 2048 tokens
+  // 50 and 32; 16 heads, 1024 29 and 21; 16, 512 behind 4000 103 and 59; 32, 256 behind 8000 206 and 113; in a round of 128
+  // pairs: 16, 2048 51 and 45; 16, 2048 behind 4000 146 and 132; but 32, 1024 30 and 39; 16, 500 + 700 + 900 29 and 37.
+  const int64_t n = (int64_t)H * pair_bound;
+  const int longest = ((window > 0 && max_keys > window + 2 * BM ? window + 2 * BM : max_keys) + BN - 1) / BN;
+  const bool split = longest >= MIN_SHARED && (2 * n <= num_sms() || (n <= num_sms() && longest >= LONG_WALK));
+  if (D == 64) return split ? launch<64, true>(mq, mkv, mr, p, H, pair_bound, stream) : launch<64, false>(mq, mkv, mr, p, H, pair_bound, stream);
+  return split ? launch<128, true>(mq, mkv, mr, p, H, pair_bound, stream) : launch<128, false>(mq, mkv, mr, p, H, pair_bound, stream);
 }

@@ -245,11 +245,11 @@ def latent_q_turn(q: torch.Tensor, positions: torch.Tensor, cos_sin: Optional[to
 def attention_latent_umma(q: torch.Tensor, out: torch.Tensor, latents: torch.Tensor, expanded: torch.Tensor,
                           cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, kv_rank: int, rope_dim: int, head_dim: int,
                           scale: float, window: int = 0, sinks: Optional[torch.Tensor] = None,
-                          pair_bound: int = 0) -> torch.Tensor:
+                          pair_bound: int = 0, max_keys: int = 0) -> torch.Tensor:
     """Causal attention of the portions (requests that bring more than one token): ``q`` [T, H * (D + P)] with its last parts
     turned, ``latents`` [rows, R + P] from ``latent_rows``, ``expanded`` [rows, H * 2 D] the keys and values of every head made
     from them; ``out`` [T, H, D], the rows of other requests untouched.  ``pair_bound``: at least the sum over the portions of
-    ceil(tokens / 256)."""
+    ceil(tokens / 256); ``max_keys``: about the keys of the longest request (0: not known)."""
     from . import gemm_ops
     require_cuda(q, out, latents, expanded, cu_seqlens, seq_lens)
     B = _check_batch(None, cu_seqlens, seq_lens)
@@ -268,8 +268,8 @@ def attention_latent_umma(q: torch.Tensor, out: torch.Tensor, latents: torch.Ten
     status = gemm_ops._state(q.device)["status"]
     lib, f = _fn("latent_expanded", "dinfer_attention_latent_umma",
                  [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                  c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p, c_void_p])
+                  c_int, c_int, c_float, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p])
     check(lib, f(ptr(q), q.stride(0), ptr(out), out.stride(0), ptr(latents), ptr(expanded), rows, ptr(cu_seqlens), ptr(seq_lens),
-                 T, B, H, kv_rank, rope_dim, head_dim, float(scale), int(window), ptr(sinks), int(pair_bound), ptr(status),
-                 stream_handle()), "attention_latent_umma")
+                 T, B, H, kv_rank, rope_dim, head_dim, float(scale), int(window), ptr(sinks), int(pair_bound), int(max_keys),
+                 ptr(status), stream_handle()), "attention_latent_umma")
     return out

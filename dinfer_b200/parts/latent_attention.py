@@ -279,7 +279,8 @@ class LatentAttention(Mixer):
         latents = latent_ops.latent_rows(kv, g.block_table, ctx.cu_seqlens, ctx.seq_lens, rows, window)
         expanded = self.ukv(latents[:, :self.R])
         latent_ops.attention_latent_umma(q, o, latents, expanded, ctx.cu_seqlens, ctx.seq_lens, self.R, self.P, self.D,
-                                         self.scale, window, sinks=self.sinks, pair_bound=tiles)
+                                         self.scale, window, sinks=self.sinks, pair_bound=tiles,
+                                         max_keys=min(ctx.max_seq_len, rows))
 
     def attend(self, q_lat, o_lat, kv, g, ctx: StepContext, singles: bool = False) -> None:
         window = int(self.window or 0)

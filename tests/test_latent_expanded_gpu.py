@@ -84,6 +84,43 @@ def test_rows_and_attention_against_plain(case):
     assert bool((lat[at:] == 0).all())
 
 
+@pytest.mark.parametrize("D,P,H,window,with_sinks,reqs", [
+    (128, 64, 3, 0, True, [(0, 640)]), (128, 64, 2, 0, False, [(0, 641), (0, 1), (500, 129), (0, 30)]),
+    (64, 32, 4, 0, True, [(5000, 257)]), (128, 64, 1, 900, False, [(2000, 300), (10, 700)]), (128, 16, 16, 0, False, [(0, 1100)]),
+    (64, 64, 1, 0, False, [(639, 2), (640, 128), (767, 2)])])
+def test_two_ctas_to_a_pair(D, P, H, window, with_sinks, reqs):
+    """Row-tile pairs whose keys two CTAs share, beside pairs too short for it, pairs with one row tile, one row of one, an odd number of
+    key tiles, histories and windows: the same as without (which the test above holds to the formula), up to the other
+    order of sums and the other maximum that weights are rounded against."""
+    from dinfer_b200.kernels import gemm_ops, latent_ops as L
+    g = torch.Generator().manual_seed(D + H)
+    cu, seq, table, pages = batch(reqs, 16, 1)
+    R, T = 64, int(cu[-1])
+    c = lambda t: None if t is None else t.cuda()
+    cache = torch.randn(pages, 1, 1, 16, R + P, generator=g).to(torch.bfloat16).cuda()
+    q = (torch.randn(T, H * (D + P), generator=g) * 1.5).to(torch.bfloat16).cuda()
+    w = (torch.randn(H * 2 * D, R, generator=g) * R ** -0.5).to(torch.bfloat16).cuda()
+    sinks = c(torch.randn(H, generator=g)) if with_sinks else None
+    portions = [(n, h + n) for h, n in reqs if n > 1]
+    lat = L.latent_rows(cache, c(table), c(cu), c(seq), L.expanded_rows(portions, window), window)
+    kv = lat[:, :R] @ w.T
+    pairs = sum((n + 255) // 256 for n, _ in portions)
+    got = []
+    for longest in (0, int(seq.max())):
+        out = torch.full((T, H, D), float("nan"), dtype=torch.bfloat16, device="cuda")
+        L.attention_latent_umma(q, out, lat, kv, c(cu), c(seq), R, P, D, (D + P) ** -0.5, window, sinks=sinks, pair_bound=pairs, max_keys=longest)
+        gemm_ops.check_status()
+        got.append(out.float())
+    for i, (h, n) in enumerate(reqs):
+        a, b = (o[int(cu[i]):int(cu[i]) + n] for o in got)
+        if n == 1:
+            assert bool(torch.isnan(b).all())
+            continue
+        # every weight and every result rounded to bfloat16 once more on either side: 2^-8 of the values' sizes
+        assert bool(((a - b).abs() <= 2.0 ** -7 * (a.abs() + kv.float().abs().max() * 0.25)).all())
+        assert float((a - b).norm() / a.norm()) < 4e-3
+
+
 @pytest.mark.parametrize("rows,pairs,bad", [(512, 3, False), (511, 3, True), (256, 3, True), (512, 2, True), (600, 7, False)])
 def test_portions_beyond_the_launch_leave_a_status(rows, pairs, bad):
     """Portions that need 512 gathered rows and three row-tile pairs: a launch made for fewer says so."""
