@@ -73,28 +73,33 @@ struct Shared {
   float blk[XCH];
   float warp_tot[32];
   int pick[4];
-  int turn;
 };
 
+// Which exchange is next, the same in all threads; -1: the cluster's first barrier phase (every CTA runs, so that its memory may be
+// written) is still to be waited for.
+struct Turn { int next = -1; };
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 // Every CTA contributes n <= XCH floats (valid in threads 0..n-1 as `mine`); afterwards
-// sh.xchg[turn][r][j] holds the contribution j of CTA r, the same in every CTA.  Returns the buffer.
-__device__ float (*exchange(Shared& sh, float mine, int n, uint32_t rank))[XCH] {
-  const int t = sh.turn;
+// sh.xchg[turn][r][j] holds the contribution j of CTA r, the same in every CTA.  Returns the buffer.  (The cluster's barrier is one of
+// every CTA's threads too.)
+__device__ float (*exchange(Shared& sh, Turn& turn, float mine, int n, uint32_t rank))[XCH] {
+  if (turn.next < 0) { cluster_wait(); turn.next = 0; }
+  const int t = turn.next;
+  turn.next = t ^ 1;
   if ((int)threadIdx.x < n) {
 #pragma unroll
     for (uint32_t r = 0; r < ROW_CTAS; ++r) st_cluster_f32(smem_u32(&sh.xchg[t][rank][threadIdx.x]), r, mine);
   }
   cluster_sync_all();
-  __syncthreads();
-  if (threadIdx.x == 0) sh.turn = t ^ 1;
-  __syncthreads();
   return sh.xchg[t];
 }
 
 // Sum over the whole row of what every segment contributes: fill(segment, v) adds segment's share to v[0..N).  Warps of
-// segments by a shuffle tree, then those in order, then the CTAs in rank order.
+// segments by a shuffle tree, then those in order, then the CTAs in rank order.  Returns the CTAs' shares.
 template <int N, typename F>
-__device__ __forceinline__ void row_sum(Shared& sh, uint32_t rank, float (&out)[N], F fill) {
+__device__ __forceinline__ float (*row_sum(Shared& sh, Turn& turn, uint32_t rank, float (&out)[N], F fill))[XCH] {
   const int lane = threadIdx.x & 31;
   __syncthreads();
 #pragma unroll 1
@@ -118,7 +123,7 @@ __device__ __forceinline__ void row_sum(Shared& sh, uint32_t rank, float (&out)[
   float mine = 0.f;
   if ((int)threadIdx.x < N)
     for (int w = 0; w < WARPS_OF_SEGMENTS; ++w) mine += sh.warp_part[w][threadIdx.x];
-  float (*x)[XCH] = exchange(sh, mine, N, rank);
+  float (*x)[XCH] = exchange(sh, turn, mine, N, rank);
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     float t = 0.f;
@@ -126,6 +131,7 @@ __device__ __forceinline__ void row_sum(Shared& sh, uint32_t rank, float (&out)[
     for (int r = 0; r < ROW_CTAS; ++r) t += x[r][j];
     out[j] = t;
   }
+  return x;
 }
 
 // order-preserving image of a float: a < b  <=>  key(a) < key(b)   (-0 is folded into +0 by the caller)
@@ -144,7 +150,7 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 
 // argmax over the row (ties to the lowest index), the same in every CTA of the cluster
 template <int THREADS>
-__device__ int row_argmax(Shared& sh, const float* xs, int n_mine, int first, uint32_t rank) {
+__device__ int row_argmax(Shared& sh, Turn& turn, const float* xs, int n_mine, int first, uint32_t rank) {
   ArgMax best{-INFINITY, 0x7fffffff};
   for (int i = threadIdx.x; i < n_mine; i += THREADS) best = better(best, ArgMax{xs[i], first + i});
 #pragma unroll
@@ -163,7 +169,7 @@ __device__ int row_argmax(Shared& sh, const float* xs, int n_mine, int first, ui
   }
   __syncthreads();
   const float mine = threadIdx.x < 2 ? sh.blk[threadIdx.x] : 0.f;
-  float (*x)[XCH] = exchange(sh, mine, 2, rank);
+  float (*x)[XCH] = exchange(sh, turn, mine, 2, rank);
   ArgMax all{-INFINITY, 0x7fffffff};
 #pragma unroll
   for (int r = 0; r < ROW_CTAS; ++r) all = better(all, ArgMax{x[r][0], __float_as_int(x[r][1])});
@@ -214,7 +220,7 @@ struct Bracket {
 // entry weighs 1 (MASS = false) or exp(x - m) (MASS = true).  Radix-16 descent over float_key - base: `above` is the
 // weight of the entries beyond the digits fixed so far.  Eight passes over the row for all floats, fewer for a bracket.
 template <bool MASS>
-__device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, float m, float floor_, float target,
+__device__ float radix_threshold(Shared& sh, Turn& turn, const Slice& sl, uint32_t rank, float m, float floor_, float target,
                                  const Bracket& where) {
   uint32_t prefix = 0;
   float above = where.above;
@@ -222,7 +228,7 @@ __device__ float radix_threshold(Shared& sh, const Slice& sl, uint32_t rank, flo
 #pragma unroll 1
   for (int shift = first; shift >= 0; shift -= 4) {
     float tot[16];
-    row_sum<16>(sh, rank, tot, [&](int u, float (&h)[16]) {
+    row_sum<16>(sh, turn, rank, tot, [&](int u, float (&h)[16]) {
       const int i1 = sl.end(u);
       for (int i = sl.begin(u); i < i1; ++i) {
         const float x = sl.at(i);
@@ -296,46 +302,61 @@ __device__ __forceinline__ void segment_scan(int (&v)[VT], int* warp_tot, int& t
 // false), or at least the share p of the mass of all kept ones (true; `denom` is then that mass).  The first pass cuts at
 // fixed distances below the maximum (x is in units of the softmax's exponent), further ones inside the gap between the lowest
 // cut that is not enough and the highest that is.  Returns whether at most CAND_MAX entries are left to look through: with
-// `whole` those from the cut up, else those of the gap, from the cut up to `below` (gap.above is what lies beyond weighs).
+// `whole` those from the cut up, else those of the gap, from the cut up to `below` (gap.above is what lies beyond weighs), and `place` how many they are.
 // Where there are more after CUT_ROUNDS passes, or equal ones crowd a gap of few floats, a descent inside the gap finds the
 // threshold.
+constexpr int UPPER = CUTS - 2;             // cuts that few entries reach
+// candidates of the CTAs before this one, and of all
+struct Place { int base, n; };
 template <bool MASS>
-__device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, float lo, float floor_, float need, bool whole,
-                         float& cut, float& below, float& denom, Bracket& gap) {
+__device__ bool find_cut(Shared& sh, Turn& turn, const Slice& sl, uint32_t rank, float m, float lo, float floor_, float need, bool whole,
+                         float& cut, float& below, float& denom, Bracket& gap, Place& place) {
   float c[CUTS] = {m - 1.f, m - 2.f, m - 4.f, m - 6.f, m - 9.f, m - 13.f, m - 18.f, floor_};
 #pragma unroll
   for (int j = 0; j < CUTS; ++j) c[j] = fmaxf(c[j], floor_);
-  float target = need, hi = m, n_above = 0.f;
+  float target = need, hi = m, n_above = 0.f, before_above = 0.f;
+  const auto before = [&](float (*x)[XCH], int j) {        // entries from cut j up in the CTAs before this one
+    float t = 0.f;
+#pragma unroll
+    for (int r = 0; r < ROW_CTAS; ++r) t += r < (int)rank ? x[r][j] : 0.f;
+    return t;
+  };
   below = INFINITY;                                        // (no cut that is not enough was met yet)
 #pragma unroll 1
   for (int round = 0; round < CUT_ROUNDS; ++round) {
     float tot[MASS ? 2 * CUTS : CUTS];
-    row_sum<MASS ? 2 * CUTS : CUTS>(sh, rank, tot, [&](int u, float (&h)[MASS ? 2 * CUTS : CUTS]) {
+    float (*x)[XCH] = row_sum<MASS ? 2 * CUTS : CUTS>(sh, turn, rank, tot, [&](int u, float (&h)[MASS ? 2 * CUTS : CUTS]) {
       const int i1 = sl.end(u);
       for (int i = sl.begin(u); i < i1; ++i) {
         const float x = sl.at(i);
         const float w = MASS ? (x >= c[CUTS - 1] ? expf(x - m) : 0.f) : 0.f;
-#pragma unroll
-        for (int j = 0; j < CUTS; ++j) {
+        // the cuts fall, and most entries of a row lie below all but the last ones
+        const auto count = [&](int j) {
           h[j] += x >= c[j] ? 1.f : 0.f;
           if (MASS) h[CUTS + j] += x >= c[j] ? w : 0.f;
+        };
+        if (x >= c[UPPER - 1]) {
+#pragma unroll
+          for (int j = 0; j < UPPER; ++j) count(j);
         }
+#pragma unroll
+        for (int j = UPPER; j < CUTS; ++j) count(j);
       }
     });
     if (MASS && round == 0) { denom = tot[(MASS ? CUTS : 0) + CUTS - 1]; target = need * denom; }
-    float n = tot[CUTS - 1];
+    float n = tot[CUTS - 1], before_cut = 0.f;
     bool reached = false;
     cut = c[CUTS - 1];
 #pragma unroll
     for (int j = 0; j < CUTS; ++j) {
       const float have = MASS ? tot[(MASS ? CUTS : 0) + j] : tot[j];
       if (!reached) {
-        if (have >= target || j == CUTS - 1) { reached = true; cut = c[j]; n = tot[j]; }
-        else { hi = below = c[j]; n_above = tot[j]; gap.above = have; }
+        if (have >= target || j == CUTS - 1) { reached = true; cut = c[j]; n = tot[j]; before_cut = before(x, j); }
+        else { hi = below = c[j]; n_above = tot[j]; before_above = before(x, j); gap.above = have; }
       }
     }
-    if (whole && n <= (float)CAND_MAX) { below = INFINITY; return true; }
-    if (!whole && n - n_above <= (float)CAND_MAX) return true;
+    if (whole && n <= (float)CAND_MAX) { below = INFINITY; place = Place{(int)before_cut, (int)n}; return true; }
+    if (!whole && n - n_above <= (float)CAND_MAX) { place = Place{(int)(before_cut - before_above), (int)(n - n_above)}; return true; }
     const float low = fmaxf(cut, lo);                      // (the floor may be -inf, and masked entries with it)
     gap.base = float_key(MASS ? low : cut);                // (masked entries have no mass, but they count)
     gap.width = hi <= lo ? 0u : float_key(hi) - (below < INFINITY ? 1u : 0u) - gap.base;
@@ -353,7 +374,7 @@ __device__ bool find_cut(Shared& sh, const Slice& sl, uint32_t rank, float m, fl
 // Fills cd.x with the entries from `cut` up and below `below` (at most CAND_MAX), in vocabulary order, and cd.s with the same
 // from the largest down; returns their number.
 template <bool GAP>
-__device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32_t rank, float cut, float below) {
+__device__ int gather_sorted(Candidates& cd, const Slice& sl, float cut, float below, const Place& place) {
   int cnt[VT], end[VT], cta_total;
 #pragma unroll
   for (int vt = 0; vt < VT; ++vt) {
@@ -366,13 +387,8 @@ __device__ int gather_sorted(Shared& sh, Candidates& cd, const Slice& sl, uint32
     cnt[vt] = end[vt] = n;
   }
   segment_scan(end, cd.warp_tot, cta_total);
-  float (*x)[XCH] = exchange(sh, threadIdx.x == 0 ? (float)cta_total : 0.f, 1, rank);
-  int base = 0, n = 0;
-#pragma unroll
-  for (int r = 0; r < ROW_CTAS; ++r) {
-    if (r < (int)rank) base += (int)x[r][0];
-    n += (int)x[r][0];
-  }
+  const int base = place.base;
+  int n = place.n;
 #pragma unroll
   for (int vt = 0; vt < VT; ++vt) {
     const int u = vt * NT + threadIdx.x, i1 = sl.end(u);
@@ -461,12 +477,10 @@ argmax_kernel(const float* __restrict__ logits, int64_t ld, int* __restrict__ ou
   const float* row = logits + (int64_t)b * ld;
   const int per = (vocab + ROW_CTAS - 1) / ROW_CTAS;
   const int first = min(vocab, (int)rank * per), n_mine = min(vocab, first + per) - first;
-  if (threadIdx.x == 0) sh.turn = 0;
-  __syncthreads();
-  cluster_sync_all();                                    // every CTA runs before any writes into its memory
-  const int r = row_argmax<BLOCK>(sh, row + first, n_mine, first, rank);
-  if (rank == 0 && threadIdx.x == 0) out[b] = r;
-  cluster_sync_all();                                    // nobody leaves while others may still write to it
+  Turn turn;
+  cluster_arrive();                                      // (waited for ahead of the first write into another CTA's memory)
+  const int r = row_argmax<BLOCK>(sh, turn, row + first, n_mine, first, rank);
+  if (rank == 0 && threadIdx.x == 0) out[b] = r;         // (behind the last barrier nobody writes to another any more)
 }
 
 // Many rows: a CTA per row (no cluster: with 8 CTAs a row, 64 rows are two waves of CTAs that mostly wait for each
@@ -529,14 +543,12 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   const float* row = logits + (int64_t)b * ld;
   const int per = (vocab + ROW_CTAS - 1) / ROW_CTAS;
   const int first = min(vocab, (int)rank * per), n_mine = min(vocab, first + per) - first;
-  if (threadIdx.x == 0) sh.turn = 0;
-  __syncthreads();
-  cluster_sync_all();                                    // every CTA runs before any writes into its memory
+  Turn turn;
+  cluster_arrive();                                      // (waited for ahead of the first write into another CTA's memory)
   const float temp = temperature[b];
   if (temp <= 1e-5f) {
-    const int r = row_argmax<NT>(sh, row + first, n_mine, first, rank);
+    const int r = row_argmax<NT>(sh, turn, row + first, n_mine, first, rank);
     if (rank == 0 && threadIdx.x == 0) out[b] = r;
-    cluster_sync_all();
     return;
   }
   const float inv_t = 1.f / temp;
@@ -569,7 +581,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
     }
     __syncthreads();
     const float mine = threadIdx.x < 2 ? sh.blk[threadIdx.x] : 0.f;
-    float (*x)[XCH] = exchange(sh, mine, 2, rank);
+    float (*x)[XCH] = exchange(sh, turn, mine, 2, rank);
     m = -INFINITY; lo = INFINITY;
 #pragma unroll
     for (int r = 0; r < ROW_CTAS; ++r) { m = fmaxf(m, x[r][0]); lo = fminf(lo, x[r][1]); }
@@ -584,15 +596,16 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
   int n_cand = -1;                                       // >= 0: cand holds every entry from the top-k threshold up
   float cut, below, denom = -1.f;
   Bracket gap;                                           // (all floats where no cut is looked for)
+  Place place{0, 0};
   if (k > 0 && k < vocab) {
     const bool whole = k <= CAND_MAX / 2;                // a small k leaves the candidates to top-p
-    if (finite && find_cut<false>(sh, sl, rank, m, lo, thr, (float)k, whole, cut, below, denom, gap)) {
-      const int n = whole ? gather_sorted<false>(sh, cand, sl, rank, cut, below) : gather_sorted<true>(sh, cand, sl, rank, cut, below);
-      const int place = whole ? k : k - (int)gap.above;
-      if (place <= n) thr = fmaxf(thr, cand.s[place - 1]);   // else all of them are kept
+    if (finite && find_cut<false>(sh, turn, sl, rank, m, lo, thr, (float)k, whole, cut, below, denom, gap, place)) {
+      const int n = whole ? gather_sorted<false>(cand, sl, cut, below, place) : gather_sorted<true>(cand, sl, cut, below, place);
+      const int kth = whole ? k : k - (int)gap.above;
+      if (kth <= n) thr = fmaxf(thr, cand.s[kth - 1]);       // else all of them are kept
       if (whole) n_cand = n;
     } else {
-      thr = fmaxf(thr, radix_threshold<false>(sh, sl, rank, m, thr, (float)k, gap));
+      thr = fmaxf(thr, radix_threshold<false>(sh, turn, sl, rank, m, thr, (float)k, gap));
     }
   }
   const float p = top_p ? top_p[b] : 1.f;
@@ -601,11 +614,11 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
       thr = fmaxf(thr, topp_of_sorted(cand, n_cand, m, thr, p, -1.f, 0.f));
     } else if (finite) {
       gap = Bracket();
-      if (find_cut<true>(sh, sl, rank, m, lo, thr, p, false, cut, below, denom, gap)) {
-        const int n = gather_sorted<true>(sh, cand, sl, rank, cut, below);
+      if (find_cut<true>(sh, turn, sl, rank, m, lo, thr, p, false, cut, below, denom, gap, place)) {
+        const int n = gather_sorted<true>(cand, sl, cut, below, place);
         thr = fmaxf(thr, topp_of_sorted(cand, n, m, thr, p, denom, gap.above));
       } else {
-        thr = fmaxf(thr, radix_threshold<true>(sh, sl, rank, m, thr, p * denom, gap));
+        thr = fmaxf(thr, radix_threshold<true>(sh, turn, sl, rank, m, thr, p * denom, gap));
       }
     }
   }
@@ -636,7 +649,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
     sh.blk[0] = s;
   }
   __syncthreads();
-  float (*x)[XCH] = exchange(sh, threadIdx.x == 0 ? sh.blk[0] : 0.f, 1, rank);
+  float (*x)[XCH] = exchange(sh, turn, threadIdx.x == 0 ? sh.blk[0] : 0.f, 1, rank);
   float total = 0.f;
 #pragma unroll
   for (int r = 0; r < ROW_CTAS; ++r) total += x[r][0];
@@ -704,8 +717,7 @@ sample_kernel(const float* __restrict__ logits, int64_t ld, const float* __restr
     }
   }
   if (owner < 0 && rank == 0 && threadIdx.x == 0) out[b] = 0;   // nothing kept at all (no finite logit)
-  cluster_sync_all();                                    // nobody leaves while others may still write to it
-}
+}                                                        // (behind the last exchange nobody writes to another any more)
 
 // history of row b: ids[offsets[b] .. offsets[b+1]), the first prompt_len[b] of them the prompt.
 __global__ void penalties_kernel(float* __restrict__ logits, int64_t ld, const int* __restrict__ ids,
