@@ -16,13 +16,13 @@
 //
 // A pair's row depends on nothing but its token and expert: where it lands inside a tile, and what else is in
 // the batch, changes no bit of it.  Router, scores, weights and the gate are 32-bit; products accumulate in 32-bit.
-#include "common.cuh"
+#include "split_umma.cuh"
 
 using namespace dinfer;
 
 namespace {
 
-enum Act : int { ACT_NONE = 0, ACT_RELU2 = 1, ACT_SILU = 2, ACT_GELU_TANH = 3, ACT_RELU = 4 };
+enum Act : int { ACT_NONE = 0, ACT_RELU2 = 1, ACT_SILU = 2, ACT_GELU_TANH = 3, ACT_RELU = 4, ACT_CLAMPED = 5 };   // (5: a gate only)
 
 __device__ __forceinline__ float activate(float z, int act) {
   switch (act) {
@@ -351,9 +351,8 @@ moe_gemm_simt_kernel(const TA* __restrict__ A, int64_t lda, const TW* __restrict
 
 // ---------------------------------------------------------------- grouped product on tensor cores (bfloat16)
 // The same tiles on mma.sync m16n8k16 with 32-bit accumulation: 4 warps, K in steps of 32 through a
-// double buffer filled with cp.async (A rows gathered by pair, the expert's weight rows as they lie).  BM = 64:
-// tile 64 x 128, warps 2 x 2, each 32 x 64; BM = 16 (decode steps: an expert gets a row or two): tile 16 x 64, each
-// warp 16 columns.
+// double buffer filled with cp.async (A rows gathered by pair, the expert's weight rows as they lie): tile 64 x 128, warps
+// 2 x 2, each 32 x 64.  Row tiles of 16 run on the kernel behind this one.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -367,23 +366,16 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-// the same, and the 256 bytes around it come into L2: a row's next 128 bytes are the next step's
-__device__ __forceinline__ void cp_async16_ahead(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// Row tiles of 16 (decode steps): bound by reading the weights of the experts that the step's tokens meet, 64 rows of them a
-// block, four stages of 64 k.  Eight tokens, 64 experts of 4096 x 2048 (8 chosen): gate and up 292 us and down 148 us with
-// two stages of 32 k, 244 and 126 us now (5.7 TB/s; 265 and 131 without the 256-byte fetch into L2).
-template <int BM, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(128)
 moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ Wall,
                     __nv_bfloat16* __restrict__ C, int64_t ldc, const int* __restrict__ sorted,
                     const int* __restrict__ tile_expert, const float* __restrict__ weights, int pairs, int top, int N,
                     int K, int act) {
-  constexpr int BN = BM == 64 ? 128 : 64, BK = BM == 64 ? 32 : 64, LD = BK + 8, ST = BM == 64 ? 2 : 4;
-  constexpr int WM = BM == 64 ? 2 : 1, WN = 4 / WM;          // warps along rows and columns
+  constexpr int BM = 64, BN = 128, BK = 32, LD = BK + 8, ST = 2;
+  constexpr int WM = 2, WN = 4 / WM;                         // warps along rows and columns
   constexpr int MTW = BM / (16 * WM), NTW = BN / (8 * WN);   // m16 and n8 tiles per warp
   __shared__ __align__(16) __nv_bfloat16 As[ST][BM][LD];
   __shared__ __align__(16) __nv_bfloat16 Bs[ST][BN][LD];
@@ -411,10 +403,7 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
         else *reinterpret_cast<uint4*>(&As[buf][r][c]) = make_uint4(0, 0, 0, 0);
       } else {
         const int n = r - BM;
-        if (n0 + n < N && in_k) {
-          if (BM == 16) cp_async16_ahead(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
-          else cp_async16(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
-        }
+        if (n0 + n < N && in_k) cp_async16(&Bs[buf][n][c], W + (int64_t)(n0 + n) * K + k0 + c);
         else *reinterpret_cast<uint4*>(&Bs[buf][n][c]) = make_uint4(0, 0, 0, 0);
       }
     }
@@ -471,6 +460,195 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
           if (n < N) C[row * ldc + n] = __float2bfloat16_rn(MODE == 0 ? activate(v, act) : v * w);
         }
     }
+}
+
+// ---------------------------------------------------------------- grouped product on row tiles of 16 (bfloat16)
+// Decode steps: an expert gets a row or two, and the product is bound by reading the weights of the experts that the step's
+// tokens meet.  Four persistent CTAs an SM stream them, each its own jobs of 64 weight rows: one warp keeps two stages of 64
+// weight rows x 128 k on their way (16 KB each, by TMA: 128 KB an SM in flight; the tile's token rows beside them, only those
+// that are there), four warps multiply 16 weight rows each by the tile's 16 tokens (mma.sync m16n8k16, the weights as its
+// rows; the second eight tokens only where there are any) and write their results while the next job's weights arrive.
+// CTA c takes the jobs (row tile, 64 weight rows) c, c + grid, ..., so that tiles of one expert read its weights at about the
+// same time.  The jobs behind the last whole round are halved or quartered while there are CTAs for the pieces: CTAs that a
+// small product leaves idle would cost more than a piece's copies of the token rows (1024 x 1024 of 16 experts, 8 tokens:
+// 11.7 us with runs of 16 rows dealt out evenly, across jobs; 9.1 with whole pieces).
+// Eight tokens, 64 experts (8 chosen), bytes of the weights met: gate and up of 4096 x 4096 240 us -> 220 (6.0 -> 6.5 TB/s),
+// down of 4096 x 2048 124 -> 108, against a CTA a job with four stages of 64 k by cp.async; 2816 x 2048 79 -> 70, 2048 x 1408
+// 49 -> 41, 1024 x 1024 of 16 experts 13.9 -> 9.7.  One CTA an SM with ten stages gets 4.4 TB/s (its warps' chain of waits and
+// products is longer than a stage's arrival), two with five 6.5 but 5.8 with 16 tokens a tile (here 6.4), three with three
+// as much as four with two up to 8 tokens and 3 % less beyond, five with two 5.2 (bound by waiting for free stages).
+constexpr int ROWS_BM = 16, ROWS_BN = 64, ROWS_BK = 128, ROWS_ST = 2, ROWS_CTAS = 4, ROWS_THREADS = 160;
+constexpr int ROWS_BOX = 16 * 64 * 2;                        // 16 weight rows x 64 k, 128-byte swizzle
+constexpr int ROWS_W = ROWS_BN * ROWS_BK * 2;                // a stage's weights: [k half][16 rows] boxes
+constexpr int ROWS_LD = ROWS_BK * 2 + 16;                    // bytes from token row to token row: eight rows meet no bank twice
+constexpr int ROWS_A = ROWS_BM * ROWS_LD;
+constexpr size_t ROWS_SMEM = 1024 + (size_t)ROWS_ST * (ROWS_W + ROWS_A);
+
+// The jobs of a CTA in order: a row tile, the first weight row, runs of 16 weight rows (1 to 4).
+struct RowJobs {
+  int nb, N, whole, unit, at, end, tile, n0, runs;
+  __device__ RowJobs(int tiles, int N_) : N(N_) {
+    nb = (N + ROWS_BN - 1) / ROWS_BN;
+    const int jobs = tiles * nb, grid = gridDim.x;
+    whole = jobs / grid * grid;
+    unit = (jobs - whole) * 2 > grid ? 4 : ((jobs - whole) * 4 > grid ? 2 : 1);
+    end = whole + (jobs - whole) * (4 / unit);
+    at = blockIdx.x;
+  }
+  __device__ bool next() {
+    if (at >= end) return false;
+    int job = at, first = 0, n = 4;
+    if (at >= whole) {
+      first = (at - whole) * unit % 4;
+      job = whole + (at - whole) * unit / 4;
+      n = unit;
+    }
+    at += gridDim.x;
+    tile = job / nb;
+    n0 = job % nb * ROWS_BN + 16 * first;
+    runs = min(n, (N - n0 + 15) / 16);                       // (may be none: the last weight rows of an odd N)
+    return true;
+  }
+};
+
+// MODE 0 and 1 as above; 2: mode 0 with weight rows in (gate, up) pairs, out [cap, N / 2] = act(gate) * up of the two results
+// rounded to bfloat16 (as a kernel of its own behind the product would find them; that kernel took 4.5 us and a launch).
+template <int MODE>
+__global__ void __launch_bounds__(ROWS_THREADS)
+moe_gemm_rows_kernel(const __grid_constant__ CUtensorMap mw, const __nv_bfloat16* __restrict__ A, int64_t lda,
+                     __nv_bfloat16* __restrict__ C, int64_t ldc, const int* __restrict__ sorted,
+                     const int* __restrict__ tile_expert, const float* __restrict__ weights, int pairs, int top, int N, int K,
+                     int max_tiles, int act, float ga, float gb, int* status) {
+  using namespace dinfer_umma;
+  extern __shared__ unsigned char rows_smem[];
+  __shared__ __align__(8) uint64_t full_bar[ROWS_ST], free_bar[ROWS_ST];
+  __shared__ int s_tiles;
+  unsigned char* sw = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(rows_smem) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sa = sw + (size_t)ROWS_ST * ROWS_W;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < ROWS_ST; ++s) { mbar_init(dinfer_umma::smem_u32(&full_bar[s]), 1); mbar_init(dinfer_umma::smem_u32(&free_bar[s]), 4); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_tiles = 0;
+  }
+  __syncthreads();
+  pdl_wait();
+  int used = 0;
+  for (int i = tid; i < max_tiles; i += ROWS_THREADS)
+    if (tile_expert[i] >= 0) used = i + 1;
+  if (used) atomicMax(&s_tiles, used);
+  __syncthreads();
+  RowJobs jobs(s_tiles, N);
+  const int steps = (K + ROWS_BK - 1) / ROWS_BK;
+  int j = 0;                                                 // stages so far
+  if (warp == 4) {
+    bool ok = true;
+    while (ok && jobs.next()) {
+      const int e = tile_expert[jobs.tile], runs = jobs.runs;
+      if (e < 0 || runs <= 0) continue;
+      const __nv_bfloat16* row = nullptr;                    // lanes 16 and up: a token row each
+      if (lane >= 16) {
+        const int pos = jobs.tile * ROWS_BM + lane - 16, p = sorted[pos];
+        if (p < pairs) row = A + (MODE == 1 ? (int64_t)pos : (int64_t)(p / top)) * lda;
+      }
+      const int rows = __popc(__ballot_sync(0xffffffffu, row != nullptr));
+      const int y = e * N + jobs.n0;
+      for (int t = 0; t < steps; ++t, ++j) {
+        const int s = j % ROWS_ST, k0 = t * ROWS_BK, left = min(ROWS_BK, K - k0), halves = left > 64 ? 2 : 1;
+        const uint32_t bar = dinfer_umma::smem_u32(&full_bar[s]);
+        if (lane == 0) {
+          ok = mbar_wait(dinfer_umma::smem_u32(&free_bar[s]), ((j / ROWS_ST) & 1) ^ 1);
+          if (ok) mbar_expect_tx(bar, halves * runs * ROWS_BOX + rows * left * 2);
+          else atomicExch(status, 46);
+        }
+        ok = __shfl_sync(0xffffffffu, (int)ok, 0);
+        if (!ok) break;
+        if (lane < 4 * halves && (lane & 3) < runs)
+          tma_load_2d(dinfer_umma::smem_u32(sw + s * ROWS_W + lane * ROWS_BOX), &mw, k0 + (lane >> 2) * 64, y + (lane & 3) * 16, bar);
+        if (row)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                       ::"r"(dinfer_umma::smem_u32(sa + s * ROWS_A + (lane - 16) * ROWS_LD)), "l"(row + k0), "r"(left * 2), "r"(bar) : "memory");
+      }
+    }
+    pdl_launch_dependents();
+    if (!ok && lane == 0)                                    // copies still on their way land before the CTA goes
+      for (int i = j < ROWS_ST ? 0 : j - ROWS_ST; i < j; ++i) mbar_wait(dinfer_umma::smem_u32(&full_bar[i % ROWS_ST]), (i / ROWS_ST) & 1);
+    return;
+  }
+  while (jobs.next()) {
+    if (tile_expert[jobs.tile] < 0 || jobs.runs <= 0) continue;
+    const bool mine = warp < jobs.runs;
+    const int pos = jobs.tile * ROWS_BM;
+    const bool second = __any_sync(0xffffffffu, lane < 8 && sorted[pos + 8 + (lane & 7)] < pairs);
+    float acc[2][4] = {};
+    for (int t = 0; t < steps; ++t, ++j) {
+      const int s = j % ROWS_ST, left = min(ROWS_BK, K - t * ROWS_BK);
+      if (!mbar_wait(dinfer_umma::smem_u32(&full_bar[s]), (j / ROWS_ST) & 1)) { atomicExch(status, 47); return; }
+      __syncwarp();
+      if (mine) {
+        const unsigned char* w = sw + s * ROWS_W + warp * ROWS_BOX + (lane & 15) * 128;
+        const unsigned char* a = sa + s * ROWS_A + (lane & 7) * ROWS_LD;
+        auto weights_of = [&](uint32_t (&f)[4], int kk) {
+          ldsm_x4(f, w + (kk >> 6) * 4 * ROWS_BOX + (((((kk & 63) >> 3) + (lane >> 4)) ^ (lane & 7)) << 4));
+        };
+        if (left == ROWS_BK) {
+          // every operand of the stage is asked for before its first product: the products are one chain
+          constexpr int KS = ROWS_BK / 16;
+          uint32_t f[KS][4], b[KS / 2][4], c[KS / 2][4];
+#pragma unroll
+          for (int u = 0; u < KS; ++u) {
+            weights_of(f[u], 16 * u);
+            if (u % 2 == 0) ldsm_x4(b[u / 2], a + u * 32 + ((lane >> 3) << 4));
+          }
+          if (second)
+#pragma unroll
+            for (int u = 0; u < KS / 2; ++u) ldsm_x4(c[u], a + 8 * ROWS_LD + u * 64 + ((lane >> 3) << 4));
+#pragma unroll
+          for (int u = 0; u < KS; ++u) mma_bf16(acc[0], f[u], b[u / 2][2 * (u & 1)], b[u / 2][2 * (u & 1) + 1]);
+          if (second)
+#pragma unroll
+            for (int u = 0; u < KS; ++u) mma_bf16(acc[1], f[u], c[u / 2][2 * (u & 1)], c[u / 2][2 * (u & 1) + 1]);
+        } else {
+          for (int kk = 0; kk < left; kk += 16) {
+            uint32_t f[4], b[4];
+            weights_of(f, kk);
+            ldsm_x4(b, a + (lane >> 4) * 8 * ROWS_LD + (((lane >> 3) & 1) << 4) + kk * 2);
+            if (kk + 8 >= left) { b[1] = 0; b[3] = 0; }      // (the weights are zero there, the tokens' bytes are old)
+            mma_bf16(acc[0], f, b[0], b[1]);
+            if (second) mma_bf16(acc[1], f, b[2], b[3]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dinfer_umma::smem_u32(&free_bar[s]));
+    }
+    if (!mine) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h && !second) break;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int at = pos + 8 * h + 2 * (lane & 3) + q, p = sorted[at];
+        float up[2] = {0.f, 0.f};
+        if (MODE == 2) { up[0] = __shfl_xor_sync(0xffffffffu, acc[h][q], 4); up[1] = __shfl_xor_sync(0xffffffffu, acc[h][2 + q], 4); }
+        if (p >= pairs || (MODE == 2 && (lane & 4))) continue;
+        __nv_bfloat16* out = C + (MODE == 1 ? (int64_t)p : (int64_t)at) * ldc;
+        const float by = MODE == 1 ? weights[p] : 1.f;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int n = jobs.n0 + 16 * warp + (lane >> 2) + 8 * u;
+          const float v = acc[h][2 * u + q];
+          if (n >= N) continue;
+          if (MODE == 2) {
+            const float g = __bfloat162float(__float2bfloat16_rn(v)), w = __bfloat162float(__float2bfloat16_rn(up[u]));
+            out[n >> 1] = __float2bfloat16_rn(act == ACT_CLAMPED ? clamped_swish_fast(g, w, ga, gb) : activate(g, act) * w);
+          } else {
+            out[n] = __float2bfloat16_rn(MODE == 0 ? activate(v, act) : v * by);
+          }
+        }
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------- combine
@@ -588,6 +766,38 @@ __global__ void xielu_bf16x8_kernel(const uint4* __restrict__ x, uint4* __restri
   }
 }
 
+// ---- host side of the products on row tiles of 16
+template <int MODE>
+int launch_rows(const __nv_bfloat16* A, int64_t lda, const void* W, __nv_bfloat16* C, int64_t ldc, const int* sorted,
+                const int* tile_expert, const float* weights, int pairs, int top, int E, int N, int K, int cap, int act,
+                float ga, float gb, int* status, cudaStream_t stream) {
+  static const auto encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(ok ? f : nullptr);
+  }();
+  static std::atomic<uint64_t> allowed{0};
+  if (!status) return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: a status word is required");
+  if (!encode) return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: cuTensorMapEncodeTiled is not available from this driver");
+  CUtensorMap map;
+  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)E * N}, strides[1] = {(cuuint64_t)K * 2};
+  const cuuint32_t box[2] = {64, 16}, ones[2] = {1, 1};
+  const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(W), dims, strides, box, ones,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: cuTensorMapEncodeTiled failed with %d", (int)r);
+  const cudaError_t e = dinfer_split::allow_shared(moe_gemm_rows_kernel<MODE>, ROWS_SMEM, allowed);
+  if (e != cudaSuccess) return refuse((int)e, "moe_gemm: shared memory opt-in failed: %s", cudaGetErrorString(e));
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int64_t jobs = (int64_t)((N + ROWS_BN - 1) / ROWS_BN) * (cap / ROWS_BM) * 4;
+  launch_pdl(moe_gemm_rows_kernel<MODE>, dim3((unsigned)(jobs < ROWS_CTAS * sms ? jobs : ROWS_CTAS * sms)), dim3(ROWS_THREADS), ROWS_SMEM, stream, map, A,
+             lda, C, ldc, sorted, tile_expert, weights, pairs, top, N, K, cap / ROWS_BM, act, ga, gb, status);
+  return cuda_status("moe_gemm");
+}
+
 }  // namespace
 
 DINFER_DEFINE_LAST_ERROR()
@@ -648,26 +858,38 @@ DINFER_API int dinfer_moe_align(const int* ids, int* sorted, int* tile_expert, i
 
 // mode 0: A = h [T, K] (row of pair p: p / top), C [cap, N] by position, epilogue activation `act`.
 // mode 1: A [cap, K] by position, C [pairs, N] by pair, each row times weights[pair].  W [E, N, K] contiguous.
+// mode 2: mode 0 with (gate, up) pairs of weight rows, C [cap, N / 2]: act(gate) * up, or (act 5) the clamped gate with its
+// limit ga > 0 and its factor gb; row tiles of 16 of bfloat16 operands that TMA can address only.
+// status: a device int that a kernel sets non-zero when one of its bounded waits ran out.
 DINFER_API int dinfer_moe_gemm(const void* A, int64_t lda, const void* W, void* C, int64_t ldc, const int* sorted,
-                               const int* tile_expert, const float* weights, int pairs, int top, int N, int K, int BM,
-                               int cap, int mode, int act, int act_dtype, int w_dtype, cudaStream_t stream) {
-  if (pairs < 0 || top <= 0 || N <= 0 || K <= 0 || (BM != 16 && BM != 64) || cap % BM || lda < K || ldc < N ||
-      (mode != 0 && mode != 1) || (mode == 1 && !weights))
+                               const int* tile_expert, const float* weights, int pairs, int top, int E, int N, int K, int BM,
+                               int cap, int mode, int act, float ga, float gb, int act_dtype, int w_dtype, int* status,
+                               cudaStream_t stream) {
+  if (pairs < 0 || top <= 0 || E <= 0 || N <= 0 || K <= 0 || (BM != 16 && BM != 64) || cap % BM || lda < K ||
+      ldc < (mode == 2 ? N / 2 : N) || mode < 0 || mode > 2 || (mode == 1 && !weights) ||
+      (mode == 2 && (N % 2 || BM != 16 || act <= 0 || act > ACT_CLAMPED || (act == ACT_CLAMPED && !(ga > 0.f)))))
     return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: bad arguments pairs=%d N=%d K=%d BM=%d cap=%d mode=%d", pairs, N, K, BM, cap, mode);
   if (pairs == 0) return 0;
   dim3 grid((N + 63) / 64, cap / BM);
   if (grid.y > 65535) return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: too many row tiles (%d)", (int)grid.y);
   if (act_dtype == DINFER_BF16 && w_dtype == DINFER_BF16 && K % 8 == 0 && lda % 8 == 0 &&
       !(reinterpret_cast<uintptr_t>(A) & 15) && !(reinterpret_cast<uintptr_t>(W) & 15)) {
-    if (BM == 64) grid.x = (N + 127) / 128;
-#define GO_MMA(BM_, MODE_)                                                                                         \
-  launch_pdl(moe_gemm_mma_kernel<BM_, MODE_>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)A, lda,           \
+    if (BM == 16 && (int64_t)grid.x * grid.y * 4 <= 0x7fffffff && (int64_t)E * N <= 0x7fffffff) {
+      auto launch = mode == 0 ? launch_rows<0> : (mode == 1 ? launch_rows<1> : launch_rows<2>);
+      return launch((const __nv_bfloat16*)A, lda, W, (__nv_bfloat16*)C, ldc, sorted, tile_expert, weights, pairs, top, E, N, K,
+                    cap, act, ga, gb, status, stream);
+    }
+    if (BM == 64) {
+      grid.x = (N + 127) / 128;
+#define GO_MMA(MODE_)                                                                                              \
+  launch_pdl(moe_gemm_mma_kernel<MODE_>, grid, dim3(128), 0, stream, (const __nv_bfloat16*)A, lda,                \
              (const __nv_bfloat16*)W, (__nv_bfloat16*)C, ldc, sorted, tile_expert, weights, pairs, top, N, K, act)
-    if (BM == 16) { if (mode == 0) GO_MMA(16, 0); else GO_MMA(16, 1); }
-    else { if (mode == 0) GO_MMA(64, 0); else GO_MMA(64, 1); }
+      if (mode == 0) GO_MMA(0); else GO_MMA(1);
 #undef GO_MMA
-    return cuda_status("moe_gemm");
+      return cuda_status("moe_gemm");
+    }
   }
+  if (mode == 2) return refuse(DINFER_BAD_ARGUMENT, "moe_gemm: a gate needs bfloat16 operands on 16 bytes, rows of multiples of 8");
 #define GO(BM_, MODE_)                                                                                              \
   launch_pdl(moe_gemm_simt_kernel<TA, TW, BM_, MODE_>, grid, dim3(256), 0, stream, (const TA*)A, lda, (const TW*)W, \
              (TA*)C, ldc, sorted, tile_expert, weights, pairs, top, N, K, act)

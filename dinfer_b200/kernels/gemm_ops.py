@@ -62,6 +62,8 @@ STATUS_MEANING = {
     43: "32-bit product: the summing warps waited for a stage's sums",
     44: "32-bit product: the TMA producer waited for a free stage",
     45: "32-bit product: the splitting warps waited for an operand tile",
+    46: "routed products: the TMA producer waited for a free stage",
+    47: "routed products: a warp waited for the experts' weights",
     51: "state-space chunks: the sums waited for their operands or their MMAs",
     52: "state-space chunks: the outputs waited for their operands or their MMAs",
 }

@@ -7,8 +7,10 @@ from typing import Optional, Tuple
 import torch
 
 from .lib import KernelError, check, dtype_code, ptr, require_cuda, stream_handle
-from .ops import _fn, _rows_contiguous
+from .ops import _fn, _rows_contiguous, _status, gate_constants
 
+_GEMM_ARGS = [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p] + [c_int] * 9 + \
+    [c_float, c_float, c_int, c_int, c_void_p, c_void_p]
 ACTIVATIONS = {"none": 0, "relu2": 1, "silu": 2, "gelu_tanh": 3, "relu": 4}
 
 
@@ -165,28 +167,43 @@ def align(ids: torch.Tensor, num_experts: int, tile: int) -> Tuple[torch.Tensor,
     return sorted_, tile_expert
 
 
+def gate_in_rows(x: torch.Tensor, w_up: torch.Tensor, tile: int, activation) -> bool:
+    """Whether ``grouped_gemm`` takes the gate of (gate, up) row pairs into the first product: row tiles of 16, bfloat16
+    operands that TMA can address."""
+    name = activation[0] if isinstance(activation, (tuple, list)) else activation
+    return (tile == 16 and (name == "clamped_swish" or ACTIVATIONS.get(name, 0) > 0) and x.dtype == torch.bfloat16
+            and w_up.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and w_up.data_ptr() % 16 == 0 and w_up.shape[0] * w_up.shape[1] < 1 << 31)
+
+
 def grouped_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, sorted_: torch.Tensor, tile_expert: torch.Tensor,
                  pairs: int, top_k: int, tile: int, mode: int, activation: str = "none",
-                 weights: Optional[torch.Tensor] = None) -> torch.Tensor:
+                 weights: Optional[torch.Tensor] = None, gate=None) -> torch.Tensor:
     """mode 0: ``out[pos] = act(a[pair // top_k] @ w[e]^T)`` for every position of the layout (a [T, K], out [cap, N]);
-    mode 1: ``out[pair] = (a[pos] @ w[e]^T) * weights[pair]`` (a [cap, K], out [pairs, N]).  w [E, N, K]."""
+    mode 1: ``out[pair] = (a[pos] @ w[e]^T) * weights[pair]`` (a [cap, K], out [pairs, N]).  w [E, N, K].  ``gate`` (mode 0,
+    where ``gate_in_rows``): the rows of w[e] are (gate, up) pairs and out is [cap, N / 2], act(gate) * up."""
     require_cuda(a, w, out, sorted_, tile_expert, weights)
     _rows_contiguous(a, "moe gemm a")
     _rows_contiguous(out, "moe gemm out")
     E, N, K = w.shape
     cap = sorted_.numel()
-    if not w.is_contiguous() or a.shape[1] != K or out.shape[1] != N or out.dtype != a.dtype:
+    act, ga, gb = ACTIVATIONS[activation], 0.0, 0.0
+    if gate is not None:
+        if mode != 0 or activation != "none" or N % 2 or not gate_in_rows(a, w, tile, gate):
+            raise KernelError("moe gemm: a gate belongs to mode 0 on row tiles of 16 (bfloat16), (gate, up) row pairs")
+        name, ga, gb = gate_constants(gate)
+        act = 5 if name == "clamped_swish" else ACTIVATIONS[name]
+        mode = 2
+    if not w.is_contiguous() or a.shape[1] != K or out.shape[1] != (N if mode != 2 else N // 2) or out.dtype != a.dtype:
         raise KernelError("moe gemm: w [E, N, K] contiguous, a [*, K], out [*, N] of a's dtype")
-    if (mode == 0 and out.shape[0] != cap) or (mode == 1 and (a.shape[0] != cap or out.shape[0] != pairs)):
+    if (mode != 1 and out.shape[0] != cap) or (mode == 1 and (a.shape[0] != cap or out.shape[0] != pairs)):
         raise KernelError("moe gemm: row counts do not fit the layout")
     if mode == 1 and (weights is None or weights.dtype != torch.float32 or weights.numel() != pairs):
         raise KernelError("moe gemm: mode 1 needs the routing weights, f32 [pairs]")
-    lib, f = _fn("moe", "dinfer_moe_gemm",
-                 [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                  c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
+    lib, f = _fn("moe", "dinfer_moe_gemm", _GEMM_ARGS)
     check(lib, f(ptr(a), a.stride(0), ptr(w), ptr(out), out.stride(0), ptr(sorted_), ptr(tile_expert), ptr(weights),
-                 pairs, top_k, N, K, tile, cap, mode, ACTIVATIONS[activation], dtype_code(a.dtype), dtype_code(w.dtype),
-                 stream_handle()), "moe_gemm")
+                 pairs, top_k, E, N, K, tile, cap, mode, act, ga, gb, dtype_code(a.dtype), dtype_code(w.dtype),
+                 _status(a.device), stream_handle()), "moe_gemm")
     return out
 
 

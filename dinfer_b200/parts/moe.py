@@ -207,9 +207,13 @@ class MoE(FeedForward):
             return self._combine(x, y, gate, identity)
         tile = moe_ops.row_tile(pairs, self.E)
         order, tile_expert = moe_ops.align(ids, self.E, tile)
-        u = torch.empty((order.numel(), wide), dtype=x.dtype, device=x.device)
-        moe_ops.grouped_gemm(x, self.w_up, u, order, tile_expert, pairs, self.top, tile, 0, first_act)
-        u, weights = self._gate(u, order, weights)
+        if self.gated and not self.weight_on_input and moe_ops.gate_in_rows(x, self.w_up, tile, self.activation):
+            u = torch.empty((order.numel(), self.ff), dtype=x.dtype, device=x.device)          # the gate in the epilogue
+            moe_ops.grouped_gemm(x, self.w_up, u, order, tile_expert, pairs, self.top, tile, 0, gate=self.activation)
+        else:
+            u = torch.empty((order.numel(), wide), dtype=x.dtype, device=x.device)
+            moe_ops.grouped_gemm(x, self.w_up, u, order, tile_expert, pairs, self.top, tile, 0, first_act)
+            u, weights = self._gate(u, order, weights)
         y = torch.empty((pairs, self.hidden), dtype=x.dtype, device=x.device)
         moe_ops.grouped_gemm(u, self.w_down, y, order, tile_expert, pairs, self.top, tile, 1, weights=weights)
         return self._combine(x, y, gate, identity)
