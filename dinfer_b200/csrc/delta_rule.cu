@@ -114,19 +114,37 @@ delta_prep_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv,
   }
 }
 
-// The same for steps of many tokens (four taps; heads of 64 or 128 key channels that fill blocks of 128 channels): a thread
-// owns a channel and walks RUN tokens with the last three inputs in registers, so that an input is read 11 / 8 times
-// instead of four, and the block's eight norms are summed in one exchange.  Bound by the exponentials and divisions of
-// silu and by its reads and writes: 2000 tokens of 16 heads of 128 (8 key heads) 40.5 us, a block per (token, head) 59.
+// The same for steps of many tokens (four taps; heads of 64 or 128 key channels that fill blocks of 128 channels): a lane
+// owns four channels, a warp 128 of them, and walks RUN tokens whose inputs it reads at once, 11 loads of four elements in
+// flight, so that an input is read 11 / 8 times instead of four; a head's norm is a sum inside the warp.  Bound by its
+// reads and writes, then by the exponentials and divisions of silu: 2000 tokens of 16 heads of 128 (8 key heads; 65 MB) 20.6
+// us, 40.8 with a channel a lane and the norms exchanged through shared memory, 59 with a block per (token, head).
+// Where an address does not take four elements (VEC false) a lane reads them one by one.
 // Tokens of a run that spans requests (or begins a portion) go one after the other, with a search and loads of their own, so
 // it is taken for portions: from RUN_FROM tokens and RUN_PORTION tokens a request on (256 for a request alone).  us, a block
-// per (token, head) and in runs, 16 heads of 128: 128 tokens 10.2 and 10.6, 256 13.4 and 12.9, 512 19.6 and 16.3; 32 requests of
-// 16 25.0 and 23.5, 64 of 8 27.3 and 31.0, 64 of 16 43.8 and 39.1; 64 single tokens and 64 of a portion 14.5 and 24.0, 16 and
-// 240 16.2 and 21.6, 16 and 496 23.8 and 22.8; 512 single tokens 45.7 and 51.8.  (16 heads of 64: 256 tokens 12.0 and 10.8, 32
-// of 16 20.9 and 18.6, 16 and 496 20.1 and 20.4.)
+// per (token, head) and in runs, 16 heads of 128: 256 tokens 13.4 and 11.3, 512 19.6 and 12.7; 32 requests of 16 25.0 and 15.3,
+// 64 of 16 43.8 and 24.9; 16 single tokens and 496 of a portion 23.8 and 15.6.  Below the lines a channel a lane lost (64 of 8
+// 27.3 and 31.0, 512 single tokens 45.7 and 51.8, 128 tokens 10.2 and 10.6): a run's tokens go one after the other there.
 constexpr int RUN = 8;
 constexpr int RUN_FROM = 512, RUN_FROM_ALONE = 256, RUN_PORTION = 16;
-template <typename TA>
+// four neighbouring elements as 32-bit values; VEC: the address is a multiple of their size
+template <bool VEC, typename T>
+__device__ __forceinline__ void load4(const T* __restrict__ p, float (&v)[4]) {
+  if constexpr (VEC && sizeof(T) == 4) {
+    const float4 f = *reinterpret_cast<const float4*>(p);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+  } else if constexpr (VEC) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = to_f32<T>(p[i]);
+  }
+}
+
+template <typename TA, bool VEC>
 __global__ void __launch_bounds__(128)
 delta_prep_run_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv, int cb, const TA* __restrict__ A,
                       int64_t lda, const float* __restrict__ conv_w, const float* __restrict__ A_log,
@@ -135,85 +153,106 @@ delta_prep_run_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int
                       float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ beta,
                       float* __restrict__ decay, int H, int G, int dk, int dv, int per_channel) {
   constexpr int TAPS = 4;
-  __shared__ float part[4][RUN];
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = blockIdx.x * RUN, n = min(RUN, T - t0);
   const int nq = G * dk, nv = H * dv, C = 2 * nq + nv;
   const int channel_blocks = (C + 127) / 128;
   if ((int)blockIdx.y >= channel_blocks) {                 // the decays, and the betas with the first of them
-    const int job = blockIdx.y - channel_blocks, nd = per_channel ? H * dk : H;
-    const int c_end = min(nd, (job + 1) * PREP_CHUNK);
-    for (int t = t0; t < t0 + n; ++t) {
-      if (job == 0)
-        for (int h = tid; h < H; h += 128) beta[(int64_t)t * H + h] = sigmoid_f(to_f32<TA>(P[(int64_t)t * ldp + cb + h]));
-      for (int c = job * PREP_CHUNK + tid; c < c_end; c += 128) {
-        const float a = to_f32<TA>(A[(int64_t)t * lda + c]) + dt_bias[c];
-        decay[(int64_t)t * nd + c] = expm1f(-expf(A_log[per_channel ? c / dk : c]) * softplus_f(a));
+    const int y = blockIdx.y - channel_blocks, job = y >> 2, nd = per_channel ? H * dk : H;
+    const int t0 = (blockIdx.x * 4 + (y & 3)) * RUN, n = min(RUN, T - t0);
+    const int c_end = min(nd, (job + 1) * PREP_CHUNK), width = c_end - job * PREP_CHUNK;
+    if (job == 0)
+      for (int i = tid; i < n * H; i += 128) {
+        const int t = t0 + i / H, h = i % H;
+        beta[(int64_t)t * H + h] = sigmoid_f(to_f32<TA>(P[(int64_t)t * ldp + cb + h]));
       }
+    for (int i = tid; i < n * width; i += 128) {
+      const int t = t0 + i / width, c = job * PREP_CHUNK + i % width;
+      const float a = to_f32<TA>(A[(int64_t)t * lda + c]) + dt_bias[c];
+      decay[(int64_t)t * nd + c] = expm1f(-expf(A_log[per_channel ? c / dk : c]) * softplus_f(a));
     }
     return;
   }
-  const int c = blockIdx.y * 128 + tid;
-  const bool live = c < C;
+  const int t0 = (blockIdx.x * 4 + warp) * RUN, n = min(RUN, T - t0);
+  const int c = blockIdx.y * 128 + 4 * lane, live = min(4, C - c);       // (VEC: four, or none)
+  if (n <= 0) return;
+  const bool all = live == 4;
+  if (blockIdx.y * 128 >= 2 * nq && live <= 0) return;
+  // (the channels of a lane lie in one of q, k and v: they are multiples of 64 wide, or of 4 at the end of v)
   const int col = c < nq ? cq + c : (c < 2 * nq ? ck + c - nq : cv + c - 2 * nq);
-  float w[TAPS], y[RUN];
+  float w[4][TAPS];                                        // w[j][TAPS - 1 - d] weighs the token d back
 #pragma unroll
-  for (int d = 0; d < TAPS; ++d) w[d] = live ? conv_w[c * TAPS + TAPS - 1 - d] : 0.f;    // w[d] weighs the token d back
+  for (int j = 0; j < 4; ++j) {
+    if (all) load4<VEC>(conv_w + (int64_t)(c + j) * TAPS, w[j]);
+    else
+#pragma unroll
+      for (int d = 0; d < TAPS; ++d) w[j][d] = j < live ? conv_w[(int64_t)(c + j) * TAPS + d] : 0.f;
+  }
+  const bool unit = (int)blockIdx.y * 128 < 2 * nq, is_q = c < nq;       // whole heads of q or k: unit vectors
+  const int64_t ldo = unit ? nq : nv;
+  float* o = (unit ? (is_q ? qn + c : kn + c - nq) : vv + c - 2 * nq) + (int64_t)t0 * ldo;
+  const float q_scale = 1.f / sqrtf((float)dk);
+  auto put = [&](int u, float (&y)[4]) {
+    if (unit) {
+      float ss = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], y[3] * y[3])));
+#pragma unroll
+      for (int m = 8; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+      if (dk == 128) ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+      float r = 1.f / sqrtf(ss + 1e-6f);
+      if (is_q) r *= q_scale;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) y[j] *= r;
+    }
+    if (VEC) *reinterpret_cast<float4*>(o + u * ldo) = make_float4(y[0], y[1], y[2], y[3]);
+    else
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < live) o[u * ldo + j] = y[j];
+  };
   const int b = request_of(cu, B, t0);
   const int i0 = t0 - cu[b];
-  if (i0 >= TAPS - 1 && t0 + n <= cu[b + 1]) {             // every tap falls into this request's tokens of the step
+  if (i0 >= TAPS - 1 && t0 + n <= cu[b + 1] && n == RUN && all) {        // every tap falls into this request's tokens of the step
     const TA* x = P + (int64_t)(t0 - (TAPS - 1)) * ldp + col;
-    float in[RUN + TAPS - 1];
+    float in[RUN + TAPS - 1][4];
 #pragma unroll
-    for (int u = 0; u < RUN + TAPS - 1; ++u) in[u] = live && u < n + TAPS - 1 ? to_f32<TA>(x[(int64_t)u * ldp]) : 0.f;
-#pragma unroll
-    for (int u = 0; u < RUN; ++u) {
-      float acc = 0.f;
-#pragma unroll
-      for (int d = 0; d < TAPS; ++d) acc = fmaf(w[d], in[u + TAPS - 1 - d], acc);
-      y[u] = silu_f(acc);
-    }
-  } else {
+    for (int u = 0; u < RUN + TAPS - 1; ++u) load4<VEC>(x + u * ldp, in[u]);
 #pragma unroll
     for (int u = 0; u < RUN; ++u) {
-      y[u] = 0.f;
-      if (u >= n || !live) continue;
-      const int t = t0 + u, bt = request_of(cu, B, t), i = t - cu[bt];
-      const float* hb = hist + (int64_t)slots[bt] * hist_stride;
-      float acc = 0.f;
-      for (int d = 0; d < TAPS; ++d) {
-        float x = 0.f;
-        if (i - d >= 0) x = to_f32<TA>(P[(int64_t)(t - d) * ldp + col]);
-        else if (!fresh[bt]) x = hb[(TAPS - 1 + i - d) * C + c];
-        acc = fmaf(conv_w[c * TAPS + TAPS - 1 - d], x, acc);
+      float y[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float acc = 0.f;
+#pragma unroll
+        for (int d = 0; d < TAPS; ++d) acc = fmaf(w[j][TAPS - 1 - d], in[u + TAPS - 1 - d][j], acc);
+        y[j] = silu_f(acc);
       }
-      y[u] = silu_f(acc);
+      put(u, y);
     }
+    return;
   }
-  if (blockIdx.y * 128 < 2 * nq) {                         // whole heads of q or k: unit vectors
+  for (int u = 0; u < n; ++u) {
+    const int t = t0 + u, bt = request_of(cu, B, t), i = t - cu[bt];
+    const float* hb = hist + (int64_t)slots[bt] * hist_stride;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int u = 0; u < RUN; ++u) {
-      const float ss = warp_sum(y[u] * y[u]);
-      if (lane == 0) part[warp][u] = ss;
+    for (int d = 0; d < TAPS; ++d) {
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (i - d >= 0) {
+        if (all) load4<VEC>(P + (int64_t)(t - d) * ldp + col, x);
+        else
+#pragma unroll
+          for (int j = 0; j < 4; ++j) if (j < live) x[j] = to_f32<TA>(P[(int64_t)(t - d) * ldp + col + j]);
+      } else if (!fresh[bt]) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (j < live) x[j] = hb[(int64_t)(TAPS - 1 + i - d) * C + c + j];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] = fmaf(w[j][TAPS - 1 - d], x[j], acc[j]);
     }
-    __syncthreads();
-    const int warps = dk / 32, w0 = warp / warps * warps;
-    const bool is_q = c < nq;
-    float* o = (is_q ? qn + c : kn + c - nq) + (int64_t)t0 * nq;
+    float y[4];
 #pragma unroll
-    for (int u = 0; u < RUN; ++u) {
-      float ss = 0.f;
-      for (int k = 0; k < warps; ++k) ss += part[w0 + k][u];
-      float r = 1.f / sqrtf(ss + 1e-6f);
-      if (is_q) r *= 1.f / sqrtf((float)dk);
-      if (u < n) o[(int64_t)u * nq] = y[u] * r;
-    }
-  } else if (live) {
-    float* o = vv + (int64_t)t0 * nv + c - 2 * nq;
-#pragma unroll
-    for (int u = 0; u < RUN; ++u)
-      if (u < n) o[(int64_t)u * nv] = y[u];
+    for (int j = 0; j < 4; ++j) y[j] = silu_f(acc[j]);
+    put(u, y);
   }
 }
 
@@ -507,6 +546,52 @@ delta_post_kernel(const float* __restrict__ o, const float* __restrict__ w, cons
   }
 }
 
+// Heads of 16, 32, 64 or 128 values on addresses that take four at a time: a lane holds four of them, a warp two sets of
+// 32 / (dv / 4) heads, everything read before the first sum.
+// 2000 tokens of 16 heads of 128, 32-bit gate: 20.7 us -> 15 from HBM (a warp per head, four loads of one element a lane, and
+// again behind the sum).
+template <typename TG, typename TA>
+__global__ void __launch_bounds__(128)
+delta_post4_kernel(const float* __restrict__ o, const float* __restrict__ w, const TG* __restrict__ gate, int64_t ldg,
+                   TA* __restrict__ y, int64_t ldy, int T, int H, int dv, float eps, int sigmoid_gate, int w_heads) {
+  constexpr int ITEMS = 2;
+  pdl_enter();
+  const int lanes = dv / 4, e = (int)threadIdx.x % lanes * 4;
+  const int64_t n = (int64_t)T * H, per = 128 / lanes, p0 = (int64_t)blockIdx.x * per * ITEMS + (int)threadIdx.x / lanes;
+  float x[ITEMS][4], z[ITEMS][4], wv[ITEMS][4];
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const int64_t p = min(p0 + k * per, n - 1), t = p / H;   // (past the end: the last head again, not stored)
+    const int h = (int)(p - t * H);
+    load4<true>(o + p * dv + e, x[k]);
+    if (gate) load4<true>(gate + t * ldg + (int64_t)h * dv + e, z[k]);
+    load4<true>(w + (w_heads ? (int64_t)h * dv : 0) + e, wv[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const int64_t p = p0 + k * per, t = p / H;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(x[k][i], x[k][i], ss);
+    for (int m = lanes / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    const float r = 1.f / sqrtf(ss / (float)dv + eps);
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float a = gate ? (sigmoid_gate ? sigmoid_f(z[k][i]) : silu_f(z[k][i])) : 1.f;
+      v[i] = x[k][i] * r * wv[k][i] * a;
+    }
+    if (p >= n) continue;
+    TA* out = y + t * ldy + (p - t * H) * dv + e;
+    if constexpr (sizeof(TA) == 4) {
+      *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+      __nv_bfloat162 q[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+      *reinterpret_cast<uint2*>(out) = *reinterpret_cast<uint2*>(q);
+    }
+  }
+}
+
 }  // namespace
 
 DINFER_DEFINE_LAST_ERROR()
@@ -531,14 +616,17 @@ DINFER_API int dinfer_delta_prep(const void* P, int64_t ldp, int cq, int ck, int
   const int nd = per_channel ? H * dk : H;
   const int jobs = 2 * G + (nv + PREP_CHUNK - 1) / PREP_CHUNK + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
   if (jobs > 65535) return refuse(DINFER_BAD_ARGUMENT, "delta_prep: too many heads for the grid");
-  const int run_jobs = (2 * nq + nv + 127) / 128 + (nd + PREP_CHUNK - 1) / PREP_CHUNK;
+  const int run_jobs = (2 * nq + nv + 127) / 128 + 4 * ((nd + PREP_CHUNK - 1) / PREP_CHUNK);
   const bool runs = dinfer_delta_prep_runs(T, B, G, dk, taps) && run_jobs <= 65535;
   DINFER_DISPATCH_DTYPE(act_dtype, TA, {
-    if (runs)
-      launch_pdl(delta_prep_run_kernel<TA>, dim3((T + RUN - 1) / RUN, run_jobs), dim3(128), 0, stream, (const TA*)P, ldp, cq, ck,
-                 cv, cb, (const TA*)A, lda, conv_w, A_log, dt_bias, (const float*)hist, hist_stride, cu, slots, fresh, B, T, qn,
-                 kn, vv, beta, decay, H, G, dk, dv, per_channel);
-    else
+    if (runs) {
+      const auto on = [](const void* q, int bytes) { return reinterpret_cast<uintptr_t>(q) % bytes == 0; };
+      const bool vec = nv % 4 == 0 && cq % 4 == 0 && ck % 4 == 0 && cv % 4 == 0 && ldp % 4 == 0 && on(P, 4 * sizeof(TA)) &&
+                       on(conv_w, 16) && on(qn, 16) && on(kn, 16) && on(vv, 16);
+      launch_pdl(vec ? delta_prep_run_kernel<TA, true> : delta_prep_run_kernel<TA, false>, dim3((T + 4 * RUN - 1) / (4 * RUN), run_jobs),
+                 dim3(128), 0, stream, (const TA*)P, ldp, cq, ck, cv, cb, (const TA*)A, lda, conv_w, A_log, dt_bias,
+                 (const float*)hist, hist_stride, cu, slots, fresh, B, T, qn, kn, vv, beta, decay, H, G, dk, dv, per_channel);
+    } else
       launch_pdl(delta_prep_kernel<TA>, dim3(T, jobs), dim3(128), smem, stream, (const TA*)P, ldp, cq, ck, cv, cb, (const TA*)A,
                  lda, conv_w, A_log, dt_bias, (const float*)hist, hist_stride, cu, slots, fresh, B, qn, kn, vv, beta,
                  decay, H, G, dk, dv, taps, per_channel);
@@ -656,6 +744,14 @@ DINFER_API int dinfer_delta_post_ex(const float* o, const float* w, const void* 
   const int64_t blocks = ((int64_t)T * H + 3) / 4;
   DINFER_DISPATCH_DTYPE(gate_dtype, TG,
     DINFER_DISPATCH_DTYPE(act_dtype, TA, {
+      const auto on = [](const void* q, int bytes) { return reinterpret_cast<uintptr_t>(q) % bytes == 0; };
+      if ((dv == 16 || dv == 32 || dv == 64 || dv == 128) && ldy % 4 == 0 && on(o, 16) && on(w, 16) && on(y, 4 * sizeof(TA)) &&
+          (!gate || (ldg % 4 == 0 && on(gate, 4 * sizeof(TG))))) {
+        const int64_t per = 2 * 128 / (dv / 4);
+        launch_pdl(delta_post4_kernel<TG, TA>, dim3((unsigned)(((int64_t)T * H + per - 1) / per)), dim3(128), 0, stream, o, w,
+                   (const TG*)gate, ldg, (TA*)y, ldy, T, H, dv, eps, sigmoid_gate, w_heads);
+        return cuda_status("delta_post");
+      }
       launch_pdl(delta_post_kernel<TG, TA>, dim3((unsigned)blocks), dim3(128), 0, stream, o, w, (const TG*)gate, ldg, (TA*)y,
                  ldy, T, H, dv, eps, sigmoid_gate, w_heads);
       return cuda_status("delta_post");

@@ -196,3 +196,32 @@ def test_which_portions_run_in_chunks(B, H, longest, chunks, monkeypatch):
                              torch.empty_like(v), longest)
     torch.cuda.synchronize()
     assert took is chunks
+
+
+@pytest.mark.parametrize("dv,H,T", [(16, 3, 11), (32, 5, 7), (64, 1, 1), (64, 3, 43), (128, 16, 9), (128, 1, 5)])
+@pytest.mark.parametrize("gate", [None, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+def test_output_norm_of_whole_heads(dv, H, T, gate, out):
+    """Four values a lane (a warp's last heads may be past the end), and the same from rows off their alignment."""
+    from dinfer_b200.kernels import delta_ops
+    g = torch.Generator().manual_seed(dv + T)
+    o = torch.randn(T, H, dv, generator=g).cuda()
+    heads = H > 1
+    w = (1 + 0.2 * torch.randn(H * dv if heads else dv, generator=g)).cuda()
+    for sigmoid in (False, True):
+        got = []
+        for shift in (0, 1):                                 # a row that starts one element in: the other kernel
+            z = None if gate is None else torch.randn(T, H * dv + 4, generator=torch.Generator().manual_seed(1)).to(gate)
+            if z is not None:
+                z = torch.cat([torch.zeros(T, 4 + shift, dtype=gate), z[:, :H * dv], torch.zeros(T, 4 - shift, dtype=gate)], 1).cuda()[:, 4 + shift:4 + shift + H * dv]
+            y = torch.empty(T, H * dv + 4, dtype=out, device="cuda")[:, shift:shift + H * dv]
+            delta_ops.post(o, w, z, 1e-5, sigmoid, y)
+            got.append(y.double().reshape(T, H, dv))
+        want = o.double() / torch.sqrt((o.double() ** 2).mean(-1, keepdim=True) + 1e-5) * w.double().reshape(H if heads else 1, dv)
+        if z is not None:
+            zz = z.double().reshape(T, H, dv)
+            want = want * (torch.sigmoid(zz) if sigmoid else zz * torch.sigmoid(zz))
+        # a dozen 32-bit roundings, then one to the output's type
+        tol = 12 * 2 ** -23 + (2 ** -8 if out == torch.bfloat16 else 0)
+        for y in got:
+            assert bool(((y - want).abs() <= tol * want.abs() + 1e-6).all())
