@@ -525,8 +525,8 @@ argmax_many_kernel(const float* __restrict__ logits, int64_t ld, int* __restrict
 // What bounds it: the instructions of its passes over the row in shared memory and the cluster barriers between them, not
 // the one read of the row (39 MB for 64 rows of 151936: 6 us).  64 rows, greedy / temperature / top-k 20 + top-p 0.95 /
 // top-p 0.9 in turn, took 165 us with eight radix rounds for the top-p threshold, a shared-memory histogram for the top-k
-// one and one block of 1024 threads to an SM; 58 us now.  Alone, at 8 and 64 rows: top-k 20 + top-p 24 and 118 -> 22 and
-// 57 us, top-p 0.9 72 and 359 -> 26 and 77 us.  Rows without likely tokens (normal, sigma 1.4 and 4.3), top-p 0.95: 80 and 397,
+// one and one block of 1024 threads to an SM; 53 us now (59 with the block's barriers in every exchange).  Alone, at 8 and 64 rows: top-k 20 + top-p 24 and 118 -> 22 and
+// 57 us, top-p 0.9 72 and 359 -> 26 and 68 us.  Rows without likely tokens (normal, sigma 1.4 and 4.3), top-p 0.95: 80 and 397,
 // 77 and 381 -> 60 and 204, 46 to 62 and 164 us (90 and 298, 101 and 318 where only whole rows' candidates and a descent over
 // all floats were known); top-k 1000 70 and 344 -> 31 to 45 and 115 to 136.
 __global__ void __launch_bounds__(NT, 2)
