@@ -173,6 +173,13 @@ __device__ __forceinline__ int request_of(const int* __restrict__ cu, int B, int
 
 constexpr int PREP_THREADS = 128, PREP_TOKENS = 16;
 
+// A decay's logarithm as the chunks add it up.  What they use are exponentials of differences of running sums, and past a
+// logarithm of minus infinity a difference is not a number, past one of -1e20 the small ones behind it are lost.  exp(-200) times
+// the largest 32-bit number is still less than half of the smallest one: a decay below it is zero with or without the floor.
+// (Something that is not a number stays so.)
+constexpr float LOG_FLOOR = -200.f;
+__device__ __forceinline__ float floored_log(float la) { return la < LOG_FLOOR ? LOG_FLOOR : la; }
+
 // grid (runs of 16 tokens, runs of channels + 1); the last blockIdx.y makes dt and the decay's logarithm.  A thread walks
 // its V channels over the run's tokens with the TAPS - 1 inputs before them in registers (TAPS = 0: any number of taps).
 template <int V, int TAPS>
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(PREP_THREADS) ssm_prep_kernel(const Params p) 
       const int t = t0 + i / p.H, h = i % p.H;
       const float dt = softplus_f(p.P[(int64_t)t * p.ldp + inner + ch + h] + p.dt_bias[h]);
       p.dt[(int64_t)t * p.H + h] = dt;
-      p.la[(int64_t)t * p.H + h] = -expf(p.A_log[h]) * dt;
+      p.la[(int64_t)t * p.H + h] = floored_log(-expf(p.A_log[h]) * dt);
     }
     return;
   }

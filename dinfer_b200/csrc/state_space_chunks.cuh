@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
         const double sum = cum[i] * 1.4426950408889634;
         const float hi = (float)sum;
         c_hi[warp][s] = hi;
-        c_lo[warp][s] = isinf(hi) ? 0.f : (float)(sum - (double)hi);
+        c_lo[warp][s] = (float)(sum - (double)hi);
         dts[warp][s] = dt4[i];
       }
     }

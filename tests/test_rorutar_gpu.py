@@ -390,6 +390,28 @@ def test_state_space_wide_chunks(H_, G, N, V, lens):
         assert float((state[i].double().cpu().reshape(H_, N, V) - S).abs().max() / S.abs().max()) < 2e-5, i
 
 
+@pytest.mark.parametrize("N, V", [(16, 64), (8, 8)])
+def test_state_space_decays_of_zero(N, V):
+    """Heads whose decay is exactly zero (the logarithm minus infinity, or -1e26 beside -1e-4): a token that follows sees what
+    came behind the last such decay, through the chunks on the tensor cores and through the others; to 2e-5 of the largest as
+    elsewhere."""
+    H_, G, lens = 3, 1, [200, 1, 300]
+    cu = [0, 200, 201, 501]
+    g = torch.Generator().manual_seed(N)
+    proj = torch.randn(cu[-1], 2 * H_ * V + 2 * G * N + H_, generator=g)
+    proj[:, -H_:] = torch.where(torch.rand(cu[-1], H_, generator=g) < 0.2, proj[:, -H_:], torch.tensor(-70.0))
+    A_log, zeros = torch.tensor([100.0, 60.0, 1.0]), torch.zeros
+    conv_b, D = zeros(H_ * V + 2 * G * N), zeros(H_)
+    start = torch.randn(len(lens), H_, N, V, generator=g)
+    state = dev(start.reshape(len(lens), -1).clone())
+    got = run_recurrence(proj, cu, [0, 0, 1], state, A_log, zeros(H_), conv_b, D, H_, G, N, V)
+    for i in range(len(lens)):
+        y, _, S = recurrence(proj[cu[i]:cu[i + 1]], A_log, zeros(H_), conv_b, H_, G, N, V, start[i].double() * (i < 2))
+        for h in range(H_):
+            assert float((got[cu[i]:cu[i + 1], h] - y[:, h]).abs().max() / y[:, h].abs().max().clamp(min=1e-30)) < 2e-5, (i, h)
+            assert float((state[i].double().cpu().reshape(H_, N, V)[h] - S[h]).abs().max() / S[h].abs().max().clamp(min=1e-30)) < 2e-5, (i, h)
+
+
 @pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
 @pytest.mark.parametrize("where", ["x", "B", "C", "dt"])
 def test_state_space_wide_chunks_keep_the_past_clean(where, bad):
