@@ -215,6 +215,13 @@ def gemv_supported(w: torch.Tensor) -> bool:
             and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0)
 
 
+def gemv_norms(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor) -> bool:
+    """Whether ``gemv`` can make its input from these: 16-byte loads of each.  (The norm's own kernel takes any address.)"""
+    return (residual.dtype == torch.float32 and residual.is_contiguous() and residual.data_ptr() % 16 == 0
+            and (delta is None or (delta.dtype == torch.bfloat16 and delta.is_contiguous() and delta.data_ptr() % 16 == 0))
+            and weight.dtype in (torch.bfloat16, torch.float32) and weight.is_contiguous() and weight.data_ptr() % 16 == 0)
+
+
 def gemv(x: Optional[torch.Tensor], w: torch.Tensor, out: torch.Tensor, gated: bool = False, norm=None) -> torch.Tensor:
     """out[1, N] = x[1, K] @ w[N, K]^T for one row in bfloat16; ``gated``: the rows of w are (gate, up) pairs and out [1, N / 2]
     gets silu(gate) * up.  With ``norm = (residual [1, K] f32, delta [1, K] bfloat16 or None, residual_out [1, K] f32 or None,
@@ -233,12 +240,11 @@ def gemv(x: Optional[torch.Tensor], w: torch.Tensor, out: torch.Tensor, gated: b
     else:
         residual, delta, residual_out, weight, eps = norm
         x = None
-        for t, dt in ((residual, torch.float32), (delta, torch.bfloat16), (residual_out, torch.float32)):
-            if t is not None and (t.dtype != dt or tuple(t.shape) != (1, K) or t.stride(1) != 1 or t.data_ptr() % 16):
-                raise KernelError("gemv: residual and residual_out float32 [1, K], delta bfloat16 [1, K], 16-byte aligned")
-        if weight.dtype not in (torch.bfloat16, torch.float32) or weight.numel() != K or not weight.is_contiguous() or weight.data_ptr() % 16 \
-                or (delta is not None and (residual_out is None or residual_out.data_ptr() == residual.data_ptr())):
-            raise KernelError("gemv: the norm's weight [K], and with a delta another buffer for the new residual")
+        if any(t is not None and tuple(t.shape) != (1, K) for t in (residual, delta, residual_out)) or weight.numel() != K \
+                or not gemv_norms(residual, delta, weight) or (residual_out is not None and not gemv_norms(residual_out, None, weight)):
+            raise KernelError("gemv: residual and residual_out float32 [1, K], delta bfloat16 [1, K], the norm's weight [K], 16-byte aligned")
+        if delta is not None and (residual_out is None or residual_out.data_ptr() == residual.data_ptr()):
+            raise KernelError("gemv: with a delta another buffer for the new residual")
     lib, f = _fn("gemv", "dinfer_gemv", [c_void_p, c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                          c_void_p, c_void_p, c_int, c_float, c_void_p])
     check(lib, f(ptr(x), ptr(w), w.stride(0), ptr(out), int(out.dtype == torch.float32), N, K, int(bool(gated)), ptr(residual),

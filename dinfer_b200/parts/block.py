@@ -3,9 +3,10 @@ from __future__ import annotations
 
 from typing import Optional
 
-from .base import BLOCKS, Block, CacheBinding, ResidualStream, StepContext, Unnormed
 import torch
 
+from ..kernels import gemm_ops
+from .base import BLOCKS, Block, CacheBinding, ResidualStream, StepContext, Unnormed
 from .norm import RMSNorm
 
 
@@ -20,12 +21,12 @@ def norm_comes_apart(producer, norm, consumer, rows: int) -> bool:
 
 def normed(stream: ResidualStream, norm, delta, consumer):
     """The input of ``consumer`` (None: of whoever) behind ``norm`` of the stream plus ``delta``: the rows, or what ``consumer``
-    makes them of."""
+    makes them of where it can read that as it lies (a part may return a slice)."""
     takes = getattr(consumer, "makes_norm", None)
     x = stream.x
     if takes is not None and x.shape[0] == 1 and takes(1) and isinstance(norm, RMSNorm) and norm.weight is not None \
-            and (delta is None or (isinstance(delta, torch.Tensor) and delta.dtype == torch.bfloat16)) \
-            and x.dtype == torch.float32 and stream.results is None:
+            and (delta is None or isinstance(delta, torch.Tensor)) and gemm_ops.gemv_norms(x, delta, norm.weight) \
+            and stream.results is None:
         return Unnormed(stream, delta, norm)
     return norm.forward(x, delta=delta)
 
