@@ -96,6 +96,17 @@ template <typename TA> __host__ __device__ constexpr uint32_t stage_bytes(int bt
 template <typename TA, typename TW> __host__ __device__ constexpr uint32_t raw_bytes(int bt) {
   return BN * raw_row<TW>() + (uint32_t)bt * raw_row<TA>();
 }
+// Dynamic shared memory of a launch.  Where CTAs share K they wait for one another, and all of tensor memory is one CTA's: two of them on
+// one SM, each ahead of the other's partner on another SM, would wait for good.  So such a CTA takes an SM's shared memory for
+// itself (more than half of it), however small its tile is; the others only wait for a CTA in front to end.
+constexpr size_t ALONE = 115 * 1024;
+template <typename TA, typename TW> __host__ constexpr size_t tile_shared(int bt, int splits) {
+  const size_t stages = (size_t)STAGES * stage_bytes<TA>(bt) + RAW_STAGES * raw_bytes<TA, TW>(bt), part = (size_t)bt * LDC_S * 4;
+  const size_t own = (stages > part ? stages : part) + 1024;
+  return splits > 1 && own < ALONE ? ALONE : own;
+}
+static_assert(2 * ALONE > 228 * 1024 && ALONE <= MAX_SMEM, "one CTA to an SM");
+static_assert(tile_shared<float, float>(BT, 1) <= MAX_SMEM, "fits a CTA");
 
 // The tile kernel: 128 weight rows (the MMA's rows) by up to 112 tokens (its columns, as many as the rows make even tiles of),
 // 32 k a stage.  FAST: TMA fetches both operands as they lie in memory (16-byte rows), else the splitting warps read them
@@ -450,7 +461,7 @@ int clusters_resident(int size) {
   int n = known[size].load(std::memory_order_relaxed);
   if (n) return n;
   auto k = gemm_tile_kernel<float, float, float, true>;
-  const size_t smem = STAGES * stage_bytes<float>(BT) + RAW_STAGES * raw_bytes<float, float>(BT) + 1024;
+  const size_t smem = tile_shared<float, float>(BT, size);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(size * num_sms()); cfg.blockDim = dim3(TILE_THREADS); cfg.dynamicSmemBytes = smem;
   cudaLaunchAttribute attr;
@@ -540,8 +551,7 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
                        make_map<TA>(&ma, A, M, K, lda, batch, sa, bt) && make_map<TW>(&mw, W, N, K, ldw, batch, sw, BN);
     const TileParams p{lda, ldw, ldc, sa, sw, sc, M, N, K, bt, splits, fast(C, sizeof(TC), ldc, sc, 4), status};
     auto k = whole ? gemm_tile_kernel<TA, TW, TC, true> : gemm_tile_kernel<TA, TW, TC, false>;
-    const size_t stages = (size_t)STAGES * stage_bytes<TA>(bt) + RAW_STAGES * raw_bytes<TA, TW>(bt), part = (size_t)bt * LDC_S * 4;
-    const size_t smem = (stages > part ? stages : part) + 1024;
+    const size_t smem = tile_shared<TA, TW>(bt, splits);
     static std::atomic<uint64_t> done[2];
     cudaError_t e = allow_shared(k, MAX_SMEM, done[whole]);
     if (e != cudaSuccess) return refuse((int)e, "gemm_f32: shared memory opt-in failed: %s", cudaGetErrorString(e));
@@ -555,6 +565,15 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
 }  // namespace
 
 DINFER_DEFINE_LAST_ERROR()
+
+// Dynamic shared memory (bytes) of a launch of tiles of bt tokens whose K `splits` CTAs share, -1: no such launch.
+DINFER_API int64_t dinfer_gemm_f32_shared(int a_dtype, int w_dtype, int bt, int splits) {
+  if (bt <= 0 || bt > BT || bt % 16 || splits < 1 || splits > MAX_SPLITS) return -1;
+  DINFER_DISPATCH_DTYPE(a_dtype, TA,
+    DINFER_DISPATCH_DTYPE(w_dtype, TW,
+      return (int64_t)tile_shared<TA, TW>(bt, splits)));
+  return -1;
+}
 
 // A [M, K] row stride lda; W [N, K] row stride ldw; C [M, N] row stride ldc (strides in elements).
 DINFER_API int dinfer_gemm_f32(const void* A, int64_t lda, int a_dtype, const void* W, int64_t ldw,
