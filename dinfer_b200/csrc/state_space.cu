@@ -59,6 +59,13 @@ template <int V> struct alignas(4 * V) Vec { float x[V]; };
 template <int V> __device__ __forceinline__ Vec<V> ldv(const float* p) { return *reinterpret_cast<const Vec<V>*>(p); }
 template <int V> __device__ __forceinline__ void stv(float* p, const Vec<V>& v) { *reinterpret_cast<Vec<V>*>(p) = v; }
 
+// A CTA that has nothing to do leaves ahead of the wait for the kernels in front, but the launch's first one waits: a launch that had
+// nothing to do at all would be over before them, and the kernel behind it, which waits for this launch alone, would start
+// on what they have not written yet.
+__device__ __forceinline__ void leave(bool first) {
+  if (first) pdl_wait();
+}
+
 // ---------------------------------------------------------------- one token
 // L lanes share a row of S, V neighbouring columns each; 256 / L rows at a time.  RPT > 0: a thread's rows (at most RPT)
 // stay in registers from the loads ahead of the wait on; RPT = 0: rows as they come.
@@ -73,7 +80,7 @@ __global__ void __launch_bounds__(THREADS, RPT == 16 ? 2 : (RPT == 8 ? 3 : 4)) s
   pdl_launch_dependents();
   const int b = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * PT;
   const int t = p.cu[b];
-  if (p.cu[b + 1] - t != 1) return;                // portions are the chunk kernels'
+  if (p.cu[b + 1] - t != 1) return leave(blockIdx.x == 0 && blockIdx.y == 0 && b == 0);   // portions are the chunk kernels'
   const int tid = threadIdx.x, col = (tid % L) * V, r0 = tid / L;
   const bool is_fresh = p.fresh[b] != 0;
   float* row_state = p.state + (int64_t)p.slots[b] * p.ld_state;

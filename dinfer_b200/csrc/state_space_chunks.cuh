@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_sums_umma_kernel(const Pa
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int c = 0;
   const int b = place_of(p.cu, p.B, blockIdx.x, c);
-  if (b < 0) return;
+  if (b < 0) return leave(blockIdx.x == 0 && blockIdx.y == 0);
   const int t_begin = p.cu[b], t_end = p.cu[b + 1], t0 = t_begin + c * CU;
   const uint32_t base = (smem_u32(umma_sm) + 1023u) & ~1023u;
   if (tid == 0) {
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int c = 0;
   const int b = place_of(p.cu, p.B, blockIdx.x, c);
-  if (b < 0) return;
+  if (b < 0) return leave(blockIdx.x == 0 && blockIdx.y == 0);
   const int t_begin = p.cu[b], t_end = p.cu[b + 1], t0 = t_begin + c * CU;
   const uint32_t base = (smem_u32(umma_sm) + 1023u) & ~1023u;
   if (tid == 0) {

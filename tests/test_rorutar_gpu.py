@@ -390,6 +390,33 @@ def test_state_space_wide_chunks(H_, G, N, V, lens):
         assert float((state[i].double().cpu().reshape(H_, N, V) - S).abs().max() / S.abs().max()) < 2e-5, i
 
 
+@pytest.mark.parametrize("lens", [[1] * 48, [300, 200]])
+@pytest.mark.parametrize("V", [64, 40])
+def test_state_space_launches_with_nothing_to_do(lens, V):
+    """A step said to hold both single tokens and portions that holds one kind only: the launches for the other kind keep the order of
+    those around them, so that results and states are those of the step as it is, bit by bit."""
+    from dinfer_b200.kernels import state_ops
+    H_, G, N, taps = 16, 2, 64, 3
+    inner, ch, B = H_ * V, H_ * V + 2 * G * N, len(lens)
+    cu = i32([sum(lens[:i]) for i in range(B + 1)])
+    g = torch.Generator().manual_seed(V)
+    proj = dev(torch.randn(sum(lens), inner + ch + H_, generator=g))
+    conv, vec, w = dev(torch.randn(ch, taps, generator=g)), dev(torch.randn(ch, generator=g)), dev(torch.ones(inner))
+    heads = dev(torch.linspace(-1.0, 1.0, H_))
+    start = dev(torch.randn(B, (H_ * N * V + (taps - 1) * ch + 3) // 4 * 4, generator=g))
+    results = []
+    for single, portion in ((1 in lens, max(lens) > 1), (True, True), (True, True)):
+        state, out = start.clone(), torch.full((sum(lens), inner), float("nan"), device="cuda")
+        args = (cu, i32(list(range(B))), i32([0] * B))
+        y = state_ops.state_space(proj, conv, vec, heads, heads, heads, state, *args, H_, G, N, V, taps, any_single=single, any_portion=portion,
+                                  max_q_len=max(lens))
+        state_ops.state_space_post(y, proj, w, 1e-5, G, out, state, *args, H_, G, N, V, taps)
+        results.append((out.cpu(), state.cpu()))
+    for out, state in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(state, results[0][1])
+    assert bool(torch.isfinite(results[0][0]).all())
+
+
 @pytest.mark.parametrize("N, V", [(16, 64), (8, 8)])
 def test_state_space_decays_of_zero(N, V):
     """Heads whose decay is exactly zero (the logarithm minus infinity, or -1e26 beside -1e-4): a token that follows sees what
