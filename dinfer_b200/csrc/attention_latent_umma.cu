@@ -587,6 +587,16 @@ DINFER_API int dinfer_attention_latent_umma_supports(int R, int P, int D, int V)
   return (D == 64 || D == 128) && V == D && P >= 0 && P <= 64 && P % 8 == 0 && R > 0 && R % 8 == 0;
 }
 
+// Whether a launch takes two CTAs to a pair: where those of all pairs run at once, or where the longest pair's walk is what a single
+// round of CTAs waits for (a cluster waits for two SMs, and a shared pair takes some 4 us more).  us alone and shared, 128 wide: 8
+// heads, 2048 tokens 50 and 32; 16 heads, 1024 29 and 21; 16, 512 behind 4000 103 and 59; 32, 256 behind 8000 206 and 113; in a
+// round of 128 pairs: 16, 2048 51 and 45; 16, 2048 behind 4000 146 and 132; but 32, 1024 30 and 39; 16, 500 + 700 + 900 29 and 37.
+DINFER_API int dinfer_attention_latent_umma_shares(int H, int pair_bound, int window, int max_keys) {
+  const int64_t n = (int64_t)H * pair_bound;
+  const int longest = ((window > 0 && max_keys > window + 2 * BM ? window + 2 * BM : max_keys) + BN - 1) / BN;
+  return longest >= MIN_SHARED && (2 * n <= num_sms() || (n <= num_sms() && longest >= LONG_WALK));
+}
+
 // Portions (more than one token) only.  q [T, H, D + P] rows of stride ldq (turned), out [T, H, D] rows of stride ldo;
 // latents [rows, R + P] as dinfer_latent_rows leaves them, expanded [rows, H, 2 D] with a head's key, then its value.
 // pair_bound >= the sum over the portions of ceil(tokens / 256); max_keys: about the keys of the longest request (0: not known).  sinks [H] f32 or null.  window <= 0: all keys.
@@ -612,13 +622,7 @@ DINFER_API int dinfer_attention_latent_umma(const void* q, int64_t ldq, void* ou
   Params p{};
   p.out = (__nv_bfloat16*)out; p.ldo = ldo; p.cu_seqlens = cu_seqlens; p.seq_lens = seq_lens; p.B = B; p.window = window; p.rows = rows;
   p.scale_log2 = scale * 1.4426950408889634f; p.sinks = sinks; p.status = status;
-  // Two CTAs to a pair where those of all pairs run at once, or where the longest pair's walk is what a single round of CTAs waits
-  // for (a cluster waits for two SMs, and a shared pair takes some 4 us more).  us alone and shared, 128 wide: 8 heads, 2048 tokens
-  // 50 and 32; 16 heads, 1024 29 and 21; 16, 512 behind 4000 103 and 59; 32, 256 behind 8000 206 and 113; in a round of 128
-  // pairs: 16, 2048 51 and 45; 16, 2048 behind 4000 146 and 132; but 32, 1024 30 and 39; 16, 500 + 700 + 900 29 and 37.
-  const int64_t n = (int64_t)H * pair_bound;
-  const int longest = ((window > 0 && max_keys > window + 2 * BM ? window + 2 * BM : max_keys) + BN - 1) / BN;
-  const bool split = longest >= MIN_SHARED && (2 * n <= num_sms() || (n <= num_sms() && longest >= LONG_WALK));
+  const bool split = dinfer_attention_latent_umma_shares(H, pair_bound, window, max_keys);
   if (D == 64) return split ? launch<64, true>(mq, mkv, mr, p, H, pair_bound, stream) : launch<64, false>(mq, mkv, mr, p, H, pair_bound, stream);
   return split ? launch<128, true>(mq, mkv, mr, p, H, pair_bound, stream) : launch<128, false>(mq, mkv, mr, p, H, pair_bound, stream);
 }

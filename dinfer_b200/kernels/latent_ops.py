@@ -242,6 +242,12 @@ def latent_q_turn(q: torch.Tensor, positions: torch.Tensor, cos_sin: Optional[to
     return q
 
 
+def shares_keys(num_heads: int, pair_bound: int, window: int, max_keys: int) -> bool:
+    """Whether ``attention_latent_umma`` takes two CTAs to a row-tile pair (``pair_bound`` and ``max_keys`` as there)."""
+    _, f = _fn("latent_expanded", "dinfer_attention_latent_umma_shares", [c_int] * 4)
+    return bool(f(int(num_heads), int(pair_bound), int(window), int(max_keys)))
+
+
 def attention_latent_umma(q: torch.Tensor, out: torch.Tensor, latents: torch.Tensor, expanded: torch.Tensor,
                           cu_seqlens: torch.Tensor, seq_lens: torch.Tensor, kv_rank: int, rope_dim: int, head_dim: int,
                           scale: float, window: int = 0, sinks: Optional[torch.Tensor] = None,

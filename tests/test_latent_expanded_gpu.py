@@ -84,14 +84,17 @@ def test_rows_and_attention_against_plain(case):
     assert bool((lat[at:] == 0).all())
 
 
-@pytest.mark.parametrize("D,P,H,window,with_sinks,reqs", [
-    (128, 64, 3, 0, True, [(0, 640)]), (128, 64, 2, 0, False, [(0, 641), (0, 1), (500, 129), (0, 30)]),
-    (64, 32, 4, 0, True, [(5000, 257)]), (128, 64, 1, 900, False, [(2000, 300), (10, 700)]), (128, 16, 16, 0, False, [(0, 1100)]),
-    (64, 64, 1, 0, False, [(639, 2), (640, 128), (767, 2)])])
-def test_two_ctas_to_a_pair(D, P, H, window, with_sinks, reqs):
+@pytest.mark.parametrize("D,P,H,window,with_sinks,reqs,shared", [
+    (128, 64, 3, 0, True, [(0, 640)], False), (128, 64, 2, 0, False, [(0, 641), (0, 1), (500, 129), (0, 30)], True),
+    (64, 32, 4, 0, True, [(5000, 257)], True), (128, 64, 1, 900, False, [(2000, 300), (10, 700)], True),
+    (128, 16, 16, 0, False, [(0, 1100)], False), (64, 64, 1, 0, False, [(639, 2), (640, 128), (767, 2)], True),
+    (128, 64, 3, 0, True, [(0, 700)], True), (128, 16, 8, 0, False, [(0, 1100)], True),
+    (128, 64, 16, 0, False, [(0, 2048)], True), (128, 32, 12, 0, True, [(1500, 2100), (0, 3)], True)])
+def test_two_ctas_to_a_pair(D, P, H, window, with_sinks, reqs, shared):
     """Row-tile pairs whose keys two CTAs share, beside pairs too short for it, pairs with one row tile, one row of one, an odd number of
-    key tiles, histories and windows: the same as without (which the test above holds to the formula), up to the other
-    order of sums and the other maximum that weights are rounded against."""
+    key tiles, histories and windows, launches whose CTAs all run at once and launches of more (and two batches whose keys are
+    not shared): the same as without (which the test above holds to the formula), up to the other order of sums and the other
+    maximum that weights are rounded against."""
     from dinfer_b200.kernels import gemm_ops, latent_ops as L
     g = torch.Generator().manual_seed(D + H)
     cu, seq, table, pages = batch(reqs, 16, 1)
@@ -105,6 +108,7 @@ def test_two_ctas_to_a_pair(D, P, H, window, with_sinks, reqs):
     lat = L.latent_rows(cache, c(table), c(cu), c(seq), L.expanded_rows(portions, window), window)
     kv = lat[:, :R] @ w.T
     pairs = sum((n + 255) // 256 for n, _ in portions)
+    assert not L.shares_keys(H, pairs, window, 0) and L.shares_keys(H, pairs, window, int(seq.max())) is shared
     got = []
     for longest in (0, int(seq.max())):
         out = torch.full((T, H, D), float("nan"), dtype=torch.bfloat16, device="cuda")
