@@ -26,6 +26,8 @@
 //
 // A request whose `fresh` flag is set starts from zeros whatever its slot holds.  What a token gets depends on how a
 // request is cut into steps through the order of sums only.
+#include <type_traits>
+
 #include "split_umma.cuh"
 
 using namespace dinfer;
@@ -327,7 +329,8 @@ __device__ __forceinline__ void chunk_log_decay(const float* la, int64_t ld, int
     const double v = __shfl_up_sync(0xffffffffu, s, d);
     if (lane >= d) s += v;
   }
-  cum[2 * lane] = s - a1;
+  const double before = __shfl_up_sync(0xffffffffu, s, 1);
+  cum[2 * lane] = lane > 0 ? before + a0 : a0;      // (not s - a1, which is not a number where the later token's is none)
   cum[2 * lane + 1] = s;
 }
 
@@ -616,8 +619,7 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
     for (int j = 0; j < 4; ++j) r[i][j] *= d;
   }
   __syncthreads();
-  const int last = min(ty * 4 + 3, n - 1);         // (A is zero beyond t, x_s beyond the chunk's tokens)
-  for (int s = 0; s <= last; s += 4) {
+  const auto add = [&](int s, auto diagonal) {
     float4 q[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) q[i] = get4(&A_s[ty * 4 + i][s]);
@@ -626,12 +628,16 @@ __global__ void __launch_bounds__(THREADS, 3) ssm_outputs_kernel(const Params p)
       const float4 x4 = get4(&x_s[s + u][tx * 4]);
       const float xw[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = decltype(diagonal)::value ? u : 0; i < 4; ++i) {
         const float qv = u == 0 ? q[i].x : u == 1 ? q[i].y : u == 2 ? q[i].z : q[i].w;
 #pragma unroll
         for (int j = 0; j < 4; ++j) r[i][j] = fmaf(qv, xw[j], r[i][j]);
       }
     }
+  };
+  if (ty * 4 < n) {                                // (x_s is zero beyond the chunk's tokens)
+    for (int s = 0; s < ty * 4; s += 4) add(s, std::false_type());
+    add(ty * 4, std::true_type());                 // a zero of A times an infinite x of a later token would not be zero
   }
   const float D = p.D[h];
 #pragma unroll
@@ -797,6 +803,20 @@ int num_sms() {                                             // of the current de
 // chunks on the tensor cores: whole column tiles and 16-byte rows, a state that fits an MMA's rows
 bool umma_takes(int N, int P) { return P % VT == 0 && N % 16 == 0 && N <= CU; }
 
+// Whether they are the faster ones for q portions of t tokens together.  Their CTAs take 9000 cycles a head and chunk of 128 however
+// few tokens it has; a block of the others takes a chunk of 64, and less the fewer there are.  So they gain where portions fill more
+// than half of a chunk (one of 64 would not do), and with them the longer a walk there is to shorten.  us on chunks of 64 and of 128,
+// heads x state channels in front:
+//   64 x 128: 1 portion of 2 tokens 31 and 26, 4 of 64 59 and 56, 8 of 80 126 and 82, 2000 tokens 337 and 189; but 64 of 2
+//             434 and 480, 64 of 32 504 and 504 (16 of 2 in between: 123 and 123; 32 x 128 the same from half as many heads on)
+//   16 x 64:  64 tokens 24.7 and 24.8, 128 25.9 and 29.0, 256 28.4 and 27.8, 2000 63.6 and 49.0; 16 of 8 36 and 44, 16 of 80 54 and
+//             47; 8 x 64: 256 25.1 and 27.1, 512 31.2 and 27.8
+//   24 x 16:  256 tokens 25 and 22, 2 of 384 34 and 38, 2 of 512 37 and 39
+bool umma_gains(int64_t q, int64_t t, int N, int64_t tiles) {
+  if (N > 64) return t > 32 * q || q * tiles <= 2048;
+  return t > 64 * q && t * tiles * N * N >= (1 << 24);
+}
+
 bool al16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
 
 }  // namespace
@@ -812,6 +832,11 @@ DINFER_API int64_t dinfer_state_space_work_floats(int64_t T, int B, int H, int G
   return r4(T * channels) + 2 * r4(T * H) + slots * H * (int64_t)N * P + r4(slots * H) + scores * G + 4;
 }
 
+// Whether portion_requests portions of portion_tokens tokens together go through chunks of 128 on the tensor cores.
+DINFER_API int dinfer_state_space_wide(int64_t portion_requests, int64_t portion_tokens, int H, int N, int P) {
+  return umma_takes(N, P) && umma_gains(portion_requests, portion_tokens, N, (int64_t)H * (P / VT));
+}
+
 // The recurrence of a step.  proj: f32 rows [z | x | B | C | dt] of stride ldp; conv_w [channels, taps], conv_b [channels],
 // dt_bias, A_log, D [H] f32; state: f32 rows of stride ld_state, S [H, N, P] first, the convolution's (taps - 1) inputs
 // [taps - 1, channels] from `hist` on (only read here: dinfer_state_space_post moves them on); cu [B + 1], slots, fresh [B];
@@ -820,8 +845,10 @@ DINFER_API int64_t dinfer_state_space_work_floats(int64_t T, int B, int H, int G
 DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* conv_w, const float* conv_b,
                                   const float* dt_bias, const float* A_log, const float* D, float* state, int64_t ld_state,
                                   int hist, const int* cu, const int* slots, const int* fresh, float* y, float* work, int T,
-                                  int B, int H, int G, int N, int P, int taps, int single, int portions, int max_q_len,
-                                  int* status, cudaStream_t stream) {
+                                  int B, int H, int G, int N, int P, int taps, int single, int portions, int portion_requests,
+                                  int max_q_len, int chunks_of, int* status, cudaStream_t stream) {
+  if (chunks_of != 0 && chunks_of != CP && (chunks_of != CU || !umma_takes(N, P) || !status || !al16(y)))
+    return refuse(DINFER_BAD_ARGUMENT, "state_space: no chunks of %d tokens here", chunks_of);
   if (T < 0 || B <= 0 || H <= 0 || G <= 0 || H % G || N <= 0 || P <= 0 || taps <= 0 || B > 65535)
     return refuse(DINFER_BAD_ARGUMENT, "state_space: bad sizes T=%d B=%d H=%d G=%d N=%d P=%d taps=%d", T, B, H, G, N, P, taps);
   Params p{};
@@ -847,7 +874,10 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
     if (!work || !al16(work) || max_q_len <= 0) return refuse(DINFER_BAD_ARGUMENT, "state_space: portions need work space and their longest");
     // 16-byte loads of the convolved rows, of the states and of y: every width and base allows them
     const bool vec = P % 4 == 0 && N % 4 == 0 && al16(y);
-    const bool wide = vec && umma_takes(N, P) && status != nullptr;
+    const int q = portion_requests > 0 && portion_requests < B ? portion_requests : B;
+    const int64_t t = single ? T - (B - q) : T;       // (about)
+    const bool wide = chunks_of ? chunks_of == CU
+                                : vec && umma_takes(N, P) && status != nullptr && umma_gains(q, t, N, (int64_t)H * (P / VT));
     const int tokens = wide ? CU : CP, chunks = (max_q_len + tokens - 1) / tokens;
     const int64_t chunk_slots = (int64_t)T / tokens + B;
     auto r4 = [](int64_t n) { return (n + 3) / 4 * 4; };
@@ -861,14 +891,14 @@ DINFER_API int dinfer_state_space(const float* proj, int64_t ldp, const float* c
     if (ch % 4 == 0 && ldp % 4 == 0 && inner % 4 == 0 && al16(proj)) launch_prep<4>(p, stream);
     else launch_prep<1>(p, stream);
     if (wide) {
-      // 2047 tokens of 64 heads of 128 x 64: sums 75 -> 22 us, walk 30 -> 17, outputs 109 -> 45 (the mixer 434 -> 350); 1024 tokens
-      // of 32 heads 113 -> 96.  Portions of 64 tokens and less take as long as they did.
-      const int per_group = H / G * (P / VT), units = units_of(T / CU + 1, G, per_group, num_sms()), runs = (per_group + units - 1) / units;
+      // (units by the portions' chunks if they are all as long: 16 portions of 4 tokens taken for one chunk were 205 us instead of 157)
+      const int per_group = H / G * (P / VT), each = (int)((t + q - 1) / q);
+      const int units = units_of(q * ((each + CU - 1) / CU), G, per_group, num_sms()), runs = (per_group + units - 1) / units;
       static std::atomic<uint64_t> sums_done, outputs_done;
       cudaError_t e = dinfer_split::allow_shared(ssm_sums_umma_kernel, SUMS_SMEM, sums_done);
       if (e == cudaSuccess) e = dinfer_split::allow_shared(ssm_outputs_umma_kernel, OUTPUTS_SMEM, outputs_done);
       if (e != cudaSuccess) return refuse((int)e, "state_space: shared memory opt-in failed: %s", cudaGetErrorString(e));
-      const unsigned places = (unsigned)(T / CU + B < (int64_t)chunks * B ? T / CU + B : chunks * B);
+      const unsigned places = (unsigned)(T / CU + q < (int64_t)chunks * q ? T / CU + q : chunks * q);
       launch_pdl(ssm_sums_umma_kernel, dim3(places, G * runs + G), dim3(UMMA_THREADS), SUMS_SMEM, stream, p, units, status);
       if (state_vec) launch_scan<4>(p, size, true, stream); else launch_scan<1>(p, size, true, stream);
       launch_pdl(ssm_outputs_umma_kernel, dim3(places, G * runs), dim3(UMMA_THREADS), OUTPUTS_SMEM, stream, p, units, status);

@@ -28,12 +28,12 @@ static_assert(A_ALL + SUM_PARTS * VT <= TMEM_ALL && 2 * A_ALL + 2 * VT <= TMEM_A
 constexpr size_t SUMS_SMEM = 2 * TILE_BYTES + 1024 + 16 * 32 * 20 * 4;   // (more than half of an SM's: the tensor memory is one CTA's)
 static_assert(SUMS_SMEM > 114 * 1024, "one CTA to an SM");
 constexpr size_t OUTPUTS_SMEM = 4 * TILE_BYTES + 1024;
-constexpr int STATUS_SUMS = 51, STATUS_OUTPUTS = 52;
+constexpr int STATUS_SUMS = 51, STATUS_OUTPUTS = 52, STATUS_PLACES = 53;
 
 __device__ __forceinline__ int64_t wide_slot(int t_begin, int b, int c) { return (int64_t)(t_begin / CU + b + c); }
 
 // Chunk number `place` of the step's portions (requests with more than one token): its request (-1: there is none) and its number
-// in it, by a whole warp.  The launches have no grid dimension for requests: beside 60 single tokens a portion's CTAs would be one in 61, and
+// in it, by a whole warp.  The launches have no grid dimension for requests, and places for the portions alone: beside 60 single tokens a portion's CTAs would be one in 61, and
 // even one that has nothing to do needs an SM's shared memory to itself (700 tokens beside 60: 95 us became 113).
 __device__ __forceinline__ int place_of(const int* __restrict__ cu, int B, int place, int& chunk) {
   const int lane = threadIdx.x & 31;
@@ -235,6 +235,10 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_sums_umma_kernel(const Pa
   __syncthreads();
   tc_fence_after();
   pdl_enter();                                     // (dependents start only now that the tensor memory is ours)
+  if (blockIdx.y == 0 && blockIdx.x == gridDim.x - 1 && warp == MMA_WARP) {     // a chunk that no CTA takes would go unnoticed
+    int beyond;
+    if (place_of(p.cu, p.B, gridDim.x, beyond) >= 0 && lane == 0) atomicExch(status, STATUS_PLACES);
+  }
   const uint32_t tmem = s_tmem, lead = dinfer_split::elect_lane(), tm = dinfer_split::uniform(tmem), lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
   const int row = (warp & 3) * 32 + lane, sub = warp >> 2;
   const int n = min(CU, t_end - t0), ch = p.channels(), inner = p.inner(), heads = p.H / p.G;

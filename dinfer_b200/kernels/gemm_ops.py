@@ -66,6 +66,7 @@ STATUS_MEANING = {
     47: "routed products: a warp waited for the experts' weights",
     51: "state-space chunks: the sums waited for their operands or their MMAs",
     52: "state-space chunks: the outputs waited for their operands or their MMAs",
+    53: "state-space chunks: the step has more portions than its launch was made for",
 }
 
 
@@ -78,7 +79,7 @@ def check_status(device=None) -> None:
     until ``reset_status``: after such a fault the step's results are not to be trusted."""
     code = device_status(device)
     if code:
-        what = "met a step beyond its launch's bounds" if code == 37 else "gave up a bounded wait and returned early"
+        what = "met a step beyond its launch's bounds" if code in (37, 53) else "gave up a bounded wait and returned early"
         raise KernelError(f"a kernel {what} (status {code}: "
                           f"{describe_status(code)}); the results of that step are invalid")
 

@@ -131,13 +131,15 @@ def _state_space_sizes(P, conv_w, state, cu_seqlens, slots, fresh, H, G, N, dv, 
 def state_space(P: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_bias: torch.Tensor, A_log: torch.Tensor,
                 D: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, fresh: torch.Tensor,
                 num_heads: int, groups: int, state_dim: int, value_dim: int, taps: int, any_single: bool = True,
-                any_portion: bool = True, max_q_len: int = 0) -> torch.Tensor:
+                any_portion: bool = True, max_q_len: int = 0, portion_requests: int = 0, chunks_of: int = 0) -> torch.Tensor:
     """``P`` float32 rows [z | x | B | C | dt] (a view with a row stride is fine): convolution with bias and silu of x, B, C,
     ``dt = softplus(dt + dt_bias)``, ``S <- exp(-exp(A_log) dt) S + dt B x^T``, ``y = S^T C + D x`` per request and head, S
     [N, P] carried in the first ``H N P`` floats of row ``slots[b]`` of ``state`` (zero for a fresh request); the
     convolution's earlier inputs are read from behind them and moved on by ``state_space_post``.  Requests that bring one
     token go through one kernel, the others' chunks of 64 or 128 tokens side by side through four; ``any_single`` /
-    ``any_portion`` say which there are, ``max_q_len`` (0: not known) bounds the longest portion.  Returns y f32 [T, H * P]."""
+    ``any_portion`` say which there are, ``max_q_len`` (0: not known) bounds the longest portion, ``portion_requests`` (0: not
+    known) the requests that do not bring one token (more of them than that leave a device status); ``chunks_of`` 64 or 128 takes
+    those chunks whatever is faster.  Returns y f32 [T, H * P]."""
     require_cuda(P, conv_w, conv_b, dt_bias, A_log, D, state, cu_seqlens, slots, fresh)
     H, G, N, dv = num_heads, groups, state_dim, value_dim
     channels, hist = _state_space_sizes(P, conv_w, state, cu_seqlens, slots, fresh, H, G, N, dv, taps)
@@ -150,7 +152,7 @@ def state_space(P: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_
     lib, f = _fn("state_space", "dinfer_state_space",
                  [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p,
                   c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                  c_int, c_void_p])
+                  c_int, c_int, c_int, c_void_p, c_void_p])
     work = None
     if any_portion:
         size = lib.dinfer_state_space_work_floats
@@ -159,8 +161,8 @@ def state_space(P: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, dt_
         work = torch.empty(size(T, B, H, G, N, dv), dtype=torch.float32, device=P.device)
     check(lib, f(ptr(P), P.stride(0), ptr(conv_w), ptr(conv_b), ptr(dt_bias), ptr(A_log), ptr(D), ptr(state),
                  state.stride(0), hist, ptr(cu_seqlens), ptr(slots), ptr(fresh), ptr(y), ptr(work), T, B, H, G, N, dv, taps,
-                 int(bool(any_single)), int(bool(any_portion)), int(max_q_len) if max_q_len > 0 else T,
-                 _status(P.device), stream_handle()), "state_space")
+                 int(bool(any_single)), int(bool(any_portion)), int(portion_requests), int(max_q_len) if max_q_len > 0 else T,
+                 int(chunks_of), _status(P.device), stream_handle()), "state_space")
     add_launches((1 if any_single else 0) + (4 if any_portion else 0) - 1)
     return y
 

@@ -95,9 +95,15 @@ class StateSpace(Mixer):
         B = ctx.cu_seqlens.numel() - 1
         slots, fresh = ctx.state_slots[:B], ctx.state_fresh[:B]
         sizes = (self.H, self.G, self.N, self.P, self.taps)
+        portions = 0
+        if ctx.any_prefill and ctx.cu_seqlens_host:          # (a captured graph's places, which a replay may leave empty)
+            if "portion_requests" not in ctx.derived:
+                cu = ctx.cu_seqlens_host
+                ctx.derived["portion_requests"] = sum(b - a != 1 for a, b in zip(cu, cu[1:]))
+            portions = ctx.derived["portion_requests"]
         y = state_ops.state_space(P, self.conv_w, self.conv_b, self.dt_bias, self.A_log, self.D, cache.state, ctx.cu_seqlens,
                                   slots, fresh, *sizes, any_single=ctx.any_decode, any_portion=ctx.any_prefill,
-                                  max_q_len=ctx.max_q_len)
+                                  max_q_len=ctx.max_q_len, portion_requests=portions)
         state_ops.state_space_post(y, P, self.norm_w, self.eps, self.parts, out, cache.state, ctx.cu_seqlens, slots, fresh, *sizes)
 
     def forward(self, x, ctx: StepContext, cache: CacheBinding):

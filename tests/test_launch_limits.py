@@ -20,3 +20,14 @@ def test_ctas_that_wait_for_one_another_have_an_sm_each(a, w):
         for splits in range(2, 9):
             assert SM_SHARED < 2 * f(a, w, bt, splits) and f(a, w, bt, splits) <= CTA_SHARED
     assert f(a, w, 128, 1) == f(a, w, 24, 1) == f(a, w, 16, 9) == -1
+
+
+@pytest.mark.parametrize("portions, tokens, heads, state, vdim, wide", [
+    (1, 2, 64, 128, 64, True), (32, 64, 64, 128, 64, True), (33, 66, 64, 128, 64, False), (64, 64 * 32, 64, 128, 64, False),
+    (64, 64 * 33, 64, 128, 64, True), (16, 64, 16, 64, 64, False), (16, 16 * 64, 16, 64, 64, False), (16, 16 * 65, 16, 64, 64, True),
+    (1, 255, 16, 64, 64, False), (1, 256, 16, 64, 64, True), (1, 511, 8, 64, 64, False), (1, 512, 8, 64, 64, True),
+    (1, 2000, 24, 16, 64, False), (1, 2731, 24, 16, 64, True), (1, 2000, 16, 128, 60, False), (1, 2000, 16, 72, 64, False), (1, 2000, 16, 144, 64, False)])
+def test_which_portions_take_chunks_of_128(portions, tokens, heads, state, vdim, wide):
+    f = library("state_space").dinfer_state_space_wide
+    f.restype, f.argtypes = c_int, [c_int64, c_int64, c_int, c_int, c_int]
+    assert bool(f(portions, tokens, heads, state, vdim)) is wide

@@ -356,19 +356,21 @@ def recurrence(proj, A_log, dt_bias, conv_b, H_, G, N, V, S):
     return torch.stack(ys), x, S
 
 
-def run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V):
+def run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V, chunks_of=0):
     from dinfer_b200.kernels import gemm_ops, state_ops
     ch, B = H_ * V + 2 * G * N, len(cu) - 1
     lens = [cu[i + 1] - cu[i] for i in range(B)]
     y = state_ops.state_space(dev(proj), torch.ones(ch, 1, device="cuda"), dev(conv_b), dev(dt_bias), dev(A_log), dev(D), state, i32(cu),
-                              i32(list(range(B))), i32(fresh), H_, G, N, V, 1, any_single=1 in lens, any_portion=max(lens) > 1, max_q_len=max(lens))
+                              i32(list(range(B))), i32(fresh), H_, G, N, V, 1, any_single=1 in lens, any_portion=max(lens) > 1, max_q_len=max(lens),
+                              portion_requests=sum(n > 1 for n in lens), chunks_of=chunks_of)
     assert gemm_ops.device_status(y.device) == 0
     return y.double().cpu().reshape(-1, H_, V)
 
 
 @pytest.mark.parametrize("H_, G, N, V", [(4, 2, 16, 64), (2, 1, 128, 128), (6, 2, 48, 64), (16, 1, 64, 64), (9, 1, 112, 64), (3, 3, 80, 192)])
 @pytest.mark.parametrize("lens", [[2, 1, 15, 16, 17], [127, 128, 129], [1, 256, 300], [64, 400]])
-def test_state_space_wide_chunks(H_, G, N, V, lens):
+@pytest.mark.parametrize("chunks_of", [64, 128])
+def test_state_space_wide_chunks(H_, G, N, V, lens, chunks_of):
     """The sizes whose chunks go through the tensor cores: edges of a chunk and of its runs of sixteen tokens, runs of heads that
     do not divide a group, several column tiles, requests that start from a state and requests that do not, single tokens
     between them; outputs and states against 64 bits, to 2e-5 of the largest (some 300 roundings of 2^-24)."""
@@ -382,12 +384,24 @@ def test_state_space_wide_chunks(H_, G, N, V, lens):
     start = torch.randn(B, H_, N, V, generator=g)
     fresh = [i % 2 for i in range(B)]
     state = dev(start.reshape(B, -1).clone())
-    got = run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V)
+    got = run_recurrence(proj, cu, fresh, state, A_log, dt_bias, conv_b, D, H_, G, N, V, chunks_of)
     for i in range(B):
         y, x, S = recurrence(proj[cu[i]:cu[i + 1]], A_log, dt_bias, conv_b, H_, G, N, V, torch.zeros_like(start[i]).double() if fresh[i] else start[i].double())
         want = y + D.double()[None, :, None] * x
         assert float((got[cu[i]:cu[i + 1]] - want).abs().max() / want.abs().max()) < 2e-5, i
         assert float((state[i].double().cpu().reshape(H_, N, V) - S).abs().max() / S.abs().max()) < 2e-5, i
+
+
+@pytest.mark.parametrize("told, bad", [(0, False), (3, False), (5, False), (2, True), (1, True)])
+def test_state_space_more_portions_than_told_leave_a_status(told, bad):
+    """Chunks beyond the launch's places would go unnoticed: a launch that was told of fewer portions says so."""
+    from dinfer_b200.kernels import gemm_ops, state_ops
+    H_, G, N, V, lens = 2, 1, 16, 64, [20, 1, 30, 40]
+    ch, cu = H_ * V + 2 * G * N, [0, 20, 21, 51, 91]
+    proj, ones = torch.zeros(91, H_ * V + ch + H_, device="cuda"), torch.ones(ch, device="cuda")
+    state_ops.state_space(proj, ones[:, None].contiguous(), ones, ones[:H_], ones[:H_], ones[:H_], torch.zeros(4, H_ * N * V, device="cuda"), i32(cu),
+                          i32([0, 1, 2, 3]), i32([1] * 4), H_, G, N, V, 1, max_q_len=40, portion_requests=told, chunks_of=128)
+    assert gemm_ops.reset_status() == (53 if bad else 0)
 
 
 @pytest.mark.parametrize("lens", [[1] * 48, [300, 200]])
@@ -417,8 +431,8 @@ def test_state_space_launches_with_nothing_to_do(lens, V):
     assert bool(torch.isfinite(results[0][0]).all())
 
 
-@pytest.mark.parametrize("N, V", [(16, 64), (8, 8)])
-def test_state_space_decays_of_zero(N, V):
+@pytest.mark.parametrize("N, V, chunks_of", [(16, 64, 128), (16, 64, 64), (8, 8, 64)])
+def test_state_space_decays_of_zero(N, V, chunks_of):
     """Heads whose decay is exactly zero (the logarithm minus infinity, or -1e26 beside -1e-4): a token that follows sees what
     came behind the last such decay, through the chunks on the tensor cores and through the others; to 2e-5 of the largest as
     elsewhere."""
@@ -431,7 +445,7 @@ def test_state_space_decays_of_zero(N, V):
     conv_b, D = zeros(H_ * V + 2 * G * N), zeros(H_)
     start = torch.randn(len(lens), H_, N, V, generator=g)
     state = dev(start.reshape(len(lens), -1).clone())
-    got = run_recurrence(proj, cu, [0, 0, 1], state, A_log, zeros(H_), conv_b, D, H_, G, N, V)
+    got = run_recurrence(proj, cu, [0, 0, 1], state, A_log, zeros(H_), conv_b, D, H_, G, N, V, chunks_of)
     for i in range(len(lens)):
         y, _, S = recurrence(proj[cu[i]:cu[i + 1]], A_log, zeros(H_), conv_b, H_, G, N, V, start[i].double() * (i < 2))
         for h in range(H_):
@@ -441,16 +455,17 @@ def test_state_space_decays_of_zero(N, V):
 
 @pytest.mark.parametrize("bad", [math.inf, -math.inf, math.nan])
 @pytest.mark.parametrize("where", ["x", "B", "C", "dt"])
-def test_state_space_wide_chunks_keep_the_past_clean(where, bad):
+@pytest.mark.parametrize("chunks_of", [64, 128])
+def test_state_space_wide_chunks_keep_the_past_clean(where, bad, chunks_of):
     """A value that is not finite at one token reaches no earlier one, and no other head (or group) than its own."""
     H_, G, N, V, T, t = 4, 2, 32, 64, 200, 77
     g = torch.Generator().manual_seed(1)
     proj = torch.randn(T, 2 * H_ * V + 2 * G * N + H_, generator=g)
     A_log, dt_bias, conv_b, D = torch.linspace(-4.0, 1.0, H_), torch.zeros(H_), torch.zeros(H_ * V + 2 * G * N), torch.ones(H_)
-    clean = run_recurrence(proj, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V)
+    clean = run_recurrence(proj, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V, chunks_of)
     broken = proj.clone()
     broken[t, {"x": H_ * V + 1, "B": 2 * H_ * V + 3, "C": 2 * H_ * V + G * N + 3, "dt": 2 * H_ * V + 2 * G * N}[where]] = bad
-    got = run_recurrence(broken, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V)
+    got = run_recurrence(broken, [0, T], [1], torch.zeros(1, H_ * N * V, device="cuda"), A_log, dt_bias, conv_b, D, H_, G, N, V, chunks_of)
     assert bool(torch.isfinite(got[:t]).all()) and bool(torch.isfinite(got[:, 2:]).all())
     scale = float(clean.abs().max())
     assert float((got[:t] - clean[:t]).abs().max()) < 1e-5 * scale and float((got[:, 2:] - clean[:, 2:]).abs().max()) < 1e-5 * scale
