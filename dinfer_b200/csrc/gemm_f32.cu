@@ -41,6 +41,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(const float* local, uint32_t ran
 
 // bfloat16 elements are one part, 32-bit ones three
 template <typename T> constexpr int parts_of() { return sizeof(T) == 4 ? PARTS : 1; }
+template <typename T> constexpr float unscale() { return sizeof(T) == 4 ? UNSCALE : 1.f; }
 template <typename T> constexpr uint32_t raw_row() { return BK * sizeof(T); }
 // Eight k of row r from a stage as TMA has laid it down: rows of 128 bytes with the 128-byte swizzle (32-bit), of 64 with the
 // 64-byte one (bfloat16)
@@ -64,12 +65,15 @@ __device__ __forceinline__ Piece<T> load_piece(const T* __restrict__ row, bool l
   for (int i = 0; i < 8; ++i) e[i] = live && k + i < k_end ? row[k + i] : from_f32<T>(0.f);
   return *reinterpret_cast<const Piece<T>*>(e);
 }
-template <typename T>
+template <typename T, bool FAST>
 __device__ __forceinline__ void split_piece(const Piece<T>& p, uint4 (&q)[PARTS]) {
   if constexpr (sizeof(T) == 4) {
-    const float x[8] = {__uint_as_float(p.v[0].x), __uint_as_float(p.v[0].y), __uint_as_float(p.v[0].z), __uint_as_float(p.v[0].w),
-                        __uint_as_float(p.v[1].x), __uint_as_float(p.v[1].y), __uint_as_float(p.v[1].z), __uint_as_float(p.v[1].w)};
-    split8(x, q);
+    float x[8] = {__uint_as_float(p.v[0].x), __uint_as_float(p.v[0].y), __uint_as_float(p.v[0].z), __uint_as_float(p.v[0].w),
+                  __uint_as_float(p.v[1].x), __uint_as_float(p.v[1].y), __uint_as_float(p.v[1].z), __uint_as_float(p.v[1].w)};
+    if (!FAST)                                     // (apart: in pairs they would cost that kernel its last registers)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] *= SCALE;
+    split8<FAST>(x, q);
   } else {
     q[0] = p.v[0];
   }
@@ -192,8 +196,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
       for (int i = 0; i < PIECES; i += 2) {
         uint4 q[2][PARTS];
-        split_piece<TW>(w[i], q[0]);
-        split_piece<TW>(w[i + 1], q[1]);
+        split_piece<TW, FAST>(w[i], q[0]);
+        split_piece<TW, FAST>(w[i + 1], q[1]);
 #pragma unroll
         for (int e = 0; e < parts_of<TW>(); ++e) tmem_st8(w_at + s * W_COLS + e * (BK / 2) + i * 4, q[0][e], q[1][e]);
       }
@@ -209,7 +213,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int ra = r + i * ROW_STEP;
         if (ra < bt) {
           uint4 q[PARTS];
-          split_piece<TA>(x[i], q);
+          split_piece<TA, FAST>(x[i], q);
 #pragma unroll
           for (int e = 0; e < parts_of<TA>(); ++e) st_shared16(ta + e * a_part + swizzled64(ra, c), q[e]);
         }
@@ -282,7 +286,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (ok) {
       float acc[HALF];
 #pragma unroll
-      for (int i = 0; i < HALF; ++i) acc[i] = __uint_as_float((uint32_t)(acc2[i / 2] >> (32 * (i & 1))));
+      for (int i = 0; i < HALF; ++i) acc[i] = __uint_as_float((uint32_t)(acc2[i / 2] >> (32 * (i & 1)))) * (unscale<TA>() * unscale<TW>());
       if (p.splits > 1) {                                       // the stages' memory takes the partial tile
 #pragma unroll
         for (int i = 0; i < HALF; ++i)

@@ -1,11 +1,14 @@
 // 32-bit operands on the tensor cores: an element x is the sum of three bfloat16 numbers h + m + l (each the rest rounded
 // to nearest; 3 x 8 bits hold the 24 of a 32-bit number), and a product of two such elements is taken as
-// h h' + h m' + m h' + m m' + h l' + l h', every one of them exact, summed in 32-bit.  What is left out (m l', l m', l l')
-// is at most 2^-23 of the product and 2^-26 on average, less than one rounding of a 32-bit sum.
+// h h' + h m' + m h' + m m' + h l' + l h', every one of them exact, summed in 32-bit.  What is left out (m l', m l', l l')
+// is at most 2^-23 of the product and 2^-26 on average, less than one rounding of a 32-bit sum.  (The method, with these six of
+// the nine products: Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision
+// Computations", 2019.)
 //
-// Limits: an element of more than 3.39e38 rounds to an infinite h, and an infinite or undefined element has parts that are
-// not numbers, so whatever such an element meets comes out as not a number: a kernel looks at its results and sums those
-// that are not finite again with plain multiply-adds.  An element below 2^-110 (7e-34) keeps its digits down to 2^-133 only.
+// Elements are split times 2^16, which a kernel takes out of its results again (UNSCALE for each 32-bit operand): the last digit of
+// the smallest 32-bit number is then the smallest bfloat16 number's, so that the parts hold every element below 2^112 whole.  An element
+// beyond, or one that is infinite or undefined, has parts that are not numbers, and a scaled sum beyond 2^128 is infinite: a
+// kernel looks at its results and sums those that are not finite again with plain multiply-adds.
 #pragma once
 #include <atomic>
 
@@ -46,6 +49,9 @@ __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {     // a - b 
   return c;
 }
 
+// what elements are split times, and back
+constexpr float SCALE = 65536.f, UNSCALE = 1.f / SCALE;
+
 // two elements: their parts packed, the first in the lower half.  LOW: what was rounded off the elements joins the rest behind
 // their first part.
 template <bool LOW = false>
@@ -61,18 +67,28 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t (&p)[PARTS], f
     }
   }
 }
-// eight elements to the 16 bytes of each part
+// eight elements to the 16 bytes of each part, times SCALE or as they are
+template <bool SCALED>
 __device__ __forceinline__ void split8(const float (&x)[8], uint4 (&p)[PARTS]) {
   uint32_t q[4][PARTS];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) split2(x[2 * i], x[2 * i + 1], q[i]);
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (SCALED) {
+      uint64_t v;
+      asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(pair(x[2 * i], x[2 * i + 1])), "l"(0x4780000047800000ull));   // (SCALE twice)
+      split2(__uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)), q[i]);
+    } else {
+      split2(x[2 * i], x[2 * i + 1], q[i]);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < PARTS; ++i) p[i] = make_uint4(q[0][i], q[1][i], q[2][i], q[3][i]);
 }
 
-// the same of x[i] * w, the products' rounding kept
+// the same of x[i] * w times SCALE, the products' rounding kept
 __device__ __forceinline__ void split8_times(const float (&x)[8], float w, uint4 (&p)[PARTS]) {
   uint32_t q[4][PARTS];
+  w *= SCALE;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float a = x[2 * i] * w, b = x[2 * i + 1] * w;

@@ -8,7 +8,9 @@
 //
 // A head's 64 value columns are the MMA's columns; while one head's MMAs run, the next one's operands are split.  Results that
 // are not finite are summed again term by term, so that a token's infinity or NaN reaches the tokens behind it and no others (a
-// zero of A times it would not be zero).
+// zero of A times it would not be zero).  The weights of x in U and A's elements, which decays make as small as they like, are split
+// times 2^16 (split_umma.cuh) at no cost; the layer's own numbers, B, C, x and S, as they are (those below 2^-110, 7e-34, with fewer digits:
+// scaled as well, a portion of 400 tokens through 16 heads took 48 us instead of 42).
 //
 // Bound by the MMAs of 64 columns (54 to 70 cycles each, where 128 x 64 x 16 would take 32) and, between them, by the splitting and
 // the making of A (9000 cycles a head and chunk, of which the MMAs take 5500).  What it takes beside plain 32-bit multiply-adds
@@ -108,7 +110,7 @@ __device__ __forceinline__ void stage_tile(uint32_t dst, const Pieces& x, const 
     const float e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     uint4 q[dinfer_split::PARTS];
     if (SCALED) dinfer_split::split8_times(e, scale[r], q);     // (0 beyond the chunk's tokens)
-    else dinfer_split::split8(e, q);
+    else dinfer_split::split8<false>(e, q);
 #pragma unroll
     for (int k = 0; k < dinfer_split::PARTS; ++k) dinfer_split::st_shared16(dst + k * PART_BYTES + dinfer_split::swizzled128(r, c), q[k]);
   }
@@ -117,8 +119,8 @@ __device__ __forceinline__ void stage_tile(uint32_t dst, const Pieces& x, const 
 __device__ __forceinline__ void put_lane(uint32_t at, int unit, const float (&x)[16]) {
   const float lo[8] = {x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]}, hi[8] = {x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]};
   uint4 a[dinfer_split::PARTS], b[dinfer_split::PARTS];
-  dinfer_split::split8(lo, a);
-  dinfer_split::split8(hi, b);
+  dinfer_split::split8<false>(lo, a);
+  dinfer_split::split8<false>(hi, b);
 #pragma unroll
   for (int e = 0; e < dinfer_split::PARTS; ++e) dinfer_split::tmem_st8(at + e * A_COLS + unit * 8, a[e], b[e]);
 }
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_sums_umma_kernel(const Pa
             x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
           }
           uint4 q[dinfer_split::PARTS];
-          dinfer_split::split8(x, q);
+          dinfer_split::split8<false>(x, q);
 #pragma unroll
           for (int k = 0; k < dinfer_split::PARTS; ++k)
             dinfer_split::st_shared16(base + half * TILE_BYTES + k * PART_BYTES + dinfer_split::swizzled128(r, piece & 7), q[k]);
@@ -396,6 +398,8 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_sums_umma_kernel(const Pa
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&read_bar));
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] *= dinfer_split::UNSCALE;
         float* U = p.U + (slot * p.H + h) * (int64_t)p.N * p.Pd + c0;
         by_rows(swap, v, [&](int, int r, int x, const float4& e) {
           const int k = (warp & 3) * 32 + r;
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
         const float hi = (float)sum;
         c_hi[warp][s] = hi;
         c_lo[warp][s] = (float)(sum - (double)hi);
-        dts[warp][s] = dt4[i];
+        dts[warp][s] = dt4[i] * dinfer_split::SCALE;
       }
     }
     fill_rows(lanes, Cp, ch, n, p.N, reinterpret_cast<float*>(umma_sm + (base - smem_u32(umma_sm)) + 2 * TILE_BYTES));   // (all meet inside)
@@ -574,7 +578,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
       const float e = exp2f(hi), D = p.D[h];
       float* y = p.y + (int64_t)t0 * inner + (int64_t)h * p.Pd + c0;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fmaf(e, v[i], w[i]);
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(e, v[i], w[i] * dinfer_split::UNSCALE);
       by_rows(reinterpret_cast<float*>(umma_sm + (tiles - smem_u32(umma_sm))) + warp * SWAP_FLOATS, v, [&](int i, int r, int col, const float4& o) {
         const int t = (warp & 3) * 32 + r;
         if (t < n)
@@ -588,7 +592,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
           for (int k = 0; k < p.N; ++k) r = fmaf(Cp[(int64_t)row * ch + k], S[(int64_t)k * p.Pd + i], r);
           r *= e;
           for (int s = 0; s <= row; ++s)
-            r = fmaf(cb[s * CU + row] * exp2f((hi - c_hi[u][s]) + (lo - c_lo[u][s])) * dts[u][s], xs[(int64_t)s * ch + h * p.Pd + c0 + i], r);
+            r = fmaf(cb[s * CU + row] * exp2f((hi - c_hi[u][s]) + (lo - c_lo[u][s])) * (dts[u][s] * dinfer_split::UNSCALE), xs[(int64_t)s * ch + h * p.Pd + c0 + i], r);
           y[(int64_t)row * inner + i] = fmaf(D, x[(int64_t)row * ch + i], r);
         }
       }

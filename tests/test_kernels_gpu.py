@@ -590,3 +590,36 @@ def test_attention_generic_without_pages(dt):
     ops.attention_generic(q[1:], alone, cache, table[1:], dev(torch.tensor([0, 1], dtype=torch.int32)), pos[1:],
                           H_, Hkv, D, D ** -0.5, 0)
     assert torch.equal(out[1], alone[0]) and torch.isfinite(out[1].float()).all()
+
+
+@pytest.mark.parametrize("e", [-100, -112, -120, -126, -135, -149])
+@pytest.mark.parametrize("small", ["a", "w"])
+@pytest.mark.parametrize("other", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("M, N, K", [(40, 72, 96), (200, 40, 1001)])
+def test_gemm_f32_small_elements(e, small, other, M, N, K):
+    """Elements far down the range of 32-bit numbers, down to the last ones, against ones that bring the products back up: K
+    products summed to 32-bit accuracy are off by at most (K + 1) 2^-24 of the sum of their sizes, wherever the elements lie."""
+    from dinfer_b200.kernels import gemm_ops, ops
+    g = torch.Generator().manual_seed(M - e)
+    tiny = (torch.randn(M if small == "a" else N, K, generator=g, dtype=torch.float64) * 2.0 ** e).float().cuda()
+    big = (torch.randn(N if small == "a" else M, K, generator=g, dtype=torch.float64) * 2.0 ** 80).to(other).cuda()
+    a, w = (tiny, big) if small == "a" else (big, tiny)
+    c = torch.empty(M, N, device="cuda")
+    ops.gemm_f32(a, w, c)
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((c.double() - want).abs() <= (K + 1) * 2.0 ** -24 * size).all())
+    assert gemm_ops.device_status() == 0
+
+
+@pytest.mark.parametrize("e, f", [(115, -20), (110, 10), (126, 0)])
+def test_gemm_f32_large_elements(e, f):
+    """Elements and sums near the top of the range, where the scaled parts are no numbers any more: summed again."""
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(e)
+    M, N, K = 50, 40, 96
+    a = (torch.rand(M, K, generator=g, dtype=torch.float64) * 2.0 ** e).float().cuda()
+    w = (torch.rand(N, K, generator=g, dtype=torch.float64) * 2.0 ** f / K).float().cuda()
+    c = torch.empty(M, N, device="cuda")
+    ops.gemm_f32(a, w, c)
+    want = a.double() @ w.double().T
+    assert bool(((c.double() - want).abs() <= (K + 1) * 2.0 ** -24 * want).all())
