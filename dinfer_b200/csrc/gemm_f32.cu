@@ -2,9 +2,9 @@
 // mode), and of a bfloat16 model whose file stores a matrix in 32-bit.  A, W and C may each be f32 or bf16 in memory.  Any M,
 // N, K.
 //
-// Two kernels: a tiled one for prompts, on the tensor cores with every 32-bit element taken as three bfloat16 parts
-// (split_umma.cuh; its results are closer to 64-bit ones than those of 32-bit multiply-adds in order), and a
-// warp-per-output-column one for the few rows of a decode step, with plain 32-bit multiply-adds.  The reference has no 32-bit
+// Three kernels: a tiled one for prompts, on the tensor cores with every 32-bit element taken as three bfloat16 parts
+// (split_umma.cuh), and with plain 32-bit multiply-adds a tiled one for short sums and a warp-per-output-column one for the few rows
+// of a decode step.  The reference has no 32-bit
 // path (its weights are bf16 and its products cuBLASLt: crates/kernels/src/gemm.rs:649-690).
 #include "split_umma.cuh"
 
@@ -359,6 +359,116 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 }
 
+// ---- short sums: 64 x 128 tiles of packed 32-bit multiply-adds, all of K in shared memory at once.  Four warps own 32 x 64 of the
+// tile each, a lane 8 x 8 (rows ly + 4 i, columns lx + 8 j), and a multiply-add works on two k (even and odd k have a sum of
+// their own), so that operands are used as they lie: 16 16-byte loads feed 128 packed multiply-adds.  Bound by one way to
+// memory and back; what the tiles above take ahead of their first MMA and behind their last is longer than these sums (times at the
+// rule).
+constexpr int SHORT_M = 64, SHORT_N = 128, SHORT_THREADS = 128, SHORT_TILE_K = 48;
+constexpr int LDK = SHORT_TILE_K + 4;          // row stride of a staged operand: eight rows' 16-byte pieces of one k lie in different banks
+constexpr int LDC_SHORT = SHORT_N + 8;
+static_assert(SHORT_M * LDC_SHORT <= (SHORT_M + SHORT_N) * LDK, "the result takes the operands' place");
+
+__device__ __forceinline__ void fma2(uint64_t& c, uint64_t a, uint64_t b, bool first) {       // two multiply-adds, each rounded once
+  if (first) asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
+  else asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+// rows [r0, r0 + ROWS) of an operand as [row][k], zeros beyond `rows` and K (a multiple of four is filled); fast: four elements a load
+template <typename T, int ROWS>
+__device__ __forceinline__ void stage_short(float* dst, const T* __restrict__ src, int64_t ld, int r0, int rows, int K, bool fast) {
+  const int pieces = (K + 3) / 4;
+  if (fast) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < ROWS * pieces; i += SHORT_THREADS) {
+      const int r = i / pieces, k = (i % pieces) * 4;
+      const bool live = r0 + r < rows;
+      const T* p = src + (live ? (int64_t)(r0 + r) * ld + k : 0);
+      if constexpr (sizeof(T) == 4) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * LDK + k)), "l"(p), "r"(live ? 16 : 0) : "memory");
+      } else {
+        const uint2 u = live ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
+        *reinterpret_cast<float4*>(dst + r * LDK + k) = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u),
+                                                                    __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+      }
+    }
+    return;
+  }
+#pragma unroll 4
+  for (int i = threadIdx.x; i < ROWS * pieces * 4; i += SHORT_THREADS) {
+    const int r = i / (pieces * 4), k = i % (pieces * 4);
+    dst[r * LDK + k] = r0 + r < rows && k < K ? to_f32<T>(src[(int64_t)(r0 + r) * ld + k]) : 0.f;
+  }
+}
+template <typename TA, typename TW, typename TC>
+__global__ void __launch_bounds__(SHORT_THREADS, 2)
+gemm_short_kernel(const TA* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw, TC* __restrict__ C, int64_t ldc, int M,
+                  int N, int K, int64_t sa, int64_t sw, int64_t sc, int a_fast, int w_fast, int c_fast) {
+  __shared__ __align__(16) float sm[(SHORT_M + SHORT_N) * LDK];
+  A += (int64_t)blockIdx.z * sa; W += (int64_t)blockIdx.z * sw; C += (int64_t)blockIdx.z * sc;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, m0 = blockIdx.y * SHORT_M, n0 = blockIdx.x * SHORT_N;
+  // (lanes 0-7 and 8-15 read the two halves of the columns' pieces: 16 lanes' 16-byte loads then take one pass over the banks)
+  const int ly = ((lane >> 2) & 1) | (lane >> 4 << 1), lx = (lane & 3) | ((lane >> 3 & 1) << 2);
+  const int wr = (warp >> 1) * 32, wc = (warp & 1) * 64;
+  stage_short<TA, SHORT_M>(sm, A, lda, m0, M, K, a_fast);
+  stage_short<TW, SHORT_N>(sm + SHORT_M * LDK, W, ldw, n0, N, K, w_fast);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float sum[8][8] = {};
+  const float* as = sm + (wr + ly) * LDK;
+  const float* ws = sm + (SHORT_M + wc + lx) * LDK;
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 8) {               // (sums of eight, then of those: 0.7 of the error of one sum in order)
+    uint64_t acc[8][8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = k0 + 4 * h;
+      if (h && k >= K) break;
+      ulonglong2 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(as + 4 * i * LDK + k);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(ws + 8 * j * LDK + k);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, b.x, h == 0);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, b.y, false);    // (a sum's two steps apart: the first takes a while)
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        sum[i][j] += __uint_as_float((uint32_t)acc[i][j]) + __uint_as_float((uint32_t)(acc[i][j] >> 32));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[(wr + ly + 4 * i) * LDC_SHORT + wc + lx + 8 * j] = sum[i][j];
+  __syncthreads();
+  for (int v = tid; v < SHORT_M * (SHORT_N / 4); v += SHORT_THREADS) {
+    const int r = v / (SHORT_N / 4), c = (v % (SHORT_N / 4)) * 4, n = n0 + c;
+    if (m0 + r >= M || n >= N) continue;
+    const float4 t = *reinterpret_cast<const float4*>(sm + r * LDC_SHORT + c);
+    const float e[4] = {t.x, t.y, t.z, t.w};
+    TC* dst = C + (int64_t)(m0 + r) * ldc + n;
+    if (c_fast && n + 3 < N) {
+      if constexpr (sizeof(TC) == 4) {
+        *reinterpret_cast<float4*>(dst) = t;
+      } else {
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(e[0], e[1]), __floats2bfloat162_rn(e[2], e[3])};
+        *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (n + u < N) dst[u] = from_f32<TC>(e[u]);
+    }
+  }
+}
+
 // The sums over the lanes of acc[m] to C[m * ldc], m < M.  32 rows are halved from step to step, a lane keeping the half with
 // its own bit: 31 exchanges instead of 160, the same additions.
 template <typename TC, int ROWS>
@@ -383,12 +493,16 @@ __device__ __forceinline__ void store_rows(float (&acc)[ROWS], TC* C, int64_t ld
   }
 }
 
-// M <= ROWS rows: one warp per output column n; lanes stride over K, the weight row is read once.
+// ROWS rows (grid: blocks of 8 columns, of ROWS rows, problems): one warp per output column n; lanes stride over K, the weight row is
+// read once a row block.
 template <typename TA, typename TW, typename TC, int ROWS>
 __global__ void __launch_bounds__(256)
 gemm_rows_kernel(const TA* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                  TC* __restrict__ C, int64_t ldc, int M, int N, int K, int64_t sa, int64_t sw, int64_t sc) {
-  A += (int64_t)blockIdx.z * sa; W += (int64_t)blockIdx.z * sw; C += (int64_t)blockIdx.z * sc;
+  A += (int64_t)blockIdx.z * sa + (int64_t)blockIdx.y * ROWS * lda;
+  W += (int64_t)blockIdx.z * sw;
+  C += (int64_t)blockIdx.z * sc + (int64_t)blockIdx.y * ROWS * ldc;
+  M = min(ROWS, M - (int)blockIdx.y * ROWS);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * 8 + warp;
   if (n >= N) return;
@@ -448,6 +562,21 @@ gemm_rows_bf16x8_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const 
 // N 128 K 128 5.5 and 4.8, 6.1 and 6.2; N 2048 K 128 5.9 and 5.5, 6.5 and 7.0; beyond, N 2048 K 192 5.8 and 7.2, 6.4 and 9.6;
 // N 4096 K 64 5.1 and 5.7, 5.6 and 6.9.  Errors against 64 bits are alike (7e-8).
 constexpr int FEW_ROWS_K = 128, FEW_ROWS_N = 2048;
+// Sums up to this long go so beyond 32 rows too, while their blocks (32 rows, 8 columns) are at most three to two SMs: what a tile takes
+// ahead of its first MMA and behind its last (5 us) is more than the sums.  us on a tile and so, in 32-bit: 333 x 48 x 16 6.4 and 3.4
+// (4.8 on tiles of multiply-adds, as they were), 1000 x 48 x 48 7.3 and 5.3, 200 x 256 x 64 7.0 and 5.4; beyond the line 333 x 256 x
+// 16 6.4 and 5.9, x 64 7.0 and 8.2, 100 x 1024 x 64 7.1 and 8.3; longer 1000 x 48 x 96 7.6 and 6.6, 100 x 128 x 128 8.0 and 7.2,
+// 2048 x 128 x 128 8.4 and 26; with a bfloat16 operand 64 x 256 x 64 5.1 and 4.8, 33 x 128 x 128 5.6 and 7.3.
+constexpr int SHORT_K = 64;
+// Beyond those blocks, sums up to which the tiles of multiply-adds are the faster ones: of two 32-bit operands, one, none.  us on the
+// tensor cores and so, 333 x 1024, 2048 x 1024 (152 tiles there, two rounds) and 7000 x 128: both 32-bit K 16 6.8 and 4.3, 12.0 and 5.7, 6.9
+// and 4.7; K 40 7.5 and 6.4, 13.5 and 9.1, 7.7 and 7.0; one K 16 6.1 and 4.5, 10.7 and
+// 5.9, 6.2 and 5.0; K 32 5.9 and 5.8, 10.5 and 7.9, 6.0 and 6.2; K 40 6.4 and 6.7, 11.4 and 9.3, 6.5 and 7.2; none K 16 5.7 and 4.6, 10.4 and
+// 6.0, 6.1 and 4.7;
+// K 24 5.9 and 5.9, 10.6 and 7.5, 6.2 and 6.0.  Errors against 64 bits are alike (K 4 4.1e-8 for 4.7e-8, K 16 5.6e-8 for 4.8e-8, K 40 6.6e-8 for
+// 6.1e-8; bfloat16 operands 2.0e-8 for 2.4e-8).
+template <typename TA, typename TW> constexpr int short_tile_k() { return sizeof(TA) + sizeof(TW) == 8 ? 40 : (sizeof(TA) + sizeof(TW) == 6 ? 32 : 16); }
+static_assert(short_tile_k<float, float>() <= SHORT_TILE_K, "all of K is staged");
 
 int num_sms() {                                             // of the current device, asked once
   static const int n = [] {
@@ -524,10 +653,19 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
   if (M <= 8) {
     gemm_rows_kernel<TA, TW, TC, 8><<<dim3((N + 7) / 8, 1, batch), 256, 0, stream>>>(
         (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
-  } else if (M <= 32 && (batch > 1 || (K <= FEW_ROWS_K && N <= FEW_ROWS_N))) {
-    // few rows against many small matrices (one per head) or one small one: each weight is read once
-    gemm_rows_kernel<TA, TW, TC, 32><<<dim3((N + 7) / 8, 1, batch), 256, 0, stream>>>(
+  } else if ((M <= 32 && (batch > 1 || (K <= FEW_ROWS_K && N <= FEW_ROWS_N))) ||
+             (batch == 1 && K <= SHORT_K && (int64_t)((N + 7) / 8) * ((M + 31) / 32) * 2 <= 3 * num_sms())) {
+    // few rows against many small matrices (one per head) or one small one, or few short sums: each weight is read once a row block
+    gemm_rows_kernel<TA, TW, TC, 32><<<dim3((N + 7) / 8, (M + 31) / 32, batch), 256, 0, stream>>>(
         (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
+  } else if (K <= short_tile_k<TA, TW>() && (M + SHORT_M - 1) / SHORT_M <= 65535) {
+    const auto fast = [](const void* q, size_t size, int64_t ld, int64_t stride) {
+      return (int)((reinterpret_cast<uintptr_t>(q) % (4 * size)) == 0 && ld % 4 == 0 && stride % 4 == 0);
+    };
+    // (no early start behind the kernel in front: beside its CTAs these share SMs while others idle, 1000 x 1000 x 40 8.3 us for 6.7)
+    gemm_short_kernel<TA, TW, TC><<<dim3((N + SHORT_N - 1) / SHORT_N, (M + SHORT_M - 1) / SHORT_M, batch), SHORT_THREADS, 0, stream>>>(
+        (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc, fast(A, sizeof(TA), lda, sa) && K % 4 == 0,
+        fast(W, sizeof(TW), ldw, sw) && K % 4 == 0, fast(C, sizeof(TC), ldc, sc));
   } else {
     if (!status) return refuse(DINFER_BAD_ARGUMENT, "gemm_f32: a status word is required");
     if (M > MAX_ROWS) return refuse(DINFER_BAD_ARGUMENT, "gemm_f32: M=%d too large", M);

@@ -623,3 +623,69 @@ def test_gemm_f32_large_elements(e, f):
     ops.gemm_f32(a, w, c)
     want = a.double() @ w.double().T
     assert bool(((c.double() - want).abs() <= (K + 1) * 2.0 ** -24 * want).all())
+
+
+@pytest.mark.parametrize("M, N, K", [(33, 1, 1), (64, 9, 16), (333, 48, 16), (335, 160, 64), (1000, 48, 33), (2048, 16, 64), (7104, 8, 64), (7105, 8, 64),
+                                     (333, 160, 65), (337, 168, 64)])
+@pytest.mark.parametrize("a_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+def test_gemm_f32_short_sums(M, N, K, a_dtype, w_dtype):
+    """Short sums of more than 32 rows, on either side of the line between a warp a column and tiles; strided rows in and out.  K
+    products summed in 32-bit are off by at most (K + 1) 2^-24 of the sum of their sizes."""
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + N)
+    a, w = torch.randn(M, K + 3, generator=g).to(a_dtype).cuda()[:, 1:K + 1], torch.randn(N, K, generator=g).to(w_dtype).cuda()
+    wide = torch.full((M, N + 5), 7.0, device="cuda")
+    ops.gemm_f32(a, w, wide[:, 2:N + 2])
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert bool(((wide[:, 2:N + 2].double() - want).abs() <= (K + 1) * 2.0 ** -24 * size).all())
+    assert bool((wide[:, :2] == 7.0).all()) and bool((wide[:, N + 2:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M, N", [(33, 1793), (65, 1000), (333, 1024), (2049, 130), (64, 3584)])
+@pytest.mark.parametrize("K", [1, 7, 8, 12, 16, 17, 32, 33, 37, 40, 41])
+@pytest.mark.parametrize("a_dtype, w_dtype, out", [(torch.float32, torch.float32, torch.float32), (torch.bfloat16, torch.float32, torch.bfloat16),
+                                                   (torch.float32, torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_gemm_f32_short_tiles(M, N, K, a_dtype, w_dtype, out, shift):
+    """Short sums of many rows and columns: tiles of multiply-adds up to a line and the tensor cores beyond, edges of a tile, rows
+    that take four elements at a time and rows that do not, several problems at once.  K products summed in 32-bit are off by
+    at most (K + 1) 2^-24 of the sum of their sizes; a bfloat16 result by 2^-8 of itself more."""
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = (torch.randn(n, (K + 7) // 4 * 4, generator=g).to(t).cuda()[:, shift:K + shift] for n, t in ((M, a_dtype), (N, w_dtype)))
+    wide = torch.full((M, (N + 11) // 4 * 4), 7.0, dtype=out, device="cuda")
+    ops.gemm_f32(a, w, wide[:, 4:N + 4])
+    want, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    bound = (K + 1) * 2.0 ** -24 * size + (2.0 ** -8 * want.abs() if out == torch.bfloat16 else 0)
+    assert bool(((wide[:, 4:N + 4].double() - want).abs() <= bound).all())
+    assert bool((wide[:, :4] == 7.0).all()) and bool((wide[:, N + 4:] == 7.0).all())
+
+
+@pytest.mark.parametrize("B, M, N, K", [(3, 70, 200, 16), (5, 33, 8, 24), (2, 300, 130, 40)])
+def test_gemm_f32_short_tiles_batched(B, M, N, K):
+    from dinfer_b200.kernels import ops
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(M, B, K, generator=g).cuda(), torch.randn(B, N, K, generator=g).cuda()
+    c = torch.empty(M, B, N, device="cuda")
+    ops.gemm_f32_batched(a, w, c)
+    want = torch.einsum("mbk,bnk->mbn", a.double(), w.double())
+    size = torch.einsum("mbk,bnk->mbn", a.double().abs(), w.double().abs())
+    assert bool(((c.double() - want).abs() <= (K + 1) * 2.0 ** -24 * size).all())
+
+
+def test_gemm_f32_short_sums_that_are_not_finite():
+    """Infinities and NaNs reach their own row or column and nothing else."""
+    import math
+    from dinfer_b200.kernels import ops
+    for M, N, K in ((333, 16, 40), (333, 1024, 40), (333, 1024, 200)):
+        a, w = torch.ones(M, K, device="cuda"), torch.ones(N, K, device="cuda")
+        a[5, 3], w[7, K - 1], a[9, 0] = math.inf, math.nan, -math.inf
+        c = torch.empty(M, N, device="cuda")
+        ops.gemm_f32(a, w, c)
+        assert bool(torch.isnan(c[:, 7]).all())
+        c[:, 7] = K
+        assert bool((c[5] == torch.where(torch.arange(N, device="cuda") == 7, K, math.inf)).all())
+        assert bool((c[9] == torch.where(torch.arange(N, device="cuda") == 7, K, -math.inf)).all())
+        c[5], c[9] = K, K
+        assert bool((c == K).all())
