@@ -30,6 +30,11 @@ static_assert(A_ALL + SUM_PARTS * VT <= TMEM_ALL && 2 * A_ALL + 2 * VT <= TMEM_A
 constexpr size_t SUMS_SMEM = 2 * TILE_BYTES + 1024 + 16 * 32 * 20 * 4;   // (more than half of an SM's: the tensor memory is one CTA's)
 static_assert(SUMS_SMEM > 114 * 1024, "one CTA to an SM");
 constexpr size_t OUTPUTS_SMEM = 4 * TILE_BYTES + 1024;
+// The MMA cuts its sums off, so that they come out too small: U by 2.4e-8 to 6e-8 of itself, the outputs, whose eight steps lie in one
+// sum, by 0.6e-7 to 2e-7 (plain sums and decayed ones, of both signs and of one, 16 to 128 tokens).  The factors that they are
+// multiplied by anyhow, the weights of x (rounded from 64 bits) and the outputs' scales, make up for the middle of that.
+constexpr double SUMS_CUT = 1.0 + 4e-8;
+constexpr float OUTPUTS_CUT = 1.f + 1.1920929e-7f;          // (the next number behind one)
 constexpr int STATUS_SUMS = 51, STATUS_OUTPUTS = 52, STATUS_PLACES = 53;
 
 __device__ __forceinline__ int64_t wide_slot(int t_begin, int b, int c) { return (int64_t)(t_begin / CU + b + c); }
@@ -366,7 +371,7 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_sums_umma_kernel(const Pa
         wide_log_decay(la4, cum);
         const double all = __shfl_sync(0xffffffffu, cum[3], 31);     // (nothing is added behind the chunk's last token)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) wgt[warp][4 * lane + i] = 4 * lane + i < n ? (float)(exp(all - cum[i]) * (double)dt4[i]) : 0.f;
+        for (int i = 0; i < 4; ++i) wgt[warp][4 * lane + i] = 4 * lane + i < n ? (float)(exp(all - cum[i]) * (double)dt4[i] * SUMS_CUT) : 0.f;
         if (lane == 0 && run.column(warp) == 0) p.decay[slot * p.H + run.head(warp, heads)] = (float)exp(all);
       }
 #pragma unroll
@@ -575,10 +580,10 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) ssm_outputs_umma_kernel(const
       load_sum(v, lanes + d1_at + sub * 16);
       load_sum(w, lanes + d2_at + sub * 16);
       if (u + 1 < run.count) hand_over(&tiles_bar);   // (head u + 1's C S may take the sums' place)
-      const float e = exp2f(hi), D = p.D[h];
+      const float e = exp2f(hi), D = p.D[h], e_cut = e * OUTPUTS_CUT;
       float* y = p.y + (int64_t)t0 * inner + (int64_t)h * p.Pd + c0;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = fmaf(e, v[i], w[i] * dinfer_split::UNSCALE);
+      for (int i = 0; i < 16; ++i) v[i] = fmaf(e_cut, v[i], w[i] * (dinfer_split::UNSCALE * OUTPUTS_CUT));
       by_rows(reinterpret_cast<float*>(umma_sm + (tiles - smem_u32(umma_sm))) + warp * SWAP_FLOATS, v, [&](int i, int r, int col, const float4& o) {
         const int t = (warp & 3) * 32 + r;
         if (t < n)
