@@ -493,16 +493,18 @@ __device__ __forceinline__ void store_rows(float (&acc)[ROWS], TC* C, int64_t ld
   }
 }
 
-// ROWS rows (grid: blocks of 8 columns, of ROWS rows, problems): one warp per output column n; lanes stride over K, the weight row is
-// read once a row block.
-template <typename TA, typename TW, typename TC, int ROWS>
+// M <= ROWS rows, or with BLOCKS any number in blocks of ROWS (grid.y): one warp per output column n; lanes stride over K, the weight
+// row is read once a block.  (Rows counted from blockIdx, not from a parameter: two rows of a 32-bit feed-forward took 94 us instead of 57.)
+template <typename TA, typename TW, typename TC, int ROWS, bool BLOCKS = false>
 __global__ void __launch_bounds__(256)
 gemm_rows_kernel(const TA* __restrict__ A, int64_t lda, const TW* __restrict__ W, int64_t ldw,
                  TC* __restrict__ C, int64_t ldc, int M, int N, int K, int64_t sa, int64_t sw, int64_t sc) {
-  A += (int64_t)blockIdx.z * sa + (int64_t)blockIdx.y * ROWS * lda;
-  W += (int64_t)blockIdx.z * sw;
-  C += (int64_t)blockIdx.z * sc + (int64_t)blockIdx.y * ROWS * ldc;
-  M = min(ROWS, M - (int)blockIdx.y * ROWS);
+  A += (int64_t)blockIdx.z * sa; W += (int64_t)blockIdx.z * sw; C += (int64_t)blockIdx.z * sc;
+  if constexpr (BLOCKS) {
+    A += (int64_t)blockIdx.y * ROWS * lda;
+    C += (int64_t)blockIdx.y * ROWS * ldc;
+    M = min(ROWS, M - (int)blockIdx.y * ROWS);
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * 8 + warp;
   if (n >= N) return;
@@ -653,10 +655,12 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int6
   if (M <= 8) {
     gemm_rows_kernel<TA, TW, TC, 8><<<dim3((N + 7) / 8, 1, batch), 256, 0, stream>>>(
         (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
-  } else if ((M <= 32 && (batch > 1 || (K <= FEW_ROWS_K && N <= FEW_ROWS_N))) ||
-             (batch == 1 && K <= SHORT_K && (int64_t)((N + 7) / 8) * ((M + 31) / 32) * 2 <= 3 * num_sms())) {
-    // few rows against many small matrices (one per head) or one small one, or few short sums: each weight is read once a row block
-    gemm_rows_kernel<TA, TW, TC, 32><<<dim3((N + 7) / 8, (M + 31) / 32, batch), 256, 0, stream>>>(
+  } else if (M <= 32 && (batch > 1 || (K <= FEW_ROWS_K && N <= FEW_ROWS_N))) {
+    // few rows against many small matrices (one per head) or one small one: each weight is read once
+    gemm_rows_kernel<TA, TW, TC, 32><<<dim3((N + 7) / 8, 1, batch), 256, 0, stream>>>(
+        (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
+  } else if (batch == 1 && K <= SHORT_K && (int64_t)((N + 7) / 8) * ((M + 31) / 32) * 2 <= 3 * num_sms()) {
+    gemm_rows_kernel<TA, TW, TC, 32, true><<<dim3((N + 7) / 8, (M + 31) / 32), 256, 0, stream>>>(
         (const TA*)A, lda, (const TW*)W, ldw, (TC*)C, ldc, M, N, K, sa, sw, sc);
   } else if (K <= short_tile_k<TA, TW>() && (M + SHORT_M - 1) / SHORT_M <= 65535) {
     const auto fast = [](const void* q, size_t size, int64_t ld, int64_t stride) {
