@@ -123,8 +123,9 @@ delta_prep_kernel(const TA* __restrict__ P, int64_t ldp, int cq, int ck, int cv,
 // Tokens of a run that spans requests (or begins a portion) go one after the other, with a search and loads of their own, so
 // it is taken for portions: from RUN_FROM tokens and RUN_PORTION tokens a request on (256 for a request alone).  us, a block
 // per (token, head) and in runs, 16 heads of 128: 256 tokens 13.4 and 11.3, 512 19.6 and 12.7; 32 requests of 16 25.0 and 15.3,
-// 64 of 16 43.8 and 24.9; 16 single tokens and 496 of a portion 23.8 and 15.6.  Below the lines a channel a lane lost (64 of 8
-// 27.3 and 31.0, 512 single tokens 45.7 and 51.8, 128 tokens 10.2 and 10.6): a run's tokens go one after the other there.
+// 64 of 16 43.8 and 24.9; 16 single tokens and 496 of a portion 23.8 and 15.6.  The lines were drawn when a lane had one channel,
+// and leave out steps that the runs would take faster now: 64 of 8 27.5 and 19.9, 512 single tokens 45.6 and 34.4, 64 of 4 18.8 and 19.7,
+// 16 of 16 15.9 and 15.0; but 128 tokens 10.0 and 11.9, 64 8.5 and 11.4, 64 single tokens and 64 of a portion 14.6 and 22.1.
 constexpr int RUN = 8;
 constexpr int RUN_FROM = 512, RUN_FROM_ALONE = 256, RUN_PORTION = 16;
 // four neighbouring elements as 32-bit values; VEC: the address is a multiple of their size

@@ -119,11 +119,16 @@ static_assert(tile_shared<float, float>(BT, 1) <= MAX_SMEM, "fits a CTA");
 // A stage's sums leave tensor memory at once and are added in registers, rounded to nearest: the MMA's own sums are cut off, and
 // over a whole K that would cost more digits than the parts keep.
 //
-// Bound by the MMAs (670 cycles a stage of about 1130) and the hand-overs between the roles: 333 x 6144 x 1024 31 us (136
-// TFLOP/s), 333 x 1024 x 3072 24, 2048 x 6144 x 1024 198; as 64 x 128 tiles of packed 32-bit multiply-adds 125, 79 and 643.
-// Small ones gain as well: 64 x 64 x 64 6.1 us for 8.0, 100 x 2048 x 1024 12.5 for 23.  Relative errors against 64 bits
-// 1.2e-7 for 4.1e-7 at K 1024, 6e-8 for 1.1e-7 at 64 (bfloat16 operands, where only the sums round: 1.1e-7 for 1.6e-7, 9e-8
-// where eight CTAs shared K before for 8.4e-8).
+// Bound by a chain of roles rather than by one of them: while an SM runs, its tensor pipe is busy 41 % of the time and its issue slots
+// 59 % (the splits; ncu, 333 x 6144 x 1024), the rest is waits from hand-over to hand-over.  333 x 6144 x 1024 29.8 us (140 TFLOP/s),
+// 333 x 1024 x 3072 22.3, 2048 x 6144 x 1024 197; as 64 x 128 tiles of packed 32-bit multiply-adds 129, 81 and 663.  Smaller ones
+// gain as well: 100 x 2048 x 1024 12.3 us for 23.8, 33 x 64 x 4096 13.6 for 38.6; rows that TMA cannot address 333 x 6144 x 1030 55 for
+// 213, 2048 x 64 x 2045 21 for 61.  Not so where a second round of tiles is nearly empty: 2048 x 1024 x 64 13.5 for 12.0.
+//
+// Relative errors against 64 bits (2-norm) beside those of the multiply-adds, operands of both signs: K 64 6.2e-8 for 1.1e-7, 1024
+// 1.2e-7 for 4.1e-7 (where eight CTAs share K 8.8e-8 for 1.6e-7), 4096 1.1e-7 for 2.9e-7; two bfloat16 operands, whose products are exact,
+// K 64 4.7e-8 for 4.3e-8, 512 7.3e-8 for 7.1e-8, from 768 on less.  The MMA cuts its sums off towards zero, and where all products
+// have one sign that adds up: K 1024 shared by CTAs 7.2e-8 for 6.0e-8, bfloat16 operands K 512 5.8e-8 for 4.0e-8.
 template <typename TA, typename TW, typename TC, bool FAST>
 __global__ void __launch_bounds__(TILE_THREADS, 1)
 gemm_tile_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const TA* __restrict__ A,

@@ -207,7 +207,13 @@ int launch(const Params& p, cudaStream_t stream) {
   return cuda_status("gemv");
 }
 template <bool GATED, bool NORM, typename OutT>
-int pick(const Params& p, cudaStream_t stream) {             // as many rows a warp as leave every SM its eight warps
+int pick(const Params& p, cudaStream_t stream) {
+  // Fewer rows a warp keep more warps busy, more of them share the reads of the input.  us a launch with 1, 2 and 4 rows, a chain over
+  // more matrices than L2 holds, plain and with the norm (gated products go as those): 1024 x 1024 2.9, 3.0, 3.1 and 3.5, 3.0, 2.8; 1024 x 3072
+  // 3.8, 5.0, 5.8 and 4.1, 4.8, 6.2; 2046 x 1024 3.1, 3.2, 3.5 and 3.9, 3.6, 3.0; 2048 x 2048 3.6, 4.1, 5.1 and 4.3, 3.9, 5.0; 2560 x
+  // 1024 4.9, 3.4, 3.7 and 5.6, 3.6, 3.0; 4094 x 1024 5.2, 3.6, 4.2 and 5.8, 4.0, 3.7; 4096 x 1536 5.5, 4.4, 5.7 and 6.2, 4.6, 5.6;
+  // 5000 x 1024 7.0, 5.3, 4.6 and 7.7, 5.6, 4.5.  So the lines suit K 1024 with the norm in front, as decode steps of such layers have it; a
+  // plain product of 2048 to 4096 rows, and K from 1536 on, would do a fifth better with half as many rows.
   if (p.N >= 4096) return launch<4, 4, GATED, NORM, OutT>(p, stream);
   if (p.N >= 2048 || GATED) return launch<2, 8, GATED, NORM, OutT>(p, stream);
   if constexpr (!GATED) return launch<1, 16, false, NORM, OutT>(p, stream);

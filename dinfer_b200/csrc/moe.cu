@@ -470,11 +470,11 @@ moe_gemm_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv
 // rows; the second eight tokens only where there are any) and write their results while the next job's weights arrive.
 // CTA c takes the jobs (row tile, 64 weight rows) c, c + grid, ..., so that tiles of one expert read its weights at about the
 // same time.  The jobs behind the last whole round are halved or quartered while there are CTAs for the pieces: CTAs that a
-// small product leaves idle would cost more than a piece's copies of the token rows (1024 x 1024 of 16 experts, 8 tokens:
-// 11.7 us with runs of 16 rows dealt out evenly, across jobs; 9.1 with whole pieces).
-// Eight tokens, 64 experts (8 chosen), bytes of the weights met: gate and up of 4096 x 4096 240 us -> 220 (6.0 -> 6.5 TB/s),
-// down of 4096 x 2048 124 -> 108, against a CTA a job with four stages of 64 k by cp.async; 2816 x 2048 79 -> 70, 2048 x 1408
-// 49 -> 41, 1024 x 1024 of 16 experts 13.9 -> 9.7.  One CTA an SM with ten stages gets 4.4 TB/s (its warps' chain of waits and
+// small product leaves idle would cost more than a piece's copies of the token rows (dealing out runs of 16 rows evenly,
+// across jobs, took a small product a quarter longer).
+// Eight tokens, 64 experts (8 chosen), one launch under ncu, against a CTA a job with four stages of 64 k by cp.async: gate and
+// up of 4096 x 4096 (1510 MB, the gate included now) 258 us -> 230 (5.9 -> 6.6 TB/s), down of 4096 x 2048 135 -> 114; 2816 x 2048
+// 99 -> 84, 2048 x 1408 54 -> 44; 1024 x 1024 of 16 experts 15.2 -> 13.3, 1024 x 512 9.8 -> 9.8.  One CTA an SM with ten stages gets 4.4 TB/s (its warps' chain of waits and
 // products is longer than a stage's arrival), two with five 6.5 but 5.8 with 16 tokens a tile (here 6.4), three with three
 // as much as four with two up to 8 tokens and 3 % less beyond, five with two 5.2 (bound by waiting for free stages).
 constexpr int ROWS_BM = 16, ROWS_BN = 64, ROWS_BK = 128, ROWS_ST = 2, ROWS_CTAS = 4, ROWS_THREADS = 160;

@@ -216,7 +216,7 @@ def _status(device):
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T to 32-bit accuracy (32-bit elements as three bfloat16 parts on the tensor cores, or
-    32-bit multiply-adds where rows are few); each operand f32 or bf16."""
+    32-bit multiply-adds where rows are few or sums short); each operand f32 or bf16."""
     require_cuda(a, w, out)
     for t, n in ((a, "a"), (w, "w"), (out, "out")):
         if t.dim() != 2:

@@ -204,13 +204,15 @@ class LatentAttention(Mixer):
         absorbed form needs H (2 R + P) multiply-adds a (token, key) pair, the expanded one H (D + P + V) and R H (D + V) a key.
         But a CTA of the expanded attention walks all keys of its 256 rows one tile after the other, so a few rows behind a
         long history are the absorbed form's.  A layer of 16 heads of 128 + 64, R 512, absorbed and expanded (us): a prompt of
-        64 tokens 52 and 37, of 2048 565 and 134; 64 tokens behind 4000 129 and 118, behind 16000 291 and 352; 256 behind
-        16000 1187 and 493; 8 heads of 64 + 32, R 256: 64 behind 4000 59 and 86.
+        64 tokens 51 and 37, of 2048 566 and 126; 64 tokens behind 4000 129 and 89, behind 8000 177 and 140, behind 16000 287 and
+        232; 32 behind 16000 225 and 234; 256 behind 16000 1187 and 305; 8 heads of 64 + 32, R 256: 64 behind 4000 59 and 60, behind
+        16000 115 and 155, 256 behind 16000 304 and 183.  (Two CTAs share a long walk where SMs are left over, which the rule does
+        not know: it charges a walk to one, and keeps 64 tokens behind 8000 and more, and 256 of the small layer's, absorbed.)
         With decoded tokens in the step the absorbing products run for them all the same, and its launches too: nothing but the
         portions' attention is saved.  Eight tokens at 1000 beside a prompt, the same layer, as a graph and kernel by kernel:
-        128 tokens 90 and 71, 200 and 258; 600 199 and 92, 216 and 265; 1024 299 and 118, 318 and 263; 2048 670 and 170, 683
-        and 262; 64 behind 4000 160 and 165, 203 and 258; 256 behind 2000 210 and 136, 224 and 259; behind 4000 323 and 200, 337
-        and 264.
+        128 tokens 90 and 71, 172 and 247; 600 158 and 93, 175 and 247; 1024 263 and 109, 278 and 248; 2048 577 and 162, 589
+        and 251; 64 behind 4000 161 and 135, 176 and 249; 256 behind 2000 211 and 112, 224 and 248; behind 4000 323 and 155, 337
+        and 248.
         In a captured graph the lengths are bounds: the tokens spread evenly over the prompt places without a history for what
         the absorbed form costs at least, every place as long as it may get for what the other one costs at most."""
         if self.ukv is None or dtype != torch.bfloat16 or not ctx.any_prefill or not ctx.cu_seqlens_host:

@@ -1,7 +1,8 @@
 """``y = x W^T`` for a weight in the PyTorch ``[out, in]`` layout (crates/layers/src/nn.rs:16-76).
 
 Which product runs follows from the dtypes and the number of rows at hand:
-  * float32 activations (the true 32-bit engine): 32-bit multiply-adds on the CUDA cores;
+  * float32 activations (the true 32-bit engine): a product to 32-bit accuracy, on the tensor cores with every element as
+    three bfloat16 parts, or 32-bit multiply-adds where rows are few or sums short;
   * bfloat16 activations and a weight the file stores in 32-bit: the same 32-bit product, the
     activations widened on the fly;
   * bfloat16 activations and weight, one row (a single chat's decode step) and a matrix of at most ``GEMV_MAX_BYTES``: a
