@@ -96,7 +96,7 @@ class StateSpace(Mixer):
         slots, fresh = ctx.state_slots[:B], ctx.state_fresh[:B]
         sizes = (self.H, self.G, self.N, self.P, self.taps)
         portions = 0
-        if ctx.any_prefill and ctx.cu_seqlens_host:          # (a captured graph's places, which a replay may leave empty)
+        if ctx.any_prefill and ctx.any_decode and ctx.cu_seqlens_host:     # (a captured graph's places, which a replay may leave empty)
             if "portion_requests" not in ctx.derived:
                 cu = ctx.cu_seqlens_host
                 ctx.derived["portion_requests"] = sum(b - a != 1 for a, b in zip(cu, cu[1:]))
